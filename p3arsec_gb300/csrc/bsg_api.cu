@@ -124,9 +124,12 @@ struct bsg_ctx {
     // each synchronous call; d_guard holds the check's {count, first index}
     bool debug = false;
     unsigned long long* d_guard = nullptr;
-    // swaption scratch: parameter table, per-block partial sums, results
+    // swaption scratch: counters, parameter table, partial sums on the device;
+    // results and the table's staging in pinned memory
     char* d_sw = nullptr;
     size_t sw_cap = 0;
+    char* h_sw = nullptr;
+    size_t h_sw_cap = 0;
 
     bsg::SoA resident(size_t n, int set = 0) const {
         (void)n;
@@ -688,6 +691,7 @@ void bsg_destroy(bsg_ctx* c) {
     if (c->d_edges) cudaFree(c->d_edges);
     if (c->d_guard) cudaFree(c->d_guard);
     if (c->d_sw) cudaFree(c->d_sw);
+    if (c->h_sw) cudaFreeHost(c->h_sw);
     if (c->seg_ev) cudaEventDestroy(c->seg_ev);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -1202,10 +1206,19 @@ int bsg_set_tune(bsg_ctx* c, const bsg_tune* t) {
 // ------------------------------------------------------------- swaptions
 // The driver's per-swaption constants, rounded as the reference rounds them
 // (HJM_Swaption_Blocking.cpp:48-62, 116-127), checked so that every index
-// the kernel uses stays inside the path and the payment vector (the
-// reference would write past its payment vector when the tenor reaches past
-// the path).  Returns an empty string when the swaption is valid.
-static std::string swaption_setup(const bsg_swaption& w, bsg::SwParams* p) {
+// stays inside the path and the payment vector (the reference would write
+// past its payment vector when the tenor reaches past the path), and from
+// them the exponents' constants and coefficients that the path kernel reads:
+// with S_k(x) the sum of factor k's first x vols, M(x) that of the first x
+// drifts times h, and f(t_0, .) the forward curve,
+//   payment at l:  -h sum_{m<l} f(t_s, m) = -h [sum_{m<l} f(t_0, t_{s+m})
+//       + sum_{i<s} (M(l+s-1-i) - M(s-1-i)
+//                    + sqrt(h) sum_k (S_k(l+s-1-i) - S_k(s-1-i)) z_ik)]
+//   own discount:  -h sum_{i<s} f(t_i, 0) = -h sum_{i<s} [f(t_0, t_i) + M(i)
+//                    + sqrt(h) sum_k S_k(s-1-i) z_ik]
+// Appends the swaption's words to `words` (the head's words_at is relative to
+// their start).  Returns an empty string when the swaption is valid.
+static std::string swaption_setup(const bsg_swaption& w, bsg::SwHead* p, std::vector<uint64_t>* words) {
     const int n = w.n_steps, nf = w.n_factors;
     if (n < 2 || n > bsg::kSwMaxSteps) return "n_steps must be 2.." + std::to_string(bsg::kSwMaxSteps);
     if (nf < 1 || nf > bsg::kSwMaxFactors)
@@ -1214,32 +1227,111 @@ static std::string swaption_setup(const bsg_swaption& w, bsg::SwParams* p) {
     if (!(w.years > 0) || !(w.maturity > 0) || !(w.tenor > 0) || !(w.payment_interval > 0) ||
         !(w.compounding >= 0))
         return "years, maturity, tenor and payment_interval must be > 0, compounding >= 0";
-    std::memset(p, 0, sizeof(*p));
-    p->h = w.years / n;
-    p->sqh = std::sqrt(p->h);
-    p->freq = (int)(w.payment_interval / p->h + 0.5);
-    p->strike_cont = w.compounding == 0 ? w.strike
-                                        : (1 / w.compounding) * std::log(1 + w.strike * w.compounding);
-    p->swap_len = (int)(n - w.maturity / p->h + 0.5);
-    p->start = (int)(w.maturity / p->h + 0.5);
-    p->swap_points = (int)(w.tenor / p->h + 0.5);
-    p->payment_interval = w.payment_interval;
-    p->n_steps = n;
-    p->n_factors = nf;
-    p->seed = w.seed;
-    if (p->freq < 1 || p->start < 1 || p->start > n - 1 || p->swap_len < 1 ||
-        p->swap_len > n - p->start || p->swap_points >= p->swap_len)
+    const double h = w.years / n, sqh = std::sqrt(h);
+    const int freq = (int)(w.payment_interval / h + 0.5);
+    const double strike_cont =
+        w.compounding == 0 ? w.strike : (1 / w.compounding) * std::log(1 + w.strike * w.compounding);
+    const int swap_len = (int)(n - w.maturity / h + 0.5);
+    const int s = (int)(w.maturity / h + 0.5);
+    const int swap_points = (int)(w.tenor / h + 0.5);
+    if (freq < 1 || s < 1 || s > n - 1 || swap_len < 1 || swap_len > n - s || swap_points >= swap_len)
         return "maturity, tenor and payment interval do not fit the grid of n_steps points over years";
-    for (int i = 0; i < n; ++i) {
-        p->yield[i] = w.yield[i];
+    for (int i = 0; i < n; ++i)
         if (!std::isfinite(w.yield[i])) return "yield is not finite";
-    }
-    for (int k = 0; k < nf; ++k)
-        for (int m = 0; m < n - 1; ++m) {
-            p->vol[k][m] = w.factors[(size_t)k * (n - 1) + m];
-            if (!std::isfinite(p->vol[k][m])) return "factors are not finite";
+    for (int i = 0; i < nf * (n - 1); ++i)
+        if (!std::isfinite(w.factors[i])) return "factors are not finite";
+    if (!std::isfinite(strike_cont)) return "strike is not finite";
+
+    // forward curve, S_k and M (HJM_Swaption_Blocking.cpp:132-140 for the payments below)
+    double fwd[bsg::kSwMaxSteps], S[bsg::kSwMaxFactors][bsg::kSwMaxSteps] = {}, M[bsg::kSwMaxSteps] = {};
+    for (int i = 0; i < n; ++i)
+        fwd[i] = i == 0 ? w.yield[0] : (double)(i + 1) * w.yield[i] - (double)i * w.yield[i - 1];
+    for (int m = 0; m < n - 1; ++m) {
+        double mu = 0.0;
+        for (int k = 0; k < nf; ++k) {
+            const double v = w.factors[(size_t)k * (n - 1) + m];
+            mu += h * v * (S[k][m] + 0.5 * v);
+            S[k][m + 1] = S[k][m] + v;
         }
-    if (!std::isfinite(p->strike_cont)) return "strike is not finite";
+        M[m + 1] = M[m] + mu * h;
+    }
+    double pay[bsg::kSwMaxExp];
+    int at[bsg::kSwMaxExp], np = 0;  // payment dates; -1 for the path's own discount
+    for (int l = freq; l <= swap_points; l += freq) {
+        const double e = std::exp(strike_cont * w.payment_interval);
+        pay[np] = l == swap_points ? e : e - 1;
+        at[np] = l;
+        if (pay[np] != 0.0) ++np;
+    }
+    double c0 = 0.0;
+    for (int i = 0; i < s; ++i) c0 += fwd[i] + M[i];
+    std::memset(p, 0, sizeof(*p));
+    p->seed = w.seed;
+    p->disc = s == 1 ? std::exp(-c0 * h) : 1.0;
+    p->disc_varies = s > 1;
+    if (np == 0) {  // nothing is paid: the payoff is max(0 - 1, 0)
+        pay[0] = 0.0;
+        at[0] = 0;
+        np = 1;
+    }
+    const int pays = np;
+    if (p->disc_varies) {
+        pay[np] = 0.0;
+        at[np++] = -1;
+    }
+    const int nz = s * nf;
+    p->n_exp = np;
+    p->n_normals = nz;
+    double c[bsg::kSwMaxExp], g[8 * 256];
+    bool wide = false;
+    for (int l = 0; l < np; ++l) {
+        double x = c0;
+        if (l < pays) {
+            x = 0.0;
+            for (int m = 0; m < at[l]; ++m) x += fwd[m + s];
+            for (int i = 0; i < s; ++i) x += M[at[l] + s - 1 - i] - M[s - 1 - i];
+        }
+        c[l] = -h * x;
+        double reach = std::fabs(c[l]);
+        for (int i = 0; i < s; ++i)
+            for (int k = 0; k < nf; ++k) {
+                const double d = l < pays ? S[k][at[l] + s - 1 - i] - S[k][s - 1 - i] : S[k][s - 1 - i];
+                const double v = -h * sqh * d;
+                g[(i * nf + k) * np + l] = v;
+                reach += 8.6 * std::fabs(v);
+                if (!(std::fabs(v) * 1.4426950408889634 < 0.999)) wide = true;
+            }
+        if (!(reach * 1.4426950408889634 < 60.0)) wide = true;
+    }
+    p->wide = wide;
+    p->words_at = (uint32_t)words->size();
+    p->n_words = (uint32_t)(np * (2 + nz));
+    auto bits = [](double d) {
+        uint64_t u;
+        std::memcpy(&u, &d, 8);
+        return u;
+    };
+    for (int l = 0; l < np; ++l) words->push_back(bits(pay[l]));
+    if (wide) {
+        for (int l = 0; l < np; ++l) words->push_back(bits(c[l]));
+        for (int i = 0; i < nz * np; ++i) words->push_back(bits(g[i]));
+        return std::string();
+    }
+    // fixed point, in powers of two: constants with 57 fraction bits, a
+    // coefficient with 63, moved by 2^63 into the unsigned range as the kernel
+    // moves a variate (58 bits) by 2^62: G Z / 2^64 = G' Z' / 2^64 - Z'/2 -
+    // G'/4 + 2^61.  The kernel's product is 1.25 units low and its Z'/2 a
+    // quarter low on average: one unit per variate goes back here.
+    const double log2e = 1.4426950408889634074;
+    const size_t at_c = words->size();
+    for (int l = 0; l < np; ++l)
+        words->push_back((uint64_t)std::llrint(std::ldexp(c[l] * log2e, 57)) + (uint64_t)nz);
+    for (int i = 0; i < nz; ++i)
+        for (int l = 0; l < np; ++l) {
+            const uint64_t G = (uint64_t)std::llrint(std::ldexp(g[i * np + l] * log2e, 63)) + (1ull << 63);
+            (*words)[at_c + l] += (1ull << 61) - ((G >> 2) + ((G >> 1) & 1));
+            words->push_back(G);
+        }
     return std::string();
 }
 
@@ -1253,57 +1345,75 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
     if (n > 65535) return fail(c, BSG_ERR_CAPACITY, "at most 65535 swaptions per call");
     if (trials < 2 || trials > ((uint64_t)1 << 40))
         return fail(c, BSG_ERR_INVALID_ARG, "trials must be 2..2^40");
-    std::vector<bsg::SwParams> tab(n);
-    int max_steps = 2;
-    for (size_t i = 0; i < n; ++i) {
-        const std::string why = swaption_setup(sw[i], &tab[i]);
-        if (!why.empty()) return fail(c, BSG_ERR_INVALID_ARG, "swaption " + std::to_string(i) + ": " + why);
-        max_steps = std::max(max_steps, sw[i].n_steps);
-    }
-    BSG_CK(c, cudaSetDevice(c->device));
-    if (int st = drain_pipeline(c)) return st;
-    // paths per thread: the most (up to 32; each block pays a set-up) that
-    // still leave 1216 blocks, four waves of 2 blocks on 152 SMs.  A fixed
-    // rule of (n, trials), so the summation order -- and the bits -- do
-    // not depend on the device.
-    int per_thread = 32;
-    while (per_thread > 1 && n * (size_t)bsg::swaption_chunks(trials, per_thread) < 1216) per_thread /= 2;
-    const size_t chunks = (size_t)bsg::swaption_chunks(trials, per_thread);
-    const size_t tab_b = round_up(n * sizeof(bsg::SwParams), 256);
-    const size_t part_b = round_up(2 * n * chunks * sizeof(double), 256);
-    const size_t out_b = round_up(2 * n * sizeof(double), 256);
-    const size_t need = tab_b + part_b + out_b;
-    if (need > c->sw_cap) {
-        if (c->d_sw) {
+    try {
+        constexpr size_t head_words = sizeof(bsg::SwHead) / 8;
+        std::vector<bsg::SwHead> heads(n);
+        std::vector<uint64_t> words;
+        bool large = false;
+        for (size_t i = 0; i < n; ++i) {
+            const std::string why = swaption_setup(sw[i], &heads[i], &words);
+            if (!why.empty())
+                return fail(c, BSG_ERR_INVALID_ARG, "swaption " + std::to_string(i) + ": " + why);
+            heads[i].words_at += (uint32_t)(n * head_words);
+            large = large || heads[i].wide || heads[i].n_exp > 4;
+        }
+        BSG_CK(c, cudaSetDevice(c->device));
+        if (int st = drain_pipeline(c)) return st;
+        // device: counters (kept zero) | table | partials; pinned: results | table
+        const size_t tab_words = n * head_words + words.size();
+        const bool inl = tab_words <= (size_t)bsg::kSwInlineWords;
+        const size_t done_b = round_up(65535 * sizeof(unsigned), 256);
+        const size_t tab_b = inl ? 0 : round_up(tab_words * 8, 256);
+        const size_t need = done_b + tab_b + bsg::swaption_partial_bytes((int)n, trials);
+        const size_t out_b = round_up(2 * n * sizeof(double), 256);
+        if (need > c->sw_cap) {
             BSG_CK(c, cudaStreamSynchronize(c->stream));
-            cudaFree(c->d_sw);
+            if (c->d_sw) cudaFree(c->d_sw);
             c->d_sw = nullptr;
             c->sw_cap = 0;
+            if (cudaMalloc(&c->d_sw, need) != cudaSuccess) {
+                cudaGetLastError();
+                return fail(c, BSG_ERR_OUT_OF_MEMORY, "swaption scratch");
+            }
+            BSG_CK(c, cudaMemsetAsync(c->d_sw, 0, done_b, c->stream));
+            c->sw_cap = need;
         }
-        if (cudaMalloc(&c->d_sw, need) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(c, BSG_ERR_OUT_OF_MEMORY, "swaption scratch");
+        if (out_b + tab_b > c->h_sw_cap) {
+            BSG_CK(c, cudaStreamSynchronize(c->stream));
+            if (c->h_sw) cudaFreeHost(c->h_sw);
+            c->h_sw = nullptr;
+            c->h_sw_cap = 0;
+            if (cudaMallocHost(&c->h_sw, out_b + tab_b) != cudaSuccess) {
+                cudaGetLastError();
+                return fail(c, BSG_ERR_OUT_OF_MEMORY, "swaption staging");
+            }
+            c->h_sw_cap = out_b + tab_b;
         }
-        c->sw_cap = need;
+        double* out = reinterpret_cast<double*>(c->h_sw);  // the kernel writes the results here itself
+        bsg::SwInline in;
+        uint64_t* d_tab = nullptr;
+        uint64_t* tab = in.words;
+        if (!inl) {
+            d_tab = reinterpret_cast<uint64_t*>(c->d_sw + done_b);
+            tab = reinterpret_cast<uint64_t*>(c->h_sw + out_b);
+        }
+        std::memcpy(tab, heads.data(), n * sizeof(bsg::SwHead));
+        if (!words.empty()) std::memcpy(tab + n * head_words, words.data(), words.size() * 8);
+        if (!inl) BSG_CK(c, cudaMemcpyAsync(d_tab, tab, tab_words * 8, cudaMemcpyHostToDevice, c->stream));
+        cudaError_t e = bsg::launch_swaptions(in, d_tab, (int)n, large, trials, c->d_sw + done_b + tab_b,
+                                              reinterpret_cast<unsigned*>(c->d_sw), out, c->sm_count,
+                                              c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "launch_swaptions");
+        c->launches++;
+        BSG_CK(c, cudaStreamSynchronize(c->stream));
+        for (size_t i = 0; i < n; ++i) {
+            price[i] = out[2 * i];
+            if (std_err) std_err[i] = out[2 * i + 1];
+        }
+        return BSG_OK;
+    } catch (const std::bad_alloc&) {
+        return fail(c, BSG_ERR_OUT_OF_MEMORY, "host allocation failed");
     }
-    bsg::SwParams* d_tab = reinterpret_cast<bsg::SwParams*>(c->d_sw);
-    double* d_part = reinterpret_cast<double*>(c->d_sw + tab_b);
-    double* d_out = reinterpret_cast<double*>(c->d_sw + tab_b + part_b);
-    BSG_CK(c, cudaMemcpyAsync(d_tab, tab.data(), n * sizeof(bsg::SwParams), cudaMemcpyHostToDevice,
-                              c->stream));
-    cudaError_t e = bsg::launch_swaptions(d_tab, (int)n, max_steps, trials, per_thread, d_part, d_out,
-                                          c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "launch_swaptions");
-    c->launches += 2;
-    std::vector<double> out(2 * n);
-    BSG_CK(c, cudaMemcpyAsync(out.data(), d_out, 2 * n * sizeof(double), cudaMemcpyDeviceToHost,
-                              c->stream));
-    BSG_CK(c, cudaStreamSynchronize(c->stream));
-    for (size_t i = 0; i < n; ++i) {
-        price[i] = out[2 * i];
-        if (std_err) std_err[i] = out[2 * i + 1];
-    }
-    return BSG_OK;
 }
 
 extern "C" int bsg_swaption_normals(bsg_ctx* c, const uint32_t* words, size_t n_pairs, double* z) {

@@ -144,29 +144,50 @@ int device_extent(const void* p, size_t bytes, int device);
 constexpr int kSwMaxSteps = 32;    // grid points of the HJM path (iN)
 constexpr int kSwMaxFactors = 8;   // volatility factors (iFactors)
 
-// One swaption as the path kernel reads it: the driver's constants, already
-// rounded as the reference rounds them, and the raw curves.
-struct SwParams {
-    double strike_cont;       // strike in continuous compounding
-    double payment_interval;  // years between swap payments
-    double h, sqh;            // grid step and its square root
-    int n_steps, n_factors;
-    int start;                // the swaption's maturity on the grid
-    int swap_len;             // forward rates of the swap curve at maturity
-    int freq, swap_points;    // payment every freq steps, the last at swap_points
+constexpr int kSwMaxExp = kSwMaxSteps;  // payments, and the path's own discount factor
+
+// One swaption as the path kernel reads it.  A path is linear in its normal
+// variates, so each exponential the payoff needs -- the discount factor of
+// each payment, then (disc_varies) the path's own down to maturity -- has an
+// exponent of a constant plus one coefficient per variate.  Its words, from
+// words_at of the table on: n_exp payments (doubles), n_exp constants, then
+// n_exp coefficients per variate.  Constants and coefficients are in powers
+// of two, fixed point (swaption_setup in bsg_api.cu), or (wide: some exponent
+// may leave the fixed-point range) natural exponents as doubles.
+struct SwHead {
     uint64_t seed;            // the paths' random stream
-    double yield[kSwMaxSteps];
-    double vol[kSwMaxFactors][kSwMaxSteps];  // [k][m], m < n_steps - 1
+    double disc;              // the path's discount factor where it is a constant, else 1
+    uint32_t words_at, n_words;
+    int n_normals;            // variates up to maturity: grid steps x factors
+    int n_exp;
+    int disc_varies;          // 0, 1
+    int wide;                 // 0, 1
+};
+// s steps to maturity and p payments share a grid of at most 32 points:
+// n_exp (2 + n_normals) <= 32 (2 + 8 s) and (p + 1) 8 s <= 8 s (32 - s)
+constexpr int kSwMaxWords = 2 * kSwMaxExp + 8 * 256;
+
+// A table small enough to travel with the launch (a copy before the kernel
+// costs 3 us of a 20 us call).
+constexpr int kSwInlineWords = 480;
+struct SwInline {
+    uint64_t words[kSwInlineWords];
 };
 
-// Blocks of trials per swaption for `trials` paths, per_thread paths per thread.
-int swaption_chunks(uint64_t trials, int per_thread);
-// Prices nsw swaptions (device table prm) with `trials` paths each:
-// out[2 i] = mean discounted payoff, out[2 i + 1] = its standard error.
-// partial: device scratch of 2 * nsw * swaption_chunks(trials, per_thread)
-// doubles.  max_steps: the largest n_steps in the table.
-cudaError_t launch_swaptions(const SwParams* prm, int nsw, int max_steps, uint64_t trials,
-                             int per_thread, double* partial, double* out, cudaStream_t st);
+// Paths per thread and blocks of paths per swaption for `trials` paths: a
+// rule of the trials alone, so that the order of a swaption's sums is too.
+int swaption_per_thread(uint64_t trials);
+uint64_t swaption_chunks(uint64_t trials);
+size_t swaption_partial_bytes(int nsw, uint64_t trials);
+// Prices nsw swaptions with `trials` paths each: out[2 i] = mean discounted
+// payoff, out[2 i + 1] = its standard error (device-writable memory).  The
+// table: nsw heads, then their words, at `table` (device memory) or in `in`
+// (table NULL).  large: some swaption has more than four exponents or is
+// wide.  partial: device scratch of swaption_partial_bytes; done: nsw device
+// counters, zero, left zero.
+cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw, bool large,
+                             uint64_t trials, void* partial, unsigned* done, double* out, int sm_count,
+                             cudaStream_t st);
 
 // z[2 i], z[2 i + 1] = the swaption kernel's normal pair of words[4 i .. 4 i + 3]
 // (device arrays), i < n.

@@ -17,22 +17,26 @@
 // with mu[m] = (h/2) sum_k (S_k(m)^2 - S_k(m-1)^2) (S_k: running sums of
 // factor k's vols), the drift that makes discounted bonds martingales.
 //
-// Work that cannot reach the payoff is not done: rows of the path after the
-// swaption's maturity t_s (the reference simulates all n_steps - 1 of them),
-// the entries of each row that no payment date of the swap reads, and the
-// discount factors of swap dates without a payment.  The variates of the
-// rows that are simulated are the same ones: each is drawn from a
-// counter-based generator (Philox4x32-10, Salmon et al., SC'11) keyed by
-// (seed, trial, index) and turned normal by Box-Muller (bsg_swmath.h:
-// table-driven -2 ln u and sin/cos(2 pi u) from the uniforms' bits), so the
-// prices equal those of a full-path simulation with the same stream.  The
-// kernel is bound by GB300's FP64 rate; the trimming and the table-driven
-// transform and exp (bsg_swmath.h) halve its double-precision work per path.
+// The path rows are linear in the variates, so the rows themselves are not
+// formed: the exponent of each payment's discount factor (and of D) is a
+// constant plus a coefficient times each variate up to maturity, the
+// coefficients differences of the S_k (swaption_setup in bsg_api.cu).  The
+// variates are the ones a full-path simulation with the same stream draws:
+// a counter-based generator (Philox4x32-10, Salmon et al., SC'11) keyed by
+// (seed, trial, index), turned normal by Box-Muller.
 //
-// Reduction: each block reduces its paths' sums (sum and sum of squares of
-// the discounted payoff) in a fixed order and writes one partial; a second
-// kernel adds a swaption's partials in a fixed order.  Results do not depend
-// on scheduling: two runs give the same bits.
+// What bounds it: in doubles the FP64 rate (2 operations a clock and SM):
+// 33.1 ms for 128 swaptions x 1M paths with 130 FP64 operations a path, that
+// pipe 85 % busy.  So the variates, the exponents and the powers of two are
+// 64-bit fixed point (bsg_swmath.h), and FP64 is left with a payment's
+// multiply-add, the floor and the two sums, 4 to 6 operations a path: 7.35 ms,
+// bound by integer issue (950 instructions a path).
+//
+// Reduction: each warp reduces its paths' sums (sum and sum of squares of
+// the discounted payoff) in a fixed order and writes one partial; the block
+// that finishes a swaption last adds its partials in a fixed order.  Which
+// paths a partial covers depends on the number of trials alone: two runs, and
+// a swaption alone or among others, give the same bits.
 #include "bsg_internal.h"
 #include "bsg_swmath.h"
 
@@ -45,6 +49,7 @@ namespace bsg {
 namespace {
 
 constexpr int kSwThreads = 256;
+constexpr int kSwWarps = kSwThreads / 32;
 
 __device__ __forceinline__ void philox4x32_10(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
                                               uint32_t k0, uint32_t k1, uint32_t out[4]) {
@@ -66,182 +71,201 @@ __device__ __forceinline__ void philox4x32_10(uint32_t x0, uint32_t x1, uint32_t
     out[3] = x3;
 }
 
-// Normal variates 2j and 2j + 1 of trial t: Box-Muller on the uniforms of
-// the Philox block (seed, t, j), evaluated from their bits (bsg_swmath.h).
-__device__ __forceinline__ void normal_pair(const bsg_sw::Tables& tab, uint64_t seed, uint64_t t,
-                                            uint32_t j, double& z0, double& z1) {
-    uint32_t x[4];
-    philox4x32_10((uint32_t)t, (uint32_t)(t >> 32), j, 0u, (uint32_t)seed, (uint32_t)(seed >> 32), x);
-    bsg_sw::normal_pair(tab, x[0], x[1], x[2], x[3], &z0, &z1);
-}
-
 __device__ const bsg_sw::Tables kSwTables = BSG_SW_TABLES;
 
 // Copies the tables of bsg_swmath.h into shared memory (all threads of the block).
 __device__ __forceinline__ void load_tables(bsg_sw::Tables& dst) {
+    static_assert(sizeof(bsg_sw::Tables) % sizeof(double2) == 0, "copied in 16-byte words");
     const double2* src = reinterpret_cast<const double2*>(&kSwTables);
     double2* d = reinterpret_cast<double2*>(&dst);
     for (int i = threadIdx.x; i < (int)(sizeof(bsg_sw::Tables) / sizeof(double2)); i += blockDim.x)
         d[i] = src[i];
 }
 
-// Per-swaption constants in shared memory: the forward curve, the drift
-// times h, the vols times sqrt(h), the swap payments.
-template <int MAXN>
+// One swaption in shared memory: its head and its words (pays, constants,
+// coefficients; bsg_internal.h).
 struct SwShared {
-    double fwd[MAXN];
-    double muh[MAXN];
-    double vol[kSwMaxFactors][MAXN];
-    double pay[MAXN];
-    double red[2][kSwThreads / 32];
     bsg_sw::Tables nt;
+    SwHead head;
+    uint64_t words[kSwMaxWords];
+    double red[2][kSwThreads];
+    int last;
 };
 
-// Paths q * kSwThreads + threadIdx.x (q < per_thread) of one block, with the
-// path rows cut to the NEED entries that reach the payoff (row i of the
-// reference's path computes all n - 1 - i; the others never reach a
-// payment date before the swap's last, so the price is the same).
-template <int MAXN, int NEED>
-__device__ __forceinline__ void price_paths(const SwParams& p, const SwShared<MAXN>& sh, uint64_t base,
-                                            int per_thread, uint64_t trials, double& sum,
-                                            double& sum_sq) {
-    const int s = p.start, nf = p.n_factors, last = p.swap_points;
-    const double h = p.h;
+__device__ __forceinline__ double as_double(uint64_t u) { return __longlong_as_double((long long)u); }
+
+// The undiscounted-by-a-constant payoff of trial t of the swaption in sh.
+// NP: the number of exponents, or with GUARD an upper bound of it.
+template <int NP, bool GUARD>
+__device__ __forceinline__ double path_payoff(const SwShared& sh, uint64_t t) {
+    const SwHead& hd = sh.head;
+    const int np = GUARD ? hd.n_exp : NP;
+    const uint64_t* c0 = sh.words + np;
+    const uint64_t* g = sh.words + 2 * np;
+    uint64_t x[NP], half = 0;
+#pragma unroll
+    for (int l = 0; l < NP; ++l) x[l] = (!GUARD || l < np) ? c0[l] : 0;
+    const int nz = hd.n_normals;
+#pragma unroll 1
+    for (int i = 0; i < nz; i += 2) {
+        uint32_t w[4];
+        philox4x32_10((uint32_t)t, (uint32_t)(t >> 32), (uint32_t)(i >> 1), 0u, (uint32_t)hd.seed,
+                      (uint32_t)(hd.seed >> 32), w);
+        // coefficients g = G 2^-63 and variates z = Z 2^-58, both moved into
+        // the unsigned range (swaption_setup's constants take that out again)
+        const bsg_sw::Root r = bsg_sw::sqrt_scaled(
+            sh.nt, bsg_sw::neg2_ln_scaled(sh.nt, bsg_sw::unit_bits(w[0], w[1])));
+        int64_t zs, zc;
+        bsg_sw::sincos_2pi_fixed(sh.nt, bsg_sw::unit_bits(w[2], w[3]), &zs, &zc);
+        const uint64_t z0 = (uint64_t)bsg_sw::times_root(r, zc) + (1ull << 62);
+        half += z0 >> 1;
+#pragma unroll
+        for (int l = 0; l < NP; ++l)
+            if (!GUARD || l < np) x[l] += bsg_sw::mulhi(g[l], z0);
+        g += np;
+        if (i + 1 < nz) {
+            const uint64_t z1 = (uint64_t)bsg_sw::times_root(r, zs) + (1ull << 62);
+            half += z1 >> 1;
+#pragma unroll
+            for (int l = 0; l < NP; ++l)
+                if (!GUARD || l < np) x[l] += bsg_sw::mulhi(g[l], z1);
+            g += np;
+        }
+    }
+    // the payments' discount factors, then the path's own if it varies
+    const int pays = hd.n_exp - hd.disc_varies;
+    double v = -1.0, disc = 1.0;
+#pragma unroll
+    for (int l = 0; l < NP; ++l)
+        if (!GUARD || l < np) {
+            const double y = bsg_sw::exp2_fixed(sh.nt, (int64_t)(x[l] - half));
+            if (l < pays) v = __fma_rn(as_double(sh.words[l]), y, v);
+            else disc = y;
+        }
+    return v > 0.0 ? __dmul_rn(v, disc) : 0.0;
+}
+
+// The same in double precision, for exponents outside the fixed-point range:
+// words hold the constants and coefficients as doubles, natural exponents.
+__device__ __noinline__ double path_payoff_wide(const SwShared& sh, uint64_t t) {
+    const SwHead& hd = sh.head;
+    const int np = hd.n_exp, nz = hd.n_normals, pays = np - hd.disc_varies;
+    double v = -1.0, disc = 1.0;
+    for (int l = 0; l < np; ++l) {
+        double x = as_double(sh.words[np + l]), z[2];
+        for (int i = 0; i < nz; ++i) {
+            if ((i & 1) == 0) {
+                uint32_t w[4];
+                philox4x32_10((uint32_t)t, (uint32_t)(t >> 32), (uint32_t)(i >> 1), 0u,
+                              (uint32_t)hd.seed, (uint32_t)(hd.seed >> 32), w);
+                bsg_sw::normal_pair(sh.nt, w[0], w[1], w[2], w[3], &z[0], &z[1]);
+            }
+            x = __fma_rn(as_double(sh.words[2 * np + i * np + l]), z[i & 1], x);
+        }
+        const double y = bsg_sw::exp_(sh.nt, x);
+        if (l < pays) v = __fma_rn(as_double(sh.words[l]), y, v);
+        else disc = y;
+    }
+    return v > 0.0 ? __dmul_rn(v, disc) : 0.0;
+}
+
+template <int NP, bool GUARD, bool WIDE = false>
+__device__ __forceinline__ void sum_paths(const SwShared& sh, uint64_t base, int per_thread,
+                                          uint64_t trials, double& sum, double& sum_sq) {
+#pragma unroll 1
     for (int q = 0; q < per_thread; ++q) {
         const uint64_t t = base + (uint64_t)q * kSwThreads + threadIdx.x;
         if (t >= trials) break;
-        double f[NEED + 1];
-#pragma unroll
-        for (int m = 0; m <= NEED; ++m) f[m] = sh.fwd[m];
-        double acc = 0.0, zc[2] = {0.0, 0.0};
-        int zi = 0;  // index of the next normal variate of this trial
-        for (int i = 0; i < s; ++i) {
-            acc += f[0];
-            double shock[NEED];
-#pragma unroll
-            for (int m = 0; m < NEED; ++m) shock[m] = 0.0;
-            for (int k = 0; k < nf; ++k, ++zi) {
-                if ((zi & 1) == 0) normal_pair(sh.nt, p.seed, t, (uint32_t)(zi >> 1), zc[0], zc[1]);
-                const double z = zc[zi & 1];
-#pragma unroll
-                for (int m = 0; m < NEED; ++m) shock[m] = __fma_rn(sh.vol[k][m], z, shock[m]);
-            }
-            // row i + 1 from row i (entries at or past NEED - i are never read)
-#pragma unroll
-            for (int m = 0; m < NEED; ++m) f[m] = f[m + 1] + sh.muh[m] + shock[m];
-        }
-        const double disc = bsg_sw::exp_(sh.nt, -acc * h);
-        double fixed = 0.0, accs = 0.0;
-#pragma unroll
-        for (int l = 0; l <= NEED; ++l) {
-            if (l <= last && sh.pay[l] != 0.0) fixed += sh.pay[l] * bsg_sw::exp_(sh.nt, -accs * h);
-            accs += f[l];
-        }
-        const double payoff = fixed - 1.0 > 0.0 ? fixed - 1.0 : 0.0;
-        const double dp = payoff * disc;
-        sum += dp;
-        sum_sq += dp * dp;
+        const double dp = WIDE ? path_payoff_wide(sh, t) : path_payoff<NP, GUARD>(sh, t);
+        sum = __dadd_rn(sum, dp);
+        sum_sq = __fma_rn(dp, dp, sum_sq);
     }
 }
 
-// One block: paths [chunk * per_block, ...) of swaption blockIdx.y.
-template <int MAXN>
-__global__ void __launch_bounds__(kSwThreads, MAXN <= 12 ? 2 : 1) swaption_paths_kernel(const SwParams* __restrict__ prm,
-                                                                    uint64_t trials, int per_thread,
-                                                                    double* __restrict__ partial) {
-    __shared__ SwShared<MAXN> sh;
-    const SwParams& p = prm[blockIdx.y];
-    const int n = p.n_steps, nf = p.n_factors;
-    const double h = p.h;
-    // set-up, the same in every block of the swaption: forward curve from the
-    // yields, drift from the vols, payments (HJM_Swaption_Blocking.cpp:132-140)
+// Persistent blocks over (swaption, chunk of per_thread x 256 paths) items.
+// LARGE: also swaptions of more than four exponents or outside the
+// fixed-point range (their registers would cost the others a block per SM).
+template <bool LARGE>
+__global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 3) swaption_paths_kernel(
+    const __grid_constant__ SwInline in, const uint64_t* __restrict__ table, int nsw, uint64_t trials,
+    int per_thread, uint64_t chunks, double2* __restrict__ partial, unsigned* __restrict__ done,
+    double* __restrict__ out) {
+    __shared__ SwShared sh;
     load_tables(sh.nt);
-    if (threadIdx.x < MAXN) {
-        const int i = threadIdx.x;
-        sh.fwd[i] = i == 0 ? p.yield[0]
-                           : (i < n ? (double)(i + 1) * p.yield[i] - (double)i * p.yield[i - 1] : 0.0);
-        double pay = 0.0;
-        if (i < p.swap_len && i >= p.freq && i <= p.swap_points && (i % p.freq) == 0)
-            pay = i == p.swap_points ? exp(p.strike_cont * p.payment_interval)
-                                     : exp(p.strike_cont * p.payment_interval) - 1;
-        sh.pay[i] = pay;
-        double mu = 0.0;
-        for (int k = 0; k < nf; ++k) {
-            double s_prev = 0.0;
-            for (int m = 0; m < i && m < n - 1; ++m) s_prev += p.vol[k][m];
-            const double vk = i < n - 1 ? p.vol[k][i] : 0.0;
-            mu += h * vk * (s_prev + 0.5 * vk);
-            sh.vol[k][i] = vk * p.sqh;
-        }
-        sh.muh[i] = mu * h;
-    }
-    __syncthreads();
-    const uint64_t base = (uint64_t)blockIdx.x * per_thread * kSwThreads;
-    double sum = 0.0, sum_sq = 0.0;
-    // rows of the path that reach the payoff: row i needs entries
-    // m < swap_points + start - 1 - i (the last payment's discount reads
-    // f[0 .. swap_points - 1] of row start); swap_points + start <= n - 1
-    switch (p.swap_points + p.start - 1) {
-        case 1: price_paths<MAXN, 1>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 2: price_paths<MAXN, 2>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 3: price_paths<MAXN, 3>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 4: price_paths<MAXN, 4>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 5: price_paths<MAXN, 5>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 6: price_paths<MAXN, 6>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 7: price_paths<MAXN, 7>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 8: price_paths<MAXN, 8>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 9: price_paths<MAXN, 9>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        case 10: price_paths<MAXN, 10>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-        default: price_paths<MAXN, MAXN - 1>(p, sh, base, per_thread, trials, sum, sum_sq); break;
-    }
-    // block reduction in a fixed order
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_down_sync(0xffffffffu, sum, o);
-        sum_sq += __shfl_down_sync(0xffffffffu, sum_sq, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        sh.red[0][threadIdx.x >> 5] = sum;
-        sh.red[1][threadIdx.x >> 5] = sum_sq;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int w = 0; w < kSwThreads / 32; ++w) {
-            a += sh.red[0][w];
-            b += sh.red[1][w];
-        }
-        partial[2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x)] = a;
-        partial[2 * ((size_t)blockIdx.y * gridDim.x + blockIdx.x) + 1] = b;
-    }
-}
-
-// One block per swaption: its chunks' partials in a fixed order, then the
-// mean and the reference's standard error (HJM_Swaption_Blocking.cpp:212-214).
-__global__ void __launch_bounds__(kSwThreads) swaption_reduce_kernel(const double* __restrict__ partial,
-                                                                     int chunks, uint64_t trials,
-                                                                     double* __restrict__ out) {
-    __shared__ double sa[kSwThreads], sb[kSwThreads];
-    double a = 0.0, b = 0.0;
-    const double* p = partial + 2 * (size_t)blockIdx.x * chunks;
-    for (int c = threadIdx.x; c < chunks; c += kSwThreads) {
-        a += p[2 * c];
-        b += p[2 * c + 1];
-    }
-    sa[threadIdx.x] = a;
-    sb[threadIdx.x] = b;
-    __syncthreads();
-    for (int w = kSwThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            sa[threadIdx.x] += sa[threadIdx.x + w];
-            sb[threadIdx.x] += sb[threadIdx.x + w];
+    const uint64_t items = chunks * (uint64_t)nsw;
+    for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint64_t sw = item / chunks, chunk = item - sw * chunks;
+        __syncthreads();  // the previous item's reads of sh are done
+        {
+            // head, then its words (from the launch's parameters when they all fit there)
+            constexpr int hw = (int)(sizeof(SwHead) / 8);
+            const uint64_t* tab = table ? table : in.words;
+            uint64_t* hd = reinterpret_cast<uint64_t*>(&sh.head);
+            if (threadIdx.x < hw) hd[threadIdx.x] = tab[sw * hw + threadIdx.x];
+            __syncthreads();
+            const uint64_t* src = tab + sh.head.words_at;
+            for (int i = threadIdx.x; i < sh.head.n_words; i += kSwThreads) sh.words[i] = src[i];
         }
         __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const double m = (double)trials, sum = sa[0], sum_sq = sb[0];
-        out[2 * blockIdx.x] = sum / m;
-        out[2 * blockIdx.x + 1] = sqrt((sum_sq - sum * sum / m) / (m - 1.0)) / sqrt(m);
+        const uint64_t base = chunk * per_thread * kSwThreads;
+        double sum = 0.0, sum_sq = 0.0;
+        if (LARGE && sh.head.wide) {
+            sum_paths<1, true, true>(sh, base, per_thread, trials, sum, sum_sq);
+        } else {
+            switch (sh.head.n_exp) {
+                case 1: sum_paths<1, false>(sh, base, per_thread, trials, sum, sum_sq); break;
+                case 2: sum_paths<2, false>(sh, base, per_thread, trials, sum, sum_sq); break;
+                case 3: sum_paths<3, false>(sh, base, per_thread, trials, sum, sum_sq); break;
+                case 4: sum_paths<4, false>(sh, base, per_thread, trials, sum, sum_sq); break;
+                default:
+                    if constexpr (LARGE) {
+                        if (sh.head.n_exp <= 8) sum_paths<8, true>(sh, base, per_thread, trials, sum, sum_sq);
+                        else sum_paths<kSwMaxExp, true>(sh, base, per_thread, trials, sum, sum_sq);
+                    }
+            }
+        }
+        // the warp's two sums in a fixed order: the lower half of the warp adds
+        // up sum, the upper half sum_sq
+        const int lane = threadIdx.x & 31;
+        const double give = lane < 16 ? sum_sq : sum, keep = lane < 16 ? sum : sum_sq;
+        double a = __dadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, 16));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) a = __dadd_rn(a, __shfl_xor_sync(0xffffffffu, a, o));
+        const double b = __shfl_sync(0xffffffffu, a, 16);
+        if (lane == 0)
+            partial[item * kSwWarps + (threadIdx.x >> 5)] =
+                make_double2(__dmul_rn(a, sh.head.disc), __dmul_rn(b, __dmul_rn(sh.head.disc, sh.head.disc)));
+        // the last block of the swaption adds its partials up
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) sh.last = atomicAdd(&done[sw], 1u) == (unsigned)(chunks - 1);
+        __syncthreads();
+        if (!sh.last) continue;
+        __threadfence();
+        double ta = 0.0, tb = 0.0;
+        const double2* p = partial + sw * chunks * kSwWarps;
+        for (uint64_t i = threadIdx.x; i < chunks * kSwWarps; i += kSwThreads) {
+            const double2 v = __ldcg(p + i);
+            ta = __dadd_rn(ta, v.x);
+            tb = __dadd_rn(tb, v.y);
+        }
+        sh.red[0][threadIdx.x] = ta;
+        sh.red[1][threadIdx.x] = tb;
+        __syncthreads();
+        for (int w = kSwThreads / 2; w > 0; w >>= 1) {
+            if (threadIdx.x < w) {
+                sh.red[0][threadIdx.x] = __dadd_rn(sh.red[0][threadIdx.x], sh.red[0][threadIdx.x + w]);
+                sh.red[1][threadIdx.x] = __dadd_rn(sh.red[1][threadIdx.x], sh.red[1][threadIdx.x + w]);
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            // the mean and the reference's standard error (HJM_Swaption_Blocking.cpp:212-214)
+            const double m = (double)trials, s1 = sh.red[0][0], s2 = sh.red[1][0];
+            out[2 * sw] = s1 / m;
+            out[2 * sw + 1] = sqrt((s2 - s1 * s1 / m) / (m - 1.0)) / sqrt(m);
+            done[sw] = 0;  // ready for the next call
+        }
     }
 }
 
@@ -265,24 +289,35 @@ cudaError_t launch_swaption_normals(const uint32_t* words, uint64_t n, double* z
     return cudaGetLastError();
 }
 
-int swaption_chunks(uint64_t trials, int per_thread) {
-    const uint64_t per_block = (uint64_t)per_thread * kSwThreads;
-    return (int)((trials + per_block - 1) / per_block);
+int swaption_per_thread(uint64_t trials) {
+    int q = 1;
+    while (q < 1024 && (trials + 2 * q * kSwThreads - 1) / ((uint64_t)2 * q * kSwThreads) >= 304) q *= 2;
+    return q;
 }
 
-cudaError_t launch_swaptions(const SwParams* prm, int nsw, int max_steps, uint64_t trials,
-                             int per_thread, double* partial, double* out, cudaStream_t st) {
-    if (nsw <= 0 || trials < 2 || per_thread < 1) return cudaErrorInvalidValue;
-    const int chunks = swaption_chunks(trials, per_thread);
-    if (nsw > 65535) return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)chunks, (unsigned)nsw);
-    if (max_steps <= 12)
-        swaption_paths_kernel<12><<<grid, kSwThreads, 0, st>>>(prm, trials, per_thread, partial);
+uint64_t swaption_chunks(uint64_t trials) {
+    const uint64_t per_block = (uint64_t)swaption_per_thread(trials) * kSwThreads;
+    return (trials + per_block - 1) / per_block;
+}
+
+size_t swaption_partial_bytes(int nsw, uint64_t trials) {
+    return (size_t)nsw * swaption_chunks(trials) * kSwWarps * sizeof(double2);
+}
+
+cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw, bool large,
+                             uint64_t trials, void* partial, unsigned* done, double* out, int sm_count,
+                             cudaStream_t st) {
+    if (nsw <= 0 || trials < 2) return cudaErrorInvalidValue;
+    const uint64_t chunks = swaption_chunks(trials), items = chunks * (uint64_t)nsw;
+    const unsigned grid = (unsigned)std::min<uint64_t>(items, (uint64_t)sm_count * (large ? 2 : 3));
+    const int per_thread = swaption_per_thread(trials);
+    double2* part = static_cast<double2*>(partial);
+    if (large)
+        swaption_paths_kernel<true><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
+                                                                 part, done, out);
     else
-        swaption_paths_kernel<kSwMaxSteps><<<grid, kSwThreads, 0, st>>>(prm, trials, per_thread, partial);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    swaption_reduce_kernel<<<(unsigned)nsw, kSwThreads, 0, st>>>(partial, chunks, trials, out);
+        swaption_paths_kernel<false><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
+                                                                  part, done, out);
     return cudaGetLastError();
 }
 

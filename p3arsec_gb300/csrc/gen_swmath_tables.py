@@ -1,10 +1,12 @@
-"""Writes bsg_swmath_tables.h: the tables of the table-driven Box-Muller
-transform and exponential in bsg_swmath.h, computed from 70-digit decimal
-values of ln 2, ln F, sin, cos and 2^(j/64) and rounded once to double.
+"""Writes bsg_swmath_tables.h: the tables of the fixed-point Box-Muller
+transform and power of two and of the double-precision exponential in
+bsg_swmath.h, computed from 70-digit decimal values of ln 2, ln c, sin, cos,
+1/sqrt(y), 2^(j/1024) and 2^(j/64) and rounded once.
 
     python gen_swmath_tables.py      # rewrites bsg_swmath_tables.h here
 
-Every double is written as a hex literal, so the header is exact."""
+Doubles are written as hex literals and fixed-point values as integers, so
+the header is exact."""
 import decimal
 import os
 from fractions import Fraction
@@ -36,6 +38,17 @@ def f64(v) -> float:
 def hexd(v) -> str:
     d = f64(v)
     return d.hex() if d != 0 else "0.0"
+
+
+def fixed(v, bits: int) -> int:
+    """v with `bits` fraction bits, rounded to nearest."""
+    return round(Fraction(v) * 2 ** bits)
+
+
+def hexu(v, bits: int) -> str:
+    x = fixed(v, bits)
+    assert 0 <= x < 1 << 64
+    return f"0x{x:016X}ull"
 
 
 def atan_inv(x: int) -> D:
@@ -77,24 +90,45 @@ def main():
     out = []
     w = out.append
     w("// bsg_swmath_tables.h -- written by gen_swmath_tables.py; do not edit.")
-    w("// Tables of the table-driven Box-Muller transform and exp in bsg_swmath.h.")
+    w("// Tables of the fixed-point Box-Muller transform, 2^x and exp in bsg_swmath.h.")
     w("#pragma once")
     w("")
-    w("// 2 pi 2^-53: the angle of one unit of the 53-bit uniform grid")
-    w(f"#define BSG_SW_TWO_PI_ULP {hexd(2 * PI / D(2) ** 53)}")
+    w("// fixed-point constants: 2 ln 2 (57 fraction bits), 2 pi (61), ln 2 (64)")
+    w(f"#define BSG_SW_2LN2_57 {hexu(2 * ln2, 57)}")
+    w(f"#define BSG_SW_2PI_61 {hexu(2 * PI, 61)}")
+    w(f"#define BSG_SW_LN2_64 {hexu(ln2, 64)}")
     w("")
-    w("// {-2/F, -2 ln F} for F = 1 + j/128, j = 0..128; ln(F/2) for j >= 64")
+    w("// {2 ln c (62 fraction bits), c (20)}, c the reciprocal of the middle of")
+    w("// interval i of [1, 2), i = 0..511; 2 ln(2 c) from i = 256 on; c = 1/2 for the last")
     w("#define BSG_SW_LOG_TABLE \\")
-    for j in range(129):
-        F = D(1) + D(j) / D(128)
-        inv = Fraction(-256, 128 + j)
-        val = D(-2) * (F / 2 if j >= 64 else F).ln()
-        w(f"    {{{hexd(inv)}, {hexd(val)}}}" + (", \\" if j < 128 else ""))
+    for i in range(512):
+        c = 2 ** 19 if i == 511 else round(Fraction(2 ** 20) * Fraction(1024, 1024 + 2 * i + 1))
+        v = 2 * (D(c) / D(2) ** 20 * (2 if i >= 256 else 1)).ln()
+        w(f"    {{{fixed(v, 62)}ll, {c}u}}" + (", \\" if i < 511 else ""))
     w("")
-    w("// 2 i ln 2, i = 0..63")
+    w("// {a, b} (30 fraction bits), i = 64..255: a - b d is at or below 1/sqrt(y)")
+    w("// for y = (i + d)/256, d in [0, 1)")
+    w("#define BSG_SW_RSQRT_TABLE \\")
+    for i in range(64, 256):
+        # the line parallel to the chord that touches the (convex) curve from below
+        y0, y1 = D(i) / 256, D(i + 1) / 256
+        f0, f1 = 1 / y0.sqrt(), 1 / y1.sqrt()
+        slope = (f1 - f0) / (y1 - y0)
+        yt = (-2 * slope) ** (D(-2) / D(3))  # f'(yt) = slope
+        a = 1 / yt.sqrt() + slope * (y0 - yt)
+        fa, fb = int(a * 2 ** 30) - 2, fixed(f0 - f1, 30) + 1  # both towards the low side
+        w(f"    {{{fa}u, {fb}u}}" + (", \\" if i < 255 else ""))
+    w("")
+    w("// {sin, cos}(2 pi j / 1024) (63 fraction bits), j = 0..255")
+    w("#define BSG_SW_ANGLE_TABLE \\")
+    for j in range(256):
+        sj, cj = sin_cos(2 * PI * D(j) / D(1024))
+        w(f"    {{{hexu(sj, 63)}, {hexu(cj, 63)}}}" + (", \\" if j < 255 else ""))
+    w("")
+    w("// 2^(j/1024) (63 fraction bits), j = 0..1023")
     w("#define BSG_SW_EXP2_TABLE \\")
-    for i in range(64):
-        w(f"    {hexd(2 * i * ln2)}" + (", \\" if i < 63 else ""))
+    for j in range(1024):
+        w(f"    {hexu((D(j) / D(1024) * ln2).exp(), 63)}" + (", \\" if j < 1023 else ""))
     w("")
     w("// exp: 64/ln 2, and ln2/64 = L1 + L2")
     L = ln2 / 64
@@ -107,12 +141,6 @@ def main():
     w("#define BSG_SW_EXP_TABLE \\")
     for j in range(64):
         w(f"    {hexd((D(j) / D(64) * ln2).exp())}" + (", \\" if j < 63 else ""))
-    w("")
-    w("// {sin, cos}(2 pi j / 256), j = 0..255")
-    w("#define BSG_SW_ANGLE_TABLE \\")
-    for j in range(256):
-        s, c = sin_cos(2 * PI * D(j) / D(256))
-        w(f"    {{{hexd(s)}, {hexd(c)}}}" + (", \\" if j < 255 else ""))
     w("")
     with open(os.path.join(HERE, "bsg_swmath_tables.h"), "w") as f:
         f.write("\n".join(out) + "\n")
