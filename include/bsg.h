@@ -449,6 +449,9 @@ int bsg_write_soa(const char* path, const bsg_book* book);
 int bsg_read_soa(const char* path, bsg_book* out);
 
 /* ---- tuning ------------------------------------------------------------
+ * A context that was never tuned picks a shape by the size of the book and the
+ * number of passes (all passes of a short book in one launch); a chosen or
+ * autotuned shape is used as it is, one launch per pass.
  * The plain map is a family of kernels: vector width per thread, block size,
  * grid size, load path and, for the resident-prefix load path, the prefix
  * size.  bsg_autotune times the candidates on the context's device for n

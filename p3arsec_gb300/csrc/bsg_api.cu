@@ -91,6 +91,7 @@ struct bsg_ctx {
     size_t cap_al = 0;  // per-array stride in the resident buffer
     char* dev_buf = nullptr;
     bsg::MapCfg tune{1, 256, 0, 0, 0};
+    bool tuned = false;  // tune was chosen (bsg_set_tune, bsg_autotune)
     std::mutex mu;
     std::string err;
     uint64_t launches = 0;
@@ -351,7 +352,13 @@ GraphKey make_key(const bsg::SoA& a, int64_t n, int runs, int mode,
 int enqueue_map_runs(bsg_ctx* c, const bsg::SoA& a, int64_t n, int runs, int mode,
                      unsigned flags) {
     if (n <= 0 || runs <= 0) return BSG_OK;
-    const bsg::MapCfg cfg = c->tune;
+    if (!c->tuned && !(flags & BSG_NO_GRAPH) && bsg::map_runs_fit(a, n, mode, runs, c->sm_count)) {
+        cudaError_t e = bsg::launch_map_runs(a, n, mode, runs, c->sm_count, c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "launch_map_runs");
+        c->launches++;
+        return BSG_OK;
+    }
+    const bsg::MapCfg cfg = c->tuned ? c->tune : bsg::map_default_cfg(a, n, runs);
     if (runs == 1 || (flags & BSG_NO_GRAPH)) {
         for (int j = 0; j < runs; ++j) {
             cudaError_t e = bsg::launch_map(a, n, mode, bsg::pass_cfg(cfg, j, runs), c->sm_count,
@@ -1198,6 +1205,7 @@ int bsg_set_tune(bsg_ctx* c, const bsg_tune* t) {
     std::lock_guard<std::mutex> lk(c->mu);
     if (!tune_valid(t)) return fail(c, BSG_ERR_INVALID_ARG, "unsupported tuning");
     c->tune = cfg_of(*t);
+    c->tuned = true;
     return BSG_OK;
 }
 
@@ -1527,6 +1535,7 @@ extern "C" int bsg_autotune(bsg_ctx* c, size_t n, bsg_tune* out) {
     bsg_tune best{};
     if (tune_cache_lookup(key, &best)) {
         c->tune = cfg_of(best);
+        c->tuned = true;
         if (out) *out = best;
         return BSG_OK;
     }
@@ -1634,6 +1643,7 @@ extern "C" int bsg_autotune(bsg_ctx* c, size_t n, bsg_tune* out) {
     if (e != cudaSuccess) return cuda_fail(c, e, "autotune launch");
     BSG_CK(c, cudaStreamSynchronize(c->stream));
     c->tune = cfg_of(best);
+    c->tuned = true;
     tune_cache_store(key, best);
     if (out) *out = best;
     return BSG_OK;

@@ -78,6 +78,12 @@ inline MapCfg pass_cfg(MapCfg c, int j, int runs) {
     c.rev = (c.load_path == 8) ? (j & 1) : 0;
     return c;
 }
+// The shape of a context that was never tuned, by the book's size and the
+// number of passes.
+MapCfg map_default_cfg(const SoA& a, int64_t n, int runs);
+// Whether launch_map_runs takes `runs` passes of this book (in one launch).
+bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count);
+cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st);
 // Reads and clears the bulk-staged kernel's error word (non-zero: a bounded
 // wait expired and some tiles were not priced).
 unsigned bulk_error_take();

@@ -176,7 +176,7 @@ __device__ __forceinline__ void price_groups(const SoA& a, int64_t g0, int64_t g
 
 // ------------------------------------------------------------- plain map
 // Vector kernel: options [0, n - n % W) in groups of W; the last n % W
-// options by block 0.  blocks_per_sm == 0: each block prices one tile of
+// options, and the `head` options before the (aligned) pointers, by block 0.  blocks_per_sm == 0: each block prices one tile of
 // blockDim.x * VPT groups; otherwise blocks stride over tiles.
 // Programmatic dependent launch: every block lets the next pass launch as
 // soon as it starts (the next pass reads only the inputs, which no pass
@@ -197,7 +197,7 @@ __device__ __forceinline__ void pdl_wait() {
 template <int M, int W, int VPT, int LP>
 __global__ void __launch_bounds__(M == MODE_LIBM_REF ? 256 : 512,
                                   M == MODE_LIBM_REF ? 4 : (VPT == 1 ? 2 : 1))
-    map_vec_kernel(SoA a, int64_t n, int64_t gres, int rev) {
+    map_vec_kernel(SoA a, int64_t n, int head, int64_t gres, int rev) {
     pdl_trigger();
     const unsigned long long pol =
         (lp_evict_first(LP) || lp_resident(LP)) ? evict_first_policy() : 0ull;
@@ -214,8 +214,94 @@ __global__ void __launch_bounds__(M == MODE_LIBM_REF ? 256 : 512,
     if (blockIdx.x == 0) {
         const int64_t i = ngroups * W + threadIdx.x;
         if (i < n) price_scalar<M>(a, i);
+        if ((int)threadIdx.x < head) price_scalar<M>(a, (int64_t)threadIdx.x - head);
     }
     pdl_wait();
+}
+
+// -------------------------------------------- several passes in one launch
+// Short books: all `runs` passes of a book in one launch.  Each thread owns W
+// neighbouring options and makes every pass over them in order, as a worker
+// of the reference's bs_thread does over its range (blackscholes.c:607-658:
+// NUM_RUNS over [start, end), no barrier between runs).  Every pass loads its
+// inputs again (volatile loads; from L1 after the first), evaluates them and
+// stores its prices.  U passes are in flight at once: their loads are issued
+// together, then the U evaluations, whose chains of dependent operations
+// (about 500 clocks each) overlap.
+// What bounds a short book is that chain and the interval between dependent
+// launches, not its bytes (65,536 options: 1.8 MB).  The whole call, 65,536
+// options x 100 passes: 41 us, 58 with one pass in flight, 91 as a graph of
+// programmatic launches, 212 as a graph of plain ones; 100 options: 31, 47,
+// 78, 155.
+template <int W>
+__device__ __forceinline__ Raw<W> ld_again(const void* p) {
+    Raw<W> r;
+    if constexpr (W == 2)
+        asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.v[0]), "=r"(r.v[1]) : "l"(p));
+    else
+        asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p));
+    return r;
+}
+
+template <int M>
+__device__ __forceinline__ float2 price2(float2 s, float2 k, float2 r, float2 v, float2 t, int o0, int o1) {
+    if constexpr (M == MODE_FAST) return price_fast2(s, k, r, v, t, o0, o1);
+    else return make_float2(price<M>(s.x, k.x, r.x, v.x, t.x, o0), price<M>(s.y, k.y, r.y, v.y, t.y, o1));
+}
+
+template <int M, int W, int U>
+__global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int head, int runs) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t o = g * W;
+    if (o + W <= n) {
+        for (int j = 0; j < runs; j += U) {
+            Raw<W> S[U], K[U], R[U], V[U], T[U], O[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j + u < runs) {
+                    S[u] = ld_again<W>(a.s + o);
+                    K[u] = ld_again<W>(a.k + o);
+                    R[u] = ld_again<W>(a.r + o);
+                    V[u] = ld_again<W>(a.v + o);
+                    T[u] = ld_again<W>(a.t + o);
+                    O[u] = ld_again<W>(a.ot + o);
+                }
+            float p[U][W];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+#pragma unroll
+                for (int e = 0; e < W; e += 2) {
+                    const float2 q = price2<M>(
+                        make_float2(__uint_as_float(S[u].v[e]), __uint_as_float(S[u].v[e + 1])),
+                        make_float2(__uint_as_float(K[u].v[e]), __uint_as_float(K[u].v[e + 1])),
+                        make_float2(__uint_as_float(R[u].v[e]), __uint_as_float(R[u].v[e + 1])),
+                        make_float2(__uint_as_float(V[u].v[e]), __uint_as_float(V[u].v[e + 1])),
+                        make_float2(__uint_as_float(T[u].v[e]), __uint_as_float(T[u].v[e + 1])),
+                        (int)O[u].v[e], (int)O[u].v[e + 1]);
+                    p[u][e] = q.x;
+                    p[u][e + 1] = q.y;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j + u < runs) {
+                    if constexpr (W == 2)
+                        asm volatile("st.global.v2.f32 [%0], {%1,%2};"
+                                     :: "l"(a.out + o), "f"(p[u][0]), "f"(p[u][1]) : "memory");
+                    else
+                        asm volatile("st.global.v4.f32 [%0], {%1,%2,%3,%4};"
+                                     :: "l"(a.out + o), "f"(p[u][0]), "f"(p[u][1]), "f"(p[u][2]), "f"(p[u][3])
+                                     : "memory");
+                }
+        }
+    }
+    // the options before the first vector and after the last: two warps of the last block
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 64) {
+        const int64_t i = threadIdx.x < 32 ? n / W * W + threadIdx.x : (int64_t)threadIdx.x - 32 - head;
+        if (threadIdx.x < 32 ? i < n : i < 0)
+            for (int j = 0; j < runs; ++j) price_scalar<M>(a, i);
+    }
 }
 
 // Scalar kernel: any 4-byte aligned pointers.
@@ -406,6 +492,27 @@ static bool aligned(const void* p, uintptr_t al) {
     return (reinterpret_cast<uintptr_t>(p) & (al - 1)) == 0;
 }
 
+// Moves the pointers up to the next `al`-byte boundary when all seven are
+// the same number of options past one (a slice of a book): the options
+// passed over, or -1 when no such move exists or the book ends before it.
+static int peel(SoA* a, int64_t* n, uintptr_t al) {
+    const uintptr_t m = reinterpret_cast<uintptr_t>(a->s) & (al - 1);
+    const void* p[6] = {a->k, a->r, a->v, a->t, a->ot, a->out};
+    for (const void* q : p)
+        if ((reinterpret_cast<uintptr_t>(q) & (al - 1)) != m) return -1;
+    const int h = m ? (int)((al - m) / 4) : 0;
+    if (h > *n) return -1;
+    a->s += h;
+    a->k += h;
+    a->r += h;
+    a->v += h;
+    a->t += h;
+    a->ot += h;
+    a->out += h;
+    *n -= h;
+    return h;
+}
+
 bool map_vectorizable(const SoA& a, const MapCfg& cfg) {
     // 256-bit loads for LP 2 and 6, and for the bulk paths' small-n fallback
     const uintptr_t al = (cfg.load_path >= 2) ? 32 : 16;
@@ -465,9 +572,10 @@ static int64_t device_l2_bytes() {
 }
 
 template <int M>
-static cudaError_t launch_map_mode(const SoA& a, int64_t n, const MapCfg& cfg_in,
+static cudaError_t launch_map_mode(const SoA& a_in, int64_t n, const MapCfg& cfg_in,
                                    int sm_count, cudaStream_t st) {
     MapCfg cfg = cfg_in;
+    SoA a = a_in;
     if constexpr (M == MODE_LIBM_REF) {
         // compute-bound (float-float exp/log): 128-bit loads and one
         // 256-thread block per tile (four resident per SM), whatever shape
@@ -478,7 +586,17 @@ static cudaError_t launch_map_mode(const SoA& a, int64_t n, const MapCfg& cfg_in
         if (cfg.block > 256) cfg.block = 256;
     }
     const int block = cfg.block;
-    if (!map_vectorizable(a, cfg)) {
+    // 256-bit loads for load paths 2 and up where a common boundary is that
+    // far, else 128-bit; a slice of a book (all seven pointers equally far
+    // from one) starts with up to 7 single options.  1,250,001 options from
+    // option 3 of a book: 10M x 100 passes 3.48 ms, 5.25 with the scalar kernel;
+    // 45M once 194 us, 237.
+    int head = peel(&a, &n, cfg.load_path >= 2 ? 32 : 16);
+    if (head < 0 && cfg.load_path >= 2 && (head = peel(&a, &n, 16)) >= 0) {
+        cfg.load_path = 0;
+        cfg.vpt = 1;
+    }
+    if (head < 0) {
         int64_t grid = (n + 255) / 256;
         const int64_t cap = (int64_t)sm_count * 8;
         if (grid > cap) grid = cap;
@@ -487,7 +605,7 @@ static cudaError_t launch_map_mode(const SoA& a, int64_t n, const MapCfg& cfg_in
         return cudaGetLastError();
     }
     if (cfg.load_path >= 3 && cfg.load_path <= 5) {
-        if constexpr (M == MODE_FAST) {
+        if constexpr (M == MODE_FAST) if (head == 0) {
             // 3: <8 options, 3 stages>, 4: <4, 4>, 5: <4, 3>
             if (cfg.load_path == 3 && n >= BulkShape<8, 3>::tile)
                 return launch_map_bulk<M, 8, 3>(a, n, cfg, sm_count, st);
@@ -499,7 +617,7 @@ static cudaError_t launch_map_mode(const SoA& a, int64_t n, const MapCfg& cfg_in
         MapCfg v8 = cfg;  // too small for a whole tile (or another mode): 256-bit loads
         v8.load_path = 2;
         v8.vpt = 1;
-        return launch_map_mode<M>(a, n, v8, sm_count, st);
+        return launch_map_mode<M>(a_in, n + head, v8, sm_count, st);
     }
     const int W = lp_v8(cfg.load_path) ? 8 : 4;
     const int64_t ngroups = n / W;
@@ -534,7 +652,7 @@ static cudaError_t launch_map_mode(const SoA& a, int64_t n, const MapCfg& cfg_in
     lc.numAttrs = cfg.pdl ? 1 : 0;
     cudaError_t le = cudaSuccess;
 #define BSG_LAUNCH(W_, V_, L_) \
-    le = cudaLaunchKernelEx(&lc, map_vec_kernel<M, W_, V_, L_>, a, n, gres, cfg.rev)
+    le = cudaLaunchKernelEx(&lc, map_vec_kernel<M, W_, V_, L_>, a, n, head, gres, cfg.rev)
     if constexpr (M == MODE_FAST) {
         switch (cfg.load_path * 10 + cfg.vpt) {
             case 1: BSG_LAUNCH(4, 1, 0); break;
@@ -581,6 +699,78 @@ cudaError_t launch_map(const SoA& a, int64_t n, int mode, const MapCfg& cfg,
         case MODE_LIBM_REF: return launch_map_mode<MODE_LIBM_REF>(a, n, cfg, sm_count, st);
         default: return cudaErrorInvalidValue;
     }
+}
+
+template <int M>
+static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cudaStream_t st) {
+    const int head = peel(&a, &n, 16);
+    if (head < 0) return cudaErrorInvalidValue;
+    // two options per thread while that needs no more than 512 threads an SM
+    // (155,000 options x 100: 57 us; four a thread would leave half the warps)
+    const bool pairs = n <= (int64_t)sm_count * 1024;
+    const int64_t ngroups = n / (pairs ? 2 : 4);
+    int64_t block = (((ngroups + sm_count - 1) / sm_count) + 31) / 32 * 32;
+    block = block < 64 ? 64 : block > 512 ? 512 : block;
+    int64_t grid = (ngroups + block - 1) / block;
+    if (grid < 1) grid = 1;
+    if (pairs) map_runs_kernel<M, 2, 4><<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs);
+    else map_runs_kernel<M, 4, 2><<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs);
+    return cudaGetLastError();
+}
+
+// Whether the n prices share memory with an input array.
+static bool in_place(const SoA& a, int64_t n) {
+    const uintptr_t o = reinterpret_cast<uintptr_t>(a.out), b = (uintptr_t)n * 4;
+    const void* p[6] = {a.s, a.k, a.r, a.v, a.t, a.ot};
+    for (const void* q : p) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(q);
+        if (x < o + b && o < x + b) return true;
+    }
+    return false;
+}
+
+// Up to 2048 options an SM (4 options a thread, 512 threads): 311,000 options x
+// 100 passes take 100 us, 117 as programmatic launches; at 622,592 both took
+// 222.  The reference-order libm mode stays with those: its evaluation fills
+// the SMs (65,536 x 100: 97 us against 140).
+bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count) {
+    SoA b = a;
+    int64_t m = n;
+    return runs > 1 && mode != MODE_LIBM_REF && n <= (int64_t)sm_count * 2048 && !in_place(a, n) &&
+           peel(&b, &m, 16) >= 0;
+}
+
+cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st) {
+    if (n <= 0 || runs <= 0) return cudaSuccess;
+    switch (mode) {
+        case MODE_FAST: return launch_runs_mode<MODE_FAST>(a, n, runs, sm_count, st);
+        case MODE_SFU_REF: return launch_runs_mode<MODE_SFU_REF>(a, n, runs, sm_count, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+MapCfg map_default_cfg(const SoA& a, int64_t n, int runs) {
+    if (in_place(a, n)) return MapCfg{1, 256, 0, 0, 0};  // passes in strict order
+    const int64_t l2 = device_l2_bytes(), bytes = n * 28;
+    // One pass: 256-bit loads, a 128-thread block per tile (2^28 options:
+    // 1047 us against 1119 with 128-bit loads; the same within 2 % below 20M).
+    if (runs == 1) return MapCfg{1, 128, 0, 2, 0};
+    // Passes launch programmatically, each while the previous one drains.  A
+    // book in half the L2: the same shape (1M x 100: 339 us, 351 with a
+    // persistent grid, 533 without programmatic launches).  Up to 2.5 L2: the
+    // resident prefix (10M x 100: 3.31 ms, 3.57 persistent, 3.82 one block per
+    // tile, 4.16 without; 4M: 1.33, 1.33, 1.42; 15M: 5.54, 5.47, 5.80).  Up to 6
+    // L2: the persistent grid (22M: 8.44, 8.45 one block per tile).  Beyond,
+    // two groups a thread (120M x 100: 45.7 ms, 45.9 with one, 46.4 persistent,
+    // 50.0 without).
+    if (bytes <= l2 / 2) return MapCfg{1, 128, 0, 2, 1};
+    if (bytes <= l2 * 5 / 2) {
+        MapCfg c{1, 128, 4, 7, 1};
+        c.res32 = 10;
+        return c;
+    }
+    if (bytes <= 6 * l2) return MapCfg{1, 256, 2, 2, 1};
+    return MapCfg{2, 128, 0, 2, 1};
 }
 
 // ------------------------------------------------------------------ FP64
