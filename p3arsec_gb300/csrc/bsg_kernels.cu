@@ -17,6 +17,7 @@
 //    multiples of the SM count (chosen by the autotuner).
 //  * No shared memory, no tensor cores: there is no reuse to stage and no
 //    contraction to run.
+#include "bsg_fx64.h"
 #include "bsg_internal.h"
 #include "bsg_math.cuh"
 
@@ -588,8 +589,8 @@ static cudaError_t launch_map_mode(const SoA& a_in, int64_t n, const MapCfg& cfg
     const int block = cfg.block;
     // 256-bit loads for load paths 2 and up where a common boundary is that
     // far, else 128-bit; a slice of a book (all seven pointers equally far
-    // from one) starts with up to 7 single options.  1,250,001 options from
-    // option 3 of a book: 10M x 100 passes 3.48 ms, 5.25 with the scalar kernel;
+    // from one) starts with up to 7 single options.  From
+    // option 3 of a book 10M x 100 passes take 3.48 ms, 5.25 with the scalar kernel;
     // 45M once 194 us, 237.
     int head = peel(&a, &n, cfg.load_path >= 2 ? 32 : 16);
     if (head < 0 && cfg.load_path >= 2 && (head = peel(&a, &n, 16)) >= 0) {
@@ -774,38 +775,94 @@ MapCfg map_default_cfg(const SoA& a, int64_t n, int runs) {
 }
 
 // ------------------------------------------------------------------ FP64
-__global__ void __launch_bounds__(256) fp64_kernel(SoA a, double* out, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = price_fp64(a.s[i], a.k[i], a.r[i], a.v[i], a.t[i], a.ot[i]);
+// Double prices: double storage in and out (the SIMD variant's NCO = 2
+// types, 52 bytes per option), or float storage in (the validation oracle).
+// In double arithmetic the kernel is bound by GB300's FP64 rate (177
+// operations an option, that pipe 85 % busy: 4M options in 1.38 ms against
+// 32 us of HBM traffic), so the elementary functions are fixed point
+// (bsg_fx64.h).  The few options that are left to the double evaluation go
+// into a queue in shared memory, which the block prices together at the end:
+// in place, one such option would hold its warp for a whole double
+// evaluation.  4M options: 175 us, bound by integer issue.
+constexpr int kF64Threads = 256;
+constexpr int kF64Queue = 1024;
+
+__device__ const bsg_sw::Tables kFxTables = BSG_SW_TABLES;
+
+__device__ __noinline__ double price_fp64_call(double s, double k, double r, double v, double t, int ot) {
+    return price_fp64(s, k, r, v, t, ot);
 }
 
-// FP64 product mode: double storage in and out (the SIMD variant's NCO = 2
-// types), 52 bytes per option; bound by GB300's FP64 rate, not by HBM.
-__global__ void __launch_bounds__(256) map_f64_kernel(SoA64 a, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        a.out[i] = price_fp64(__ldg(a.s + i), __ldg(a.k + i), __ldg(a.r + i), __ldg(a.v + i),
-                              __ldg(a.t + i), __ldg(a.ot + i));
+__device__ __forceinline__ uint64_t dbits(double d) { return (uint64_t)__double_as_longlong(d); }
+
+template <typename T>
+struct F64View {
+    const T* s;
+    const T* k;
+    const T* r;
+    const T* v;
+    const T* t;
+    const int32_t* ot;
+    double* out;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kF64Threads, 3) map_f64_kernel(F64View<T> a, int64_t n) {
+    __shared__ bsg_sw::Tables tab;
+    __shared__ uint32_t queue[kF64Queue];
+    __shared__ int queued;
+    {
+        const double2* src = reinterpret_cast<const double2*>(&kFxTables);
+        double2* dst = reinterpret_cast<double2*>(&tab);
+        for (int i = threadIdx.x; i < (int)(sizeof(tab) / sizeof(double2)); i += kF64Threads) dst[i] = src[i];
+        if (threadIdx.x == 0) queued = 0;
+    }
+    __syncthreads();
+    const int64_t base = (int64_t)blockIdx.x * kF64Threads, stride = (int64_t)gridDim.x * kF64Threads;
+    uint32_t at = threadIdx.x;  // the option's place among the block's: 256 per pass of the grid
+    for (int64_t i = base + threadIdx.x; i < n; i += stride, at += kF64Threads) {
+        const double s = __ldg(a.s + i), k = __ldg(a.k + i), r = __ldg(a.r + i), v = __ldg(a.v + i),
+                     t = __ldg(a.t + i);
+        const int ot = __ldg(a.ot + i);
+        double p;
+        bool done = bsg_fx::fx64_domain(dbits(s), dbits(k), dbits(r), dbits(v), dbits(t));
+        if (done) done = bsg_fx::price_fx64(tab, dbits(s), dbits(k), dbits(r), dbits(v), dbits(t), ot, &p);
+        if (!done) {
+            const int q = atomicAdd(&queued, 1);
+            if (q < kF64Queue) {
+                queue[q] = at;
+                continue;
+            }
+            p = price_fp64_call(s, k, r, v, t, ot);
+        }
+        a.out[i] = p;
+    }
+    __syncthreads();
+    const int m = queued < kF64Queue ? queued : kF64Queue;
+    for (int q = threadIdx.x; q < m; q += kF64Threads) {
+        const int64_t i = base + (int64_t)(queue[q] / kF64Threads) * stride + queue[q] % kF64Threads;
+        a.out[i] = price_fp64_call(__ldg(a.s + i), __ldg(a.k + i), __ldg(a.r + i), __ldg(a.v + i),
+                                   __ldg(a.t + i), __ldg(a.ot + i));
+    }
+}
+
+template <typename T>
+static cudaError_t launch_f64_view(const F64View<T>& a, int64_t n, int sm_count, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    int64_t grid = (n + kF64Threads - 1) / kF64Threads;
+    const int64_t cap = (int64_t)sm_count * 3;
+    if (grid > cap) grid = cap;
+    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, 0, st>>>(a, n);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    int64_t grid = (n + 255) / 256;
-    const int64_t cap = (int64_t)sm_count * 8;
-    if (grid > cap) grid = cap;
-    map_f64_kernel<<<(unsigned)grid, 256, 0, st>>>(a, n);
-    return cudaGetLastError();
+    return launch_f64_view(F64View<double>{a.s, a.k, a.r, a.v, a.t, a.ot, a.out}, n, sm_count, st);
 }
 
 cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count,
                         cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    int64_t grid = (n + 255) / 256;
-    const int64_t cap = (int64_t)sm_count * 8;
-    if (grid > cap) grid = cap;
-    fp64_kernel<<<(unsigned)grid, 256, 0, st>>>(a, out, n);
-    return cudaGetLastError();
+    return launch_f64_view(F64View<float>{a.s, a.k, a.r, a.v, a.t, a.ot, out}, n, sm_count, st);
 }
 
 // ------------------------------------------------------------ batched books
