@@ -198,12 +198,17 @@ SIGNATURES = {
                                                                        ctypes.c_long, _I, _I]),
 }
 
+# The functions csrc/bsg_pycall.cpp calls, in bind()'s order.
+_PYCALL = ("bsg_price_soa", "bsg_price_soa_f64", "bsg_price_batch", "bsg_price_books_plain",
+           "bsg_server_submit", "bsg_server_wait", "bsg_price_swaptions")
+
 _lib = None
+_call = None  # p3arsec_gb300._pycall, bound to _lib
 
 
 def load(path: str = LIB_PATH) -> ctypes.CDLL:
     """Load libbsgpu.so (once).  Raises if it has not been built."""
-    global _lib
+    global _lib, _call
     if _lib is not None:
         return _lib
     if not os.path.exists(path):
@@ -215,6 +220,9 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
+    from . import _pycall
+    _pycall.bind(*[ctypes.cast(getattr(lib, name), _P).value for name in _PYCALL])
+    _call = _pycall
     _lib = lib
     return lib
 
@@ -267,6 +275,7 @@ class Context:
         if st != 0:
             raise BsgError(st, self.lib.bsg_strerror(st).decode())
         self.h = h
+        self._addr = h.value
         self.device = device
         self.max_options = max_options
         _live.add(self)
@@ -274,7 +283,7 @@ class Context:
     def close(self):
         if getattr(self, "h", None):
             self.lib.bsg_destroy(self.h)
-            self.h = None
+            self.h = self._addr = None
 
     def __enter__(self):
         return self
@@ -313,15 +322,10 @@ class Context:
             flags |= ASYNC
         if not graph:
             flags |= NO_GRAPH
-        if not device:
-            for a, dt in ((s, np.float32), (k, np.float32), (r, np.float32), (v, np.float32),
-                          (t, np.float32), (otype, np.int32), (prices, np.float32)):
-                if not (isinstance(a, np.ndarray) and a.dtype == dt and a.flags.c_contiguous
-                        and a.shape[0] >= n):
-                    raise TypeError("host arrays must be C-contiguous float32 (otype int32) of length >= n")
-        st = self.lib.bsg_price_soa(self.h, ptr(s), ptr(k), ptr(r), ptr(v), ptr(t), ptr(otype),
-                                    ptr(prices), n, num_runs, flags)
-        _check(self.lib, self.h, st)
+        # host arrays: C-contiguous float32 (otype int32) of length >= n, else TypeError
+        st = _call.price_soa(self._addr, s, k, r, v, t, otype, prices, n, num_runs, flags, False)
+        if st:
+            _check(self.lib, self.h, st)
         return prices
 
     def price_book(self, book, num_runs=1, mode="fast"):
@@ -345,26 +349,19 @@ class Context:
         if n is None:
             n = len(s)
         flags = (DEVICE_PTRS if device else HOST_PTRS) | (ASYNC if asynchronous else 0)
-        st = self.lib.bsg_price_soa_f64(self.h, ptr(s), ptr(k), ptr(r), ptr(v), ptr(t),
-                                        ptr(otype), ptr(prices), n, num_runs, flags)
+        st = _call.price_soa(self._addr, s, k, r, v, t, otype, prices, n, num_runs, flags, True)
         _check(self.lib, self.h, st)
         return prices
 
     def price_batch(self, pool, prices, pool_len, segments, num_runs=1, mode="fast",
                     plain=False, asynchronous=False, graph=True):
         """Batched books over a device pool (pool = 6 device pointers)."""
-        segs = (Segment * max(len(segments), 1))()
-        for i, (o, l) in enumerate(segments):
-            segs[i].offset = int(o)
-            segs[i].len = int(l)
         flags = MODES[mode] | DEVICE_PTRS
         if asynchronous:
             flags |= ASYNC
         if not graph:
             flags |= NO_GRAPH
-        fn = self.lib.bsg_price_books_plain if plain else self.lib.bsg_price_batch
-        st = fn(self.h, *[ptr(x) for x in pool], ptr(prices), pool_len, segs, len(segments),
-                num_runs, flags)
+        st = _call.price_batch(self._addr, pool, prices, pool_len, segments, num_runs, flags, bool(plain))
         _check(self.lib, self.h, st)
 
     def autotune_batch(self, pool, prices, pool_len, segments) -> dict:
@@ -432,11 +429,10 @@ class Context:
     def price_swaptions(self, swaptions, trials: int):
         """bsg_price_swaptions over p3arsec_gb300.swaptions.Swaption objects;
         returns (prices, standard errors) as float64 arrays."""
-        arr, keep = swaption_structs(swaptions)
         n = len(swaptions)
         price = np.empty(n)
         err = np.empty(n)
-        st = self.lib.bsg_price_swaptions(self.h, arr, n, trials, ptr(price), ptr(err))
+        st = _call.price_swaptions(self._addr, swaptions, trials, price, err)
         _check(self.lib, self.h, st)
         return price, err
 
@@ -473,12 +469,13 @@ class Server:
         if st != 0:
             raise BsgError(st, self.lib.bsg_strerror(st).decode())
         self.h = h
+        self._addr = h.value
         _live.add(self)
 
     def close(self):
         if getattr(self, "h", None):
             self.lib.bsg_server_destroy(self.h)
-            self.h = None
+            self.h = self._addr = None
 
     def __enter__(self):
         return self
@@ -495,18 +492,14 @@ class Server:
     def submit(self, s, k, r, v, t, otype, prices, n=None) -> int:
         if n is None:
             n = len(s)
-        req = Request(ptr(s), ptr(k), ptr(r), ptr(v), ptr(t), ptr(otype), ptr(prices), n)
-        rid = ctypes.c_uint64()
-        st = self.lib.bsg_server_submit(self.h, ctypes.byref(req), ctypes.byref(rid))
+        st, rid = _call.server_submit(self._addr, s, k, r, v, t, otype, prices, n)
         if st != 0:
             raise BsgError(st, self.lib.bsg_strerror(st).decode())
-        return int(rid.value)
+        return rid
 
     def wait(self, rid: int, timeout_s: float = -1.0):
         """Returns (status, latency_s); status BSG_ERR_TIMEOUT leaves it pending."""
-        lat = ctypes.c_double(float("nan"))
-        st = self.lib.bsg_server_wait(self.h, rid, timeout_s, ctypes.byref(lat))
-        return st, lat.value
+        return _call.server_wait(self._addr, rid, timeout_s)
 
     def cancel(self, rid: int) -> int:
         return self.lib.bsg_server_cancel(self.h, rid)

@@ -1,5 +1,5 @@
-"""In-tree build of libbsgpu.so (sm_103a) and the drop-in blackscholes and
-swaptions CLIs.
+"""In-tree build of libbsgpu.so (sm_103a), the Python binding's native half and
+the drop-in blackscholes and swaptions CLIs.
 
 Compiles each translation unit with nvcc in parallel, links the shared
 library next to this file and the CLIs into ``p3arsec_gb300/bin/``.  No
@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -20,6 +21,7 @@ HOST = os.path.join(PKG, "host")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libbsgpu.so")
 CLI = os.path.join(PKG, "bin", "blackscholes_gpu")
+PYCALL = os.path.join(PKG, "_pycall.so")  # the Python binding's native half
 SWAPTIONS_CLI = os.path.join(PKG, "bin", "swaptions_gpu")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -96,11 +98,18 @@ def _build_locked(verbose: bool, force: bool) -> str:
         objs.append(o)
         if force or _stale(o, [s] + heads):
             jobs.append(["g++"] + CXX_FLAGS + ["-c", s, "-o", o])
+    pycall_src = os.path.join(CSRC, "bsg_pycall.cpp")
+    pycall = force or _stale(PYCALL, [pycall_src] + heads)
+    if pycall:
+        jobs.append(["g++"] + CXX_FLAGS + ["-I" + sysconfig.get_paths()["include"], "-shared",
+                                           pycall_src, "-o", PYCALL + ".tmp"])
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=len(jobs)) as ex:
             for out in ex.map(_run, jobs):
                 if verbose and out.strip():
                     print(out)
+    if pycall:
+        os.replace(PYCALL + ".tmp", PYCALL)
     if force or jobs or _stale(LIB, objs):
         tmp = LIB + ".tmp"
         _run([nv] + ARCH + ["-shared", "-o", tmp] + objs + ["-lpthread"])

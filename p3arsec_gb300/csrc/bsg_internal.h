@@ -100,7 +100,8 @@ cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count,
 // One pass of the FP64 product mode over n options.
 cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st);
 
-// Persistent batched pricing.  seg_off/seg_len/tile_prefix are device arrays
+// Persistent batched pricing.  seg_off/seg_len/tile_prefix (not read where
+// tile_bounds is given) are device arrays
 // of nseg (tile_prefix: nseg + 1 entries, exclusive prefix of tiles of
 // tile_opts options per segment); tile_bounds (optional, NULL = search the
 // prefix instead) holds each tile's [begin, end) in the pool, 2 * ntiles
