@@ -69,6 +69,21 @@ int mode_of(unsigned flags) {
 
 size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Host calls of up to this many options go through the context's pinned
+// staging: the host copies the six arrays there, the kernel reads them over the
+// host link and writes the prices back there.  A call of 16 options: 14 us
+// against 31 with six copies in, a launch and a copy out; 4,096: 18 against 39;
+// at 65,536 the host's copy (1.6 MB at 20 GB/s) would cost more than the six
+// pageable ones (83 us in all).
+constexpr size_t kStageOptions = 32768;
+constexpr size_t kStageBytes = 7 * kStageOptions * sizeof(float);
+// Host arrays in pinned memory are read in place (one pass: 65,536 options 22
+// us against 54, 10M 1.17 ms against 1.43), or gathered into the resident
+// arrays by one kernel (several passes: 65,536 x 2 32 us against 51, 1M x 2
+// 167 against 189) up to this many options; beyond, six copies reach the same
+// rate (3M x 2: 460 against 472).
+constexpr size_t kGatherOptions = (size_t)1 << 21;
+
 constexpr size_t kGuardWords = 64;        // guard words after each resident array
 constexpr int kGuardByte = 0xA5;          // guard fill byte
 constexpr uint32_t kGuardWord = 0xA5A5A5A5u;
@@ -102,7 +117,9 @@ struct bsg_ctx {
     uint64_t* h_tb = nullptr;
     size_t tb_cap = 0;  // tiles
     cudaEvent_t seg_ev = nullptr;
-    unsigned long long* d_cursor = nullptr;  // one work counter per pass
+    char* d_small = nullptr;                     // small scratch of every context
+    unsigned long long* d_cursor = nullptr;      // one work counter per pass (in d_small
+    unsigned long long* d_cursor_own = nullptr;  // while 128 are enough, else here)
     size_t cursor_cap = 0;
     // error-report scratch
     bsg::ErrAcc* d_acc = nullptr;
@@ -116,13 +133,16 @@ struct bsg_ctx {
     cudaEvent_t ev_out[2] = {nullptr, nullptr};
     int next_set = 0;
     bool pipelined = false;  // pipelined work may be in flight
+    // pinned memory for the arrays of short host calls (kStageOptions); used
+    // only inside a synchronous call
+    char* h_stage = nullptr;
     // debug guards (BSG_DEBUG set at bsg_create): every resident array is
     // followed by at least kGuardWords words of kGuardByte, checked after
     // each synchronous call; d_guard holds the check's {count, first index}
     bool debug = false;
     unsigned long long* d_guard = nullptr;
     // swaption scratch: counters, parameter table, partial sums on the device;
-    // results and the table's staging in pinned memory
+    // results and the table's staging in pinned memory (h_sw where h_stage is too small)
     char* d_sw = nullptr;
     size_t sw_cap = 0;
     char* h_sw = nullptr;
@@ -475,6 +495,64 @@ int ensure_pipeline(bsg_ctx* c) {
     return BSG_OK;
 }
 
+// The device's addresses of a host book whose seven arrays each lie inside
+// one pinned allocation or registration, and whose prices overlap no input;
+// false otherwise.
+bool pinned_view(const bsg::SoA& h, size_t n, bsg::SoA* d) {
+    static PointerGetAttributeFn get_attr =
+        driver_entry<PointerGetAttributeFn>("cuPointerGetAttribute");
+    if (!get_attr) return false;
+    const void* p[7] = {h.s, h.k, h.r, h.v, h.t, h.ot, h.out};
+    void* q[7];
+    const size_t b = n * 4;
+    for (int i = 0; i < 7; ++i) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(p[i]);
+        if (x & 3) return false;
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p[i]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeHost || !a.devicePointer) return false;
+        CUdeviceptr start = 0;
+        size_t size = 0;
+        if (get_attr(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)x) != CUDA_SUCCESS ||
+            get_attr(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)x) != CUDA_SUCCESS ||
+            x < (uintptr_t)start || b > size || x - (uintptr_t)start > size - b)
+            return false;
+        q[i] = a.devicePointer;
+        if (i < 6) {
+            const uintptr_t o = reinterpret_cast<uintptr_t>(h.out);
+            if (x < o + b && o < x + b) return false;
+        }
+    }
+    *d = bsg::SoA{(const float*)q[0], (const float*)q[1], (const float*)q[2], (const float*)q[3],
+                  (const float*)q[4], (const int32_t*)q[5], (float*)q[6]};
+    return true;
+}
+
+// A synchronous host call over memory that the GPU reads and writes in place
+// (`src`: device addresses of pinned arrays).
+int price_in_place(bsg_ctx* c, const bsg::SoA& src, size_t n, int runs, int mode, unsigned flags) {
+    int st;
+    if (runs == 1) {
+        // the tuned shapes are for device memory: plain 256-bit loads here
+        cudaError_t e = bsg::launch_map(src, (int64_t)n, mode, bsg::MapCfg{1, 128, 0, 2, 0}, c->sm_count,
+                                        c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "launch_map (host memory)");
+        c->launches++;
+    } else {
+        const bsg::SoA d = c->resident(n);
+        cudaError_t e = bsg::launch_gather(src, d, (int64_t)n, c->sm_count, c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "launch_gather");
+        c->launches++;
+        if ((st = enqueue_map_runs(c, d, (int64_t)n, runs, mode, flags))) return st;
+        BSG_CK(c, cudaMemcpyAsync(src.out, d.out, n * 4, cudaMemcpyDeviceToHost, c->stream));
+    }
+    BSG_CK(c, cudaStreamSynchronize(c->stream));
+    return check_bulk_error(c);
+}
+
 // A pipelined host call: inputs copied into the next of two resident sets on
 // the copy-in stream, the passes on the compute stream, prices copied out on
 // the copy-out stream; events order each set's reuse.  Successive calls
@@ -607,15 +685,20 @@ int bsg_create(bsg_ctx** out, int device, size_t max_options) {
         return BSG_ERR_NO_DEVICE;
     }
     if (device < 0 || device >= ndev) return BSG_ERR_NO_DEVICE;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return BSG_ERR_NO_DEVICE;
-    if (!(prop.major == 10 && prop.minor == 3)) return BSG_ERR_NO_DEVICE;  // sm_103a cubin only
+    int major = 0, minor = 0, sms = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return BSG_ERR_NO_DEVICE;
+    }
+    if (!(major == 10 && minor == 3)) return BSG_ERR_NO_DEVICE;  // sm_103a cubin only
     if (max_options > ((size_t)1 << 36)) return BSG_ERR_INVALID_ARG;
 
     bsg_ctx* c = new (std::nothrow) bsg_ctx();
     if (!c) return BSG_ERR_OUT_OF_MEMORY;
     c->device = device;
-    c->sm_count = prop.multiProcessorCount;
+    c->sm_count = sms;
     int rc = BSG_OK;
     do {
         if (cudaSetDevice(device) != cudaSuccess) { rc = BSG_ERR_NO_DEVICE; break; }
@@ -630,10 +713,14 @@ int bsg_create(bsg_ctx** out, int device, size_t max_options) {
             if (cudaMalloc(&c->d_guard, 16) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
             if (cudaMemsetAsync(c->dev_buf, kGuardByte, 7 * c->cap_al * sizeof(float), c->stream) != cudaSuccess) { rc = BSG_ERR_CUDA; break; }
         }
+        if (cudaMallocHost(&c->h_stage, kStageBytes) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
+        // the small device scratch in one allocation: work counters, error accumulators, edges
         c->cursor_cap = 128;
-        if (cudaMalloc(&c->d_cursor, c->cursor_cap * 8) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
-        if (cudaMalloc(&c->d_acc, sizeof(bsg::ErrAcc) * bsg::kMaxErrBuckets) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
-        if (cudaMalloc(&c->d_edges, sizeof(double) * (bsg::kMaxErrBuckets + 1)) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
+        const size_t cur_b = c->cursor_cap * 8, acc_b = sizeof(bsg::ErrAcc) * bsg::kMaxErrBuckets;
+        if (cudaMalloc(&c->d_small, cur_b + acc_b + sizeof(double) * (bsg::kMaxErrBuckets + 1)) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
+        c->d_cursor = reinterpret_cast<unsigned long long*>(c->d_small);
+        c->d_acc = reinterpret_cast<bsg::ErrAcc*>(c->d_small + cur_b);
+        c->d_edges = reinterpret_cast<double*>(c->d_small + cur_b + acc_b);
         const int bps = bsg::batch_blocks_per_sm();
         if (bps > 0) c->batch_blocks_per_sm = bps;
     } while (0);
@@ -664,12 +751,12 @@ void bsg_destroy(bsg_ctx* c) {
     if (c->dev_buf) cudaFree(c->dev_buf);
     if (c->d_tb) cudaFree(c->d_tb);
     if (c->h_tb) cudaFreeHost(c->h_tb);
-    if (c->d_cursor) cudaFree(c->d_cursor);
-    if (c->d_acc) cudaFree(c->d_acc);
-    if (c->d_edges) cudaFree(c->d_edges);
+    if (c->d_cursor_own) cudaFree(c->d_cursor_own);
+    if (c->d_small) cudaFree(c->d_small);
     if (c->d_guard) cudaFree(c->d_guard);
     if (c->d_sw) cudaFree(c->d_sw);
     if (c->h_sw) cudaFreeHost(c->h_sw);
+    if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->seg_ev) cudaEventDestroy(c->seg_ev);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -726,9 +813,23 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
         if (n > c->cap) return fail(c, BSG_ERR_CAPACITY, "n exceeds the context's max_options");
         if (flags & BSG_ASYNC) return enqueue_host_pipelined(c, a, n, num_runs, mode, flags);
         if ((st = drain_pipeline(c))) return st;
+        const size_t b = n * 4;
+        if (!c->debug && n <= kStageOptions) {
+            float* f = reinterpret_cast<float*>(c->h_stage);
+            const size_t al = round_up(n, 64);
+            const void* in[6] = {s, k, r, v, t, otype};
+            for (int i = 0; i < 6; ++i) std::memcpy(f + i * al, in[i], b);
+            const bsg::SoA h{f, f + al, f + 2 * al, f + 3 * al, f + 4 * al,
+                             reinterpret_cast<const int32_t*>(f + 5 * al), f + 6 * al};
+            if ((st = price_in_place(c, h, n, num_runs, mode, flags))) return st;
+            std::memcpy(prices, h.out, b);
+            return BSG_OK;
+        }
+        bsg::SoA view;
+        if (!c->debug && (num_runs == 1 || n <= kGatherOptions) && pinned_view(a, n, &view))
+            return price_in_place(c, view, n, num_runs, mode, flags);
         if ((st = debug_arm(c, n))) return st;
         const bsg::SoA d = c->resident(n);
-        const size_t b = n * 4;
         BSG_CK(c, cudaMemcpyAsync((void*)d.s, s, b, cudaMemcpyHostToDevice, c->stream));
         BSG_CK(c, cudaMemcpyAsync((void*)d.k, k, b, cudaMemcpyHostToDevice, c->stream));
         BSG_CK(c, cudaMemcpyAsync((void*)d.r, r, b, cudaMemcpyHostToDevice, c->stream));
@@ -896,10 +997,12 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
         if ((size_t)num_runs > c->cursor_cap) {
             BSG_CK(c, cudaStreamSynchronize(c->stream));
             graph_drop_all(c);
-            cudaFree(c->d_cursor);
+            if (c->d_cursor_own) cudaFree(c->d_cursor_own);
+            c->d_cursor_own = nullptr;
             c->d_cursor = nullptr;
             c->cursor_cap = 0;
-            BSG_CK(c, cudaMalloc(&c->d_cursor, (size_t)num_runs * 8));
+            BSG_CK(c, cudaMalloc(&c->d_cursor_own, (size_t)num_runs * 8));
+            c->d_cursor = c->d_cursor_own;
             c->cursor_cap = (size_t)num_runs;
         }
         auto all_runs = [&]() -> cudaError_t {
@@ -1350,7 +1453,9 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
             BSG_CK(c, cudaMemsetAsync(c->d_sw, 0, done_b, c->stream));
             c->sw_cap = need;
         }
-        if (out_b + tab_b > c->h_sw_cap) {
+        // pinned: the staging (no other call's work uses it now), or their own
+        char* pin = c->h_stage;
+        if (out_b + tab_b > kStageBytes && out_b + tab_b > c->h_sw_cap) {
             BSG_CK(c, cudaStreamSynchronize(c->stream));
             if (c->h_sw) cudaFreeHost(c->h_sw);
             c->h_sw = nullptr;
@@ -1361,13 +1466,14 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
             }
             c->h_sw_cap = out_b + tab_b;
         }
-        double* out = reinterpret_cast<double*>(c->h_sw);  // the kernel writes the results here itself
+        if (out_b + tab_b > kStageBytes) pin = c->h_sw;
+        double* out = reinterpret_cast<double*>(pin);  // the kernel writes the results here itself
         bsg::SwInline in;
         uint64_t* d_tab = nullptr;
         uint64_t* tab = in.words;
         if (!inl) {
             d_tab = reinterpret_cast<uint64_t*>(c->d_sw + done_b);
-            tab = reinterpret_cast<uint64_t*>(c->h_sw + out_b);
+            tab = reinterpret_cast<uint64_t*>(pin + out_b);
         }
         std::memcpy(tab, heads.data(), n * sizeof(bsg::SwHead));
         if (!words.empty()) std::memcpy(tab + n * head_words, words.data(), words.size() * 8);

@@ -84,6 +84,9 @@ MapCfg map_default_cfg(const SoA& a, int64_t n, int runs);
 // Whether launch_map_runs takes `runs` passes of this book (in one launch).
 bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count);
 cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st);
+// Copies n options' six input arrays from src (pinned host memory, its device
+// addresses) into dst's, by one kernel.
+cudaError_t launch_gather(const SoA& src, const SoA& dst, int64_t n, int sm_count, cudaStream_t st);
 // Reads and clears the bulk-staged kernel's error word (non-zero: a bounded
 // wait expired and some tiles were not priced).
 unsigned bulk_error_take();

@@ -305,6 +305,38 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
     }
 }
 
+// Host arrays into device arrays: blockIdx.y picks the array, so that the link
+// carries all six at once; 16-byte words where the source allows (dst is
+// aligned), four in flight per thread.
+__global__ void __launch_bounds__(256) gather_kernel(SoA src, SoA dst, int64_t n) {
+    const void* ps[6] = {src.s, src.k, src.r, src.v, src.t, src.ot};
+    const void* pd[6] = {dst.s, dst.k, dst.r, dst.v, dst.t, dst.ot};
+    const uint32_t* s = static_cast<const uint32_t*>(ps[blockIdx.y]);
+    uint32_t* d = const_cast<uint32_t*>(static_cast<const uint32_t*>(pd[blockIdx.y]));
+    const int64_t n4 = (reinterpret_cast<uintptr_t>(s) & 15) == 0 ? n / 4 : 0;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int64_t i = i0;
+    for (; i + 3 * stride < n4; i += 4 * stride) {
+        uint4 x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = __ldg(reinterpret_cast<const uint4*>(s) + i + j * stride);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(d)[i + j * stride] = x[j];
+    }
+    for (; i < n4; i += stride) reinterpret_cast<uint4*>(d)[i] = __ldg(reinterpret_cast<const uint4*>(s) + i);
+    for (int64_t k = 4 * n4 + i0; k < n; k += stride) d[k] = __ldg(s + k);
+}
+
+cudaError_t launch_gather(const SoA& src, const SoA& dst, int64_t n, int sm_count, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    int64_t gx = (n / 4 + 255) / 256;
+    if (gx > sm_count) gx = sm_count;
+    if (gx < 1) gx = 1;
+    gather_kernel<<<dim3((unsigned)gx, 6), 256, 0, st>>>(src, dst, n);
+    return cudaGetLastError();
+}
+
 // Scalar kernel: any 4-byte aligned pointers.
 template <int M>
 __global__ void __launch_bounds__(256) map_scalar_kernel(SoA a, int64_t n) {
