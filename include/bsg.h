@@ -56,7 +56,8 @@ typedef enum bsg_status {
 } bsg_status;
 
 /* ---- flags ------------------------------------------------------------ */
-#define BSG_HOST_PTRS     0x000u /* host arrays: copied in and out inside the call */
+#define BSG_HOST_PTRS     0x000u /* host arrays: copied in and out inside the call, or read
+                                    and written in place by the GPU where it can */
 #define BSG_DEVICE_PTRS   0x001u /* device arrays on the context's device */
 #define BSG_ASYNC         0x002u /* return once enqueued (see bsg_price_soa) */
 #define BSG_MODE_FAST     0x000u /* compensated FP32 with SFU approximations */

@@ -29,6 +29,9 @@
 #include <string>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 namespace {
 
 constexpr size_t kGraphCacheSize = 8;
@@ -72,13 +75,14 @@ size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // Host calls of up to this many options go through the context's pinned
 // staging: the host copies the six arrays there, the kernel reads them over the
 // host link and writes the prices back there.  A call of 16 options: 14 us
-// against 31 with six copies in, a launch and a copy out; 4,096: 18 against 39;
-// at 65,536 the host's copy (1.6 MB at 20 GB/s) would cost more than the six
-// pageable ones (83 us in all).
-constexpr size_t kStageOptions = 32768;
+// against 31 with six copies in, a launch and a copy out; 8,192: 22 against 50;
+// 32,768 would take 51 (0.8 MB at the host's 20 GB/s), 22 in place.
+constexpr size_t kStageOptions = 8192;
 constexpr size_t kStageBytes = 7 * kStageOptions * sizeof(float);
-// Host arrays in pinned memory are read in place (one pass: 65,536 options 22
-// us against 54, 10M 1.17 ms against 1.43), or gathered into the resident
+// Host arrays in pinned memory, or in pageable memory whose page tables the
+// GPU walks, are read in place (one pass: 65,536 pinned options 22 us against
+// 54, 10M 1.17 ms against 1.43; pageable 23 us against 92, 1M 150 against 239,
+// 10M 1.31 ms against 1.72), or gathered into the resident
 // arrays by one kernel (several passes: 65,536 x 2 32 us against 51, 1M x 2
 // 167 against 189) up to this many options; beyond, six copies reach the same
 // rate (3M x 2: 460 against 472).
@@ -133,6 +137,7 @@ struct bsg_ctx {
     cudaEvent_t ev_out[2] = {nullptr, nullptr};
     int next_set = 0;
     bool pipelined = false;  // pipelined work may be in flight
+    bool host_tables = false;  // the GPU reads pageable memory through the process's page tables
     // pinned memory for the arrays of short host calls (kStageOptions); used
     // only inside a synchronous call
     char* h_stage = nullptr;
@@ -531,8 +536,39 @@ bool pinned_view(const bsg::SoA& h, size_t n, bsg::SoA* d) {
     return true;
 }
 
+// Whether the GPU may read a pageable host book's inputs, and write its prices
+// when `write`, in place: it walks the process's own page tables
+// (bsg_ctx::host_tables), and the kernel has just made every page of the
+// arrays present with the access needed.  A range that is not mapped, not
+// readable or writable, or no ordinary memory (device files) fails there, and
+// the call copies.
+bool populated(const void* p, size_t bytes, bool write) {
+#ifndef MADV_POPULATE_READ
+    constexpr int MADV_POPULATE_READ = 22, MADV_POPULATE_WRITE = 23;
+#endif
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t b = reinterpret_cast<uintptr_t>(p), b0 = b & ~(page - 1);
+    return madvise(reinterpret_cast<void*>(b0), b + bytes - b0,
+                   write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) == 0;
+}
+
+bool pageable_view(const bsg_ctx* c, const bsg::SoA& h, size_t n, bool write) {
+    if (!c->host_tables) return false;
+    const void* p[6] = {h.s, h.k, h.r, h.v, h.t, h.ot};
+    const uintptr_t o = reinterpret_cast<uintptr_t>(h.out);
+    const size_t b = n * 4;
+    if (o & 3) return false;
+    for (const void* q : p) {
+        const uintptr_t x = reinterpret_cast<uintptr_t>(q);
+        if ((x & 3) || (x < o + b && o < x + b)) return false;
+    }
+    for (const void* q : p)
+        if (!populated(q, b, false)) return false;
+    return !write || populated(h.out, b, true);
+}
+
 // A synchronous host call over memory that the GPU reads and writes in place
-// (`src`: device addresses of pinned arrays).
+// (`src`: the device's addresses of the arrays).
 int price_in_place(bsg_ctx* c, const bsg::SoA& src, size_t n, int runs, int mode, unsigned flags) {
     int st;
     if (runs == 1) {
@@ -704,6 +740,9 @@ int bsg_create(bsg_ctx** out, int device, size_t max_options) {
         if (cudaSetDevice(device) != cudaSuccess) { rc = BSG_ERR_NO_DEVICE; break; }
         if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { rc = BSG_ERR_CUDA; break; }
         if (cudaEventCreateWithFlags(&c->seg_ev, cudaEventDisableTiming) != cudaSuccess) { rc = BSG_ERR_CUDA; break; }
+        int ats = 0;
+        c->host_tables = cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables,
+                                                device) == cudaSuccess && ats != 0;
         c->cap = max_options;
         c->debug = debug_env();
         // 256-byte aligned arrays, each followed by guard words in debug mode
@@ -826,8 +865,11 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
             return BSG_OK;
         }
         bsg::SoA view;
-        if (!c->debug && (num_runs == 1 || n <= kGatherOptions) && pinned_view(a, n, &view))
-            return price_in_place(c, view, n, num_runs, mode, flags);
+        if (!c->debug && (num_runs == 1 || n <= kGatherOptions)) {
+            if (pinned_view(a, n, &view)) return price_in_place(c, view, n, num_runs, mode, flags);
+            if (pageable_view(c, a, n, num_runs == 1))
+                return price_in_place(c, a, n, num_runs, mode, flags);
+        }
         if ((st = debug_arm(c, n))) return st;
         const bsg::SoA d = c->resident(n);
         BSG_CK(c, cudaMemcpyAsync((void*)d.s, s, b, cudaMemcpyHostToDevice, c->stream));

@@ -11,7 +11,7 @@ from p3arsec_gb300 import Context, books
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-STAGE, GATHER = 32768, 1 << 21  # kStageOptions, kGatherOptions
+STAGE, GATHER = 8192, 1 << 21  # kStageOptions, kGatherOptions
 N_MAX = GATHER + 9
 
 
@@ -66,6 +66,21 @@ def test_pinned_prices_over_an_input(ctx, book, n):
     want = _want(ctx, book, 0, n, "fast")
     ctx.price_soa(*arrays, keep[0].numpy()[1:], n=n)
     assert np.array_equal(keep[0].numpy()[1:].view(np.uint32), want.view(np.uint32))
+
+
+def test_read_only_file_mappings(ctx, book, tmp_path):
+    """Inputs mapped read-only from files, prices in a fresh allocation whose
+    pages nobody has touched."""
+    n = 150_001
+    arrays = []
+    for i, a in enumerate(book.arrays()):
+        a[:n].tofile(tmp_path / f"{i}.bin")
+        arrays.append(np.memmap(tmp_path / f"{i}.bin", dtype=a.dtype, mode="r"))
+    want = _want(ctx, book, 0, n, "fast")
+    for runs in (1, 2):
+        out = np.empty(n, np.float32)
+        ctx.price_soa(*arrays, out, num_runs=runs)
+        assert np.array_equal(out.view(np.uint32), want.view(np.uint32))
 
 
 def test_wrong_host_arrays_are_refused(ctx, book):
