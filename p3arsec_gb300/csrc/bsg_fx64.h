@@ -4,20 +4,22 @@
 //
 // Why: GB300 issues 2 double-precision operations per clock and SM; the
 // formula takes 177 of them (four divisions, a square root, a log, three
-// exps and two polynomials).  Here sqrt, log, exp, the division and the
-// polynomial are integer work on the multiply-add pipes (as bsg_swmath.h,
-// whose tables these share), and six double operations are left: the
+// exps and two polynomials).  Here sqrt, log, exp and the division are integer
+// work on the multiply-add pipes (as bsg_swmath.h, whose tables these share),
+// the tail of N -- exp and polynomial together -- comes from a table of its
+// Taylor coefficients (15 integer multiply-adds; 46 with exp, reciprocal and
+// polynomial evaluated: 173 us), and six double operations are left: the
 // products and the difference of the reference's last line, on N rounded to
 // 2^-53 as the reference's 1 - (1 - N(|d|)) rounds it.
 //
-// 4M options: 1368 us in doubles, 175 us here.
+// 4M options: 1368 us in doubles, 133 us here.
 //
 // Precision (against long double, over max(s, k)): root mean square 6.0e-17
 // and at most 3.2e-16 on strikes to 1.5 times the spot price, 1.1e-16 and
 // 7.2e-16 in doubles; 5.7e-17 and 3.4e-16 on strikes to 20 times, 6.2e-17 and
 // 5.4e-16 in doubles.  num = (r + v^2/2) t + ln(s/k), d1 and d2 carry 58 fraction bits
 // (the double evaluation rounds ln(s/k) near 2^-53 and N to 2^-53), the
-// tails of N 60; v sqrt(t) and 1/(v sqrt t) have 61 significant bits.
+// tails of N 60; v sqrt(t) and 1/(v sqrt t) have 55 significant bits.
 //
 // Where the double evaluation is kept: one unit of N, 2^-53, is worth 2^-53 s
 // or 2^-53 k e^(-rt), and for an option far out of the money that may be more
@@ -34,6 +36,7 @@
 // Anything else (zeros, negative or enormous times, infinities, NaN) is
 // priced by price_fp64 itself.
 #pragma once
+#include "bsg_fx64_tables.h"
 #include "bsg_swmath.h"
 
 namespace bsg_fx {
@@ -44,19 +47,10 @@ using bsg_sw::mul_64x32;
 using bsg_sw::mulhi;
 using bsg_sw::wide;
 
-#if defined(__CUDA_ARCH__)
-// A reciprocal seed of y (62 fraction bits, [1, 4)) a few units of 2^-22 low:
-// 1/y with 31 fraction bits.
-BSG_SW_FN uint32_t rcp_seed(uint64_t y) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint2float_rn(hi32(y))));
-    return __float2uint_rz(__fmul_rn(r, 2305841909702066176.0f));  // 2^61 (1 - 2^-21)
-}
-#else
-inline uint32_t rcp_seed(uint64_t y) {
-    return (uint32_t)((1.0f / (float)hi32(y)) * 2305841909702066176.0f);
-}
-#endif
+// Taylor coefficients of the upper tail on [i/64, (i + 1)/64): 64 fraction
+// bits, then 59 (gen_fx64_tables.py).
+struct alignas(16) TailEntry { uint64_t a0; int64_t a1, a2, a3; int32_t a4, a5, a6, a7; };
+struct alignas(16) TailTable { TailEntry at[BSG_FX_TAIL_ENTRIES]; };  // 26,112 bytes
 
 BSG_SW_FN int exponent_of(uint64_t b) { return (int)(b >> 52) & 2047; }
 // The significand with its top bit at bit 63 (zero for a zero or denormal).
@@ -74,62 +68,30 @@ BSG_SW_FN bool fx64_domain(uint64_t s, uint64_t k, uint64_t r, uint64_t v, uint6
            (unsigned)(2 * ev + et - 3 * 1023 + 52) <= 53u && er + et - 2 * 1023 < 1;
 }
 
-// -2 ln of x = m 2^-63 in [1, 2) (for x >= 1.5 of x/2: *half = 1), 62 fraction bits.
-BSG_SW_FN int64_t neg2_ln_significand(const bsg_sw::Tables& t, uint64_t m, int* half) {
-    const int i = (int)((m >> 54) & 511);
-    *half = i >> 8;
-    const bsg_sw::LogEntry le = t.lg[i];
-    const uint64_t lo = wide((uint32_t)m, le.c);
-    const uint64_t hi = wide(hi32(m), le.c) + (lo >> 32);
-    const int64_t r = (int64_t)((hi << 22) | ((uint32_t)lo >> 10));  // 73, as in neg2_ln_scaled
-    const int32_t rh = (int32_t)(r >> 32);
-    int32_t q = 858993459 - (bsg_sw::shi32x32(rh, 715827883) >> 9);
-    q = 1073741824 - (bsg_sw::shi32x32(rh, q) >> 9);
-    q = 1431655765 - (bsg_sw::shi32x32(rh, q) >> 9);
-    const uint64_t q63 = (1ull << 63) - (uint64_t)(((int64_t)rh * q) >> 9);
-    const uint64_t r2 = (uint64_t)((int64_t)rh * rh + 4) +
-                        (uint64_t)((int64_t)bsg_sw::shi32x32(rh, (int32_t)((uint32_t)r >> 1)) * 4);
-    return le.ln + (int64_t)(mulhi(r2, q63) >> 19) - (r >> 10);
+// a + s e: s with 64 fraction bits, e with 32 (|e| <= 1/2); up to 3 units off.
+BSG_SW_FN int64_t horner(int64_t a, int64_t s, int32_t e) {
+    return a + (int64_t)(int32_t)(s >> 32) * e + (int64_t)bsg_sw::shi32x32((int32_t)((uint32_t)s >> 1), e) * 2;
 }
 
-// 2^(-x 2^-57) as a significand in [1, 2) (63 fraction bits) and *n >= 0, the
-// power of two taken out; 0 < x 2^-57 < 63.
-BSG_SW_FN uint64_t exp2_neg(const bsg_sw::Tables& t, uint64_t x, int* n) {
-    const uint64_t f = 0ull - x;                                      // the fraction of -x
-    const uint64_t a = (f & ((1ull << 47) - 1)) << 17;                // 74
-    const uint64_t tt = mulhi(a, BSG_SW_LN2_64);
-    const uint32_t th = hi32(tt);
-    const uint64_t t2 = wide(th, th) + ((uint64_t)hi32x32(th, (uint32_t)tt) << 1);
-    const uint32_t g = 2863311531u + hi32x32(th, 699051u);
-    const uint64_t t3g = wide(hi32(t2), hi32x32(th, g));
-    const uint64_t p = tt + (t2 >> 11) + (t3g >> 22);
-    const uint64_t e = t.e2[(f >> 47) & 1023];
-    *n = -(int)((int64_t)f >> 57);
-    return e + (mulhi(e, p) >> 10);
-}
-
-// N's upper tail at x >= 0 (58 fraction bits) in units of 2^-53, rounded: the
-// polynomial of Abramowitz and Stegun 26.2.17 with 1/sqrt(2 pi) multiplied
-// into its coefficients.  Sets *near where the rounding is in doubt (above).
-BSG_SW_FN uint64_t tail_units(const bsg_sw::Tables& t, uint64_t x, bool* near) {
-    const uint64_t top = 2680624789467443200ull;         // 9.3: beyond it the tail is under 2^-66
+// N's upper tail at x >= 0 (58 fraction bits) in units of 2^-53, rounded, from
+// the table's Taylor polynomial of degree 7 (its error is under 2^-64).  Sets
+// *near where the rounding is in doubt (above).
+BSG_SW_FN uint64_t tail_units(const TailTable& t, uint64_t x, bool* near) {
+    const uint64_t top = (17ull << 57) - 1;              // 8.5: from there on 0 units
     x = x < top ? x : top;
-    // k = 1/(1 + c0 x): a seed 2^-21 low, then k0 (1 + e + e^2)
-    const uint64_t y = (1ull << 62) + mulhi(x << 2, 0x3B4CE230E2201C00ull) * 4;  // 62
-    const uint32_t k0 = rcp_seed(y);                     // 31
-    const uint64_t e = (1ull << 61) - mul_64x32(y, k0);  // 61, in (0, 2^-20)
-    const uint32_t eh = (uint32_t)(e >> 9);              // 52
-    const uint64_t c = (e << 11) + hi32x32(eh, eh);      // e + e^2, 72
-    const uint64_t k = ((uint64_t)k0 << 33) + (mul_64x32(c, k0) >> 7);  // 64
-    const uint64_t a4 = 0xBA00E2B624772872ull - mulhi(k, 0x87DC2211AA9F6974ull);
-    const uint64_t a3 = 0xB5F0E2AE93BD6878ull - mulhi(k, a4);
-    const uint64_t a1 = 0x209E418D66AFA2E4ull + mulhi(k, mulhi(k, a3)) - mulhi(k, 0x246A6399C19DCB8Eull);
-    const uint64_t p = mulhi(k, a1);                     // 64, at most 1/2
-    // exp(-x^2/2) = 2^-(x^2 log2(e)/2); x in 60 bits, x^2 in 56
-    const uint64_t xx = mulhi(x << 2, x << 2) << 1;
-    int n;
-    const uint64_t g = exp2_neg(t, mulhi(xx, 0xB8AA3B295C17F0BCull) | 1, &n);  // n >= 1
-    const uint64_t q = mulhi(g, p) >> (n - 1);           // 64
+    const TailEntry& p = t.at[(int)(x >> 52)];
+    const int32_t e = (int32_t)((uint32_t)(x >> 20) ^ 0x80000000u);   // 64 (x - middle), 32 bits
+    int32_t h = p.a6 + bsg_sw::shi32x32(p.a7, e);
+    h = p.a5 + bsg_sw::shi32x32(h, e);
+    h = p.a4 + bsg_sw::shi32x32(h, e);
+    const int64_t s3 = p.a3 + (int64_t)bsg_sw::shi32x32(h, e) * 32;
+    const int64_t s2 = horner(p.a2, s3, e);
+    const int64_t s1 = horner(p.a1, s2, e);
+    // x's last 20 bits times the slope s1 + e (s2 + e s3)
+    const int32_t slope = (int32_t)(s1 >> 32) +
+        bsg_sw::shi32x32((int32_t)(s2 >> 32) + bsg_sw::shi32x32((int32_t)(s3 >> 32), e), e);
+    const int32_t low = (int32_t)(((uint32_t)x & 0xFFFFFu) << 11);
+    const uint64_t q = (uint64_t)(horner((int64_t)p.a0, s1, e) + (int64_t)bsg_sw::shi32x32(low, slope) * 2);  // 64
     // |q - middle| in 2^-11 units against 2^11 4.5 q (x^2 + 4), and this
     // evaluation's own 2^-60
     const uint32_t x16 = (uint32_t)(x >> 54), x2 = (x16 * x16) >> 8;
@@ -156,24 +118,22 @@ struct Seed2 { uint64_t root, rroot; int e; };
 
 // sqrt and 1/sqrt of w = x 2^-s (x's top bit set): root 2^(e - 62) and
 // rroot 2^(-e - 62).
-BSG_SW_FN Seed2 sqrt_both(const bsg_sw::Tables& t, uint64_t x, int s) {
+template <typename Tables>
+BSG_SW_FN Seed2 sqrt_both(const Tables& t, uint64_t x, int s) {
     const int b = 64 - s;
     const int odd = b & 1;
     const uint64_t y = x >> odd;
-    const bsg_sw::SeedEntry se = t.rs[(int)(y >> 56) - 64];
-    const uint32_t y0 = se.a - hi32x32(se.b, (uint32_t)(y >> 24));  // 30
-    const uint64_t e = (1ull << 60) - mulhi(y, wide(y0, y0));
-    const uint32_t eh = (uint32_t)(e >> 14);
-    const uint32_t g = 805306368u + (hi32x32(eh, 671088640u) >> 14);
-    const uint64_t corr = (e >> 1) + ((uint64_t)hi32x32(hi32(wide(eh, eh)), g) << 1);  // 60
-    const uint64_t s0 = mul_64x32(y, y0);                            // 62
-    return {s0 + (mulhi(s0, corr << 17) >> 13), ((uint64_t)y0 << 32) + (mul_64x32(corr << 17, y0) >> 13),
+    uint32_t c;
+    const uint32_t y0 = bsg_sw::rsqrt_seed(t, y, &c);
+    const uint64_t s0 = mul_64x32(y, y0);
+    return {s0 + (wide((uint32_t)(s0 >> 30), c) >> 26), ((uint64_t)y0 << 32) + (wide(y0, c) >> 24),
             (b + odd) / 2};
 }
 
 // The price for fields inside the domain (their bits), otype 0 = call; false
 // where it is left to price_fp64.
-BSG_SW_FN bool price_fx64(const bsg_sw::Tables& t, uint64_t bs, uint64_t bk, uint64_t br, uint64_t bv,
+template <typename Tables>  // bsg_sw::Tables, or one with its lg, rs and e2
+BSG_SW_FN bool price_fx64(const Tables& t, const TailTable& tails, uint64_t bs, uint64_t bk, uint64_t br, uint64_t bv,
                           uint64_t bt, int otype, double* price) {
     const uint64_t ms = significand(bs), mk = significand(bk), mt = significand(bt), mv = significand(bv);
     const int es = exponent_of(bs), ek = exponent_of(bk), et = exponent_of(bt) - 1023, ev = exponent_of(bv) - 1023;
@@ -184,9 +144,10 @@ BSG_SW_FN bool price_fx64(const bsg_sw::Tables& t, uint64_t bs, uint64_t bk, uin
     const int sw = 61 + nw - 2 * ev - et;                // w 2^-sw
     const Seed2 den = sqrt_both(t, w, sw);
     // ln(s/k) = n ln 2 + (L(k) - L(s))/2
-    int hs, hk;
-    const int64_t ls = neg2_ln_significand(t, ms, &hs), lk = neg2_ln_significand(t, mk, &hk);
-    const int n = es + hs - ek - hk;
+    int is, ik;
+    int64_t r;
+    const int64_t ls = bsg_sw::neg2_ln_core(t, ms, &is, &r), lk = bsg_sw::neg2_ln_core(t, mk, &ik, &r);
+    const int n = es + (is >> 8) - ek - (ik >> 8);
     int64_t num = ((lk - ls) >> 5) + n * 0x02C5C85FDF473DE8ll;       // 58
     // r t
     const int er = exponent_of(br) - 1023;
@@ -210,8 +171,8 @@ BSG_SW_FN bool price_fx64(const bsg_sw::Tables& t, uint64_t bs, uint64_t bk, uin
     const int64_t d2s = (dneg ? -(int64_t)d1 : (int64_t)d1) - (int64_t)dd;
     const bool d2neg = d2s < 0;
     bool near = false;
-    const uint64_t q1 = tail_units(t, d1, &near);
-    const uint64_t q2 = tail_units(t, d2neg ? 0ull - (uint64_t)d2s : (uint64_t)d2s, &near);
+    const uint64_t q1 = tail_units(tails, d1, &near);
+    const uint64_t q2 = tail_units(tails, d2neg ? 0ull - (uint64_t)d2s : (uint64_t)d2s, &near);
     // N(d1), N(d2) for a call, N(-d1), N(-d2) for a put, in units of 2^-53:
     // the tail where the sign says so, else 2^53 less the tail
     const bool put = otype != 0;
@@ -234,3 +195,6 @@ BSG_SW_FN bool price_fx64(const bsg_sw::Tables& t, uint64_t bs, uint64_t bk, uin
 }
 
 }  // namespace bsg_fx
+
+// The table's initializer: `const bsg_fx::TailTable t = BSG_FX_TAILS;`
+#define BSG_FX_TAILS {{BSG_FX_TAIL_TABLE}}

@@ -554,24 +554,30 @@ bool map_vectorizable(const SoA& a, const MapCfg& cfg) {
            aligned(a.out, al);
 }
 
-template <int M, int OPT, int STAGES>
-static cudaError_t launch_map_bulk(const SoA& a, int64_t n, const MapCfg& cfg, int sm_count,
-                                  cudaStream_t st, uint64_t wait_ns = kBulkWaitNs,
-                                  uint32_t tx_extra = 0) {
-    using B = BulkShape<OPT, STAGES>;
-    // opt in to the dynamic shared memory, once per device (contexts on
-    // several host threads may race here: setting the attribute twice is
-    // harmless, the bit mask is atomic)
+// Opts kernel K in to `bytes` of dynamic shared memory, once per device
+// (contexts on several host threads may race here: setting the attribute
+// twice is harmless, the bit mask is atomic).
+template <auto* K>
+static cudaError_t opt_in_smem(size_t bytes) {
     static std::atomic<unsigned long long> opted{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 64 || !(opted.load(std::memory_order_acquire) & (1ull << dev))) {
-        e = cudaFuncSetAttribute(map_bulk_kernel<M, OPT, STAGES>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, B::smem);
+        e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return e;
         if (dev < 64) opted.fetch_or(1ull << dev, std::memory_order_release);
     }
+    return cudaSuccess;
+}
+
+template <int M, int OPT, int STAGES>
+static cudaError_t launch_map_bulk(const SoA& a, int64_t n, const MapCfg& cfg, int sm_count,
+                                  cudaStream_t st, uint64_t wait_ns = kBulkWaitNs,
+                                  uint32_t tx_extra = 0) {
+    using B = BulkShape<OPT, STAGES>;
+    cudaError_t e = opt_in_smem<map_bulk_kernel<M, OPT, STAGES>>(B::smem);
+    if (e != cudaSuccess) return e;
     const int64_t ntiles = n / B::tile;
     int64_t grid = (int64_t)sm_count * (220 * 1024 / B::smem);  // CTAs that fit per SM
     if (grid > ntiles) grid = ntiles;
@@ -815,11 +821,31 @@ MapCfg map_default_cfg(const SoA& a, int64_t n, int runs) {
 // (bsg_fx64.h).  The few options that are left to the double evaluation go
 // into a queue in shared memory, which the block prices together at the end:
 // in place, one such option would hold its warp for a whole double
-// evaluation.  4M options: 175 us, bound by integer issue.
+// evaluation.  4M options: 133 us, bound by the pipe of the integer
+// multiply-adds (173 us before N came from a table, that pipe 73 % busy).
 constexpr int kF64Threads = 256;
 constexpr int kF64Queue = 1024;
 
 __device__ const bsg_sw::Tables kFxTables = BSG_SW_TABLES;
+__device__ const bsg_fx::TailTable kFxTails = BSG_FX_TAILS;
+
+// The block's copy of the tables the price reads (48,640 bytes: dynamic shared
+// memory, four blocks an SM), and its queue.
+struct F64Shared {
+    bsg_sw::LogEntry lg[512];
+    bsg_sw::SeedEntry rs[384];
+    uint64_t e2[1024];
+    bsg_fx::TailTable tails;
+    uint32_t queue[kF64Queue];
+    int queued;
+};
+
+template <typename T>
+__device__ __forceinline__ void copy_table(T& dst, const T& src) {
+    static_assert(sizeof(T) % 16 == 0, "copied in 16-byte words");
+    for (int i = threadIdx.x; i < (int)(sizeof(T) / 16); i += kF64Threads)
+        reinterpret_cast<uint4*>(&dst)[i] = __ldg(reinterpret_cast<const uint4*>(&src) + i);
+}
 
 __device__ __noinline__ double price_fp64_call(double s, double k, double r, double v, double t, int ot) {
     return price_fp64(s, k, r, v, t, ot);
@@ -839,16 +865,14 @@ struct F64View {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kF64Threads, 3) map_f64_kernel(F64View<T> a, int64_t n) {
-    __shared__ bsg_sw::Tables tab;
-    __shared__ uint32_t queue[kF64Queue];
-    __shared__ int queued;
-    {
-        const double2* src = reinterpret_cast<const double2*>(&kFxTables);
-        double2* dst = reinterpret_cast<double2*>(&tab);
-        for (int i = threadIdx.x; i < (int)(sizeof(tab) / sizeof(double2)); i += kF64Threads) dst[i] = src[i];
-        if (threadIdx.x == 0) queued = 0;
-    }
+__global__ void __launch_bounds__(kF64Threads, 4) map_f64_kernel(F64View<T> a, int64_t n) {
+    extern __shared__ __align__(16) char f64_smem[];
+    F64Shared& sh = *reinterpret_cast<F64Shared*>(f64_smem);
+    copy_table(sh.lg, kFxTables.lg);
+    copy_table(sh.rs, kFxTables.rs);
+    copy_table(sh.e2, kFxTables.e2);
+    copy_table(sh.tails, kFxTails);
+    if (threadIdx.x == 0) sh.queued = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * kF64Threads, stride = (int64_t)gridDim.x * kF64Threads;
     uint32_t at = threadIdx.x;  // the option's place among the block's: 256 per pass of the grid
@@ -858,11 +882,11 @@ __global__ void __launch_bounds__(kF64Threads, 3) map_f64_kernel(F64View<T> a, i
         const int ot = __ldg(a.ot + i);
         double p;
         bool done = bsg_fx::fx64_domain(dbits(s), dbits(k), dbits(r), dbits(v), dbits(t));
-        if (done) done = bsg_fx::price_fx64(tab, dbits(s), dbits(k), dbits(r), dbits(v), dbits(t), ot, &p);
+        if (done) done = bsg_fx::price_fx64(sh, sh.tails, dbits(s), dbits(k), dbits(r), dbits(v), dbits(t), ot, &p);
         if (!done) {
-            const int q = atomicAdd(&queued, 1);
+            const int q = atomicAdd(&sh.queued, 1);
             if (q < kF64Queue) {
-                queue[q] = at;
+                sh.queue[q] = at;
                 continue;
             }
             p = price_fp64_call(s, k, r, v, t, ot);
@@ -870,9 +894,9 @@ __global__ void __launch_bounds__(kF64Threads, 3) map_f64_kernel(F64View<T> a, i
         a.out[i] = p;
     }
     __syncthreads();
-    const int m = queued < kF64Queue ? queued : kF64Queue;
+    const int m = sh.queued < kF64Queue ? sh.queued : kF64Queue;
     for (int q = threadIdx.x; q < m; q += kF64Threads) {
-        const int64_t i = base + (int64_t)(queue[q] / kF64Threads) * stride + queue[q] % kF64Threads;
+        const int64_t i = base + (int64_t)(sh.queue[q] / kF64Threads) * stride + sh.queue[q] % kF64Threads;
         a.out[i] = price_fp64_call(__ldg(a.s + i), __ldg(a.k + i), __ldg(a.r + i), __ldg(a.v + i),
                                    __ldg(a.t + i), __ldg(a.ot + i));
     }
@@ -881,10 +905,12 @@ __global__ void __launch_bounds__(kF64Threads, 3) map_f64_kernel(F64View<T> a, i
 template <typename T>
 static cudaError_t launch_f64_view(const F64View<T>& a, int64_t n, int sm_count, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
+    cudaError_t e = opt_in_smem<map_f64_kernel<T>>(sizeof(F64Shared));
+    if (e != cudaSuccess) return e;
     int64_t grid = (n + kF64Threads - 1) / kF64Threads;
-    const int64_t cap = (int64_t)sm_count * 3;
+    const int64_t cap = (int64_t)sm_count * 4;
     if (grid > cap) grid = cap;
-    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, 0, st>>>(a, n);
+    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, sizeof(F64Shared), st>>>(a, n);
     return cudaGetLastError();
 }
 

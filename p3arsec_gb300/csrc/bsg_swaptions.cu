@@ -29,8 +29,10 @@
 // 33.1 ms for 128 swaptions x 1M paths with 130 FP64 operations a path, that
 // pipe 85 % busy.  So the variates, the exponents and the powers of two are
 // 64-bit fixed point (bsg_swmath.h), and FP64 is left with a payment's
-// multiply-add, the floor and the two sums, 4 to 6 operations a path: 7.35 ms,
-// bound by integer issue (950 instructions a path).
+// multiply-add, the floor and the two sums, 4 to 6 operations a path: 5.28 ms.
+// Its bound is the pipe that takes the integer multiply-adds (two thirds busy,
+// 170 of them a path, 40 in the generator).  Four blocks of 64 registers an SM:
+// 5.34 ms, three of 80 5.53, two of 128 5.54.
 //
 // Reduction: each warp reduces its paths' sums (sum and sum of squares of
 // the discounted payoff) in a fixed order and writes one partial; the block
@@ -83,21 +85,23 @@ __device__ __forceinline__ void load_tables(bsg_sw::Tables& dst) {
 }
 
 // One swaption in shared memory: its head and its words (pays, constants,
-// coefficients; bsg_internal.h).
+// coefficients; bsg_internal.h).  Swaptions of up to four exponents have at
+// most 4 (2 + 8 x 31) words.
+template <bool LARGE>
 struct SwShared {
     bsg_sw::Tables nt;
     SwHead head;
-    uint64_t words[kSwMaxWords];
-    double red[2][kSwThreads];
+    uint64_t words[LARGE ? kSwMaxWords : 1000];
+    double red[2][kSwWarps];
     int last;
 };
 
 __device__ __forceinline__ double as_double(uint64_t u) { return __longlong_as_double((long long)u); }
 
-// The undiscounted-by-a-constant payoff of trial t of the swaption in sh.
+// The payoff of trial t of the swaption in sh, less its constant discount.
 // NP: the number of exponents, or with GUARD an upper bound of it.
-template <int NP, bool GUARD>
-__device__ __forceinline__ double path_payoff(const SwShared& sh, uint64_t t) {
+template <int NP, bool GUARD, typename Sh>
+__device__ __forceinline__ double path_payoff(const Sh& sh, uint64_t t) {
     const SwHead& hd = sh.head;
     const int np = GUARD ? hd.n_exp : NP;
     const uint64_t* c0 = sh.words + np;
@@ -105,31 +109,30 @@ __device__ __forceinline__ double path_payoff(const SwShared& sh, uint64_t t) {
     uint64_t x[NP], half = 0;
 #pragma unroll
     for (int l = 0; l < NP; ++l) x[l] = (!GUARD || l < np) ? c0[l] : 0;
+    // coefficients g = G 2^-63 and variates z = Z 2^-58 enter as G + 2^63 and
+    // Z + 2^62 (swaption_setup's constants take that out again)
+    auto take = [&](int64_t z) {
+        const uint64_t zu = (uint64_t)z + (1ull << 62);
+        half += zu >> 1;
+#pragma unroll
+        for (int l = 0; l < NP; ++l)
+            if (!GUARD || l < np) x[l] += bsg_sw::mulhi(g[l], zu);
+        g += np;
+    };
     const int nz = hd.n_normals;
 #pragma unroll 1
     for (int i = 0; i < nz; i += 2) {
         uint32_t w[4];
         philox4x32_10((uint32_t)t, (uint32_t)(t >> 32), (uint32_t)(i >> 1), 0u, (uint32_t)hd.seed,
                       (uint32_t)(hd.seed >> 32), w);
-        // coefficients g = G 2^-63 and variates z = Z 2^-58, both moved into
-        // the unsigned range (swaption_setup's constants take that out again)
-        const bsg_sw::Root r = bsg_sw::sqrt_scaled(
-            sh.nt, bsg_sw::neg2_ln_scaled(sh.nt, bsg_sw::unit_bits(w[0], w[1])));
-        int64_t zs, zc;
-        bsg_sw::sincos_2pi_fixed(sh.nt, bsg_sw::unit_bits(w[2], w[3]), &zs, &zc);
-        const uint64_t z0 = (uint64_t)bsg_sw::times_root(r, zc) + (1ull << 62);
-        half += z0 >> 1;
-#pragma unroll
-        for (int l = 0; l < NP; ++l)
-            if (!GUARD || l < np) x[l] += bsg_sw::mulhi(g[l], z0);
-        g += np;
+        int64_t z0, z1;
         if (i + 1 < nz) {
-            const uint64_t z1 = (uint64_t)bsg_sw::times_root(r, zs) + (1ull << 62);
-            half += z1 >> 1;
-#pragma unroll
-            for (int l = 0; l < NP; ++l)
-                if (!GUARD || l < np) x[l] += bsg_sw::mulhi(g[l], z1);
-            g += np;
+            bsg_sw::normal_pair_fixed<true>(sh.nt, w[0], w[1], w[2], w[3], &z0, &z1);
+            take(z0);
+            take(z1);
+        } else {
+            bsg_sw::normal_pair_fixed<false>(sh.nt, w[0], w[1], w[2], w[3], &z0, &z1);
+            take(z0);
         }
     }
     // the payments' discount factors, then the path's own if it varies
@@ -147,7 +150,8 @@ __device__ __forceinline__ double path_payoff(const SwShared& sh, uint64_t t) {
 
 // The same in double precision, for exponents outside the fixed-point range:
 // words hold the constants and coefficients as doubles, natural exponents.
-__device__ __noinline__ double path_payoff_wide(const SwShared& sh, uint64_t t) {
+template <typename Sh>
+__device__ __noinline__ double path_payoff_wide(const Sh& sh, uint64_t t) {
     const SwHead& hd = sh.head;
     const int np = hd.n_exp, nz = hd.n_normals, pays = np - hd.disc_varies;
     double v = -1.0, disc = 1.0;
@@ -169,32 +173,53 @@ __device__ __noinline__ double path_payoff_wide(const SwShared& sh, uint64_t t) 
     return v > 0.0 ? __dmul_rn(v, disc) : 0.0;
 }
 
-template <int NP, bool GUARD, bool WIDE = false>
-__device__ __forceinline__ void sum_paths(const SwShared& sh, uint64_t base, int per_thread,
-                                          uint64_t trials, double& sum, double& sum_sq) {
+// A warp's two sums in a fixed order: the lower half of the warp adds up a,
+// the upper half b.
+__device__ __forceinline__ double2 warp_sums(double a, double b) {
+    const bool low = (threadIdx.x & 31) < 16;
+    const double give = low ? b : a, keep = low ? a : b;
+    double v = __dadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, 16));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return make_double2(v, __shfl_sync(0xffffffffu, v, 16));  // lane 0's are the sums
+}
+
+// Chunks [chunk, end) of the swaption in sh: one partial per warp and chunk.
+template <int NP, bool GUARD, bool WIDE, typename Sh>
+__device__ __forceinline__ void sum_chunks(const Sh& sh, uint64_t chunk, uint64_t end, int per_thread,
+                                           uint64_t trials, double2* partial) {
 #pragma unroll 1
-    for (int q = 0; q < per_thread; ++q) {
-        const uint64_t t = base + (uint64_t)q * kSwThreads + threadIdx.x;
-        if (t >= trials) break;
-        const double dp = WIDE ? path_payoff_wide(sh, t) : path_payoff<NP, GUARD>(sh, t);
-        sum = __dadd_rn(sum, dp);
-        sum_sq = __fma_rn(dp, dp, sum_sq);
+    for (; chunk < end; ++chunk) {
+        double sum = 0.0, sum_sq = 0.0;
+        uint64_t t = chunk * per_thread * kSwThreads + threadIdx.x;
+#pragma unroll 1
+        for (int q = 0; q < per_thread && t < trials; ++q, t += kSwThreads) {
+            const double dp = WIDE ? path_payoff_wide(sh, t) : path_payoff<NP, GUARD>(sh, t);
+            sum = __dadd_rn(sum, dp);
+            sum_sq = __fma_rn(dp, dp, sum_sq);
+        }
+        const double2 v = warp_sums(sum, sum_sq);
+        const double d = sh.head.disc;
+        if ((threadIdx.x & 31) == 0)
+            partial[chunk * kSwWarps + (threadIdx.x >> 5)] =
+                make_double2(__dmul_rn(v.x, d), __dmul_rn(v.y, __dmul_rn(d, d)));
     }
 }
 
-// Persistent blocks over (swaption, chunk of per_thread x 256 paths) items.
-// LARGE: also swaptions of more than four exponents or outside the
-// fixed-point range (their registers would cost the others a block per SM).
+// Persistent blocks over (swaption, `span` consecutive chunks of per_thread x
+// 256 paths).  LARGE: also swaptions of more than four exponents or outside
+// the fixed-point range (their registers would cost the others a block per SM).
 template <bool LARGE>
-__global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 3) swaption_paths_kernel(
+__global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 4) swaption_paths_kernel(
     const __grid_constant__ SwInline in, const uint64_t* __restrict__ table, int nsw, uint64_t trials,
-    int per_thread, uint64_t chunks, double2* __restrict__ partial, unsigned* __restrict__ done,
-    double* __restrict__ out) {
-    __shared__ SwShared sh;
+    int per_thread, uint64_t chunks, unsigned span, double2* __restrict__ partial,
+    unsigned* __restrict__ done, double* __restrict__ out) {
+    __shared__ SwShared<LARGE> sh;
     load_tables(sh.nt);
-    const uint64_t items = chunks * (uint64_t)nsw;
+    const uint64_t spans = (chunks + span - 1) / span, items = spans * (uint64_t)nsw;
     for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
-        const uint64_t sw = item / chunks, chunk = item - sw * chunks;
+        const uint64_t sw = item / spans, chunk = (item - sw * spans) * span;
+        const uint64_t end = chunk + span < chunks ? chunk + span : chunks;
         __syncthreads();  // the previous item's reads of sh are done
         {
             // head, then its words (from the launch's parameters when they all fit there)
@@ -207,61 +232,52 @@ __global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 3) swaption_paths_kern
             for (int i = threadIdx.x; i < sh.head.n_words; i += kSwThreads) sh.words[i] = src[i];
         }
         __syncthreads();
-        const uint64_t base = chunk * per_thread * kSwThreads;
-        double sum = 0.0, sum_sq = 0.0;
+        double2* part = partial + sw * chunks * kSwWarps;
         if (LARGE && sh.head.wide) {
-            sum_paths<1, true, true>(sh, base, per_thread, trials, sum, sum_sq);
+            sum_chunks<1, true, true>(sh, chunk, end, per_thread, trials, part);
         } else {
             switch (sh.head.n_exp) {
-                case 1: sum_paths<1, false>(sh, base, per_thread, trials, sum, sum_sq); break;
-                case 2: sum_paths<2, false>(sh, base, per_thread, trials, sum, sum_sq); break;
-                case 3: sum_paths<3, false>(sh, base, per_thread, trials, sum, sum_sq); break;
-                case 4: sum_paths<4, false>(sh, base, per_thread, trials, sum, sum_sq); break;
+                case 1: sum_chunks<1, false, false>(sh, chunk, end, per_thread, trials, part); break;
+                case 2: sum_chunks<2, false, false>(sh, chunk, end, per_thread, trials, part); break;
+                case 3: sum_chunks<3, false, false>(sh, chunk, end, per_thread, trials, part); break;
+                case 4: sum_chunks<4, false, false>(sh, chunk, end, per_thread, trials, part); break;
                 default:
                     if constexpr (LARGE) {
-                        if (sh.head.n_exp <= 8) sum_paths<8, true>(sh, base, per_thread, trials, sum, sum_sq);
-                        else sum_paths<kSwMaxExp, true>(sh, base, per_thread, trials, sum, sum_sq);
+                        if (sh.head.n_exp <= 8)
+                            sum_chunks<8, true, false>(sh, chunk, end, per_thread, trials, part);
+                        else
+                            sum_chunks<kSwMaxExp, true, false>(sh, chunk, end, per_thread, trials, part);
                     }
             }
         }
-        // the warp's two sums in a fixed order: the lower half of the warp adds
-        // up sum, the upper half sum_sq
-        const int lane = threadIdx.x & 31;
-        const double give = lane < 16 ? sum_sq : sum, keep = lane < 16 ? sum : sum_sq;
-        double a = __dadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, 16));
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) a = __dadd_rn(a, __shfl_xor_sync(0xffffffffu, a, o));
-        const double b = __shfl_sync(0xffffffffu, a, 16);
-        if (lane == 0)
-            partial[item * kSwWarps + (threadIdx.x >> 5)] =
-                make_double2(__dmul_rn(a, sh.head.disc), __dmul_rn(b, __dmul_rn(sh.head.disc, sh.head.disc)));
-        // the last block of the swaption adds its partials up
-        __threadfence();
+        // the block that finishes the swaption's last chunk adds the partials up
+        if ((threadIdx.x & 31) == 0) __threadfence();
         __syncthreads();
-        if (threadIdx.x == 0) sh.last = atomicAdd(&done[sw], 1u) == (unsigned)(chunks - 1);
+        if (threadIdx.x == 0)
+            sh.last = atomicAdd(&done[sw], (unsigned)(end - chunk)) + (unsigned)(end - chunk) == (unsigned)chunks;
         __syncthreads();
         if (!sh.last) continue;
         __threadfence();
         double ta = 0.0, tb = 0.0;
-        const double2* p = partial + sw * chunks * kSwWarps;
         for (uint64_t i = threadIdx.x; i < chunks * kSwWarps; i += kSwThreads) {
-            const double2 v = __ldcg(p + i);
+            const double2 v = __ldcg(part + i);
             ta = __dadd_rn(ta, v.x);
             tb = __dadd_rn(tb, v.y);
         }
-        sh.red[0][threadIdx.x] = ta;
-        sh.red[1][threadIdx.x] = tb;
-        __syncthreads();
-        for (int w = kSwThreads / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) {
-                sh.red[0][threadIdx.x] = __dadd_rn(sh.red[0][threadIdx.x], sh.red[0][threadIdx.x + w]);
-                sh.red[1][threadIdx.x] = __dadd_rn(sh.red[1][threadIdx.x], sh.red[1][threadIdx.x + w]);
-            }
-            __syncthreads();
+        const double2 v = warp_sums(ta, tb);
+        if ((threadIdx.x & 31) == 0) {
+            sh.red[0][threadIdx.x >> 5] = v.x;
+            sh.red[1][threadIdx.x >> 5] = v.y;
         }
+        __syncthreads();
         if (threadIdx.x == 0) {
+            double s1 = sh.red[0][0], s2 = sh.red[1][0];
+            for (int w = 1; w < kSwWarps; ++w) {
+                s1 = __dadd_rn(s1, sh.red[0][w]);
+                s2 = __dadd_rn(s2, sh.red[1][w]);
+            }
             // the mean and the reference's standard error (HJM_Swaption_Blocking.cpp:212-214)
-            const double m = (double)trials, s1 = sh.red[0][0], s2 = sh.red[1][0];
+            const double m = (double)trials;
             out[2 * sw] = s1 / m;
             out[2 * sw + 1] = sqrt((s2 - s1 * s1 / m) / (m - 1.0)) / sqrt(m);
             done[sw] = 0;  // ready for the next call
@@ -309,15 +325,19 @@ cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw,
                              cudaStream_t st) {
     if (nsw <= 0 || trials < 2) return cudaErrorInvalidValue;
     const uint64_t chunks = swaption_chunks(trials), items = chunks * (uint64_t)nsw;
-    const unsigned grid = (unsigned)std::min<uint64_t>(items, (uint64_t)sm_count * (large ? 2 : 3));
+    const uint64_t room = (uint64_t)sm_count * (large ? 2 : 4);
     const int per_thread = swaption_per_thread(trials);
+    // chunks per visit of a block: the fewer the better for the last wave, so
+    // the most that leave 16 visits per block
+    const unsigned span = (unsigned)std::min<uint64_t>(std::max<uint64_t>(items / (16 * room), 1), 16);
+    const unsigned grid = (unsigned)std::min<uint64_t>((chunks + span - 1) / span * (uint64_t)nsw, room);
     double2* part = static_cast<double2*>(partial);
     if (large)
         swaption_paths_kernel<true><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
-                                                                 part, done, out);
+                                                                 span, part, done, out);
     else
         swaption_paths_kernel<false><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
-                                                                  part, done, out);
+                                                                  span, part, done, out);
     return cudaGetLastError();
 }
 

@@ -8,8 +8,10 @@
 // operations (measured), so a 64-bit product truncated to its high half
 // (three multiply-adds) costs a fifth of a double multiply and carries 11
 // more bits, and the high-order terms of a series fit 32 bits at a thirtieth
-// of the cost.  Every value here has at least 57 fraction bits; a normal
-// variate is within 2e-17 + half an ulp of the exact one.
+// of the cost.  Each series is cut where its terms pass 2^-60, and each term
+// has the bits it needs for that and no more.  A normal variate, as a double,
+// is within 1.5e-16 of max(1, |z|) of the exact one (5.0e-16 when every step was
+// a double operation).
 //
 // The uniforms are u = (2k + 1) 2^-53 for a 52-bit integer k (the grid of
 // midpoints in (0, 1)); a pair (u1, u2) gives z0 = sqrt(-2 ln u1) cos(2 pi u2)
@@ -24,13 +26,14 @@
 //    alone, as small as it is, from a normalised r.  This is the table-driven
 //    logarithm of P. T. P. Tang, ACM TOMS 16(4), 1990, with the reciprocal
 //    table's exact products.
-//  sqrt: a linear table seed at or below 1/sqrt(y) (192 intervals), then
-//    s = y y0 (1 + e/2 + 3 e^2/8), e = 1 - y y0^2 < 2^-14 (the binomial series
-//    of (1 - e)^(-1/2); its cubic term, folded into the quadratic's factor).
-//  sin/cos(2 pi u): the quadrant and the nearest 1/1024 turn of u from k's
-//    bits, the rest an exact integer; the angle-addition formulas combine the
+//  sqrt: a quadratic table seed at or below 1/sqrt(y) (384 intervals), then
+//    s = y y0 (1 + e/2 + 3 e^2/8), e = 1 - y y0^2 < 2^-24 (the binomial series
+//    of (1 - e)^(-1/2)).
+//  sin/cos(2 pi u): the quadrant and the 1/2048 turn below u from k's bits,
+//    the rest an exact integer; the angle-addition formulas combine the
 //    table's sin and cos with Taylor polynomials of sin phi (to phi^5) and
-//    1 - cos phi (to phi^6), |phi| <= pi/1024.
+//    cos phi (to phi^6), 0 < phi < 2 pi/2048: nothing is negative inside a
+//    quadrant, so signs are set once, at the end.
 //  2^x: the integer part, a table of 2^(j/1024), and the Taylor polynomial of
 //    e^t - 1 to t^4, t = r ln 2 < 2^-10.
 //  e^x (double): x = (64 m + j) ln2/64 + r with k = 64 m + j the integer
@@ -58,14 +61,14 @@
 namespace bsg_sw {
 
 struct alignas(16) LogEntry { int64_t ln; uint32_t c; };
-struct alignas(8) SeedEntry { uint32_t a, b; };
+struct alignas(16) SeedEntry { uint32_t a, b, c, unused; };
 struct alignas(16) Angle { uint64_t s, c; };
 
-// 22,528 bytes: the kernels copy it into shared memory once per block.
+// 31,232 bytes: the kernels copy it into shared memory once per block.
 struct alignas(16) Tables {
     LogEntry lg[512];
-    SeedEntry rs[192];  // y in [i/256, (i + 1)/256), i = 64..255
-    Angle ang[256];     // the first quadrant
+    SeedEntry rs[384];  // y in [i/512, (i + 1)/512), i = 128..511
+    Angle ang[512];     // the first quadrant
     uint64_t e2[1024];  // 2^(j/1024)
     double e64[64];     // 2^(j/64)
 };
@@ -109,30 +112,47 @@ BSG_SW_FN uint64_t mul_64x32(uint64_t a, uint32_t b) {
 // 20 bits of a, all of b).
 BSG_SW_FN uint64_t unit_bits(uint32_t a, uint32_t b) { return ((uint64_t)(a >> 12) << 32) | b; }
 
+// -2 ln of x = m 2^-63 in [1, 2) with 62 fraction bits; for the upper half of
+// the table (*i >= 256) that of x/2.  *r: x c - 1 (the table's c) with 63 bits.
+template <typename T>
+BSG_SW_FN int64_t neg2_ln_core(const T& t, uint64_t m, int* i, int64_t* r) {
+    *i = (int)(m >> 54) & 511;
+    const LogEntry le = t.lg[*i];
+    // x c 2^83 = hi 2^32 + (lo mod 2^32); r = that less 2^83, exact before the shifts
+    const uint64_t lo = wide((uint32_t)m, le.c);
+    const uint64_t hi = wide(hi32(m), le.c) + (lo >> 32);
+    *r = (int64_t)(((hi << 12) | ((uint32_t)lo >> 20)) ^ (1ull << 63));
+    const int32_t rh = (int32_t)(uint32_t)(hi >> 10);    // r 2^41
+    const int32_t nr = -(rh >> 9);                       // -r 2^32
+    // -2 ln(1 + r) = -2 r + r^2 - r^2 r (2/3 - r (1/2 - r (2/5 - r/3)))
+    int32_t q = 858993459 + shi32x32(nr, 715827883);     // 2/5 - r/3, 31 fraction bits
+    q = 1073741824 + shi32x32(nr, q);
+    q = 1431655765 + shi32x32(nr, q);
+    const int32_t rq = (int32_t)(((int64_t)rh * q + (1ll << 30)) >> 31);  // 41
+    const uint32_t rl = (uint32_t)((uint64_t)*r << 10);  // r 2^73 below rh's last bit
+    // r^2 2^82, the cross term rounded down by at most 4: + 4 keeps it positive
+    const uint64_t r2 = (uint64_t)((int64_t)rh * rh + 4) +
+                        (uint64_t)((int64_t)shi32x32(rh, (int32_t)(rl >> 1)) * 4);
+    uint32_t rs = (uint32_t)(r2 >> 31);                  // 51, below 2^31 but for |r| next to 2^-10
+    rs = rs < 0x7FFFFFFFu ? rs : 0x7FFFFFFFu;
+    const int64_t r3q = (int64_t)(int32_t)rs * rq;       // 51 + 41
+    return le.ln + (int64_t)(r2 >> 20) - (r3q >> 30) - *r;
+}
+
 // -2 ln u for u = (2k + 1) 2^-53, k < 2^52, as x 2^-s with x's top bit set.
 struct Scaled { uint64_t x; int s; };
 
 BSG_SW_FN Scaled neg2_ln_scaled(const Tables& t, uint64_t k) {
     const uint64_t v = 2 * k + 1;                        // u = v 2^-53, v odd
     const int lz = clz64(v);                             // 11..63
-    const uint64_t m = v << lz;                          // u = (m 2^-63) 2^(10 - lz)
-    const int i = (int)((m >> 54) & 511);
-    const LogEntry le = t.lg[i];
+    int i;
+    int64_t r;
+    const uint64_t w = (uint64_t)neg2_ln_core(t, v << lz, &i, &r);
     const int ne = lz - 10 - (i >> 8);                   // powers of two taken out, negated: 0..53
-    // r 2^73, exact: m c 2^20 - 2^83 (a multiple of 2^73 times 2^10, mod 2^64 after the shift)
-    const uint64_t lo = wide((uint32_t)m, le.c);
-    const uint64_t hi = wide(hi32(m), le.c) + (lo >> 32);
-    const int64_t r = (int64_t)((hi << 22) | ((uint32_t)lo >> 10));
-    const int32_t rh = (int32_t)(r >> 32);               // r 2^41
-    // -2 ln(1 + r) = -2 r + r^2 q, q = 1 - r (2/3 - r (1/2 - r (2/5 - r/3)))
-    int32_t q = 858993459 - (shi32x32(rh, 715827883) >> 9);  // 2/5 - r/3, 31 fraction bits
-    q = 1073741824 - (shi32x32(rh, q) >> 9);
-    q = 1431655765 - (shi32x32(rh, q) >> 9);
-    const uint64_t q63 = (1ull << 63) - (uint64_t)(((int64_t)rh * q) >> 9);
     if (ne == 0 && i == 511) {
         // u near 1: -2 ln u = 2 |r| (1 + c), c = |r|/2 + r^2/3 + |r|^3/4 + r^4/5,
-        // from |r| = 1 - u (2^-53 and up) with its top bit moved up
-        const uint64_t ar = 0ull - (uint64_t)r;          // |r| 2^73
+        // |r| = 1 - u = (2^53 - v) 2^-53 with its top bit moved up
+        const uint64_t ar = ((1ull << 53) - v) << 20;    // |r| 2^73
         const uint32_t ah = hi32(ar);                    // 41
         const uint64_t a2 = wide(ah, ah) + ((uint64_t)hi32x32(ah, (uint32_t)ar) << 1);  // r^2, 82
         const uint32_t g = hi32x32(ah, 1073741824u + (hi32x32(ah, 858993459u) >> 9));   // |r| (1/4 + |r|/5), 41
@@ -144,14 +164,10 @@ BSG_SW_FN Scaled neg2_ln_scaled(const Tables& t, uint64_t k) {
         const int top = (int)(y >> 63);
         return {y << (1 - top), n + 72 - top};
     }
-    // r^2 2^82, the cross term rounded down by at most 4: + 4 keeps it positive
-    const uint64_t r2 = (uint64_t)((int64_t)rh * rh + 4) +
-                        (uint64_t)((int64_t)shi32x32(rh, (int32_t)((uint32_t)r >> 1)) * 4);
-    const uint64_t w = (uint64_t)le.ln + (mulhi(r2, q63) >> 19) - (uint64_t)(r >> 10);      // 62 bits
     // below 2 at ne = 0, where it may be small; below 73.5 otherwise
     const uint64_t x = ne == 0 ? w
                                : (uint64_t)((int64_t)w >> 5) + wide((uint32_t)BSG_SW_2LN2_57, (uint32_t)ne) +
-                                     (wide(hi32(BSG_SW_2LN2_57), (uint32_t)ne) << 32);
+                                     ((uint64_t)(hi32(BSG_SW_2LN2_57) * (uint32_t)ne) << 32);
     const int n = clz64(x);
     return {x << n, (ne == 0 ? 62 : 57) + n};
 }
@@ -167,63 +183,67 @@ BSG_SW_FN double neg2_ln_unit(const Tables& t, uint64_t k) {
     return scaled_to_double(w.x, w.s);
 }
 
-// sqrt(x 2^-w.s) = s 2^(e - 62), s in [2^61, 2^62].
+// sqrt(w.x 2^-w.s) = s 2^(e - 62), s in [2^61, 2^62].
 struct Root { uint64_t s; int e; };
+
+// The seed and its correction: y (1/4..1, 64 fraction bits) -> y0 at or below
+// 1/sqrt(y) (30) and c with 1/sqrt(y) = y0 (1 + c) (56).
+template <typename T>
+BSG_SW_FN uint32_t rsqrt_seed(const T& t, uint64_t y, uint32_t* c) {
+    const SeedEntry se = t.rs[(int)(y >> 55) - 128];
+    const uint32_t d = (uint32_t)(y >> 23);
+    const uint32_t y0 = se.a - hi32x32(d, se.b - hi32x32(d, se.c));
+    const uint64_t e = (1ull << 60) - mulhi(y, wide(y0, y0));        // 1 - y y0^2 in [0, 2^-24)
+    const uint32_t h = (uint32_t)(e >> 5);               // e 2^55 = e/2 2^56
+    *c = h + hi32x32(hi32x32(h, h), 384u);               // + 3 e^2/8: 78, 3/8 2^10, 56
+    return y0;
+}
 
 BSG_SW_FN Root sqrt_scaled(const Tables& t, Scaled w) {
     const int b = 64 - w.s;                              // the value is (x 2^-64) 2^b
     const int odd = b & 1;
     const uint64_t y = w.x >> odd;                       // [1/4, 1), 64 fraction bits
-    const SeedEntry se = t.rs[(int)(y >> 56) - 64];
-    const uint32_t y0 = se.a - hi32x32(se.b, (uint32_t)(y >> 24));  // 30 bits, at or below 1/sqrt(y)
-    const uint64_t e = (1ull << 60) - mulhi(y, wide(y0, y0));       // 1 - y y0^2 in [0, 2^-14), 60 bits
-    const uint32_t eh = (uint32_t)(e >> 14);             // e 2^46
-    const uint32_t g = 805306368u + (hi32x32(eh, 671088640u) >> 14);  // 3/8 + 5/16 e, 31 bits
-    const uint64_t corr = (e >> 1) + ((uint64_t)hi32x32(hi32(wide(eh, eh)), g) << 1);  // 60 bits
-    const uint64_t s0 = mul_64x32(y, y0);                // 62 bits
-    return {s0 + (mulhi(s0, corr << 17) >> 13), (b + odd) / 2};
+    uint32_t c;
+    const uint32_t y0 = rsqrt_seed(t, y, &c);
+    const uint64_t s0 = mul_64x32(y, y0);                // 62, below 2^62
+    return {s0 + (wide((uint32_t)(s0 >> 30), c) >> 26), (b + odd) / 2};
 }
 
-// |sin| and |cos| of 2 pi u (u = (2k + 1) 2^-53) with 63 fraction bits up to
-// the quadrant: in quadrant q (0..3) the angle is q quarter turns past the
-// one whose sine and cosine these are.  Both may be off the first quadrant by
-// half a table step, so they are signed: 62 fraction bits.
-BSG_SW_FN void sincos_quadrant(const Tables& t, uint64_t k, int* quadrant, int64_t* s, int64_t* c) {
-    const uint32_t j = (uint32_t)((k + (1ull << 41)) >> 42);  // nearest 1/1024: 0..1024
-    const int64_t x = (int64_t)(2 * k + 1) - ((int64_t)j << 43);  // odd, |x| < 2^42
-    const uint64_t neg = (uint64_t)(x >> 63);
-    const uint64_t ax = ((uint64_t)x ^ neg) - neg;
-    const uint64_t ph = mulhi(ax << 22, BSG_SW_2PI_61);  // |phi| = |x| 2 pi 2^-53, 72 fraction bits
-    const uint32_t phh = hi32(ph);                       // 40
-    const uint64_t p = wide(phh, phh) + ((uint64_t)hi32x32(phh, (uint32_t)ph) << 1);  // phi^2, 80
+// 2 pi u (u = (2k + 1) 2^-53) less its whole quarter turns (k >> 50) as a
+// table angle (63 fraction bits) and sin and cos (64) of the rest.
+struct Turn { Angle a; uint64_t sn, cs; };
+
+BSG_SW_FN Turn turn_of(const Tables& t, uint64_t k) {
+    // phi = x 2 pi 2^-53, x = 2 (k mod 2^41) + 1: x 2^22 drops k's higher bits
+    const uint64_t ph = mulhi((k << 23) | (1ull << 22), BSG_SW_2PI_53);  // 64
+    const uint32_t phh = (uint32_t)(ph >> 24);           // 40
+    const uint64_t p = wide(phh, phh) + ((uint64_t)hi32x32(phh, (uint32_t)ph << 8) << 1);  // phi^2, 80
     const uint32_t pp = hi32(p);                         // 48
-    // sin = phi - phi sg, sg = phi^2 (1/6 - phi^2/120)
-    const uint32_t mu = 2863311531u - hi32x32(pp, 2185u);             // 34
-    const uint32_t sg = (uint32_t)(wide(pp, mu) >> 31);               // 51
-    const uint64_t sp = ph - (wide(phh, sg) >> 19);                   // 72
-    // 1 - cos = phi^2 (1/2 - phi^2 (1/24 - phi^2/720))
-    const uint32_t la = 2863311531u - hi32x32(pp, 1456u);             // 36
-    const uint64_t ka = (1ull << 62) - (wide(pp, la) >> 21);          // 63
-    const uint64_t cm = mulhi(p, ka);                                 // 79
-    const Angle a = t.ang[j & 255];
-    // a.s, a.c: 63 bits; products with sp: 71, with cm: 78
-    const uint64_t csp = mulhi(a.c, sp) >> 9, ssp = mulhi(a.s, sp) >> 9;  // 62
-    *s = (int64_t)((a.s >> 1) - (mulhi(a.s, cm) >> 16) + ((csp ^ neg) - neg));
-    *c = (int64_t)((a.c >> 1) - (mulhi(a.c, cm) >> 16) - ((ssp ^ neg) - neg));
-    *quadrant = (int)(j >> 8) & 3;
+    // sin = phi - phi phi^2 (1/6 - phi^2/120); the product with 58 bits
+    const uint32_t sg = hi32x32(pp, 2863311531u - hi32x32(pp, 2185u));    // 34, 50
+    const uint64_t sn = ph - ((uint64_t)hi32x32(phh, sg) << 6);           // 64
+    // cos = 1 - phi^2/2 + phi^4 (1/24 - phi^2/720), less one unit: below 2^64
+    const uint32_t f = hi32x32(pp, hi32x32(pp, 178956971u - hi32x32(pp, 91u)));  // 32, 48, 64
+    return {t.ang[(int)(k >> 41) & 511], sn, f + ~(p >> 17)};
+}
+
+// sin and cos of the angle less its quarter turns, both >= 0, 63 bits.
+BSG_SW_FN void sincos_quadrant(const Turn& r, uint64_t* s, uint64_t* c) {
+    *s = mulhi(r.a.s, r.cs) + mulhi(r.a.c, r.sn);
+    *c = mulhi(r.a.c, r.cs) - mulhi(r.a.s, r.sn);
 }
 
 // cos and sin of 2 pi u with 62 fraction bits.
 BSG_SW_FN void sincos_2pi_fixed(const Tables& t, uint64_t k, int64_t* s, int64_t* c) {
-    int q;
-    int64_t s1, c1;
-    sincos_quadrant(t, k, &q, &s1, &c1);
-    const int64_t ss = (q & 1) ? c1 : s1, cc = (q & 1) ? s1 : c1;
+    uint64_t s1, c1;
+    sincos_quadrant(turn_of(t, k), &s1, &c1);
+    const int q = (int)(k >> 50);
+    const int64_t ss = (int64_t)(((q & 1) ? c1 : s1) >> 1), cc = (int64_t)(((q & 1) ? s1 : c1) >> 1);
     *s = (q & 2) ? -ss : ss;
     *c = ((q + 1) & 2) ? -cc : cc;
 }
 
-// A 62-bit fixed-point value of magnitude at most 1 as a double.
+// A fixed-point value as a double.
 BSG_SW_FN double fixed_to_double(int64_t a, int bits) {
     if (a == 0) return 0.0;
     const uint64_t neg = (uint64_t)(a >> 63), m = ((uint64_t)a ^ neg) - neg;
@@ -238,25 +258,30 @@ BSG_SW_FN void sincos_2pi_unit(const Tables& t, uint64_t k, double* s, double* c
     *c = fixed_to_double(cf, 62);
 }
 
-// r f, f in [-1, 1] with 62 fraction bits, as a fixed-point variate of 58
-// fraction bits (|z| < 8.6).
+// Normal variates with 58 fraction bits (|z| < 8.6) from four random words:
+// u1 from (w0, w1), u2 from (w2, w3).  Negative ones are complemented, not
+// negated: one unit of 2^-58 off.  With BOTH false *z1 is not computed.
 constexpr int kZBits = 58;
-BSG_SW_FN int64_t times_root(Root r, int64_t f) {
-    const uint64_t neg = (uint64_t)(f >> 63), m = ((uint64_t)f ^ neg) - neg;
-    const uint64_t z = mulhi(r.s << 1, m << 1) >> (4 - r.e);  // 62 + e bits before the shift, e <= 4
-    return (int64_t)((z ^ neg) - neg);
-}
 
-// Normal variates z0, z1 (58 fraction bits) from four random words: u1 from
-// (w0, w1), u2 from (w2, w3).  With BOTH false z1 is not computed.
 template <bool BOTH>
 BSG_SW_FN void normal_pair_fixed(const Tables& t, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3,
                                  int64_t* z0, int64_t* z1) {
     const Root r = sqrt_scaled(t, neg2_ln_scaled(t, unit_bits(w0, w1)));
-    int64_t s, c;
-    sincos_2pi_fixed(t, unit_bits(w2, w3), &s, &c);
-    *z0 = times_root(r, c);
-    if (BOTH) *z1 = times_root(r, s);
+    const Turn u = turn_of(t, unit_bits(w2, w3));
+    const uint64_t r59 = (r.s << 1) >> (4 - r.e);        // e <= 4
+    const bool odd = (w2 >> 30) & 1, upper = (w2 >> 31) & 1;
+    const uint64_t m0 = 0ull - (uint64_t)(odd != upper), m1 = 0ull - (uint64_t)upper;
+    uint64_t f0;                                         // |cos|: 59 + 63 - 64 bits times r
+    if (BOTH) {
+        uint64_t s, c;
+        sincos_quadrant(u, &s, &c);
+        f0 = odd ? s : c;
+        *z1 = (int64_t)(mulhi(r59, odd ? c : s) ^ m1);
+    } else {
+        const uint64_t x = mulhi(odd ? u.a.s : u.a.c, u.cs), y = mulhi(odd ? u.a.c : u.a.s, u.sn);
+        f0 = odd ? x + y : x - y;
+    }
+    *z0 = (int64_t)(mulhi(r59, f0) ^ m0);
 }
 
 // The same as doubles.
@@ -268,18 +293,23 @@ BSG_SW_FN void normal_pair(const Tables& t, uint32_t w0, uint32_t w1, uint32_t w
     *z1 = fixed_to_double(b, kZBits);
 }
 
+// 2^(f 2^-57) for the fraction of f 2^-57 alone: [1, 2), 63 fraction bits.
+template <typename T>
+BSG_SW_FN uint64_t exp2_fraction(const T& t, uint64_t f) {
+    const uint64_t tt = mulhi(f << 17, BSG_SW_LN2_54);   // t = r ln 2, r < 2^-10 (74 bits): 64
+    const uint32_t th = (uint32_t)(tt >> 22);            // 42
+    const uint64_t t2 = wide(th, th) + ((uint64_t)hi32x32(th, (uint32_t)tt << 10) << 1);  // t^2, 84
+    // t^3 (1/6 + t/24): 34, 44, then 52 + 44 - 32 = 64
+    const uint32_t t3 = hi32x32(hi32(t2), hi32x32(th, 2863311531u + hi32x32(th, 699051u)));
+    const uint64_t e = t.e2[(int)(f >> 47) & 1023];
+    return e + mulhi(e, tt + (t2 >> 21) + t3);
+}
+
 // 2^(x 2^-57), |x 2^-57| < 64, as a double.
 constexpr int kXBits = 57;
-BSG_SW_FN double exp2_fixed(const Tables& t, int64_t x) {
-    const uint64_t a = ((uint64_t)x & ((1ull << 47) - 1)) << 17;      // r < 2^-10, 74 fraction bits
-    const uint64_t tt = mulhi(a, BSG_SW_LN2_64);                      // t = r ln 2, 74
-    const uint32_t th = hi32(tt);                                     // 42
-    const uint64_t t2 = wide(th, th) + ((uint64_t)hi32x32(th, (uint32_t)tt) << 1);  // t^2, 84
-    const uint32_t g = 2863311531u + hi32x32(th, 699051u);            // 1/6 + t/24, 34
-    const uint64_t t3g = wide(hi32(t2), hi32x32(th, g));              // t^3 g, 52 + 44 = 96
-    const uint64_t p = tt + (t2 >> 11) + (t3g >> 22);                 // e^t - 1, 74
-    const uint64_t e = t.e2[(x >> 47) & 1023];                        // 63
-    const uint64_t y = e + (mulhi(e, p) >> 10);                       // [1, 2), 63
+template <typename T>
+BSG_SW_FN double exp2_fixed(const T& t, int64_t x) {
+    const uint64_t y = exp2_fraction(t, (uint64_t)x);
     return from_bits((y >> 11) + ((y >> 10) & 1) + ((uint64_t)(1022 + (x >> kXBits)) << 52));
 }
 

@@ -93,10 +93,10 @@ def main():
     w("// Tables of the fixed-point Box-Muller transform, 2^x and exp in bsg_swmath.h.")
     w("#pragma once")
     w("")
-    w("// fixed-point constants: 2 ln 2 (57 fraction bits), 2 pi (61), ln 2 (64)")
+    w("// fixed-point constants: 2 ln 2 (57 fraction bits), 2 pi (53), ln 2 (54)")
     w(f"#define BSG_SW_2LN2_57 {hexu(2 * ln2, 57)}")
-    w(f"#define BSG_SW_2PI_61 {hexu(2 * PI, 61)}")
-    w(f"#define BSG_SW_LN2_64 {hexu(ln2, 64)}")
+    w(f"#define BSG_SW_2PI_53 {hexu(2 * PI, 53)}")
+    w(f"#define BSG_SW_LN2_54 {hexu(ln2, 54)}")
     w("")
     w("// {2 ln c (62 fraction bits), c (20)}, c the reciprocal of the middle of")
     w("// interval i of [1, 2), i = 0..511; 2 ln(2 c) from i = 256 on; c = 1/2 for the last")
@@ -106,24 +106,30 @@ def main():
         v = 2 * (D(c) / D(2) ** 20 * (2 if i >= 256 else 1)).ln()
         w(f"    {{{fixed(v, 62)}ll, {c}u}}" + (", \\" if i < 511 else ""))
     w("")
-    w("// {a, b} (30 fraction bits), i = 64..255: a - b d is at or below 1/sqrt(y)")
-    w("// for y = (i + d)/256, d in [0, 1)")
+    w("// {a, b, c} (30 fraction bits), i = 128..511: a - d (b - c d) is at or")
+    w("// below 1/sqrt(y) for y = (i + d)/512, d in [0, 1)")
     w("#define BSG_SW_RSQRT_TABLE \\")
-    for i in range(64, 256):
-        # the line parallel to the chord that touches the (convex) curve from below
-        y0, y1 = D(i) / 256, D(i + 1) / 256
-        f0, f1 = 1 / y0.sqrt(), 1 / y1.sqrt()
-        slope = (f1 - f0) / (y1 - y0)
-        yt = (-2 * slope) ** (D(-2) / D(3))  # f'(yt) = slope
-        a = 1 / yt.sqrt() + slope * (y0 - yt)
-        fa, fb = int(a * 2 ** 30) - 2, fixed(f0 - f1, 30) + 1  # both towards the low side
-        w(f"    {{{fa}u, {fb}u}}" + (", \\" if i < 255 else ""))
+    for i in range(128, 512):
+        # the parabola through the curve at the three Chebyshev points, moved
+        # down by its largest error (three 30-bit units for the roundings)
+        y0, h = D(i) / 512, D(1) / 512
+        f = lambda d: 1 / (y0 + h * d).sqrt()  # noqa: E731
+        c3 = D(3).sqrt() / 4
+        x = [D("0.5") - c3, D("0.5"), D("0.5") + c3]
+        f0, f1, f2 = (f(v) for v in x)
+        d01, d12 = (f1 - f0) / (x[1] - x[0]), (f2 - f1) / (x[2] - x[1])
+        q = (d12 - d01) / (x[2] - x[0])
+        lin = d01 - q * (x[0] + x[1])
+        con = f0 - x[0] * d01 + q * x[0] * x[1]
+        over = max(con + lin * D(k) / 64 + q * (D(k) / 64) ** 2 - f(D(k) / 64) for k in range(65))
+        a = int((con - over) * 2 ** 30) - 3
+        w(f"    {{{a}u, {fixed(-lin, 30)}u, {fixed(q, 30)}u, 0u}}" + (", \\" if i < 511 else ""))
     w("")
-    w("// {sin, cos}(2 pi j / 1024) (63 fraction bits), j = 0..255")
+    w("// {sin, cos}(2 pi j / 2048) (63 fraction bits), j = 0..511")
     w("#define BSG_SW_ANGLE_TABLE \\")
-    for j in range(256):
-        sj, cj = sin_cos(2 * PI * D(j) / D(1024))
-        w(f"    {{{hexu(sj, 63)}, {hexu(cj, 63)}}}" + (", \\" if j < 255 else ""))
+    for j in range(512):
+        sj, cj = sin_cos(2 * PI * D(j) / D(2048))
+        w(f"    {{{hexu(sj, 63)}, {hexu(cj, 63)}}}" + (", \\" if j < 511 else ""))
     w("")
     w("// 2^(j/1024) (63 fraction bits), j = 0..1023")
     w("#define BSG_SW_EXP2_TABLE \\")

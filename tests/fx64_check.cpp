@@ -16,6 +16,7 @@
 namespace {
 
 const bsg_sw::Tables kT = BSG_SW_TABLES;
+const bsg_fx::TailTable kTails = BSG_FX_TAILS;
 
 template <typename F>
 F upper_tail(F x) {  // the reference's polynomial, blackscholes.simd.c:134-216
@@ -83,7 +84,7 @@ int main(int argc, char** argv) {
                                bsg_sw::to_bits(v), bsg_sw::to_bits(t)};
         double f;
         if (!bsg_fx::fx64_domain(b[0], b[1], b[2], b[3], b[4]) ||
-            !bsg_fx::price_fx64(kT, b[0], b[1], b[2], b[3], b[4], put, &f)) {
+            !bsg_fx::price_fx64(kT, kTails, b[0], b[1], b[2], b[3], b[4], put, &f)) {
             ++left;
             continue;
         }

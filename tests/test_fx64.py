@@ -38,6 +38,18 @@ def test_no_further_off_than_doubles(checker, dist, left_at_most):
         assert test <= 1.0, r.stdout
 
 
+def test_table_header_is_what_the_generator_writes(tmp_path):
+    """bsg_fx64_tables.h is generated: regenerating it changes nothing."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("gen_fx64", os.path.join(CSRC, "gen_fx64_tables.py"))
+    gen = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(gen)
+    gen.HERE = str(tmp_path)
+    gen.main()
+    with open(os.path.join(CSRC, "bsg_fx64_tables.h")) as a, open(tmp_path / "bsg_fx64_tables.h") as b:
+        assert a.read() == b.read()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 255, 257, 152 * 3 * 256 + 1, 400_003])
 def test_domain_ends_on_the_gpu(gpu_ctx, oracle_lib, n):
