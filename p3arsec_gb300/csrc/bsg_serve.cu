@@ -75,7 +75,8 @@ struct Desc {
     float* out;
     uint64_t off;  // pool offset in options
     uint64_t n;
-    uint64_t vec;  // 1: every host array 16-byte aligned (float4 transfers)
+    uint64_t vec;  // 1 + h: every host array is 16-byte aligned h options on
+                   // (float4 transfers from there); 0: they differ
 };
 
 __device__ __forceinline__ int find_segment(const uint64_t* pre, int m, uint64_t tile) {
@@ -106,7 +107,7 @@ __global__ void __launch_bounds__(kThreads) ingest_kernel(const Desc* __restrict
         const uint64_t e = (b + kTile < q.n) ? b + kTile : q.n;
         // float4 body when the host arrays allow it (pool offsets are 64-
         // option aligned and b is a multiple of 4), scalar rest
-        const uint64_t e4 = q.vec ? b + ((e - b) & ~3ull) : b;
+        const uint64_t e4 = q.vec == 1 ? b + ((e - b) & ~3ull) : b;
         for (uint64_t g = b / 4 + threadIdx.x; g < e4 / 4; g += kThreads) {
             const uint64_t o = q.off / 4 + g;
             reinterpret_cast<float4*>(ps)[o] = reinterpret_cast<const float4*>(q.src[0])[g];
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(kThreads) egress_kernel(const Desc* __restrict
         const Desc q = d[sh_q];
         const uint64_t b = (tile - pre[sh_q]) * kTile;
         const uint64_t e = (b + kTile < q.n) ? b + kTile : q.n;
-        const uint64_t e4 = q.vec ? b + ((e - b) & ~3ull) : b;
+        const uint64_t e4 = q.vec == 1 ? b + ((e - b) & ~3ull) : b;
         for (uint64_t g = b / 4 + threadIdx.x; g < e4 / 4; g += kThreads)
             reinterpret_cast<float4*>(q.out)[g] = reinterpret_cast<const float4*>(pool_out)[q.off / 4 + g];
         for (uint64_t i = e4 + threadIdx.x; i < e; i += kThreads) q.out[i] = pool_out[q.off + i];
@@ -149,45 +150,58 @@ __global__ void __launch_bounds__(kThreads) egress_kernel(const Desc* __restrict
     }
 }
 
-// Prices options [b, min(b + kTile, n)) of request q: inputs read from the
-// request's (host) arrays, prices written to its (host) output.  A thread
-// issues the loads of both of its 4-option groups of a full tile before
+// Prices the tile of request q that starts at option b (a multiple of kTile):
+// inputs read from the request's (host) arrays, prices written to its (host)
+// output.  A request whose arrays are all h < 4 options past a 16-byte boundary
+// (a slice of a book) has its tiles start at that boundary, the first with the
+// h options before it: scalar loads would fetch a fifth sector over the link
+// for every four (64 requests of a burst, sliced anywhere: 842 us, 885).  A
+// thread issues the loads of both of its 4-option groups of a full tile before
 // pricing either, so a block keeps 12 requests per thread in flight.
 template <int M>
 __device__ __forceinline__ void price_request_tile(const Desc& q, uint64_t b) {
     static_assert(kTile == 8 * kThreads, "two 4-option groups per thread per tile");
-    const uint64_t e = (b + kTile < q.n) ? b + kTile : q.n;
+    const uint64_t h = q.vec ? (q.vec - 1 < q.n ? q.vec - 1 : q.n) : 0;
+    const float* const src[5] = {q.src[0] + h, q.src[1] + h, q.src[2] + h, q.src[3] + h, q.src[4] + h};
+    const int32_t* const ot = q.ot + h;
+    float* const out = q.out + h;
+    const uint64_t n = q.n - h;  // from the boundary on
+    if (b == 0 && threadIdx.x < h) {
+        const uint64_t i = threadIdx.x;
+        q.out[i] = bsg::price<M>(q.src[0][i], q.src[1][i], q.src[2][i], q.src[3][i], q.src[4][i], q.ot[i]);
+    }
+    const uint64_t e = (b + kTile < n) ? b + kTile : n;
+    if (b >= e) return;
     const uint64_t e4 = q.vec ? b + ((e - b) & ~3ull) : b;
     if (e4 - b == kTile) {  // a full vector tile: both groups' loads first
         const uint64_t g0 = b / 4 + threadIdx.x, g1 = g0 + kThreads;
-        const float4 S0 = reinterpret_cast<const float4*>(q.src[0])[g0];
-        const float4 K0 = reinterpret_cast<const float4*>(q.src[1])[g0];
-        const float4 R0 = reinterpret_cast<const float4*>(q.src[2])[g0];
-        const float4 V0 = reinterpret_cast<const float4*>(q.src[3])[g0];
-        const float4 T0 = reinterpret_cast<const float4*>(q.src[4])[g0];
-        const int4 O0 = reinterpret_cast<const int4*>(q.ot)[g0];
-        const float4 S1 = reinterpret_cast<const float4*>(q.src[0])[g1];
-        const float4 K1 = reinterpret_cast<const float4*>(q.src[1])[g1];
-        const float4 R1 = reinterpret_cast<const float4*>(q.src[2])[g1];
-        const float4 V1 = reinterpret_cast<const float4*>(q.src[3])[g1];
-        const float4 T1 = reinterpret_cast<const float4*>(q.src[4])[g1];
-        const int4 O1 = reinterpret_cast<const int4*>(q.ot)[g1];
-        reinterpret_cast<float4*>(q.out)[g0] = bsg::price4<M>(S0, K0, R0, V0, T0, O0);
-        reinterpret_cast<float4*>(q.out)[g1] = bsg::price4<M>(S1, K1, R1, V1, T1, O1);
+        const float4 S0 = reinterpret_cast<const float4*>(src[0])[g0];
+        const float4 K0 = reinterpret_cast<const float4*>(src[1])[g0];
+        const float4 R0 = reinterpret_cast<const float4*>(src[2])[g0];
+        const float4 V0 = reinterpret_cast<const float4*>(src[3])[g0];
+        const float4 T0 = reinterpret_cast<const float4*>(src[4])[g0];
+        const int4 O0 = reinterpret_cast<const int4*>(ot)[g0];
+        const float4 S1 = reinterpret_cast<const float4*>(src[0])[g1];
+        const float4 K1 = reinterpret_cast<const float4*>(src[1])[g1];
+        const float4 R1 = reinterpret_cast<const float4*>(src[2])[g1];
+        const float4 V1 = reinterpret_cast<const float4*>(src[3])[g1];
+        const float4 T1 = reinterpret_cast<const float4*>(src[4])[g1];
+        const int4 O1 = reinterpret_cast<const int4*>(ot)[g1];
+        reinterpret_cast<float4*>(out)[g0] = bsg::price4<M>(S0, K0, R0, V0, T0, O0);
+        reinterpret_cast<float4*>(out)[g1] = bsg::price4<M>(S1, K1, R1, V1, T1, O1);
         return;
     }
     for (uint64_t g = b / 4 + threadIdx.x; g < e4 / 4; g += kThreads) {
-        const float4 S = reinterpret_cast<const float4*>(q.src[0])[g];
-        const float4 K = reinterpret_cast<const float4*>(q.src[1])[g];
-        const float4 R = reinterpret_cast<const float4*>(q.src[2])[g];
-        const float4 V = reinterpret_cast<const float4*>(q.src[3])[g];
-        const float4 T = reinterpret_cast<const float4*>(q.src[4])[g];
-        const int4 O = reinterpret_cast<const int4*>(q.ot)[g];
-        reinterpret_cast<float4*>(q.out)[g] = bsg::price4<M>(S, K, R, V, T, O);
+        const float4 S = reinterpret_cast<const float4*>(src[0])[g];
+        const float4 K = reinterpret_cast<const float4*>(src[1])[g];
+        const float4 R = reinterpret_cast<const float4*>(src[2])[g];
+        const float4 V = reinterpret_cast<const float4*>(src[3])[g];
+        const float4 T = reinterpret_cast<const float4*>(src[4])[g];
+        const int4 O = reinterpret_cast<const int4*>(ot)[g];
+        reinterpret_cast<float4*>(out)[g] = bsg::price4<M>(S, K, R, V, T, O);
     }
     for (uint64_t i = e4 + threadIdx.x; i < e; i += kThreads)
-        q.out[i] = bsg::price<M>(q.src[0][i], q.src[1][i], q.src[2][i], q.src[3][i],
-                                 q.src[4][i], q.ot[i]);
+        out[i] = bsg::price<M>(src[0][i], src[1][i], src[2][i], src[3][i], src[4][i], ot[i]);
 }
 
 // Fused path: one kernel per batch reads each request's inputs from host
@@ -1169,7 +1183,7 @@ int submit_impl(bsg_server* s, const bsg_request* r, uint64_t* id, bool auto_rel
     q->lat_slot = lat_slot;
     std::lock_guard<std::mutex> lk(s->mu);
     if (!s->cfg.plain && r->n) {
-        bool vec = true;
+        uint64_t vec = ~0ull;  // 1 + h of the first array; 0 once another differs
         const size_t b = r->n * 4;
         const void* arrs[7] = {r->sptprice, r->strike, r->rate, r->volatility,
                                r->otime, r->otype, r->prices};
@@ -1180,12 +1194,13 @@ int submit_impl(bsg_server* s, const bsg_request* r, uint64_t* id, bool auto_rel
                 return BSG_ERR_INVALID_ARG;  // not inside registered host memory
             }
             const uintptr_t dev = reinterpret_cast<uintptr_t>(arrs[j]) + h->delta;
-            if ((dev & 15) != 0) vec = false;
+            const uint64_t v = (dev & 3) ? 0 : 1 + ((16 - (dev & 15)) & 15) / 4;
+            vec = (j == 0 || vec == v) ? v : 0;
             if (j < 5) q->desc.src[j] = reinterpret_cast<const float*>(dev);
             else if (j == 5) q->desc.ot = reinterpret_cast<const int32_t*>(dev);
             else q->desc.out = reinterpret_cast<float*>(dev);
         }
-        q->desc.vec = vec ? 1 : 0;
+        q->desc.vec = vec;
     }
     if (s->stop || s->broken) {
         delete q;
