@@ -74,7 +74,7 @@ size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Host calls of up to this many options go through the context's pinned
 // staging: the host copies the six arrays there, the kernel reads them over the
-// host link and writes the prices back there.  A call of 16 options: 14 us
+// host link and writes the prices back there.  A call of 16 options: 12 us
 // against 31 with six copies in, a launch and a copy out; 8,192: 22 against 50;
 // 32,768 would take 51 (0.8 MB at the host's 20 GB/s), 22 in place.
 constexpr size_t kStageOptions = 8192;
@@ -139,8 +139,12 @@ struct bsg_ctx {
     bool pipelined = false;  // pipelined work may be in flight
     bool host_tables = false;  // the GPU reads pageable memory through the process's page tables
     // pinned memory for the arrays of short host calls (kStageOptions); used
-    // only inside a synchronous call
+    // only inside a synchronous call.  After it, the word that a kernel stores
+    // the call's number to when it is done, and the kernel's counter of parts.
     char* h_stage = nullptr;
+    unsigned* h_flag = nullptr;
+    unsigned* d_parts = nullptr;
+    unsigned call = 0;
     // debug guards (BSG_DEBUG set at bsg_create): every resident array is
     // followed by at least kGuardWords words of kGuardByte, checked after
     // each synchronous call; d_guard holds the check's {count, first index}
@@ -500,6 +504,19 @@ int ensure_pipeline(bsg_ctx* c) {
     return BSG_OK;
 }
 
+// Waits for the kernel of this call (number c->call) to store that number to
+// *h_flag: by polling the word, which sees it 2 us before the driver's stream
+// synchronisation would return, and after 2 ms by that (which also returns
+// the error of a kernel that failed).
+cudaError_t wait_flag(bsg_ctx* c) {
+    const auto t0 = std::chrono::steady_clock::now();
+    for (unsigned i = 1;; ++i) {
+        if (__atomic_load_n(c->h_flag, __ATOMIC_ACQUIRE) == c->call) return cudaSuccess;
+        if ((i & 1023) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(2))
+            return cudaStreamSynchronize(c->stream);
+    }
+}
+
 // The device's addresses of a host book whose seven arrays each lie inside
 // one pinned allocation or registration, and whose prices overlap no input;
 // false otherwise.
@@ -752,12 +769,17 @@ int bsg_create(bsg_ctx** out, int device, size_t max_options) {
             if (cudaMalloc(&c->d_guard, 16) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
             if (cudaMemsetAsync(c->dev_buf, kGuardByte, 7 * c->cap_al * sizeof(float), c->stream) != cudaSuccess) { rc = BSG_ERR_CUDA; break; }
         }
-        if (cudaMallocHost(&c->h_stage, kStageBytes) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
-        // the small device scratch in one allocation: work counters, error accumulators, edges
+        if (cudaMallocHost(&c->h_stage, kStageBytes + 64) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
+        c->h_flag = reinterpret_cast<unsigned*>(c->h_stage + kStageBytes);
+        *c->h_flag = 0;
+        // the small device scratch in one allocation: work counters (and one for
+        // kernels' parts), error accumulators, edges
         c->cursor_cap = 128;
-        const size_t cur_b = c->cursor_cap * 8, acc_b = sizeof(bsg::ErrAcc) * bsg::kMaxErrBuckets;
+        const size_t cur_b = c->cursor_cap * 8 + 64, acc_b = sizeof(bsg::ErrAcc) * bsg::kMaxErrBuckets;
         if (cudaMalloc(&c->d_small, cur_b + acc_b + sizeof(double) * (bsg::kMaxErrBuckets + 1)) != cudaSuccess) { rc = BSG_ERR_OUT_OF_MEMORY; break; }
+        if (cudaMemsetAsync(c->d_small, 0, cur_b, c->stream) != cudaSuccess) { rc = BSG_ERR_CUDA; break; }
         c->d_cursor = reinterpret_cast<unsigned long long*>(c->d_small);
+        c->d_parts = reinterpret_cast<unsigned*>(c->d_small + c->cursor_cap * 8);
         c->d_acc = reinterpret_cast<bsg::ErrAcc*>(c->d_small + cur_b);
         c->d_edges = reinterpret_cast<double*>(c->d_small + cur_b + acc_b);
         const int bps = bsg::batch_blocks_per_sm();
@@ -860,7 +882,14 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
             for (int i = 0; i < 6; ++i) std::memcpy(f + i * al, in[i], b);
             const bsg::SoA h{f, f + al, f + 2 * al, f + 3 * al, f + 4 * al,
                              reinterpret_cast<const int32_t*>(f + 5 * al), f + 6 * al};
-            if ((st = price_in_place(c, h, n, num_runs, mode, flags))) return st;
+            if (num_runs == 1) {
+                cudaError_t e = bsg::launch_map_stage(h, (int)n, mode, c->d_parts, c->h_flag, ++c->call, c->stream);
+                if (e != cudaSuccess) return cuda_fail(c, e, "launch_map_stage");
+                c->launches++;
+                BSG_CK(c, wait_flag(c));
+            } else if ((st = price_in_place(c, h, n, num_runs, mode, flags))) {
+                return st;
+            }
             std::memcpy(prices, h.out, b);
             return BSG_OK;
         }
@@ -1521,11 +1550,11 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
         if (!words.empty()) std::memcpy(tab + n * head_words, words.data(), words.size() * 8);
         if (!inl) BSG_CK(c, cudaMemcpyAsync(d_tab, tab, tab_words * 8, cudaMemcpyHostToDevice, c->stream));
         cudaError_t e = bsg::launch_swaptions(in, d_tab, (int)n, large, trials, c->d_sw + done_b + tab_b,
-                                              reinterpret_cast<unsigned*>(c->d_sw), out, c->sm_count,
-                                              c->stream);
+                                              reinterpret_cast<unsigned*>(c->d_sw), out, c->d_parts,
+                                              c->h_flag, ++c->call, c->sm_count, c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "launch_swaptions");
         c->launches++;
-        BSG_CK(c, cudaStreamSynchronize(c->stream));
+        BSG_CK(c, wait_flag(c));
         for (size_t i = 0; i < n; ++i) {
             price[i] = out[2 * i];
             if (std_err) std_err[i] = out[2 * i + 1];

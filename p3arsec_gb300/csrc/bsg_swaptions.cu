@@ -213,7 +213,7 @@ template <bool LARGE>
 __global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 4) swaption_paths_kernel(
     const __grid_constant__ SwInline in, const uint64_t* __restrict__ table, int nsw, uint64_t trials,
     int per_thread, uint64_t chunks, unsigned span, double2* __restrict__ partial,
-    unsigned* __restrict__ done, double* __restrict__ out) {
+    unsigned* __restrict__ done, double* __restrict__ out, unsigned* count, unsigned* flag, unsigned seq) {
     __shared__ SwShared<LARGE> sh;
     load_tables(sh.nt);
     const uint64_t spans = (chunks + span - 1) / span, items = spans * (uint64_t)nsw;
@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 4) swaption_paths_kern
             out[2 * sw] = s1 / m;
             out[2 * sw + 1] = sqrt((s2 - s1 * s1 / m) / (m - 1.0)) / sqrt(m);
             done[sw] = 0;  // ready for the next call
+            signal_host(count, (unsigned)nsw, flag, seq);
         }
     }
 }
@@ -321,8 +322,8 @@ size_t swaption_partial_bytes(int nsw, uint64_t trials) {
 }
 
 cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw, bool large,
-                             uint64_t trials, void* partial, unsigned* done, double* out, int sm_count,
-                             cudaStream_t st) {
+                             uint64_t trials, void* partial, unsigned* done, double* out, unsigned* count,
+                             unsigned* flag, unsigned seq, int sm_count, cudaStream_t st) {
     if (nsw <= 0 || trials < 2) return cudaErrorInvalidValue;
     const uint64_t chunks = swaption_chunks(trials), items = chunks * (uint64_t)nsw;
     const uint64_t room = (uint64_t)sm_count * (large ? 2 : 4);
@@ -334,10 +335,10 @@ cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw,
     double2* part = static_cast<double2*>(partial);
     if (large)
         swaption_paths_kernel<true><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
-                                                                 span, part, done, out);
+                                                                 span, part, done, out, count, flag, seq);
     else
         swaption_paths_kernel<false><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
-                                                                  span, part, done, out);
+                                                                  span, part, done, out, count, flag, seq);
     return cudaGetLastError();
 }
 
