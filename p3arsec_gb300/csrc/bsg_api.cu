@@ -44,7 +44,6 @@ struct GraphKey {
     bsg::MapCfg cfg;
     int kind;  // 0 plain map, 1 batch
     uint64_t ntiles;
-    int nseg;
     uint64_t btile;  // batch tile (options) and grid
     int bgrid;
     bool operator==(const GraphKey& o) const {
@@ -250,7 +249,7 @@ bool vmm_piece_rw(uintptr_t p, int device) {
 
 namespace bsg {
 
-int device_extent(const void* p, size_t bytes, int device) {
+int device_extent(const void* p, size_t bytes, int device, Range* alloc) {
     const uintptr_t want = reinterpret_cast<uintptr_t>(p) + bytes;
     if (want < reinterpret_cast<uintptr_t>(p)) return kExtentOverrun;
     MemGetAddressRangeFn range = mem_get_address_range();
@@ -271,6 +270,10 @@ int device_extent(const void* p, size_t bytes, int device) {
         if (range(&base, &size, (CUdeviceptr)cur) != CUDA_SUCCESS)
             return piece ? kExtentOverrun : kExtentUnknown;
         const uintptr_t end = (uintptr_t)base + size;
+        if (!piece && want <= end) {
+            if (alloc) *alloc = Range{(uintptr_t)base, end};
+            return kExtentOk;
+        }
         // a piece of a virtual range must itself be readable and writable
         // by the device; one cudaMalloc allocation is
         const bool vmm = attr.type == cudaMemoryTypeDevice && vmm_piece_rw(cur, device);
@@ -290,12 +293,17 @@ namespace {
 
 // Checks that [p, p + bytes) is device memory of the context's device:
 // inside one allocation, or across consecutive mapped pieces of a virtual
-// range (bsg::device_extent).
-int check_dev_range(bsg_ctx* c, const void* p, size_t bytes, const char* name) {
+// range (bsg::device_extent).  seen: the allocation that the previous array of
+// the same call was found in, which the next often shares (a look-up in the
+// driver takes 0.3 us).
+int check_dev_range(bsg_ctx* c, const void* p, size_t bytes, const char* name,
+                    bsg::Range* seen = nullptr) {
     if (!p) return fail(c, BSG_ERR_INVALID_ARG, std::string(name) + " is NULL");
     if ((reinterpret_cast<uintptr_t>(p) & 3) != 0)
         return fail(c, BSG_ERR_MISALIGNED, std::string(name) + " is not 4-byte aligned");
-    switch (bsg::device_extent(p, bytes, c->device)) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(p);
+    if (seen && x >= seen->b && x < seen->e && bytes <= seen->e - x) return BSG_OK;
+    switch (bsg::device_extent(p, bytes, c->device, seen)) {
         case bsg::kExtentOk: return BSG_OK;
         case bsg::kExtentNotDevice:
             return fail(c, BSG_ERR_INVALID_ARG, std::string(name) + " is not device memory");
@@ -313,13 +321,14 @@ int check_dev_range(bsg_ctx* c, const void* p, size_t bytes, const char* name) {
 int check_soa_dev(bsg_ctx* c, const bsg::SoA& a, size_t n, size_t out_elem) {
     const size_t b = n * 4;
     int st;
-    if ((st = check_dev_range(c, a.s, b, "sptprice"))) return st;
-    if ((st = check_dev_range(c, a.k, b, "strike"))) return st;
-    if ((st = check_dev_range(c, a.r, b, "rate"))) return st;
-    if ((st = check_dev_range(c, a.v, b, "volatility"))) return st;
-    if ((st = check_dev_range(c, a.t, b, "otime"))) return st;
-    if ((st = check_dev_range(c, a.ot, b, "otype"))) return st;
-    if (out_elem && (st = check_dev_range(c, a.out, n * out_elem, "prices"))) return st;
+    bsg::Range seen;
+    if ((st = check_dev_range(c, a.s, b, "sptprice", &seen))) return st;
+    if ((st = check_dev_range(c, a.k, b, "strike", &seen))) return st;
+    if ((st = check_dev_range(c, a.r, b, "rate", &seen))) return st;
+    if ((st = check_dev_range(c, a.v, b, "volatility", &seen))) return st;
+    if ((st = check_dev_range(c, a.t, b, "otime", &seen))) return st;
+    if ((st = check_dev_range(c, a.ot, b, "otype", &seen))) return st;
+    if (out_elem && (st = check_dev_range(c, a.out, n * out_elem, "prices", &seen))) return st;
     return BSG_OK;
 }
 
@@ -355,7 +364,7 @@ void graph_put(bsg_ctx* c, const GraphKey& k, cudaGraphExec_t exec) {
 }
 
 GraphKey make_key(const bsg::SoA& a, int64_t n, int runs, int mode,
-                  const bsg::MapCfg& cfg, int kind, uint64_t ntiles, int nseg,
+                  const bsg::MapCfg& cfg, int kind, uint64_t ntiles,
                   uint64_t btile = 0, int bgrid = 0) {
     GraphKey k;
     std::memset(static_cast<void*>(&k), 0, sizeof(k));  // padding must compare equal
@@ -366,7 +375,6 @@ GraphKey make_key(const bsg::SoA& a, int64_t n, int runs, int mode,
     k.cfg = cfg;
     k.kind = kind;
     k.ntiles = ntiles;
-    k.nseg = nseg;
     k.btile = btile;
     k.bgrid = bgrid;
     return k;
@@ -393,7 +401,7 @@ int enqueue_map_runs(bsg_ctx* c, const bsg::SoA& a, int64_t n, int runs, int mod
         }
         return BSG_OK;
     }
-    GraphKey key = make_key(a, n, runs, mode, cfg, 0, 0, 0);
+    GraphKey key = make_key(a, n, runs, mode, cfg, 0, 0);
     cudaGraphExec_t exec = graph_find(c, key);
     if (!exec) {
         cudaGraph_t g = nullptr;
@@ -657,45 +665,51 @@ int grow_tile_scratch(bsg_ctx* c, size_t ntiles) {
 }
 
 // Validates the segments and writes every tile's [begin, end) into the pinned
-// staging buffer.  Returns the counts of non-empty segments and of tiles.
+// staging buffer.  Books that follow one another in the pool without a gap
+// share tiles.
 int build_segments(bsg_ctx* c, const bsg_segment* segs, size_t nseg, size_t pool_len,
-                   uint64_t tile, int* nseg_out, uint64_t* ntiles_out) {
-    std::vector<std::pair<uint64_t, uint64_t>> v;
+                   uint64_t tile, uint64_t* ntiles_out) {
+    typedef std::pair<uint64_t, uint64_t> Span;
+    std::vector<Span> v;  // [begin, end)
     v.reserve(nseg);
+    bool ordered = true;
     for (size_t i = 0; i < nseg; ++i) {
         const uint64_t o = segs[i].offset, l = segs[i].len;
         if (o > pool_len || l > pool_len - o)
             return fail(c, BSG_ERR_INVALID_ARG, "segment " + std::to_string(i) + " lies outside the pool");
-        if (l) v.emplace_back(o, l);
-    }
-    // overlaps show between neighbours in order of offset; a pool is mostly
-    // given in that order already (sorting 4,096 books took 50 us)
-    auto overlap = [](const std::vector<std::pair<uint64_t, uint64_t>>& x) {
-        for (size_t i = 1; i < x.size(); ++i)
-            if (x[i - 1].first + x[i - 1].second > x[i].first) return true;
-        return false;
-    };
-    if (overlap(v)) {
-        std::vector<std::pair<uint64_t, uint64_t>> sorted(v);
-        std::sort(sorted.begin(), sorted.end());
-        if (overlap(sorted)) return fail(c, BSG_ERR_INVALID_ARG, "segments overlap");
-    }
-    if (v.size() > 0x7fffffff) return fail(c, BSG_ERR_INVALID_ARG, "too many segments");
-    if (c->seg_ev) BSG_CK(c, cudaEventSynchronize(c->seg_ev));  // staging reuse
-    const size_t m = v.size();
-    uint64_t acc = 0;
-    for (size_t i = 0; i < m; ++i) acc += (v[i].second + tile - 1) / tile;
-    if (int st = grow_tile_scratch(c, acc)) return st;
-    uint64_t* tb = c->h_tb;
-    for (size_t i = 0; i < m; ++i) {
-        const uint64_t e = v[i].first + v[i].second;
-        for (uint64_t b = v[i].first; b < e; b += tile, tb += 2) {
-            tb[0] = b;
-            tb[1] = (e - b > tile) ? b + tile : e;
+        if (!l) continue;
+        if (!v.empty()) {
+            if (o == v.back().second) {
+                v.back().second = o + l;
+                continue;
+            }
+            ordered = ordered && o > v.back().second;
         }
+        v.emplace_back(o, o + l);
     }
-    *nseg_out = (int)m;
-    *ntiles_out = acc;
+    if (!ordered) {
+        // overlaps show between neighbours in order of offset; a pool is mostly
+        // given in that order already (sorting 4,096 books took 50 us)
+        std::sort(v.begin(), v.end());
+        for (size_t i = 1; i < v.size(); ++i)
+            if (v[i - 1].second > v[i].first) return fail(c, BSG_ERR_INVALID_ARG, "segments overlap");
+    }
+    if (c->seg_ev) BSG_CK(c, cudaEventSynchronize(c->seg_ev));  // staging reuse
+    uint64_t total = 0;
+    if ((tile & (tile - 1)) == 0) {
+        const int sh = 63 - __builtin_clzll(tile);
+        for (const Span& x : v) total += (x.second - x.first + tile - 1) >> sh;
+    } else {
+        for (const Span& x : v) total += (x.second - x.first + tile - 1) / tile;
+    }
+    if (int st = grow_tile_scratch(c, total)) return st;
+    uint64_t* tb = c->h_tb;
+    for (const Span& x : v)
+        for (uint64_t b = x.first; b < x.second; b += tile, tb += 2) {
+            tb[0] = b;
+            tb[1] = (x.second - b > tile) ? b + tile : x.second;
+        }
+    *ntiles_out = total;
     return BSG_OK;
 }
 
@@ -991,10 +1005,11 @@ int bsg_price_soa_f64(bsg_ctx* c, const double* s, const double* k, const double
     int st;
     if (flags & BSG_DEVICE_PTRS) {
         const size_t b = n * 8;
-        if ((st = check_dev_range(c, s, b, "sptprice")) || (st = check_dev_range(c, k, b, "strike")) ||
-            (st = check_dev_range(c, r, b, "rate")) || (st = check_dev_range(c, v, b, "volatility")) ||
-            (st = check_dev_range(c, t, b, "otime")) || (st = check_dev_range(c, otype, n * 4, "otype")) ||
-            (st = check_dev_range(c, prices, b, "prices")))
+        bsg::Range seen;
+        if ((st = check_dev_range(c, s, b, "sptprice", &seen)) || (st = check_dev_range(c, k, b, "strike", &seen)) ||
+            (st = check_dev_range(c, r, b, "rate", &seen)) || (st = check_dev_range(c, v, b, "volatility", &seen)) ||
+            (st = check_dev_range(c, t, b, "otime", &seen)) || (st = check_dev_range(c, otype, n * 4, "otype", &seen)) ||
+            (st = check_dev_range(c, prices, b, "prices", &seen)))
             return st;
         const bsg::SoA64 a{s, k, r, v, t, otype, prices};
         for (int j = 0; j < num_runs; ++j) {
@@ -1057,10 +1072,9 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
         const int bps = (c->batch_bps > 0 && c->batch_bps < c->batch_blocks_per_sm)
                             ? c->batch_bps : c->batch_blocks_per_sm;
         const int grid = c->sm_count * bps;
-        int m = 0;
         uint64_t ntiles = 0;
-        if ((st = build_segments(c, segs, nseg, pool_len, topt, &m, &ntiles))) return st;
-        if (m == 0) return finish(c, flags);
+        if ((st = build_segments(c, segs, nseg, pool_len, topt, &ntiles))) return st;
+        if (ntiles == 0) return finish(c, flags);
         BSG_CK(c, cudaMemcpyAsync(c->d_tb, c->h_tb, ntiles * 16, cudaMemcpyHostToDevice, c->stream));
         BSG_CK(c, cudaEventRecord(c->seg_ev, c->stream));
         // one work counter per pass, zeroed together, so that pass j + 1 can
@@ -1079,8 +1093,8 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
         auto all_runs = [&]() -> cudaError_t {
             cudaError_t e = cudaMemsetAsync(c->d_cursor, 0, (size_t)num_runs * 8, c->stream);
             for (int j = 0; j < num_runs && e == cudaSuccess; ++j)
-                e = bsg::launch_batch(a, nullptr, nullptr, nullptr, c->d_tb, m, ntiles, topt,
-                                      c->d_cursor + j, mode, grid, j > 0 ? 1 : 0, c->stream);
+                e = bsg::launch_batch(a, c->d_tb, ntiles, c->d_cursor + j,
+                                      mode, grid, j > 0 ? 1 : 0, c->stream);
             return e;
         };
         if (num_runs == 1 || (flags & BSG_NO_GRAPH)) {
@@ -1089,7 +1103,7 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
             c->launches += (uint64_t)num_runs;
             return finish(c, flags);
         }
-        GraphKey key = make_key(a, (int64_t)pool_len, num_runs, mode, c->tune, 1, ntiles, m,
+        GraphKey key = make_key(a, (int64_t)pool_len, num_runs, mode, c->tune, 1, ntiles,
                                 topt, grid);
         cudaGraphExec_t exec = graph_find(c, key);
         if (!exec) {

@@ -121,19 +121,17 @@ cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count,
 // One pass of the FP64 product mode over n options.
 cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st);
 
-// Persistent batched pricing.  seg_off/seg_len/tile_prefix (not read where
-// tile_bounds is given) are device arrays
-// of nseg (tile_prefix: nseg + 1 entries, exclusive prefix of tiles of
-// tile_opts options per segment); tile_bounds (optional, NULL = search the
-// prefix instead) holds each tile's [begin, end) in the pool, 2 * ntiles
-// entries; cursor is a device counter that must be 0 at launch.  pdl: launch
-// with programmatic stream serialization (the next pass may start while
-// this one drains; it must use its own cursor).
-cudaError_t launch_batch(const SoA& pool, const uint64_t* seg_off,
-                         const uint64_t* seg_len, const uint64_t* tile_prefix,
-                         const uint64_t* tile_bounds, int nseg, uint64_t ntiles,
-                         uint64_t tile_opts, unsigned long long* cursor, int mode, int grid,
-                         int pdl, cudaStream_t st);
+// Persistent batched pricing over a device table of ntiles tiles, each its
+// [begin, end) in the pool.  cursor is a device counter that must be 0 at
+// launch.  pdl: launch with programmatic stream serialization (the next pass
+// may start while this one drains; it must use its own cursor).
+cudaError_t launch_batch(const SoA& pool, const uint64_t* tiles, uint64_t ntiles,
+                         unsigned long long* cursor, int mode, int grid, int pdl, cudaStream_t st);
+// The same over device arrays of nseg segments (tile_prefix: nseg + 1 entries,
+// exclusive prefix of tiles of tile_opts options per segment).
+cudaError_t launch_batch_segments(const SoA& pool, const uint64_t* seg_off, const uint64_t* seg_len,
+                                  const uint64_t* tile_prefix, int nseg, uint64_t ntiles, uint64_t tile_opts,
+                                  unsigned long long* cursor, int mode, int grid, cudaStream_t st);
 // Default options per batch tile.
 uint64_t batch_tile_options();
 // Resident blocks per SM of the batch kernel (its persistent grid = this x SMs).
@@ -166,7 +164,9 @@ enum Extent : int {
     kExtentUnknown = 3,
     kExtentOverrun = 4,
 };
-int device_extent(const void* p, size_t bytes, int device);
+// *alloc (optional): on kExtentOk within one allocation, its [begin, end).
+struct Range { uintptr_t b = 0, e = 0; };
+int device_extent(const void* p, size_t bytes, int device, Range* alloc = nullptr);
 
 // ---- swaptions (HJM Monte Carlo) -------------------------------------------
 constexpr int kSwMaxSteps = 32;    // grid points of the HJM path (iN)

@@ -118,20 +118,20 @@ __device__ __forceinline__ void price_scalar(const SoA& a, int64_t i) {
                         __ldg(a.v + i), __ldg(a.t + i), __ldg(a.ot + i));
 }
 
-// Prices vector groups [g0, g1) (group = W options) of one block's range:
-// each thread loads VPT groups (stride blockDim.x) of all six arrays, then
+// Prices vector groups [g0, g1) (group = W options) as thread `tid` of `bd`
+// that share them: each loads VPT groups (stride bd) of all six arrays, then
 // computes and stores them.  pol is the L2 policy of the hinted load paths;
 // for LP 7, groups below gres use pol_res instead.
 template <int M, int W, int VPT, int LP>
 __device__ __forceinline__ void price_groups(const SoA& a, int64_t g0, int64_t g1,
                                              unsigned long long pol,
-                                             unsigned long long pol_res, int64_t gres) {
-    const int64_t bd = blockDim.x;
+                                             unsigned long long pol_res, int64_t gres,
+                                             unsigned tid, unsigned bd) {
     for (int64_t base = g0; base < g1; base += bd * VPT) {
         Raw<W> S[VPT], K[VPT], R[VPT], V[VPT], T[VPT], O[VPT];
 #pragma unroll
         for (int j = 0; j < VPT; ++j) {
-            const int64_t g = base + threadIdx.x + j * bd;
+            const int64_t g = base + tid + (int64_t)j * bd;
             if (g < g1) {
                 const int64_t o = g * W;
                 const unsigned long long pl = (lp_resident(LP) && g < gres) ? pol_res : pol;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void price_groups(const SoA& a, int64_t g0, int64_t g
         }
 #pragma unroll
         for (int j = 0; j < VPT; ++j) {
-            const int64_t g = base + threadIdx.x + j * bd;
+            const int64_t g = base + tid + (int64_t)j * bd;
             if (g < g1) {
                 float p[W];
 #pragma unroll
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(M == MODE_LIBM_REF ? 256 : 512,
         // LP 8's odd passes take the tiles from the last to the first
         const int64_t t0 = (lp_alternating(LP) && rev ? ntiles - 1 - ti : ti) * tile;
         const int64_t t1 = (t0 + tile < ngroups) ? t0 + tile : ngroups;
-        price_groups<M, W, VPT, LP>(a, t0, t1, pol, pol_res, gres);
+        price_groups<M, W, VPT, LP>(a, t0, t1, pol, pol_res, gres, threadIdx.x, blockDim.x);
     }
     if (blockIdx.x == 0) {
         const int64_t i = ngroups * W + threadIdx.x;
@@ -970,39 +970,32 @@ constexpr uint64_t kBatchTileOptions = 8192;
 
 uint64_t batch_tile_options() { return kBatchTileOptions; }
 
-// Prices options [b, e) of the pool with the whole block: an unaligned head
-// and tail one option per thread, the aligned body in groups of W options
-// (W = 4: 16-byte loads, VPT = 2 groups per thread; W = 8: 256-bit loads,
-// one group per thread).
+// Prices options [b, e) of the pool as thread `tid` of `nt` that share them: an
+// unaligned head and tail one option per thread, the aligned body in groups of
+// W options (W = 4: 16-byte loads; W = 8: 256-bit loads).
 template <int M, int W>
-__device__ __forceinline__ void price_range(const SoA& pool, uint64_t b, uint64_t e) {
+__device__ __forceinline__ void price_range(const SoA& pool, uint64_t b, uint64_t e, unsigned tid, unsigned nt) {
     constexpr uint64_t mask = W - 1;
     const uint64_t head_end = ((b + mask) & ~mask) < e ? ((b + mask) & ~mask) : e;
     const uint64_t body_end = (e & ~mask) > head_end ? (e & ~mask) : head_end;
-    const uint64_t i_head = b + threadIdx.x;
+    const uint64_t i_head = b + tid;
     if (i_head < head_end) price_scalar<M>(pool, (int64_t)i_head);
-    if constexpr (W == 8)
-        price_groups<M, 8, 1, 2>(pool, (int64_t)(head_end / 8), (int64_t)(body_end / 8), 0ull, 0ull, 0);
-    else
-        price_groups<M, 4, kBatchVpt, 0>(pool, (int64_t)(head_end / 4), (int64_t)(body_end / 4), 0ull, 0ull, 0);
-    const uint64_t i_tail = body_end + threadIdx.x;
+    price_groups<M, W, W == 8 ? 1 : kBatchVpt, W == 8 ? 2 : 0>(
+        pool, (int64_t)(head_end / W), (int64_t)(body_end / W), 0ull, 0ull, 0, tid, nt);
+    const uint64_t i_tail = body_end + tid;
     if (i_tail < e) price_scalar<M>(pool, (int64_t)i_tail);
 }
 
-// Persistent kernel: each block takes the next tile from the device work
-// counter and prices it.  With a per-tile bounds table (tile_bounds[2 t],
-// [2 t + 1] = the tile's [b, e) in the pool) a tile costs thread 0 one load;
-// without it, a binary search over the tile prefix finds its segment.  The
-// claim of the next tile is issued before the current one is priced, so the
-// counter's round trip overlaps the pricing.  No block ever waits on another;
-// the loop ends when the counter passes the last tile.  (Four blocks per SM
-// hold the registers to 64; the libm mode's float-float exp/log get up to
-// 128.)
+// Persistent kernel over a table of tiles ([b, e) in the pool, two words
+// each): each block takes the next tile from the device work counter and
+// prices it.  The claim of the next tile is issued before the current one is
+// priced, so the counter's round trip overlaps the pricing.  No block ever
+// waits on another; the loop ends when the counter passes the last tile.
+// (Four blocks per SM hold the registers to 64; the libm mode's float-float
+// exp/log get up to 128.)
 template <int M, int W>
 __global__ void __launch_bounds__(kBatchBlock, M == MODE_LIBM_REF ? 2 : 4) batch_kernel(
-    SoA pool, const uint64_t* __restrict__ seg_off, const uint64_t* __restrict__ seg_len,
-    const uint64_t* __restrict__ tile_prefix, const uint64_t* __restrict__ tile_bounds, int nseg,
-    uint64_t ntiles, uint64_t topt, unsigned long long* cursor) {
+    SoA pool, const uint64_t* __restrict__ tiles, uint64_t ntiles, unsigned long long* cursor) {
     __shared__ uint64_t sh_b, sh_e;
     __shared__ int sh_done;
     pdl_trigger();
@@ -1011,25 +1004,11 @@ __global__ void __launch_bounds__(kBatchBlock, M == MODE_LIBM_REF ? 2 : 4) batch
     for (;;) {
         if (threadIdx.x == 0) {
             const unsigned long long tile = next;
-            if (tile >= ntiles) {
-                sh_done = 1;
-            } else {
+            sh_done = tile >= ntiles;
+            if (!sh_done) {
                 next = atomicAdd(cursor, 1ull);  // travels while this tile is priced
-                if (tile_bounds) {
-                    sh_b = tile_bounds[2 * tile];
-                    sh_e = tile_bounds[2 * tile + 1];
-                } else {
-                    int lo = 0, hi = nseg - 1;
-                    while (lo < hi) {  // largest segment whose first tile <= tile
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (tile_prefix[mid] <= tile) lo = mid; else hi = mid - 1;
-                    }
-                    const uint64_t b = seg_off[lo] + (tile - tile_prefix[lo]) * topt;
-                    const uint64_t send = seg_off[lo] + seg_len[lo];
-                    sh_b = b;
-                    sh_e = (b + topt < send) ? b + topt : send;
-                }
-                sh_done = 0;
+                sh_b = tiles[2 * tile];
+                sh_e = tiles[2 * tile + 1];
             }
         }
         __syncthreads();
@@ -1037,9 +1016,47 @@ __global__ void __launch_bounds__(kBatchBlock, M == MODE_LIBM_REF ? 2 : 4) batch
         const uint64_t b = sh_b, e = sh_e;
         __syncthreads();
         if (done) break;
-        price_range<M, W>(pool, b, e);
+        price_range<M, W>(pool, b, e, threadIdx.x, kBatchBlock);
     }
     pdl_wait();
+}
+
+// The same over a table of segments (the serving loop's unfused path, whose
+// tiles have no table): thread 0 finds a tile's segment by a binary search of
+// the tile prefix.
+template <int M, int W>
+__global__ void __launch_bounds__(kBatchBlock, M == MODE_LIBM_REF ? 2 : 4) batch_segments_kernel(
+    SoA pool, const uint64_t* __restrict__ seg_off, const uint64_t* __restrict__ seg_len,
+    const uint64_t* __restrict__ tile_prefix, int nseg, uint64_t ntiles, uint64_t topt,
+    unsigned long long* cursor) {
+    __shared__ uint64_t sh_b, sh_e;
+    __shared__ int sh_done;
+    unsigned long long next = 0;
+    if (threadIdx.x == 0) next = atomicAdd(cursor, 1ull);
+    for (;;) {
+        if (threadIdx.x == 0) {
+            const unsigned long long tile = next;
+            sh_done = tile >= ntiles;
+            if (!sh_done) {
+                next = atomicAdd(cursor, 1ull);  // travels while this tile is priced
+                int lo = 0, hi = nseg - 1;
+                while (lo < hi) {  // largest segment whose first tile <= tile
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (tile_prefix[mid] <= tile) lo = mid; else hi = mid - 1;
+                }
+                const uint64_t b = seg_off[lo] + (tile - tile_prefix[lo]) * topt;
+                const uint64_t send = seg_off[lo] + seg_len[lo];
+                sh_b = b;
+                sh_e = (b + topt < send) ? b + topt : send;
+            }
+        }
+        __syncthreads();
+        const int done = sh_done;
+        const uint64_t b = sh_b, e = sh_e;
+        __syncthreads();
+        if (done) break;
+        price_range<M, W>(pool, b, e, threadIdx.x, kBatchBlock);
+    }
 }
 
 int batch_blocks_per_sm() {
@@ -1051,13 +1068,15 @@ int batch_blocks_per_sm() {
     return n > 0 ? n : 1;
 }
 
-cudaError_t launch_batch(const SoA& pool, const uint64_t* seg_off,
-                         const uint64_t* seg_len, const uint64_t* tile_prefix,
-                         const uint64_t* tile_bounds, int nseg, uint64_t ntiles,
-                         uint64_t tile_opts, unsigned long long* cursor, int mode, int grid,
-                         int pdl, cudaStream_t st) {
-    if (ntiles == 0 || nseg <= 0) return cudaSuccess;
-    if (tile_opts == 0) return cudaErrorInvalidValue;
+// 256-bit loads need every pool array 32-byte aligned; the libm mode keeps
+// 128-bit loads (fewer registers: it is compute-bound)
+static bool batch_w8(const SoA& pool, int mode) {
+    return mode != MODE_LIBM_REF && map_vectorizable(pool, MapCfg{1, kBatchBlock, 0, 2, 0});
+}
+
+cudaError_t launch_batch(const SoA& pool, const uint64_t* tiles, uint64_t ntiles,
+                         unsigned long long* cursor, int mode, int grid, int pdl, cudaStream_t st) {
+    if (ntiles == 0) return cudaSuccess;
     if ((uint64_t)grid > ntiles) grid = (int)ntiles;  // no block without a tile
     if (grid < 1) grid = 1;
     cudaLaunchConfig_t lc = {};
@@ -1069,14 +1088,10 @@ cudaError_t launch_batch(const SoA& pool, const uint64_t* seg_off,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = pdl ? 1 : 0;
-    // 256-bit loads need every pool array 32-byte aligned; the libm mode
-    // keeps 128-bit loads (fewer registers: it is compute-bound)
-    const bool w8 = mode != MODE_LIBM_REF && map_vectorizable(pool, MapCfg{1, kBatchBlock, 0, 2, 0});
+    const bool w8 = batch_w8(pool, mode);
 #define BSG_BATCH(M_) \
-    (w8 ? cudaLaunchKernelEx(&lc, batch_kernel<M_, 8>, pool, seg_off, seg_len, tile_prefix, \
-                             tile_bounds, nseg, ntiles, tile_opts, cursor) \
-        : cudaLaunchKernelEx(&lc, batch_kernel<M_, 4>, pool, seg_off, seg_len, tile_prefix, \
-                             tile_bounds, nseg, ntiles, tile_opts, cursor))
+    (w8 ? cudaLaunchKernelEx(&lc, batch_kernel<M_, 8>, pool, tiles, ntiles, cursor) \
+        : cudaLaunchKernelEx(&lc, batch_kernel<M_, 4>, pool, tiles, ntiles, cursor))
     switch (mode) {
         case MODE_FAST: return BSG_BATCH(MODE_FAST);
         case MODE_SFU_REF: return BSG_BATCH(MODE_SFU_REF);
@@ -1084,6 +1099,31 @@ cudaError_t launch_batch(const SoA& pool, const uint64_t* seg_off,
         default: return cudaErrorInvalidValue;
     }
 #undef BSG_BATCH
+}
+
+cudaError_t launch_batch_segments(const SoA& pool, const uint64_t* seg_off, const uint64_t* seg_len,
+                                  const uint64_t* tile_prefix, int nseg, uint64_t ntiles, uint64_t tile_opts,
+                                  unsigned long long* cursor, int mode, int grid, cudaStream_t st) {
+    if (ntiles == 0 || nseg <= 0) return cudaSuccess;
+    if (tile_opts == 0) return cudaErrorInvalidValue;
+    if ((uint64_t)grid > ntiles) grid = (int)ntiles;  // no block without a tile
+    if (grid < 1) grid = 1;
+    const bool w8 = batch_w8(pool, mode);
+#define BSG_BATCH(M_) \
+    do { \
+        if (w8) batch_segments_kernel<M_, 8><<<grid, kBatchBlock, 0, st>>>(pool, seg_off, seg_len, tile_prefix, \
+                                                                          nseg, ntiles, tile_opts, cursor); \
+        else batch_segments_kernel<M_, 4><<<grid, kBatchBlock, 0, st>>>(pool, seg_off, seg_len, tile_prefix, \
+                                                                       nseg, ntiles, tile_opts, cursor); \
+    } while (0)
+    switch (mode) {
+        case MODE_FAST: BSG_BATCH(MODE_FAST); break;
+        case MODE_SFU_REF: BSG_BATCH(MODE_SFU_REF); break;
+        case MODE_LIBM_REF: BSG_BATCH(MODE_LIBM_REF); break;
+        default: return cudaErrorInvalidValue;
+    }
+#undef BSG_BATCH
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------- error report

@@ -96,6 +96,10 @@ bool host_array(PyObject* x, char fmt, size_t n, Py_buffer* b) {
 }
 
 bool whole(PyObject* x, uint64_t* out) {  // int(x), modulo 2^64 as ctypes stores it
+    if (PyLong_CheckExact(x) && PyUnstable_Long_IsCompact((PyLongObject*)x)) {
+        *out = (uint64_t)PyUnstable_Long_CompactValue((PyLongObject*)x);
+        return true;
+    }
     if (PyLong_Check(x)) {
         *out = PyLong_AsUnsignedLongLongMask(x);
         return !PyErr_Occurred();
