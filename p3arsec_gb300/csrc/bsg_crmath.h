@@ -13,7 +13,7 @@
 // exponential function in IEEE floating-point arithmetic", ACM TOMS 15(2),
 // 1989, and its logarithm counterpart, ACM TOMS 16(4), 1990), written here
 // from the mathematics: Taylor polynomials, error-free transformations
-// (Knuth's two-sum, the fma two-product), and tables of 2^(j/32) and
+// (Dekker's two-sum, the fma two-product), and tables of 2^(j/32) and
 // ln(256/k) computed exactly by gen_crmath_tables.py.
 //
 // Compiles as CUDA device code and as host C++ (compile the host side with
@@ -61,14 +61,7 @@ inline float fallback_exp(float x) { return expf(x); }
 inline float fallback_log(float x) { return logf(x); }
 #endif
 
-// a + b = s + e exactly (Knuth), any magnitudes
-BSG_CR_FN F2 two_sum(float a, float b) {
-    const float s = add(a, b);
-    const float bb = sub(s, a);
-    const float e = add(sub(a, sub(s, bb)), sub(b, bb));
-    return {s, e};
-}
-// a + b = s + e exactly when |a| >= |b| (Dekker)
+// a + b = s + e exactly when |a| >= |b|, or their exponents are equal, or a is 0 (Dekker)
 BSG_CR_FN F2 fast_two_sum(float a, float b) {
     const float s = add(a, b);
     return {s, sub(b, sub(s, a))};
@@ -110,9 +103,10 @@ constexpr uint32_t kShifterBits = 0x4B400000u;
 // e^x.  Arguments outside [-87, 88.5] (subnormal or overflowing results,
 // NaN) go to the platform's expf.
 //   x = (32 m + j) ln2/32 + r, |r| <~ ln2/64; e^x = 2^m 2^(j/32) e^r.
-//   r = x - n L1 - n L2 - n L3 as a float pair: x - n L1 is exact (L1 has
-//   12 bits, |n| < 2^12, the difference has at most 24 bits), n L2 is an
-//   exact two-product.  e^r - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120)
+//   r = x - n L1 - n L2 - n L3 as a float pair: the fma x - n L1 is exact (its
+//   last bit is at 2^-29 or x's own, and |x - n L1| < 2^-6), n L2 < 2^-21 is
+//   taken off it twice, once rounded and once for what that lost (x - n L1
+//   less the rounded result is exact).  e^r - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120)
 //   (truncation below 2^-48 for |r| <= 0.011), with r^2/2 exact.
 BSG_CR_FN float exp(float x) {
     if (!(x >= -87.0f && x <= 88.5f)) return fallback_exp(x);
@@ -120,10 +114,8 @@ BSG_CR_FN float exp(float x) {
     const float nf = sub(sh, kShifter);
     const int n = (int)(float_to_bits(sh) - kShifterBits);
     const float r1 = fma_(-nf, BSG_CR_L1, x);
-    const F2 p = two_prod(nf, BSG_CR_L2);
-    const F2 rs = two_sum(r1, -p.hi);
-    const float rh = rs.hi;
-    const float rl = fma_(-nf, BSG_CR_L3, sub(rs.lo, p.lo));
+    const float rh = fma_(-nf, BSG_CR_L2, r1);
+    const float rl = fma_(-nf, BSG_CR_L3, fma_(-nf, BSG_CR_L2, sub(r1, rh)));
     const F2 s2 = two_prod(rh, rh);
     float c = fma_(rh, 1.0f / 120.0f, 1.0f / 24.0f);
     c = fma_(rh, c, 1.0f / 6.0f);
@@ -163,9 +155,10 @@ BSG_CR_FN float log(float x) {
     const float alo = add(a.lo, fma_(s2.lo, -0.5f, c));
     const float ef = sub(bits_to_float(kShifterBits + (uint32_t)e), kShifter);  // (float)e
     const F2 em = two_prod(ef, BSG_CR_LN2M);
-    const F2 s1 = two_sum(mul(ef, BSG_CR_LN2H), tab.hi);
-    const F2 s2s = two_sum(s1.hi, a.hi);
-    const F2 s3 = two_sum(s2s.hi, em.hi);
+    // each sum's first term is 0 or no smaller (in exponent) than its second
+    const F2 s1 = fast_two_sum(mul(ef, BSG_CR_LN2H), tab.hi);
+    const F2 s2s = fast_two_sum(s1.hi, a.hi);
+    const F2 s3 = fast_two_sum(s2s.hi, em.hi);
     const float lo = add(add(add(s1.lo, s2s.lo), s3.lo),
                          add(add(tab.lo, alo), fma_(ef, BSG_CR_LN2L, em.lo)));
     return add(s3.hi, lo);

@@ -412,14 +412,12 @@ __device__ __forceinline__ float price_libm_ref(float s, float k, float r, float
 // rounds a product and then adds it: the toolchain fuses an f32x2 multiply
 // into the f32x2 add or subtract that is its only use (even from inline
 // PTX mul.rn.f32x2 / add.rn.f32x2, and under -fmad=false), which would skip
-// that rounding.
+// that rounding.  Bound by instructions issued, not by memory (20M options'
+// 28 B take 82 us): 215 us a pass with every exp's out-of-domain lanes
+// selected around and exact two-sums throughout, 192 without the selects,
+// 178 with r and the sums in the shorter exact forms.
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return add2(a, neg2(b)); }
 struct FF2 { float2 hi, lo; };
-__device__ __forceinline__ FF2 two_sum2(float2 a, float2 b) {
-    const float2 s = add2(a, b);
-    const float2 bb = sub2(s, a);
-    return {s, add2(sub2(a, sub2(s, bb)), sub2(b, bb))};
-}
 __device__ __forceinline__ FF2 fast_two_sum2(float2 a, float2 b) {
     const float2 s = add2(a, b);
     return {s, sub2(b, sub2(s, a))};
@@ -428,25 +426,19 @@ __device__ __forceinline__ FF2 two_prod2(float2 a, float2 b) {
     const float2 p = mul2(a, b);
     return {p, fma2(a, b, neg2(p))};
 }
-__device__ __forceinline__ bool cr_exp_in_range(float x) { return x >= -87.0f && x <= 88.5f; }
 __device__ __forceinline__ bool cr_log_in_range(float x) {
     return x >= 1.17549435e-38f && x <= 3.40282347e38f;
 }
 
-// A lane whose argument is outside bsg_cr::exp's domain takes the platform's
-// expf, as bsg_cr::exp does; the packed evaluation runs on 0 in its place.
-__device__ __forceinline__ float2 cr_exp2(float2 xin) {
-    const bool in0 = cr_exp_in_range(xin.x), in1 = cr_exp_in_range(xin.y);
-    const float2 x = make_float2(in0 ? xin.x : 0.0f, in1 ? xin.y : 0.0f);
+// bsg_cr::exp on two arguments inside its domain.
+__device__ __forceinline__ float2 cr_exp2_in(float2 x) {
     const float2 sh = fma2(x, f2(BSG_CR_INV_L), f2(bsg_cr::kShifter));
     const float2 nf = sub2(sh, f2(bsg_cr::kShifter));
-    const int n0 = (int)(__float_as_uint(sh.x) - bsg_cr::kShifterBits);
-    const int n1 = (int)(__float_as_uint(sh.y) - bsg_cr::kShifterBits);
+    // n in sh's low bits (kShifterBits is a multiple of 2^22)
+    const uint32_t n0 = __float_as_uint(sh.x), n1 = __float_as_uint(sh.y);
     const float2 r1 = fma2(neg2(nf), f2(BSG_CR_L1), x);
-    const FF2 p = two_prod2(nf, f2(BSG_CR_L2));
-    const FF2 rs = two_sum2(r1, neg2(p.hi));
-    const float2 rh = rs.hi;
-    const float2 rl = fma2(neg2(nf), f2(BSG_CR_L3), sub2(rs.lo, p.lo));
+    const float2 rh = fma2(neg2(nf), f2(BSG_CR_L2), r1);
+    const float2 rl = fma2(neg2(nf), f2(BSG_CR_L3), fma2(neg2(nf), f2(BSG_CR_L2), sub2(r1, rh)));
     const FF2 s2 = two_prod2(rh, rh);
     float2 c = fma2(rh, f2(1.0f / 120.0f), f2(1.0f / 24.0f));
     c = fma2(rh, c, f2(1.0f / 6.0f));
@@ -454,17 +446,27 @@ __device__ __forceinline__ float2 cr_exp2(float2 xin) {
     const FF2 q = fast_two_sum2(rh, mul2(s2.hi, f2(0.5f)));
     const float2 ql =
         add2(q.lo, add2(rl, fma2(s2.lo, f2(0.5f), fma2(rh, rl, mul2(s2.hi, c)))));
-    const bsg_cr::F2 t0 = bsg_cr::exp_tab(n0 & 31), t1 = bsg_cr::exp_tab(n1 & 31);
+    const bsg_cr::F2 t0 = bsg_cr::exp_tab((int)(n0 & 31)), t1 = bsg_cr::exp_tab((int)(n1 & 31));
     const float2 thi = make_float2(t0.hi, t1.hi), tlo = make_float2(t0.lo, t1.lo);
     const FF2 tq = two_prod2(thi, q.hi);
     const FF2 sm = fast_two_sum2(thi, tq.hi);
     const float2 lo = add2(sm.lo, add2(tq.lo, add2(tlo, fma2(thi, ql, mul2(tlo, q.hi)))));
     const float2 y = add2(sm.hi, lo);
-    float2 e = mul2(y, make_float2(__uint_as_float((uint32_t)((n0 >> 5) + 127) << 23),
-                                   __uint_as_float((uint32_t)((n1 >> 5) + 127) << 23)));
-    if (!in0) e.x = bsg_cr::fallback_exp(xin.x);
-    if (!in1) e.y = bsg_cr::fallback_exp(xin.y);
-    return e;
+    // times 2^(n >> 5), a normal result: added to the exponent
+    return make_float2(__uint_as_float(__float_as_uint(y.x) + ((n0 << 18) & 0xFF800000u)),
+                       __uint_as_float(__float_as_uint(y.y) + ((n1 << 18) & 0xFF800000u)));
+}
+
+// The larger of a and b, NaN if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+__device__ __forceinline__ float2 cr_exp2(float2 x) {
+    if (!(max_nan(fabsf(x.x), fabsf(x.y)) <= 87.0f)) return make_float2(bsg_cr::exp(x.x), bsg_cr::exp(x.y));
+    return cr_exp2_in(x);
 }
 
 __device__ __forceinline__ float2 cr_log2(float2 x) {
@@ -489,9 +491,9 @@ __device__ __forceinline__ float2 cr_log2(float2 x) {
                                        __uint_as_float(bsg_cr::kShifterBits + (uint32_t)e1)),
                            f2(bsg_cr::kShifter));
     const FF2 em = two_prod2(ef, f2(BSG_CR_LN2M));
-    const FF2 s1 = two_sum2(mul2(ef, f2(BSG_CR_LN2H)), make_float2(g0.hi, g1.hi));
-    const FF2 s2s = two_sum2(s1.hi, a.hi);
-    const FF2 s3 = two_sum2(s2s.hi, em.hi);
+    const FF2 s1 = fast_two_sum2(mul2(ef, f2(BSG_CR_LN2H)), make_float2(g0.hi, g1.hi));
+    const FF2 s2s = fast_two_sum2(s1.hi, a.hi);
+    const FF2 s3 = fast_two_sum2(s2s.hi, em.hi);
     const float2 lo = add2(add2(add2(s1.lo, s2s.lo), s3.lo),
                            add2(add2(make_float2(g0.lo, g1.lo), alo),
                                 fma2(ef, f2(BSG_CR_LN2L), em.lo)));
@@ -502,15 +504,27 @@ __device__ __forceinline__ float2 dmul_finite2(float2 x, FF c) {
     return fma2(f2(c.hi), x, mul2(f2(c.lo), x));
 }
 
+// The smaller of a and b, NaN if either is.
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 __device__ __forceinline__ float2 cndf_libm_ref2(float2 xin) {
     constexpr FF c0 = split(BSG_C0), c1 = split(BSG_C1), c2 = split(BSG_C2);
     constexpr FF c3 = split(BSG_C3), c4 = split(BSG_C4), c5 = split(BSG_C5);
     constexpr FF isp = split(BSG_INV_SQRT_2PI);
     const bool neg0 = xin.x < 0.0f, neg1 = xin.y < 0.0f;
-    const float2 x = make_float2(neg0 ? -xin.x : xin.x, neg1 ? -xin.y : xin.y);
-    const float2 e = cr_exp2(mul2(mul2(f2(-0.5f), x), x));
+    // Neither an infinite |d| nor an exponent under -87 needs a path of its
+    // own: with |d| held to 3e38 and the exponent to -87 the product l1 np is
+    // under 2^-125, and 1 less it rounds to 1 as it does with exp's own 0 or
+    // subnormal (a NaN passes through k).
+    const float2 x = make_float2(min_nan(fabsf(xin.x), 3e38f), min_nan(fabsf(xin.y), 3e38f));
+    const float2 a = mul2(mul2(f2(-0.5f), x), x);
+    const float2 e = cr_exp2_in(make_float2(fmaxf(a.x, -87.0f), fmaxf(a.y, -87.0f)));
     const float2 np = dmul_finite2(e, isp);
-    float2 k = make_float2(dmul(x.x, c0), dmul(x.y, c0));
+    float2 k = dmul_finite2(x, c0);
     k = add2(f2(1.0f), k);
     k = make_float2(__frcp_rn(k.x), __frcp_rn(k.y));
     const float2 k2 = mul2(k, k), k3 = mul2(k2, k);

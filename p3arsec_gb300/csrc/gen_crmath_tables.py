@@ -44,7 +44,7 @@ def split2(v: Fraction):
 def main():
     ln2 = Fraction(D(2).ln())
     L = ln2 / 32
-    L1 = round_bits(L, 12)       # n * L1 exact for |n| < 2^12
+    L1 = f32(L)
     L2 = f32(L - L1)
     L3 = f32(L - L1 - L2)
     inv_l = f32(1 / L)
@@ -70,7 +70,7 @@ def main():
     w("// Constants and tables of the float-float exp and log in bsg_crmath.h.")
     w("#pragma once")
     w("")
-    w("// ln2/32 = kL1 + kL2 + kL3 (kL1 has 12 significant bits), and 32/ln2")
+    w("// ln2/32 = kL1 + kL2 + kL3, and 32/ln2")
     w(f"#define BSG_CR_L1 {hexf(L1)}")
     w(f"#define BSG_CR_L2 {hexf(L2)}")
     w(f"#define BSG_CR_L3 {hexf(L3)}")
