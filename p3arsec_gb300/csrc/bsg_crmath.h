@@ -121,11 +121,11 @@ BSG_CR_FN float exp(float x) {
     c = fma_(rh, c, 1.0f / 6.0f);
     c = mul(rh, c);
     const F2 q = fast_two_sum(rh, mul(s2.hi, 0.5f));
-    const float ql = add(q.lo, add(rl, fma_(s2.lo, 0.5f, fma_(rh, rl, mul(s2.hi, c)))));
+    const float ql = add(q.lo, fma_(s2.lo, 0.5f, fma_(s2.hi, c, fma_(rh, rl, rl))));
     const F2 t = exp_tab(n & 31);
     const F2 tq = two_prod(t.hi, q.hi);
     const F2 s = fast_two_sum(t.hi, tq.hi);
-    const float lo = add(s.lo, add(tq.lo, add(t.lo, fma_(t.hi, ql, mul(t.lo, q.hi)))));
+    const float lo = add(s.lo, add(tq.lo, fma_(t.hi, ql, fma_(t.lo, q.hi, t.lo))));
     const float y = add(s.hi, lo);
     const int m = n >> 5;  // floor(n / 32): m in [-126, 127] on this domain
     return mul(y, bits_to_float((uint32_t)(m + 127) << 23));
@@ -142,10 +142,9 @@ BSG_CR_FN float exp(float x) {
 BSG_CR_FN float log(float x) {
     if (!(x >= 1.17549435e-38f && x <= 3.40282347e38f)) return fallback_log(x);
     const uint32_t u = float_to_bits(x);
-    const uint32_t i = (u >> 15) & 0xFFu;
-    const int e = (int)(u >> 23) - 127 + (int)(i >> 7);
-    const float m = bits_to_float((u & 0x7FFFFFu) | (i >= 128 ? 0x3F000000u : 0x3F800000u));
-    const LogEntry tab = log_tab((int)i);
+    const uint32_t v = u + 0x400000u;  // e + 127 from bit 23 on
+    const float m = bits_to_float(u + 0x3F800000u - (v & 0xFF800000u));
+    const LogEntry tab = log_tab((int)((u >> 15) & 0xFFu));
     const float r = fma_(m, tab.c, -1.0f);
     const F2 s2 = two_prod(r, r);
     float c = fma_(r, 0.2f, -0.25f);
@@ -153,15 +152,17 @@ BSG_CR_FN float log(float x) {
     c = mul(mul(s2.hi, r), c);
     const F2 a = fast_two_sum(r, mul(s2.hi, -0.5f));
     const float alo = add(a.lo, fma_(s2.lo, -0.5f, c));
-    const float ef = sub(bits_to_float(kShifterBits + (uint32_t)e), kShifter);  // (float)e
-    const F2 em = two_prod(ef, BSG_CR_LN2M);
-    // each sum's first term is 0 or no smaller (in exponent) than its second
-    const F2 s1 = fast_two_sum(mul(ef, BSG_CR_LN2H), tab.hi);
-    const F2 s2s = fast_two_sum(s1.hi, a.hi);
-    const F2 s3 = fast_two_sum(s2s.hi, em.hi);
-    const float lo = add(add(add(s1.lo, s2s.lo), s3.lo),
-                         add(add(tab.lo, alo), fma_(ef, BSG_CR_LN2L, em.lo)));
-    return add(s3.hi, lo);
+    const float ef = sub(bits_to_float(kShifterBits - 127u + (v >> 23)), kShifter);  // (float)e
+    // e LN2H and e LN2M are exact (within an fma too); each sum's first term
+    // is 0 or no smaller (in exponent) than its second
+    const float s1 = fma_(ef, BSG_CR_LN2H, tab.hi);
+    const float s1l = sub(tab.hi, fma_(-ef, BSG_CR_LN2H, s1));
+    const F2 s2s = fast_two_sum(s1, a.hi);
+    const float s3 = fma_(ef, BSG_CR_LN2M, s2s.hi);
+    const float s3l = fma_(ef, BSG_CR_LN2M, sub(s2s.hi, s3));
+    const float lo = add(add(add(s1l, s2s.lo), s3l),
+                         fma_(ef, BSG_CR_LN2L, add(tab.lo, alo)));
+    return add(s3, lo);
 }
 
 }  // namespace bsg_cr

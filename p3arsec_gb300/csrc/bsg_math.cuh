@@ -407,15 +407,16 @@ __device__ __forceinline__ float price_libm_ref(float s, float k, float r, float
 // Two options at a time: the operations of cndf_libm_ref / price_libm_ref
 // and of bsg_cr::exp / bsg_cr::log, each as one packed f32x2 operation
 // where the scalar code has a float operation (componentwise the same
-// rounding: the same bits), per lane where it has a division, a square
-// root, integer work or a table load -- and per lane where the reference
-// rounds a product and then adds it: the toolchain fuses an f32x2 multiply
-// into the f32x2 add or subtract that is its only use (even from inline
-// PTX mul.rn.f32x2 / add.rn.f32x2, and under -fmad=false), which would skip
-// that rounding.  Bound by instructions issued, not by memory (20M options'
-// 28 B take 82 us): 215 us a pass with every exp's out-of-domain lanes
-// selected around and exact two-sums throughout, 192 without the selects,
-// 178 with r and the sums in the shorter exact forms.
+// rounding: the same bits), per lane where it has integer work or a table
+// load -- and per lane where the reference rounds a product and then adds
+// it: the toolchain fuses an f32x2 multiply into the f32x2 add or subtract
+// that is its only use (even from inline PTX mul.rn.f32x2 / add.rn.f32x2,
+// and under -fmad=false), which would skip that rounding.  Bound by
+// instructions issued, not by memory (20M options' 28 B take 82 us): 215 us
+// a pass with every exp's out-of-domain lanes selected around and exact
+// two-sums throughout, 192 without the selects, 178 with r and the sums in
+// the shorter exact forms, 159 with the divisions, the square root and the
+// reciprocals packed too and one test of the operands' range per pair.
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return add2(a, neg2(b)); }
 struct FF2 { float2 hi, lo; };
 __device__ __forceinline__ FF2 fast_two_sum2(float2 a, float2 b) {
@@ -426,10 +427,6 @@ __device__ __forceinline__ FF2 two_prod2(float2 a, float2 b) {
     const float2 p = mul2(a, b);
     return {p, fma2(a, b, neg2(p))};
 }
-__device__ __forceinline__ bool cr_log_in_range(float x) {
-    return x >= 1.17549435e-38f && x <= 3.40282347e38f;
-}
-
 // bsg_cr::exp on two arguments inside its domain.
 __device__ __forceinline__ float2 cr_exp2_in(float2 x) {
     const float2 sh = fma2(x, f2(BSG_CR_INV_L), f2(bsg_cr::kShifter));
@@ -444,42 +441,26 @@ __device__ __forceinline__ float2 cr_exp2_in(float2 x) {
     c = fma2(rh, c, f2(1.0f / 6.0f));
     c = mul2(rh, c);
     const FF2 q = fast_two_sum2(rh, mul2(s2.hi, f2(0.5f)));
-    const float2 ql =
-        add2(q.lo, add2(rl, fma2(s2.lo, f2(0.5f), fma2(rh, rl, mul2(s2.hi, c)))));
+    const float2 ql = add2(q.lo, fma2(s2.lo, f2(0.5f), fma2(s2.hi, c, fma2(rh, rl, rl))));
     const bsg_cr::F2 t0 = bsg_cr::exp_tab((int)(n0 & 31)), t1 = bsg_cr::exp_tab((int)(n1 & 31));
     const float2 thi = make_float2(t0.hi, t1.hi), tlo = make_float2(t0.lo, t1.lo);
     const FF2 tq = two_prod2(thi, q.hi);
     const FF2 sm = fast_two_sum2(thi, tq.hi);
-    const float2 lo = add2(sm.lo, add2(tq.lo, add2(tlo, fma2(thi, ql, mul2(tlo, q.hi)))));
+    const float2 lo = add2(sm.lo, add2(tq.lo, fma2(thi, ql, fma2(tlo, q.hi, tlo))));
     const float2 y = add2(sm.hi, lo);
     // times 2^(n >> 5), a normal result: added to the exponent
     return make_float2(__uint_as_float(__float_as_uint(y.x) + ((n0 << 18) & 0xFF800000u)),
                        __uint_as_float(__float_as_uint(y.y) + ((n1 << 18) & 0xFF800000u)));
 }
 
-// The larger of a and b, NaN if either is.
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
-__device__ __forceinline__ float2 cr_exp2(float2 x) {
-    if (!(max_nan(fabsf(x.x), fabsf(x.y)) <= 87.0f)) return make_float2(bsg_cr::exp(x.x), bsg_cr::exp(x.y));
-    return cr_exp2_in(x);
-}
-
-__device__ __forceinline__ float2 cr_log2(float2 x) {
-    if (!(cr_log_in_range(x.x) && cr_log_in_range(x.y)))
-        return make_float2(bsg_cr::log(x.x), bsg_cr::log(x.y));
+// bsg_cr::log on two positive normal finite arguments.
+__device__ __forceinline__ float2 cr_log2_in(float2 x) {
     const uint32_t u0 = __float_as_uint(x.x), u1 = __float_as_uint(x.y);
-    const uint32_t i0 = (u0 >> 15) & 0xFFu, i1 = (u1 >> 15) & 0xFFu;
-    const int e0 = (int)(u0 >> 23) - 127 + (int)(i0 >> 7);
-    const int e1 = (int)(u1 >> 23) - 127 + (int)(i1 >> 7);
-    const float2 m = make_float2(
-        __uint_as_float((u0 & 0x7FFFFFu) | (i0 >= 128 ? 0x3F000000u : 0x3F800000u)),
-        __uint_as_float((u1 & 0x7FFFFFu) | (i1 >= 128 ? 0x3F000000u : 0x3F800000u)));
-    const bsg_cr::LogEntry g0 = bsg_cr::log_tab((int)i0), g1 = bsg_cr::log_tab((int)i1);
+    const uint32_t v0 = u0 + 0x400000u, v1 = u1 + 0x400000u;
+    const float2 m = make_float2(__uint_as_float(u0 + 0x3F800000u - (v0 & 0xFF800000u)),
+                                 __uint_as_float(u1 + 0x3F800000u - (v1 & 0xFF800000u)));
+    const bsg_cr::LogEntry g0 = bsg_cr::log_tab((int)((u0 >> 15) & 0xFFu));
+    const bsg_cr::LogEntry g1 = bsg_cr::log_tab((int)((u1 >> 15) & 0xFFu));
     const float2 r = fma2(m, make_float2(g0.c, g1.c), f2(-1.0f));
     const FF2 s2 = two_prod2(r, r);
     float2 c = fma2(r, f2(0.2f), f2(-0.25f));
@@ -487,46 +468,82 @@ __device__ __forceinline__ float2 cr_log2(float2 x) {
     c = mul2(mul2(s2.hi, r), c);
     const FF2 a = fast_two_sum2(r, mul2(s2.hi, f2(-0.5f)));
     const float2 alo = add2(a.lo, fma2(s2.lo, f2(-0.5f), c));
-    const float2 ef = sub2(make_float2(__uint_as_float(bsg_cr::kShifterBits + (uint32_t)e0),
-                                       __uint_as_float(bsg_cr::kShifterBits + (uint32_t)e1)),
-                           f2(bsg_cr::kShifter));
-    const FF2 em = two_prod2(ef, f2(BSG_CR_LN2M));
-    const FF2 s1 = fast_two_sum2(mul2(ef, f2(BSG_CR_LN2H)), make_float2(g0.hi, g1.hi));
-    const FF2 s2s = fast_two_sum2(s1.hi, a.hi);
-    const FF2 s3 = fast_two_sum2(s2s.hi, em.hi);
-    const float2 lo = add2(add2(add2(s1.lo, s2s.lo), s3.lo),
-                           add2(add2(make_float2(g0.lo, g1.lo), alo),
-                                fma2(ef, f2(BSG_CR_LN2L), em.lo)));
-    return add2(s3.hi, lo);
+    // (e + 127 shifted without its sign: with an arithmetic shift of e itself
+    // nvcc 13.0.88 left the shift out in one lane)
+    const float2 ef =
+        sub2(make_float2(__uint_as_float(bsg_cr::kShifterBits - 127u + (v0 >> 23)),
+                         __uint_as_float(bsg_cr::kShifterBits - 127u + (v1 >> 23))),
+             f2(bsg_cr::kShifter));
+    const float2 th = make_float2(g0.hi, g1.hi);
+    const float2 s1 = fma2(ef, f2(BSG_CR_LN2H), th);
+    const float2 s1l = sub2(th, fma2(neg2(ef), f2(BSG_CR_LN2H), s1));
+    const FF2 s2s = fast_two_sum2(s1, a.hi);
+    const float2 s3 = fma2(ef, f2(BSG_CR_LN2M), s2s.hi);
+    const float2 s3l = fma2(ef, f2(BSG_CR_LN2M), sub2(s2s.hi, s3));
+    const float2 lo = add2(add2(add2(s1l, s2s.lo), s3l),
+                           fma2(ef, f2(BSG_CR_LN2L), add2(make_float2(g0.lo, g1.lo), alo)));
+    return add2(s3, lo);
 }
 
 __device__ __forceinline__ float2 dmul_finite2(float2 x, FF c) {
     return fma2(f2(c.hi), x, mul2(f2(c.lo), x));
 }
 
-// The smaller of a and b, NaN if either is.
-__device__ __forceinline__ float min_nan(float a, float b) {
+// 1/b, a/b and sqrt(t), each rounded to nearest as __frcp_rn, __fdiv_rn and
+// __fsqrt_rn round it, two at a time and without their tests for operands
+// near the ends of the float range: the caller has made sure that no step
+// comes near those.  The corrections are P. W. Markstein's ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34(1), 1990): a residual that one fma gives exactly, times the
+// approximate reciprocal.  1/b: every float in [2^-60, 2^110], and sqrt(t):
+// every float in [2^-40, 2^40], compared with the functions above.  a/b: from
+// a correctly rounded 1/b and a quotient within an ulp (which the first
+// correction makes of q) the second correction is his theorem; 2^36 random
+// and near-power-of-two pairs compared.
+__device__ __forceinline__ float2 rcp2_rn(float2 b) {
+    const float2 y = make_float2(rcp_approx(b.x), rcp_approx(b.y));
+    return fma2(fma2(neg2(b), y, f2(1.0f)), y, y);
+}
+__device__ __forceinline__ float2 div2_rn(float2 a, float2 b) {
+    const float2 y = rcp2_rn(b);
+    float2 q = mul2(a, y);
+    q = fma2(fma2(neg2(b), q, a), y, q);
+    return fma2(fma2(neg2(b), q, a), y, q);
+}
+__device__ __forceinline__ float2 sqrt2_rn(float2 t) {
+    const float2 y = make_float2(rsqrt_approx(t.x), rsqrt_approx(t.y));
+    const float2 g = mul2(t, y);
+    return fma2(fma2(neg2(g), g, t), mul2(f2(0.5f), y), g);
+}
+
+// The smallest and the largest of three, NaN if any is.
+__device__ __forceinline__ float min3_nan(float a, float b, float c) {
     float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
 
+// |d| < 2^76 here (price_libm_ref2).
 __device__ __forceinline__ float2 cndf_libm_ref2(float2 xin) {
     constexpr FF c0 = split(BSG_C0), c1 = split(BSG_C1), c2 = split(BSG_C2);
     constexpr FF c3 = split(BSG_C3), c4 = split(BSG_C4), c5 = split(BSG_C5);
     constexpr FF isp = split(BSG_INV_SQRT_2PI);
     const bool neg0 = xin.x < 0.0f, neg1 = xin.y < 0.0f;
-    // Neither an infinite |d| nor an exponent under -87 needs a path of its
-    // own: with |d| held to 3e38 and the exponent to -87 the product l1 np is
-    // under 2^-125, and 1 less it rounds to 1 as it does with exp's own 0 or
-    // subnormal (a NaN passes through k).
-    const float2 x = make_float2(min_nan(fabsf(xin.x), 3e38f), min_nan(fabsf(xin.y), 3e38f));
+    const float2 x = make_float2(fabsf(xin.x), fabsf(xin.y));
+    // An exponent under -87 needs no path of its own: held to -87 the product
+    // l1 np is under 2^-125, and 1 less it rounds to 1 as it does with exp's
+    // own 0 or subnormal.
     const float2 a = mul2(mul2(f2(-0.5f), x), x);
     const float2 e = cr_exp2_in(make_float2(fmaxf(a.x, -87.0f), fmaxf(a.y, -87.0f)));
     const float2 np = dmul_finite2(e, isp);
     float2 k = dmul_finite2(x, c0);
     k = add2(f2(1.0f), k);
-    k = make_float2(__frcp_rn(k.x), __frcp_rn(k.y));
+    k = rcp2_rn(k);
     const float2 k2 = mul2(k, k), k3 = mul2(k2, k);
     const float2 k4 = mul2(k3, k), k5 = mul2(k4, k);
     float2 l1 = dmul_finite2(k, c1);
@@ -546,17 +563,31 @@ __device__ __forceinline__ float2 cndf_libm_ref2(float2 xin) {
 
 __device__ __forceinline__ float2 price_libm_ref2(float2 s, float2 k, float2 r, float2 v,
                                                   float2 t, int ot0, int ot1) {
-    const float2 sq = make_float2(__fsqrt_rn(t.x), __fsqrt_rn(t.y));
-    const float2 lg = cr_log2(make_float2(__fdiv_rn(s.x, k.x), __fdiv_rn(s.y, k.y)));
+    const float2 sq = sqrt2_rn(t);
+    const float2 lg = cr_log2_in(div2_rn(s, k));
     float2 pw = mul2(v, v);
     pw = mul2(pw, f2(0.5f));
     float2 d1 = add2(r, pw);
     d1 = make_float2(__fadd_rn(__fmul_rn(d1.x, t.x), lg.x), __fadd_rn(__fmul_rn(d1.y, t.y), lg.y));
+    const float2 rt = mul2(neg2(r), t);
+    // Inside these bounds no operation below or above leaves the range that
+    // its packed form is good for: s/k in 2^+-60, v sqrt(t) in 2^+-45, d1 in
+    // 2^-75 .. 2^75 and all residuals whole multiples of 2^-77.  Both
+    // options of a pair with anything else (a numerator of 0 too) are priced
+    // one by one.
+    const float a0 = fabsf(d1.x), a1 = fabsf(d1.y);
+    const float lo = min3_nan(min3_nan(s.x, k.x, v.x), min3_nan(t.x, a0, s.y),
+                              min3_nan(min3_nan(k.y, v.y, t.y), a1, a1));
+    const float hi = max3_nan(max3_nan(s.x, k.x, v.x), max3_nan(t.x, a0, s.y),
+                              max3_nan(max3_nan(k.y, v.y, t.y), a1, a1));
+    if (!(lo >= 0x1p-30f && hi <= 0x1p30f && max3_nan(fabsf(rt.x), fabsf(rt.y), 0.0f) <= 87.0f))
+        return make_float2(price_libm_ref(s.x, k.x, r.x, v.x, t.x, ot0),
+                           price_libm_ref(s.y, k.y, r.y, v.y, t.y, ot1));
     const float2 den = mul2(v, sq);
-    d1 = make_float2(__fdiv_rn(d1.x, den.x), __fdiv_rn(d1.y, den.y));
+    d1 = div2_rn(d1, den);
     const float2 d2 = sub2(d1, den);
     const float2 n1 = cndf_libm_ref2(d1), n2 = cndf_libm_ref2(d2);
-    const float2 fv = mul2(k, cr_exp2(mul2(neg2(r), t)));
+    const float2 fv = mul2(k, cr_exp2_in(rt));
     const float2 nn1 = sub2(f2(1.0f), n1), nn2 = sub2(f2(1.0f), n2);
     const float p0 = ot0 == 0 ? __fsub_rn(__fmul_rn(s.x, n1.x), __fmul_rn(fv.x, n2.x))
                               : __fsub_rn(__fmul_rn(fv.x, nn2.x), __fmul_rn(s.x, nn1.x));

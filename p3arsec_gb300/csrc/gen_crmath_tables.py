@@ -49,7 +49,7 @@ def main():
     L3 = f32(L - L1 - L2)
     inv_l = f32(1 / L)
     LN2H = round_bits(ln2, 16)   # e * LN2H exact for |e| <= 2^8
-    LN2M = f32(ln2 - LN2H)
+    LN2M = round_bits(ln2 - LN2H, 16)
     LN2L = f32(ln2 - LN2H - LN2M)
     exp_tab = [split2(Fraction(D(2) ** (D(j) / D(32)))) for j in range(32)]
     # log: m in [1, 2) indexed by its top 8 fraction bits i; for i >= 128
@@ -75,7 +75,7 @@ def main():
     w(f"#define BSG_CR_L2 {hexf(L2)}")
     w(f"#define BSG_CR_L3 {hexf(L3)}")
     w(f"#define BSG_CR_INV_L {hexf(inv_l)}")
-    w("// ln2 = kLN2H + kLN2M + kLN2L (kLN2H has 16 significant bits)")
+    w("// ln2 = kLN2H + kLN2M + kLN2L (the first two of 16 significant bits)")
     w(f"#define BSG_CR_LN2H {hexf(LN2H)}")
     w(f"#define BSG_CR_LN2M {hexf(LN2M)}")
     w(f"#define BSG_CR_LN2L {hexf(LN2L)}")
