@@ -152,7 +152,7 @@ struct bsg_ctx {
     // swaption scratch: counters, parameter table, partial sums on the device;
     // results and the table's staging in pinned memory (h_sw where h_stage is too small)
     char* d_sw = nullptr;
-    size_t sw_cap = 0;
+    size_t sw_cap = 0, sw_done_cap = 0;
     char* h_sw = nullptr;
     size_t h_sw_cap = 0;
 
@@ -1517,27 +1517,42 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
             heads[i].words_at += (uint32_t)(n * head_words);
             large = large || heads[i].wide || heads[i].n_exp > 4;
         }
+        // Longest paths first (in instructions, about): the last paths of a
+        // call, which leave the GPU half empty, are then its shortest.  Of no
+        // use to a call with enough swaptions to fill it many times over.
+        std::vector<uint32_t> order(n);
+        for (size_t i = 0; i < n; ++i) order[i] = (uint32_t)i;
+        if (n <= 1024) {
+            auto cost = [&](uint32_t i) {
+                const int nz = heads[i].n_normals, np = heads[i].n_exp;
+                return (nz + 1) / 2 * 230 + np * (8 * nz + 45);
+            };
+            std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost(a) > cost(b); });
+        }
         BSG_CK(c, cudaSetDevice(c->device));
         if (int st = drain_pipeline(c)) return st;
-        // device: counters (kept zero) | table | partials; pinned: results | table
+        // device: counters (kept zero) | table | partials; pinned: sums | table
         const size_t tab_words = n * head_words + words.size();
         const bool inl = tab_words <= (size_t)bsg::kSwInlineWords;
-        const size_t done_b = round_up(65535 * sizeof(unsigned), 256);
+        const size_t done_b = round_up(8 + bsg::swaption_counters((int)n, trials) * sizeof(unsigned), 256);
         const size_t tab_b = inl ? 0 : round_up(tab_words * 8, 256);
-        const size_t need = done_b + tab_b + bsg::swaption_partial_bytes((int)n, trials);
+        const size_t rest_b = tab_b + bsg::swaption_partial_bytes((int)n, trials);
         const size_t out_b = round_up(2 * n * sizeof(double), 256);
-        if (need > c->sw_cap) {
+        if (done_b > c->sw_done_cap || rest_b > c->sw_cap) {
+            const size_t done_cap = std::max(done_b, c->sw_done_cap), cap = std::max(rest_b, c->sw_cap);
             BSG_CK(c, cudaStreamSynchronize(c->stream));
             if (c->d_sw) cudaFree(c->d_sw);
             c->d_sw = nullptr;
-            c->sw_cap = 0;
-            if (cudaMalloc(&c->d_sw, need) != cudaSuccess) {
+            c->sw_cap = c->sw_done_cap = 0;
+            if (cudaMalloc(&c->d_sw, done_cap + cap) != cudaSuccess) {
                 cudaGetLastError();
                 return fail(c, BSG_ERR_OUT_OF_MEMORY, "swaption scratch");
             }
-            BSG_CK(c, cudaMemsetAsync(c->d_sw, 0, done_b, c->stream));
-            c->sw_cap = need;
+            BSG_CK(c, cudaMemsetAsync(c->d_sw, 0, done_cap, c->stream));
+            c->sw_cap = cap;
+            c->sw_done_cap = done_cap;
         }
+        char* const d_rest = c->d_sw + c->sw_done_cap;
         // pinned: the staging (no other call's work uses it now), or their own
         char* pin = c->h_stage;
         if (out_b + tab_b > kStageBytes && out_b + tab_b > c->h_sw_cap) {
@@ -1552,26 +1567,32 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
             c->h_sw_cap = out_b + tab_b;
         }
         if (out_b + tab_b > kStageBytes) pin = c->h_sw;
-        double* out = reinterpret_cast<double*>(pin);  // the kernel writes the results here itself
+        double2* sums = reinterpret_cast<double2*>(pin);  // the kernel writes them here itself
         bsg::SwInline in;
         uint64_t* d_tab = nullptr;
         uint64_t* tab = in.words;
         if (!inl) {
-            d_tab = reinterpret_cast<uint64_t*>(c->d_sw + done_b);
+            d_tab = reinterpret_cast<uint64_t*>(d_rest);
             tab = reinterpret_cast<uint64_t*>(pin + out_b);
         }
-        std::memcpy(tab, heads.data(), n * sizeof(bsg::SwHead));
+        for (size_t i = 0; i < n; ++i) std::memcpy(tab + i * head_words, &heads[order[i]], sizeof(bsg::SwHead));
         if (!words.empty()) std::memcpy(tab + n * head_words, words.data(), words.size() * 8);
         if (!inl) BSG_CK(c, cudaMemcpyAsync(d_tab, tab, tab_words * 8, cudaMemcpyHostToDevice, c->stream));
-        cudaError_t e = bsg::launch_swaptions(in, d_tab, (int)n, large, trials, c->d_sw + done_b + tab_b,
-                                              reinterpret_cast<unsigned*>(c->d_sw), out, c->d_parts,
+        cudaError_t e = bsg::launch_swaptions(in, d_tab, (int)n, large, trials, d_rest + tab_b,
+                                              reinterpret_cast<unsigned*>(c->d_sw + 8),
+                                              reinterpret_cast<unsigned long long*>(c->d_sw), sums, c->d_parts,
                                               c->h_flag, ++c->call, c->sm_count, c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "launch_swaptions");
         c->launches++;
         BSG_CK(c, wait_flag(c));
+        // the mean and the reference's standard error (HJM_Swaption_Blocking.cpp:212-214);
+        // three divisions and two square roots in a row in doubles, at the end of
+        // the kernel, kept a small call waiting 2 us
+        const double m = (double)trials, rm = std::sqrt(m);
         for (size_t i = 0; i < n; ++i) {
-            price[i] = out[2 * i];
-            if (std_err) std_err[i] = out[2 * i + 1];
+            const double2 s = sums[i];
+            price[order[i]] = s.x / m;
+            if (std_err) std_err[order[i]] = std::sqrt((s.y - s.x * s.x / m) / (m - 1.0)) / rm;
         }
         return BSG_OK;
     } catch (const std::bad_alloc&) {

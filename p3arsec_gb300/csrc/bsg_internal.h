@@ -87,11 +87,14 @@ cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_
 #if defined(__CUDACC__)
 // One thread of each of `parts` parts of a kernel, once the part's stores are
 // made (and seen by this thread): the last one zeroes the count and stores seq
-// to *flag in pinned host memory, where the host then sees every part's stores.
-__device__ __forceinline__ void signal_host(unsigned* count, unsigned parts, unsigned* flag, unsigned seq) {
+// (and zeroes *queue if there is one: no part takes from it any more) to *flag
+// in pinned host memory, where the host then sees every part's stores.
+__device__ __forceinline__ void signal_host(unsigned* count, unsigned parts, unsigned* flag, unsigned seq,
+                                            unsigned long long* queue = nullptr) {
     __threadfence_system();
     if (atomicAdd(count, 1u) != parts - 1) return;
     *count = 0;
+    if (queue) *queue = 0;
     __threadfence_system();
     asm volatile("st.release.sys.global.u32 [%0], %1;" :: "l"(flag), "r"(seq) : "memory");
 }
@@ -207,16 +210,18 @@ struct SwInline {
 int swaption_per_thread(uint64_t trials);
 uint64_t swaption_chunks(uint64_t trials);
 size_t swaption_partial_bytes(int nsw, uint64_t trials);
-// Prices nsw swaptions with `trials` paths each: out[2 i] = mean discounted
-// payoff, out[2 i + 1] = its standard error (pinned or device memory).  The
+size_t swaption_counters(int nsw, uint64_t trials);
+// Runs nsw swaptions with `trials` paths each: sums[i] = the sums of the
+// discounted payoffs and of their squares (pinned or device memory).  The
 // table: nsw heads, then their words, at `table` (device memory) or in `in`
 // (table NULL).  large: some swaption has more than four exponents or is
-// wide.  partial: device scratch of swaption_partial_bytes; done: nsw device
-// counters, zero, left zero.
+// wide.  partial: device scratch of swaption_partial_bytes; done:
+// swaption_counters device counters, and queue another: zero, left zero.
 // At the end it stores seq to *flag in pinned memory (signal_host over count).
 cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw, bool large,
-                             uint64_t trials, void* partial, unsigned* done, double* out, unsigned* count,
-                             unsigned* flag, unsigned seq, int sm_count, cudaStream_t st);
+                             uint64_t trials, void* partial, unsigned* done, unsigned long long* queue,
+                             double2* sums, unsigned* count, unsigned* flag, unsigned seq, int sm_count,
+                             cudaStream_t st);
 
 // z[2 i], z[2 i + 1] = the swaption kernel's normal pair of words[4 i .. 4 i + 3]
 // (device arrays), i < n.

@@ -32,19 +32,22 @@
 // multiply-add, the floor and the two sums, 4 to 6 operations a path: 5.28 ms.
 // Its bound is the pipe that takes the integer multiply-adds (two thirds busy,
 // 170 of them a path, 40 in the generator).  Four blocks of 64 registers an SM:
-// 5.34 ms, three of 80 5.53, two of 128 5.54.
+// 5.34 ms, three of 80 5.53, two of 128 5.54.  With warps that take their own
+// work (below) instead of blocks: 4.74 ms.
 //
 // Reduction: each warp reduces its paths' sums (sum and sum of squares of
-// the discounted payoff) in a fixed order and writes one partial; the block
-// that finishes a swaption last adds its partials in a fixed order.  Which
-// paths a partial covers depends on the number of trials alone: two runs, and
-// a swaption alone or among others, give the same bits.
+// the discounted payoff) in a fixed order to one part; the warp that finishes
+// a group of parts, and then a swaption, last adds them up in a fixed order.
+// Which paths a part covers and how parts are grouped depends on the number of
+// trials alone: two runs, and a swaption alone or among others, give the same
+// bits.
 #include "bsg_internal.h"
 #include "bsg_swmath.h"
 
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 namespace bsg {
 
@@ -52,6 +55,16 @@ namespace {
 
 constexpr int kSwThreads = 256;
 constexpr int kSwWarps = kSwThreads / 32;
+
+// How many of a swaption's parts one warp adds up before the swaption's last
+// warp adds up the groups' sums: all of up to 256 (eight loads a lane, at once),
+// else 32.  16 swaptions x 5,000 paths (160 parts): 38.9 us in groups of 32,
+// 37.9 in one; x 20,000 (632): 52.0 in groups of 32, 53.8 of 256.
+__host__ __device__ __forceinline__ unsigned group_size(uint64_t parts) { return parts <= 256 ? 256 : 32; }
+__host__ __device__ __forceinline__ uint64_t group_count(uint64_t parts) {
+    return parts <= 256 ? 1 : (parts + 31) / 32;
+}
+constexpr int kHeadWords = sizeof(SwHead) / sizeof(uint64_t);
 
 __device__ __forceinline__ void philox4x32_10(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
                                               uint32_t k0, uint32_t k1, uint32_t out[4]) {
@@ -84,28 +97,25 @@ __device__ __forceinline__ void load_tables(bsg_sw::Tables& dst) {
         d[i] = src[i];
 }
 
-// One swaption in shared memory: its head and its words (pays, constants,
-// coefficients; bsg_internal.h).  Swaptions of up to four exponents have at
-// most 4 (2 + 8 x 31) words.
-template <bool LARGE>
+// What a block keeps in shared memory: the tables, and the swaptions when
+// they came with the launch.
+template <bool INLINE>
 struct SwShared {
     bsg_sw::Tables nt;
-    SwHead head;
-    uint64_t words[LARGE ? kSwMaxWords : 1000];
-    double red[2][kSwWarps];
-    int last;
+    uint64_t words[INLINE ? kSwInlineWords : 1];
 };
 
 __device__ __forceinline__ double as_double(uint64_t u) { return __longlong_as_double((long long)u); }
 
-// The payoff of trial t of the swaption in sh, less its constant discount.
+// The payoff of trial t of the swaption with head hd and these words (pays,
+// constants, coefficients; bsg_internal.h), less its constant discount.
 // NP: the number of exponents, or with GUARD an upper bound of it.
-template <int NP, bool GUARD, typename Sh>
-__device__ __forceinline__ double path_payoff(const Sh& sh, uint64_t t) {
-    const SwHead& hd = sh.head;
+template <int NP, bool GUARD>
+__device__ __forceinline__ double path_payoff(const bsg_sw::Tables& nt, const SwHead& hd,
+                                              const uint64_t* words, uint64_t t) {
     const int np = GUARD ? hd.n_exp : NP;
-    const uint64_t* c0 = sh.words + np;
-    const uint64_t* g = sh.words + 2 * np;
+    const uint64_t* c0 = words + np;
+    const uint64_t* g = words + 2 * np;
     uint64_t x[NP], half = 0;
 #pragma unroll
     for (int l = 0; l < NP; ++l) x[l] = (!GUARD || l < np) ? c0[l] : 0;
@@ -127,11 +137,11 @@ __device__ __forceinline__ double path_payoff(const Sh& sh, uint64_t t) {
                       (uint32_t)(hd.seed >> 32), w);
         int64_t z0, z1;
         if (i + 1 < nz) {
-            bsg_sw::normal_pair_fixed<true>(sh.nt, w[0], w[1], w[2], w[3], &z0, &z1);
+            bsg_sw::normal_pair_fixed<true>(nt, w[0], w[1], w[2], w[3], &z0, &z1);
             take(z0);
             take(z1);
         } else {
-            bsg_sw::normal_pair_fixed<false>(sh.nt, w[0], w[1], w[2], w[3], &z0, &z1);
+            bsg_sw::normal_pair_fixed<false>(nt, w[0], w[1], w[2], w[3], &z0, &z1);
             take(z0);
         }
     }
@@ -141,8 +151,8 @@ __device__ __forceinline__ double path_payoff(const Sh& sh, uint64_t t) {
 #pragma unroll
     for (int l = 0; l < NP; ++l)
         if (!GUARD || l < np) {
-            const double y = bsg_sw::exp2_fixed(sh.nt, (int64_t)(x[l] - half));
-            if (l < pays) v = __fma_rn(as_double(sh.words[l]), y, v);
+            const double y = bsg_sw::exp2_fixed(nt, (int64_t)(x[l] - half));
+            if (l < pays) v = __fma_rn(as_double(words[l]), y, v);
             else disc = y;
         }
     return v > 0.0 ? __dmul_rn(v, disc) : 0.0;
@@ -150,24 +160,23 @@ __device__ __forceinline__ double path_payoff(const Sh& sh, uint64_t t) {
 
 // The same in double precision, for exponents outside the fixed-point range:
 // words hold the constants and coefficients as doubles, natural exponents.
-template <typename Sh>
-__device__ __noinline__ double path_payoff_wide(const Sh& sh, uint64_t t) {
-    const SwHead& hd = sh.head;
+__device__ __noinline__ double path_payoff_wide(const bsg_sw::Tables& nt, const SwHead& hd,
+                                                const uint64_t* words, uint64_t t) {
     const int np = hd.n_exp, nz = hd.n_normals, pays = np - hd.disc_varies;
     double v = -1.0, disc = 1.0;
     for (int l = 0; l < np; ++l) {
-        double x = as_double(sh.words[np + l]), z[2];
+        double x = as_double(words[np + l]), z[2];
         for (int i = 0; i < nz; ++i) {
             if ((i & 1) == 0) {
                 uint32_t w[4];
                 philox4x32_10((uint32_t)t, (uint32_t)(t >> 32), (uint32_t)(i >> 1), 0u,
                               (uint32_t)hd.seed, (uint32_t)(hd.seed >> 32), w);
-                bsg_sw::normal_pair(sh.nt, w[0], w[1], w[2], w[3], &z[0], &z[1]);
+                bsg_sw::normal_pair(nt, w[0], w[1], w[2], w[3], &z[0], &z[1]);
             }
-            x = __fma_rn(as_double(sh.words[2 * np + i * np + l]), z[i & 1], x);
+            x = __fma_rn(as_double(words[2 * np + i * np + l]), z[i & 1], x);
         }
-        const double y = bsg_sw::exp_(sh.nt, x);
-        if (l < pays) v = __fma_rn(as_double(sh.words[l]), y, v);
+        const double y = bsg_sw::exp_(nt, x);
+        if (l < pays) v = __fma_rn(as_double(words[l]), y, v);
         else disc = y;
     }
     return v > 0.0 ? __dmul_rn(v, disc) : 0.0;
@@ -184,104 +193,124 @@ __device__ __forceinline__ double2 warp_sums(double a, double b) {
     return make_double2(v, __shfl_sync(0xffffffffu, v, 16));  // lane 0's are the sums
 }
 
-// Chunks [chunk, end) of the swaption in sh: one partial per warp and chunk.
-template <int NP, bool GUARD, bool WIDE, typename Sh>
-__device__ __forceinline__ void sum_chunks(const Sh& sh, uint64_t chunk, uint64_t end, int per_thread,
-                                           uint64_t trials, double2* partial) {
+// The sums of a warp's per_thread paths a lane from trial t on, kSwThreads apart.
+template <int NP, bool GUARD, bool WIDE>
+__device__ __forceinline__ double2 sum_paths(const bsg_sw::Tables& nt, const SwHead& hd, const uint64_t* words,
+                                             uint64_t t, int per_thread, uint64_t trials) {
+    double sum = 0.0, sum_sq = 0.0;
 #pragma unroll 1
-    for (; chunk < end; ++chunk) {
-        double sum = 0.0, sum_sq = 0.0;
-        uint64_t t = chunk * per_thread * kSwThreads + threadIdx.x;
-#pragma unroll 1
-        for (int q = 0; q < per_thread && t < trials; ++q, t += kSwThreads) {
-            const double dp = WIDE ? path_payoff_wide(sh, t) : path_payoff<NP, GUARD>(sh, t);
-            sum = __dadd_rn(sum, dp);
-            sum_sq = __fma_rn(dp, dp, sum_sq);
-        }
-        const double2 v = warp_sums(sum, sum_sq);
-        const double d = sh.head.disc;
-        if ((threadIdx.x & 31) == 0)
-            partial[chunk * kSwWarps + (threadIdx.x >> 5)] =
-                make_double2(__dmul_rn(v.x, d), __dmul_rn(v.y, __dmul_rn(d, d)));
+    for (int q = 0; q < per_thread && t < trials; ++q, t += kSwThreads) {
+        const double dp = WIDE ? path_payoff_wide(nt, hd, words, t) : path_payoff<NP, GUARD>(nt, hd, words, t);
+        sum = __dadd_rn(sum, dp);
+        sum_sq = __fma_rn(dp, dp, sum_sq);
     }
+    __syncwarp();
+    return warp_sums(sum, sum_sq);
 }
 
-// Persistent blocks over (swaption, `span` consecutive chunks of per_thread x
-// 256 paths).  LARGE: also swaptions of more than four exponents or outside
-// the fixed-point range (their registers would cost the others a block per SM).
-template <bool LARGE>
+// Lane 0's value v to *at; true in the warp that is the last of `of` to come
+// here with this counter, which then sees all their values and leaves it zero.
+__device__ __forceinline__ bool last_of(unsigned lane, double2* at, double2 v, unsigned* counter, unsigned of) {
+    unsigned before = 0;
+    if (lane == 0) {
+        *at = v;
+        __threadfence();
+        before = atomicAdd(counter, 1u);
+        if (before == of - 1) *counter = 0;
+    }
+    if (__shfl_sync(0xffffffffu, before, 0) != of - 1) return false;
+    __threadfence();
+    return true;
+}
+
+// The sum of p[0 .. n) in a fixed order, eight loads a lane in flight.
+__device__ __forceinline__ double2 sum_parts(unsigned lane, const double2* p, unsigned n) {
+    double a = 0.0, b = 0.0;
+#pragma unroll 8
+    for (unsigned i = lane; i < n; i += 32) {
+        const double2 v = __ldcg(p + i);
+        a = __dadd_rn(a, v.x);
+        b = __dadd_rn(b, v.y);
+    }
+    return warp_sums(a, b);
+}
+
+// Persistent blocks whose warps each take the next 32 x per_thread paths from
+// a queue: no warp waits for another, and what is left over at the end is a
+// part's work, not a block's.  Blocks that took 256 x per_thread paths at a
+// time, with a barrier on either side, spent a quarter of a round of one path
+// per thread outside the paths, and a round more for a remainder: 16 swaptions
+// x 20,000 paths 56 -> 52 us, x 80,000 139 -> 93, 64 x 100,000 494 -> 361, 128 x
+// 1M 5.17 -> 4.74 ms.  (Counting a part only when the next is done, so that the
+// warp does not wait for its store, took more registers: 4.88 ms.)
+// LARGE: also swaptions of more than four exponents or outside the fixed-point
+// range (their registers would cost the others two blocks per SM).  INLINE:
+// the table came in the launch's parameters.
+template <bool LARGE, bool INLINE>
 __global__ void __launch_bounds__(kSwThreads, LARGE ? 2 : 4) swaption_paths_kernel(
     const __grid_constant__ SwInline in, const uint64_t* __restrict__ table, int nsw, uint64_t trials,
-    int per_thread, uint64_t chunks, unsigned span, double2* __restrict__ partial,
-    unsigned* __restrict__ done, double* __restrict__ out, unsigned* count, unsigned* flag, unsigned seq) {
-    __shared__ SwShared<LARGE> sh;
+    int per_thread, uint64_t nparts, double2* __restrict__ partial, unsigned* __restrict__ done,
+    unsigned long long* queue, double2* __restrict__ sums, unsigned* count, unsigned* flag, unsigned seq) {
+    __shared__ SwShared<INLINE> sh;
     load_tables(sh.nt);
-    const uint64_t spans = (chunks + span - 1) / span, items = spans * (uint64_t)nsw;
-    for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
-        const uint64_t sw = item / spans, chunk = (item - sw * spans) * span;
-        const uint64_t end = chunk + span < chunks ? chunk + span : chunks;
-        __syncthreads();  // the previous item's reads of sh are done
+    if (INLINE)
+        for (int i = threadIdx.x; i < kSwInlineWords; i += kSwThreads) sh.words[i] = in.words[i];
+    __syncthreads();
+    const uint64_t* tab = INLINE ? sh.words : table;
+    const unsigned lane = threadIdx.x & 31;
+    // an item: 32 x per_thread paths, one part of one swaption's sums
+    using Item = typename std::conditional<LARGE, uint64_t, uint32_t>::type;
+    using Take = typename std::conditional<LARGE, unsigned long long, unsigned>::type;
+    const Item parts = (Item)nparts, items = parts * (Item)nsw;
+    for (Item item = blockIdx.x * kSwWarps + (threadIdx.x >> 5); item < items;) {
+        // asked for now, looked at when this item is done
+        Item next = 0;
+        if (lane == 0) next = (Item)atomicAdd(reinterpret_cast<Take*>(queue), (Take)1);
+        const uint64_t* words;
+        uint64_t t;
         {
-            // head, then its words (from the launch's parameters when they all fit there)
-            constexpr int hw = (int)(sizeof(SwHead) / 8);
-            const uint64_t* tab = table ? table : in.words;
-            uint64_t* hd = reinterpret_cast<uint64_t*>(&sh.head);
-            if (threadIdx.x < hw) hd[threadIdx.x] = tab[sw * hw + threadIdx.x];
-            __syncthreads();
-            const uint64_t* src = tab + sh.head.words_at;
-            for (int i = threadIdx.x; i < sh.head.n_words; i += kSwThreads) sh.words[i] = src[i];
+            const Item sw = item / parts, part = item - sw * parts;
+            t = (uint64_t)(part / kSwWarps) * per_thread * kSwThreads + (part % kSwWarps) * 32 + lane;
+            words = tab + (uint64_t)sw * kHeadWords;
         }
-        __syncthreads();
-        double2* part = partial + sw * chunks * kSwWarps;
-        if (LARGE && sh.head.wide) {
-            sum_chunks<1, true, true>(sh, chunk, end, per_thread, trials, part);
+        const SwHead& hd = *reinterpret_cast<const SwHead*>(words);
+        words = tab + hd.words_at;
+        double2 v;
+        if (LARGE && hd.wide) {
+            v = sum_paths<1, true, true>(sh.nt, hd, words, t, per_thread, trials);
         } else {
-            switch (sh.head.n_exp) {
-                case 1: sum_chunks<1, false, false>(sh, chunk, end, per_thread, trials, part); break;
-                case 2: sum_chunks<2, false, false>(sh, chunk, end, per_thread, trials, part); break;
-                case 3: sum_chunks<3, false, false>(sh, chunk, end, per_thread, trials, part); break;
-                case 4: sum_chunks<4, false, false>(sh, chunk, end, per_thread, trials, part); break;
+            switch (hd.n_exp) {
+                case 1: v = sum_paths<1, false, false>(sh.nt, hd, words, t, per_thread, trials); break;
+                case 2: v = sum_paths<2, false, false>(sh.nt, hd, words, t, per_thread, trials); break;
+                case 3: v = sum_paths<3, false, false>(sh.nt, hd, words, t, per_thread, trials); break;
                 default:
-                    if constexpr (LARGE) {
-                        if (sh.head.n_exp <= 8)
-                            sum_chunks<8, true, false>(sh, chunk, end, per_thread, trials, part);
-                        else
-                            sum_chunks<kSwMaxExp, true, false>(sh, chunk, end, per_thread, trials, part);
-                    }
+                    if (!LARGE || hd.n_exp == 4)
+                        v = sum_paths<4, false, false>(sh.nt, hd, words, t, per_thread, trials);
+                    else if (hd.n_exp <= 8)
+                        v = sum_paths<8, true, false>(sh.nt, hd, words, t, per_thread, trials);
+                    else
+                        v = sum_paths<kSwMaxExp, true, false>(sh.nt, hd, words, t, per_thread, trials);
             }
         }
-        // the block that finishes the swaption's last chunk adds the partials up
-        if ((threadIdx.x & 31) == 0) __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0)
-            sh.last = atomicAdd(&done[sw], (unsigned)(end - chunk)) + (unsigned)(end - chunk) == (unsigned)chunks;
-        __syncthreads();
-        if (!sh.last) continue;
-        __threadfence();
-        double ta = 0.0, tb = 0.0;
-        for (uint64_t i = threadIdx.x; i < chunks * kSwWarps; i += kSwThreads) {
-            const double2 v = __ldcg(part + i);
-            ta = __dadd_rn(ta, v.x);
-            tb = __dadd_rn(tb, v.y);
+        v = make_double2(__dmul_rn(v.x, hd.disc), __dmul_rn(v.y, __dmul_rn(hd.disc, hd.disc)));
+        const Item sw = item / parts, part = item - sw * parts;
+        // the warp that finishes a group of parts adds them up, the one that
+        // finishes a swaption's last group adds the groups up
+        const unsigned size = group_size(parts);
+        const Item groups = (Item)group_count(parts), group = part / size;
+        double2* mine = partial + (uint64_t)sw * (parts + groups);
+        unsigned* left = done + (uint64_t)sw * (groups + 1);
+        const unsigned in_group = group + 1 < groups ? size : (unsigned)(parts - size * group);
+        item = (Item)(gridDim.x * kSwWarps) + __shfl_sync(0xffffffffu, next, 0);
+        if (!last_of(lane, mine + part, v, left + group, in_group)) continue;
+        v = sum_parts(lane, mine + size * group, in_group);
+        if (groups > 1) {
+            if (!last_of(lane, mine + parts + group, v, left + groups, (unsigned)groups)) continue;
+            v = sum_parts(lane, mine + parts, (unsigned)groups);
         }
-        const double2 v = warp_sums(ta, tb);
-        if ((threadIdx.x & 31) == 0) {
-            sh.red[0][threadIdx.x >> 5] = v.x;
-            sh.red[1][threadIdx.x >> 5] = v.y;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s1 = sh.red[0][0], s2 = sh.red[1][0];
-            for (int w = 1; w < kSwWarps; ++w) {
-                s1 = __dadd_rn(s1, sh.red[0][w]);
-                s2 = __dadd_rn(s2, sh.red[1][w]);
-            }
-            // the mean and the reference's standard error (HJM_Swaption_Blocking.cpp:212-214)
-            const double m = (double)trials;
-            out[2 * sw] = s1 / m;
-            out[2 * sw + 1] = sqrt((s2 - s1 * s1 / m) / (m - 1.0)) / sqrt(m);
-            done[sw] = 0;  // ready for the next call
-            signal_host(count, (unsigned)nsw, flag, seq);
+        if (lane == 0) {
+            sums[sw] = v;
+            signal_host(count, (unsigned)nsw, flag, seq, queue);
         }
     }
 }
@@ -318,27 +347,27 @@ uint64_t swaption_chunks(uint64_t trials) {
 }
 
 size_t swaption_partial_bytes(int nsw, uint64_t trials) {
-    return (size_t)nsw * swaption_chunks(trials) * kSwWarps * sizeof(double2);
+    const size_t parts = swaption_chunks(trials) * kSwWarps;
+    return (size_t)nsw * (parts + group_count(parts)) * sizeof(double2);
+}
+
+size_t swaption_counters(int nsw, uint64_t trials) {
+    return (size_t)nsw * (group_count(swaption_chunks(trials) * kSwWarps) + 1);
 }
 
 cudaError_t launch_swaptions(const SwInline& in, const uint64_t* table, int nsw, bool large,
-                             uint64_t trials, void* partial, unsigned* done, double* out, unsigned* count,
-                             unsigned* flag, unsigned seq, int sm_count, cudaStream_t st) {
+                             uint64_t trials, void* partial, unsigned* done, unsigned long long* queue,
+                             double2* sums, unsigned* count, unsigned* flag, unsigned seq, int sm_count,
+                             cudaStream_t st) {
     if (nsw <= 0 || trials < 2) return cudaErrorInvalidValue;
-    const uint64_t chunks = swaption_chunks(trials), items = chunks * (uint64_t)nsw;
-    const uint64_t room = (uint64_t)sm_count * (large ? 2 : 4);
-    const int per_thread = swaption_per_thread(trials);
-    // chunks per visit of a block: the fewer the better for the last wave, so
-    // the most that leave 16 visits per block
-    const unsigned span = (unsigned)std::min<uint64_t>(std::max<uint64_t>(items / (16 * room), 1), 16);
-    const unsigned grid = (unsigned)std::min<uint64_t>((chunks + span - 1) / span * (uint64_t)nsw, room);
-    double2* part = static_cast<double2*>(partial);
-    if (large)
-        swaption_paths_kernel<true><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
-                                                                 span, part, done, out, count, flag, seq);
-    else
-        swaption_paths_kernel<false><<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, per_thread, chunks,
-                                                                  span, part, done, out, count, flag, seq);
+    const uint64_t chunks = swaption_chunks(trials);
+    large = large || chunks * kSwWarps * nsw >> 31;  // counts items in 64 bits
+    const unsigned grid = (unsigned)std::min<uint64_t>(chunks * nsw, (uint64_t)sm_count * (large ? 2 : 4));
+    auto* kernel = large ? (table ? swaption_paths_kernel<true, false> : swaption_paths_kernel<true, true>)
+                         : (table ? swaption_paths_kernel<false, false> : swaption_paths_kernel<false, true>);
+    kernel<<<grid, kSwThreads, 0, st>>>(in, table, nsw, trials, swaption_per_thread(trials),
+                                        chunks * kSwWarps, static_cast<double2*>(partial), done, queue, sums,
+                                        count, flag, seq);
     return cudaGetLastError();
 }
 
