@@ -1592,7 +1592,14 @@ extern "C" int bsg_price_swaptions(bsg_ctx* c, const bsg_swaption* sw, size_t n,
         for (size_t i = 0; i < n; ++i) {
             const double2 s = sums[i];
             price[order[i]] = s.x / m;
-            if (std_err) std_err[order[i]] = std::sqrt((s.y - s.x * s.x / m) / (m - 1.0)) / rm;
+            if (!std_err) continue;
+            // s.y - s.x^2 / m, the quotient q + what it leaves: the difference
+            // is a thousandth of either and would show their last bits (and no
+            // sign of its own where every path pays the same)
+            const double p = s.x * s.x, q = p / m;
+            const double rest = (std::fma(-q, m, p) + std::fma(s.x, s.x, -p)) / m;
+            const double var = s.y - q - rest;
+            std_err[order[i]] = std::sqrt((var < 0.0 ? 0.0 : var) / (m - 1.0)) / rm;
         }
         return BSG_OK;
     } catch (const std::bad_alloc&) {
