@@ -858,25 +858,45 @@ MapCfg map_default_cfg(const SoA& a, int64_t n, int runs) {
 // operations an option, that pipe 85 % busy: 4M options in 1.38 ms against
 // 32 us of HBM traffic), so the elementary functions are fixed point
 // (bsg_fx64.h).  The few options that are left to the double evaluation go
-// into a queue in shared memory, which the block prices together at the end:
-// in place, one such option would hold its warp for a whole double
-// evaluation.  4M options: 133 us, bound by the pipe of the integer
-// multiply-adds (173 us before N came from a table, that pipe 73 % busy).
-constexpr int kF64Threads = 256;
+// into a queue of the block's: the warp whose option is a 32nd prices 32 of
+// them together, between the other warps' integer work, and the block the rest
+// at the end.  In place, one such option would hold its warp for a whole
+// double evaluation.  4M options: 124 us, bound by the pipe of the integer
+// multiply-adds (173 us before N came from a table).
+//
+// One block of 32 warps an SM; each warp takes the SM's next 32 options when it
+// is done with its last, and has the ones after copied into shared memory
+// meanwhile.  With a fixed share per warp (256-thread blocks, four an SM) the
+// scheduler, which prefers older warps, left the younger ones alone at the
+// end (25 of 32 warps resident on average), a fifth of the stalls were for
+// loads, and the queue waited for the end: 136 us, 155 where 3 % go into the
+// queue (now 136), 16M of those 533 (446).
+constexpr int kF64Threads = 1024;
+constexpr int kF64Warps = kF64Threads / 32;
 constexpr int kF64Queue = 1024;
+constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 
 __device__ const bsg_sw::Tables kFxTables = BSG_SW_TABLES;
 __device__ const bsg_fx::TailTable kFxTails = BSG_FX_TAILS;
 
-// The block's copy of the tables the price reads (48,640 bytes: dynamic shared
-// memory, four blocks an SM), and its queue.
+// One warp's options on their way in.
+template <typename T>
+struct F64Slot {
+    T s[32], k[32], r[32], v[32], t[32];
+    int32_t ot[32];
+};
+
+// The block's copy of the tables the price reads (48,640 bytes), two slots a
+// warp, and the options left to the double evaluation: dynamic shared memory.
+template <typename T>
 struct F64Shared {
     bsg_sw::LogEntry lg[512];
     bsg_sw::SeedEntry rs[384];
     uint64_t e2[1024];
     bsg_fx::TailTable tails;
+    F64Slot<T> slot[2][kF64Warps];
     uint32_t queue[kF64Queue];
-    int queued;
+    uint32_t queued, next;
 };
 
 template <typename T>
@@ -904,52 +924,98 @@ struct F64View {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kF64Threads, 4) map_f64_kernel(F64View<T> a, int64_t n) {
+__device__ __forceinline__ void copy_async(T* dst, const T* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(sizeof(T))
+                 : "memory");
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kF64Threads, 1) map_f64_kernel(F64View<T> a, int64_t n) {
     extern __shared__ __align__(16) char f64_smem[];
-    F64Shared& sh = *reinterpret_cast<F64Shared*>(f64_smem);
+    F64Shared<T>& sh = *reinterpret_cast<F64Shared<T>*>(f64_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the block's j-th 32 options begin here
+    auto begin = [&](uint32_t j) { return ((int64_t)j * gridDim.x + blockIdx.x) * 32; };
+    auto fetch = [&](uint32_t j, int b) {
+        const int64_t i = begin(j) + lane;
+        if (i < n) {
+            F64Slot<T>& d = sh.slot[b][warp];
+            copy_async(&d.s[lane], a.s + i);
+            copy_async(&d.k[lane], a.k + i);
+            copy_async(&d.r[lane], a.r + i);
+            copy_async(&d.v[lane], a.v + i);
+            copy_async(&d.t[lane], a.t + i);
+            copy_async(&d.ot[lane], a.ot + i);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint32_t j = warp;
+    int b = 0;
+    fetch(j, b);
     copy_table(sh.lg, kFxTables.lg);
     copy_table(sh.rs, kFxTables.rs);
     copy_table(sh.e2, kFxTables.e2);
     copy_table(sh.tails, kFxTails);
-    if (threadIdx.x == 0) sh.queued = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kF64Threads, stride = (int64_t)gridDim.x * kF64Threads;
-    uint32_t at = threadIdx.x;  // the option's place among the block's: 256 per pass of the grid
-    for (int64_t i = base + threadIdx.x; i < n; i += stride, at += kF64Threads) {
-        const double s = __ldg(a.s + i), k = __ldg(a.k + i), r = __ldg(a.r + i), v = __ldg(a.v + i),
-                     t = __ldg(a.t + i);
-        const int ot = __ldg(a.ot + i);
-        double p;
-        bool done = bsg_fx::fx64_domain(dbits(s), dbits(k), dbits(r), dbits(v), dbits(t));
-        if (done) done = bsg_fx::price_fx64(sh, sh.tails, dbits(s), dbits(k), dbits(r), dbits(v), dbits(t), ot, &p);
-        if (!done) {
-            const int q = atomicAdd(&sh.queued, 1);
-            if (q < kF64Queue) {
-                sh.queue[q] = at;
-                continue;
-            }
-            p = price_fp64_call(s, k, r, v, t, ot);
-        }
-        a.out[i] = p;
+    for (int q = threadIdx.x; q < kF64Queue; q += kF64Threads) sh.queue[q] = kEmpty;
+    if (threadIdx.x == 0) {
+        sh.queued = 0;
+        sh.next = kF64Warps;
     }
     __syncthreads();
-    const int m = sh.queued < kF64Queue ? sh.queued : kF64Queue;
-    for (int q = threadIdx.x; q < m; q += kF64Threads) {
-        const int64_t i = base + (int64_t)(sh.queue[q] / kF64Threads) * stride + sh.queue[q] % kF64Threads;
+    auto price_left = [&](uint32_t at) {
+        const int64_t i = begin(at / 32) + at % 32;
         a.out[i] = price_fp64_call(__ldg(a.s + i), __ldg(a.k + i), __ldg(a.r + i), __ldg(a.v + i),
                                    __ldg(a.t + i), __ldg(a.ot + i));
+    };
+    while (begin(j) < n) {
+        uint32_t after = 0;
+        if (lane == 0) after = atomicAdd(&sh.next, 1u);
+        after = __shfl_sync(0xffffffffu, after, 0);
+        fetch(after, b ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // each lane reads what it copied itself
+        const int64_t i = begin(j) + lane;
+        bool done = true;
+        if (i < n) {
+            const F64Slot<T>& d = sh.slot[b][warp];
+            const uint64_t s = dbits(d.s[lane]), k = dbits(d.k[lane]), r = dbits(d.r[lane]),
+                           v = dbits(d.v[lane]), t = dbits(d.t[lane]);
+            double p;
+            done = bsg_fx::fx64_domain(s, k, r, v, t);
+            if (done) done = bsg_fx::price_fx64(sh, sh.tails, s, k, r, v, t, d.ot[lane], &p);
+            if (done) a.out[i] = p;
+        }
+        uint32_t q = 0;
+        if (!done) {
+            q = atomicAdd(&sh.queued, 1u);
+            if (atomicCAS(&sh.queue[q % kF64Queue], kEmpty, j * 32 + lane) != kEmpty) price_left(j * 32 + lane);
+        }
+        // whoever fills up 32 entries prices those that are there (one whose
+        // writer is not that far yet stays until the end), unless the block is
+        // nearly through: then the rest is priced side by side at the end
+        const bool fills = q % 32 == 31 && begin(j + 4 * kF64Warps) < n;
+        for (unsigned full = __ballot_sync(0xffffffffu, fills); full; full &= full - 1) {
+            const uint32_t last = __shfl_sync(0xffffffffu, q, __ffs(full) - 1);
+            const uint32_t at = atomicExch(&sh.queue[(last - lane) % kF64Queue], kEmpty);
+            if (at != kEmpty) price_left(at);
+            __syncwarp();
+        }
+        j = after;
+        b ^= 1;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    for (int q = threadIdx.x; q < kF64Queue; q += kF64Threads)
+        if (sh.queue[q] != kEmpty) price_left(sh.queue[q]);
 }
 
 template <typename T>
 static cudaError_t launch_f64_view(const F64View<T>& a, int64_t n, int sm_count, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    cudaError_t e = opt_in_smem<map_f64_kernel<T>>(sizeof(F64Shared));
+    cudaError_t e = opt_in_smem<map_f64_kernel<T>>(sizeof(F64Shared<T>));
     if (e != cudaSuccess) return e;
-    int64_t grid = (n + kF64Threads - 1) / kF64Threads;
-    const int64_t cap = (int64_t)sm_count * 4;
-    if (grid > cap) grid = cap;
-    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, sizeof(F64Shared), st>>>(a, n);
+    const int64_t grid = std::min<int64_t>((n + 31) / 32, sm_count);
+    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, sizeof(F64Shared<T>), st>>>(a, n);
     return cudaGetLastError();
 }
 
