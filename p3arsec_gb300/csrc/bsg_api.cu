@@ -592,6 +592,13 @@ bool pageable_view(const bsg_ctx* c, const bsg::SoA& h, size_t n, bool write) {
     return !write || populated(h.out, b, true);
 }
 
+// Whether all passes of a host call over memory that the GPU reaches are one
+// launch.
+bool one_launch(const bsg_ctx* c, size_t n, int runs, int mode, unsigned flags) {
+    return runs > 1 && !c->tuned && !(flags & BSG_NO_GRAPH) &&
+           bsg::map_runs_fit(c->resident(n), (int64_t)n, mode, runs, c->sm_count);
+}
+
 // A synchronous host call over memory that the GPU reads and writes in place
 // (`src`: the device's addresses of the arrays).
 int price_in_place(bsg_ctx* c, const bsg::SoA& src, size_t n, int runs, int mode, unsigned flags) {
@@ -602,6 +609,13 @@ int price_in_place(bsg_ctx* c, const bsg::SoA& src, size_t n, int runs, int mode
                                         c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "launch_map (host memory)");
         c->launches++;
+    } else if (one_launch(c, n, runs, mode, flags)) {
+        const bsg::HostBook book{src, c->d_parts, c->h_flag, ++c->call};
+        cudaError_t e = bsg::launch_map_runs(c->resident(n), (int64_t)n, mode, runs, c->sm_count, c->stream, &book);
+        if (e != cudaSuccess) return cuda_fail(c, e, "launch_map_runs (host memory)");
+        c->launches++;
+        BSG_CK(c, wait_flag(c));
+        return BSG_OK;
     } else {
         const bsg::SoA d = c->resident(n);
         cudaError_t e = bsg::launch_gather(src, d, (int64_t)n, c->sm_count, c->stream);
@@ -910,7 +924,7 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
         bsg::SoA view;
         if (!c->debug && (num_runs == 1 || n <= kGatherOptions)) {
             if (pinned_view(a, n, &view)) return price_in_place(c, view, n, num_runs, mode, flags);
-            if (pageable_view(c, a, n, num_runs == 1))
+            if (pageable_view(c, a, n, num_runs == 1 || one_launch(c, n, num_runs, mode, flags)))
                 return price_in_place(c, a, n, num_runs, mode, flags);
         }
         if ((st = debug_arm(c, n))) return st;

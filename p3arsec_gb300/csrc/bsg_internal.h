@@ -83,7 +83,18 @@ inline MapCfg pass_cfg(MapCfg c, int j, int runs) {
 MapCfg map_default_cfg(const SoA& a, int64_t n, int runs);
 // Whether launch_map_runs takes `runs` passes of this book (in one launch).
 bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count);
-cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st);
+// A host book's arrays, as the device sees them, and how to tell the host that
+// the prices are there (signal_host).
+struct HostBook {
+    SoA at;
+    unsigned* count;
+    unsigned* flag;
+    unsigned seq;
+};
+// All passes in one launch; with `host` over its book, by way of the device
+// arrays a (16-byte aligned), where the kernel stores seq to *flag at its end.
+cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st,
+                            const HostBook* host = nullptr);
 #if defined(__CUDACC__)
 // One thread of each of `parts` parts of a kernel, once the part's stores are
 // made (and seen by this thread): the last one zeroes the count and stores seq

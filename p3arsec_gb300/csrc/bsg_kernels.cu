@@ -233,12 +233,19 @@ __global__ void __launch_bounds__(M == MODE_LIBM_REF ? 256 : 512,
 // launches, not its bytes (65,536 options: 1.8 MB).  The whole call, 65,536
 // options x 100 passes: 41 us, 58 with one pass in flight, 91 as a graph of
 // programmatic launches, 212 as a graph of plain ones; 100 options: 31, 47,
-// 78, 155.
-template <int W>
+// 78, 155.  Of a host book of 65,536 pinned options x 100 passes a launch that
+// first gathered it (14 us), this kernel (29) and a copy of the prices took 65;
+// with HOST, the kernel that does all three, 54; x 2, 40 and 30.
+template <int W, bool OWN>  // OWN: written by this thread before
 __device__ __forceinline__ Raw<W> ld_again(const void* p) {
     Raw<W> r;
-    if constexpr (W == 2)
+    if constexpr (W == 2 && OWN)
+        asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(r.v[0]), "=r"(r.v[1]) : "l"(p) : "memory");
+    else if constexpr (W == 2)
         asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.v[0]), "=r"(r.v[1]) : "l"(p));
+    else if constexpr (OWN)
+        asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p) : "memory");
     else
         asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]) : "l"(p));
@@ -251,22 +258,61 @@ __device__ __forceinline__ float2 price2(float2 s, float2 k, float2 r, float2 v,
     else return make_float2(price<M>(s.x, k.x, r.x, v.x, t.x, o0), price<M>(s.y, k.y, r.y, v.y, t.y, o1));
 }
 
-template <int M, int W, int U>
-__global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int head, int runs) {
+// W words from host memory (s + o) to device memory (d + o).
+template <int W>
+__device__ __forceinline__ void take_words(const void* s, const void* d, int64_t o) {
+    using V = typename std::conditional<W == 2, uint2, uint4>::type;
+    const uint32_t* from = static_cast<const uint32_t*>(s) + o;
+    uint32_t* to = const_cast<uint32_t*>(static_cast<const uint32_t*>(d)) + o;
+    if ((reinterpret_cast<uintptr_t>(s) & (4 * W - 1)) == 0) {
+        *reinterpret_cast<V*>(to) = __ldg(reinterpret_cast<const V*>(from));
+    } else {
+        uint32_t x[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) x[i] = __ldg(from + i);
+#pragma unroll
+        for (int i = 0; i < W; ++i) to[i] = x[i];
+    }
+}
+
+template <int W>
+__device__ __forceinline__ void give_words(float* to, const float* p) {
+    if ((reinterpret_cast<uintptr_t>(to) & (4 * W - 1)) == 0) {
+        if constexpr (W == 2) *reinterpret_cast<float2*>(to) = make_float2(p[0], p[1]);
+        else *reinterpret_cast<float4*>(to) = make_float4(p[0], p[1], p[2], p[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < W; ++i) to[i] = p[i];
+    }
+}
+
+// HOST: the book is the host's: each thread first brings its options into a
+// (device arrays, aligned), and the last pass's prices go to the host too.
+template <int M, int W, int U, bool HOST>
+__global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int head, int runs,
+                                                                        HostBook host) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t o = g * W;
     if (o + W <= n) {
+        if constexpr (HOST) {
+            take_words<W>(host.at.s, a.s, o);
+            take_words<W>(host.at.k, a.k, o);
+            take_words<W>(host.at.r, a.r, o);
+            take_words<W>(host.at.v, a.v, o);
+            take_words<W>(host.at.t, a.t, o);
+            take_words<W>(host.at.ot, a.ot, o);
+        }
         for (int j = 0; j < runs; j += U) {
             Raw<W> S[U], K[U], R[U], V[U], T[U], O[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (j + u < runs) {
-                    S[u] = ld_again<W>(a.s + o);
-                    K[u] = ld_again<W>(a.k + o);
-                    R[u] = ld_again<W>(a.r + o);
-                    V[u] = ld_again<W>(a.v + o);
-                    T[u] = ld_again<W>(a.t + o);
-                    O[u] = ld_again<W>(a.ot + o);
+                    S[u] = ld_again<W, HOST>(a.s + o);
+                    K[u] = ld_again<W, HOST>(a.k + o);
+                    R[u] = ld_again<W, HOST>(a.r + o);
+                    V[u] = ld_again<W, HOST>(a.v + o);
+                    T[u] = ld_again<W, HOST>(a.t + o);
+                    O[u] = ld_again<W, HOST>(a.ot + o);
                 }
             float p[U][W];
 #pragma unroll
@@ -294,14 +340,51 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
                         asm volatile("st.global.v4.f32 [%0], {%1,%2,%3,%4};"
                                      :: "l"(a.out + o), "f"(p[u][0]), "f"(p[u][1]), "f"(p[u][2]), "f"(p[u][3])
                                      : "memory");
+                    if (HOST && j + u == runs - 1) give_words<W>(host.at.out + o, p[u]);
                 }
         }
     }
-    // the options before the first vector and after the last: two warps of the last block
+    // the options before the first vector and after the last: two warps of the
+    // last block, which has no others then
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 64) {
         const int64_t i = threadIdx.x < 32 ? n / W * W + threadIdx.x : (int64_t)threadIdx.x - 32 - head;
-        if (threadIdx.x < 32 ? i < n : i < 0)
-            for (int j = 0; j < runs; ++j) price_scalar<M>(a, i);
+        if (threadIdx.x < 32 ? i < n : i < 0) {
+            if constexpr (HOST) {
+                const_cast<float*>(a.s)[i] = host.at.s[i];
+                const_cast<float*>(a.k)[i] = host.at.k[i];
+                const_cast<float*>(a.r)[i] = host.at.r[i];
+                const_cast<float*>(a.v)[i] = host.at.v[i];
+                const_cast<float*>(a.t)[i] = host.at.t[i];
+                const_cast<int32_t*>(a.ot)[i] = host.at.ot[i];
+            }
+            auto f = [&](const float* x) { return *const_cast<const volatile float*>(x + i); };
+            constexpr int kTail = 4;  // passes in flight
+            float p = 0.0f;
+            for (int j = 0; j < runs; j += kTail) {
+                float in[kTail][5], q[kTail];
+                int ot[kTail];
+#pragma unroll
+                for (int u = 0; u < kTail; ++u) {
+                    in[u][0] = f(a.s);
+                    in[u][1] = f(a.k);
+                    in[u][2] = f(a.r);
+                    in[u][3] = f(a.v);
+                    in[u][4] = f(a.t);
+                    ot[u] = *const_cast<const volatile int32_t*>(a.ot + i);
+                }
+#pragma unroll
+                for (int u = 0; u < kTail; ++u)
+                    q[u] = price<M>(in[u][0], in[u][1], in[u][2], in[u][3], in[u][4], ot[u]);
+#pragma unroll
+                for (int u = 0; u < kTail; ++u)
+                    if (j + u < runs) *const_cast<volatile float*>(a.out + i) = p = q[u];
+            }
+            if constexpr (HOST) host.at.out[i] = p;
+        }
+    }
+    if constexpr (HOST) {
+        __syncthreads();
+        if (threadIdx.x == 0) signal_host(host.count, gridDim.x, host.flag, host.seq);
     }
 }
 
@@ -780,19 +863,24 @@ cudaError_t launch_map(const SoA& a, int64_t n, int mode, const MapCfg& cfg,
 }
 
 template <int M>
-static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cudaStream_t st) {
+static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cudaStream_t st, const HostBook* host) {
     const int head = peel(&a, &n, 16);
-    if (head < 0) return cudaErrorInvalidValue;
+    if (head < 0 || (host && head)) return cudaErrorInvalidValue;
     // two options per thread while that needs no more than 512 threads an SM
     // (155,000 options x 100: 57 us; four a thread would leave half the warps)
     const bool pairs = n <= (int64_t)sm_count * 1024;
     const int64_t ngroups = n / (pairs ? 2 : 4);
     int64_t block = (((ngroups + sm_count - 1) / sm_count) + 31) / 32 * 32;
     block = block < 64 ? 64 : block > 512 ? 512 : block;
-    int64_t grid = (ngroups + block - 1) / block;
+    // (a block of its own for the options before and after the vectors, so that
+    // their passes run beside the others': 20,001 options x 100 on the device 49 us without)
+    const bool odd = head || n % (pairs ? 2 : 4);
+    int64_t grid = (ngroups + block - 1) / block + odd;
     if (grid < 1) grid = 1;
-    if (pairs) map_runs_kernel<M, 2, 4><<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs);
-    else map_runs_kernel<M, 4, 2><<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs);
+    const HostBook h = host ? *host : HostBook{};
+    auto* kernel = pairs ? (host ? map_runs_kernel<M, 2, 4, true> : map_runs_kernel<M, 2, 4, false>)
+                         : (host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>);
+    kernel<<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs, h);
     return cudaGetLastError();
 }
 
@@ -818,11 +906,12 @@ bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count) {
            peel(&b, &m, 16) >= 0;
 }
 
-cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st) {
-    if (n <= 0 || runs <= 0) return cudaSuccess;
+cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st,
+                            const HostBook* host) {
+    if (n <= 0 || runs <= 0) return host ? cudaErrorInvalidValue : cudaSuccess;
     switch (mode) {
-        case MODE_FAST: return launch_runs_mode<MODE_FAST>(a, n, runs, sm_count, st);
-        case MODE_SFU_REF: return launch_runs_mode<MODE_SFU_REF>(a, n, runs, sm_count, st);
+        case MODE_FAST: return launch_runs_mode<MODE_FAST>(a, n, runs, sm_count, st, host);
+        case MODE_SFU_REF: return launch_runs_mode<MODE_SFU_REF>(a, n, runs, sm_count, st, host);
         default: return cudaErrorInvalidValue;
     }
 }

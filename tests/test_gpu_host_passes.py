@@ -1,0 +1,35 @@
+"""Several passes over a short host book are one kernel that brings the book in,
+makes the passes and writes the last one's prices to the host: the bits of a
+device call, nothing written beside them, at its edges (two and four options a
+thread, options left over at the end, arrays off the vector boundary)."""
+import numpy as np
+import pytest
+
+from p3arsec_gb300 import Context, books
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("pinned", [False, True], ids=["pageable", "pinned"])
+@pytest.mark.parametrize("n", [2, 8193, 155_648, 155_651, 311_296])
+def test_host_passes(n, pinned):
+    pad = 9
+    book = books.generate(n + pad, seed=8)
+    with Context(0, n + pad) as ctx:
+        for mode, lo in (("fast", 0), ("sfu_ref", 1), ("fast", 2)):
+            dev = [torch.from_numpy(a[lo:lo + n].copy()).cuda() for a in book.arrays()]
+            out = torch.zeros(n, device="cuda:0")
+            torch.cuda.synchronize()
+            ctx.price_soa(*dev, out, n=n, mode=mode, device=True)
+            want = out.cpu().numpy()
+            whole = np.empty(n + pad, np.float32)
+            arrays = [np.ascontiguousarray(a) for a in book.arrays()]
+            if pinned:
+                keep = [torch.from_numpy(a).pin_memory() for a in arrays + [whole]]
+                arrays, whole = [k.numpy() for k in keep[:6]], keep[6].numpy()
+            for runs in (2, 5, 100):
+                whole[:] = -1
+                ctx.price_soa(*[a[lo:lo + n] for a in arrays], whole[lo:lo + n], num_runs=runs, mode=mode)
+                assert np.array_equal(whole[lo:lo + n].view(np.uint32), want.view(np.uint32)), (mode, runs)
+                assert (whole[:lo] == -1).all() and (whole[lo + n:] == -1).all()
