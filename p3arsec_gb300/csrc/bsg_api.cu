@@ -77,6 +77,11 @@ size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // against 31 with six copies in, a launch and a copy out; 8,192: 22 against 50;
 // 32,768 would take 51 (0.8 MB at the host's 20 GB/s), 22 in place.
 constexpr size_t kStageOptions = 8192;
+// A pageable book of this many options or more is priced in two launches, so
+// that making most of its pages present (15 us for a book of 1M) goes on beside
+// the first.  131,072 options take 48 us either way, 200,001 57 against 62, 1M
+// 158 against 173, 16M 1,927 against 2,080.
+constexpr size_t kOverlapOptions = (size_t)1 << 17;
 constexpr size_t kStageBytes = 7 * kStageOptions * sizeof(float);
 // Host arrays in pinned memory, or in pageable memory whose page tables the
 // GPU walks, are read in place (one pass: 65,536 pinned options 22 us against
@@ -577,7 +582,7 @@ bool populated(const void* p, size_t bytes, bool write) {
                    write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) == 0;
 }
 
-bool pageable_view(const bsg_ctx* c, const bsg::SoA& h, size_t n, bool write) {
+bool pageable_book(const bsg_ctx* c, const bsg::SoA& h, size_t n) {
     if (!c->host_tables) return false;
     const void* p[6] = {h.s, h.k, h.r, h.v, h.t, h.ot};
     const uintptr_t o = reinterpret_cast<uintptr_t>(h.out);
@@ -587,9 +592,15 @@ bool pageable_view(const bsg_ctx* c, const bsg::SoA& h, size_t n, bool write) {
         const uintptr_t x = reinterpret_cast<uintptr_t>(q);
         if ((x & 3) || (x < o + b && o < x + b)) return false;
     }
+    return true;
+}
+
+// The pages of options [lo, lo + n) of a pageable_book.
+bool populated_book(const bsg::SoA& h, size_t lo, size_t n, bool write) {
+    const void* p[6] = {h.s, h.k, h.r, h.v, h.t, h.ot};
     for (const void* q : p)
-        if (!populated(q, b, false)) return false;
-    return !write || populated(h.out, b, true);
+        if (!populated(static_cast<const char*>(q) + 4 * lo, 4 * n, false)) return false;
+    return !write || populated(h.out + lo, 4 * n, true);
 }
 
 // Whether all passes of a host call over memory that the GPU reaches are one
@@ -599,16 +610,23 @@ bool one_launch(const bsg_ctx* c, size_t n, int runs, int mode, unsigned flags) 
            bsg::map_runs_fit(c->resident(n), (int64_t)n, mode, runs, c->sm_count);
 }
 
+// One pass over memory that the GPU reads and writes in place, behind what the
+// stream holds or (beside) as soon as there is room beside it.
+int enqueue_in_place(bsg_ctx* c, const bsg::SoA& src, size_t n, int mode, bool beside) {
+    // the tuned shapes are for device memory: plain 256-bit loads here
+    cudaError_t e = bsg::launch_map(src, (int64_t)n, mode, bsg::MapCfg{1, 128, 0, 2, beside}, c->sm_count,
+                                    c->stream);
+    if (e != cudaSuccess) return cuda_fail(c, e, "launch_map (host memory)");
+    c->launches++;
+    return BSG_OK;
+}
+
 // A synchronous host call over memory that the GPU reads and writes in place
 // (`src`: the device's addresses of the arrays).
 int price_in_place(bsg_ctx* c, const bsg::SoA& src, size_t n, int runs, int mode, unsigned flags) {
     int st;
     if (runs == 1) {
-        // the tuned shapes are for device memory: plain 256-bit loads here
-        cudaError_t e = bsg::launch_map(src, (int64_t)n, mode, bsg::MapCfg{1, 128, 0, 2, 0}, c->sm_count,
-                                        c->stream);
-        if (e != cudaSuccess) return cuda_fail(c, e, "launch_map (host memory)");
-        c->launches++;
+        if ((st = enqueue_in_place(c, src, n, mode, false))) return st;
     } else if (one_launch(c, n, runs, mode, flags)) {
         const bsg::HostBook book{src, c->d_parts, c->h_flag, ++c->call};
         cudaError_t e = bsg::launch_map_runs(c->resident(n), (int64_t)n, mode, runs, c->sm_count, c->stream, &book);
@@ -924,8 +942,22 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
         bsg::SoA view;
         if (!c->debug && (num_runs == 1 || n <= kGatherOptions)) {
             if (pinned_view(a, n, &view)) return price_in_place(c, view, n, num_runs, mode, flags);
-            if (pageable_view(c, a, n, num_runs == 1 || one_launch(c, n, num_runs, mode, flags)))
-                return price_in_place(c, a, n, num_runs, mode, flags);
+            if (pageable_book(c, a, n)) {
+                size_t first = n;
+                if (num_runs == 1 && n >= kOverlapOptions) first = round_up(n / 8, 1024);
+                const bool write = num_runs == 1 || one_launch(c, n, num_runs, mode, flags);
+                if (populated_book(a, 0, first, write)) {
+                    if (first == n) return price_in_place(c, a, n, num_runs, mode, flags);
+                    if ((st = enqueue_in_place(c, a, first, mode, false))) return st;
+                    if (populated_book(a, first, n - first, true)) {
+                        const bsg::SoA rest{a.s + first, a.k + first, a.r + first, a.v + first,
+                                            a.t + first, a.ot + first, a.out + first};
+                        if ((st = enqueue_in_place(c, rest, n - first, mode, true))) return st;
+                        BSG_CK(c, cudaStreamSynchronize(c->stream));
+                        return BSG_OK;
+                    }
+                }
+            }
         }
         if ((st = debug_arm(c, n))) return st;
         const bsg::SoA d = c->resident(n);

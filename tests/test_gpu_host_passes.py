@@ -33,3 +33,23 @@ def test_host_passes(n, pinned):
                 ctx.price_soa(*[a[lo:lo + n] for a in arrays], whole[lo:lo + n], num_runs=runs, mode=mode)
                 assert np.array_equal(whole[lo:lo + n].view(np.uint32), want.view(np.uint32)), (mode, runs)
                 assert (whole[:lo] == -1).all() and (whole[lo + n:] == -1).all()
+
+
+@pytest.mark.parametrize("n", [(1 << 17) - 1, 1 << 17, (1 << 17) + 1025, 400_007])
+def test_pageable_book_in_two_launches(n):
+    """From 2^17 options a pageable book's first eighth is priced while the rest
+    of its pages are made present: the bits of a device call at the seam and at
+    the ends, for arrays off the vector boundary too, nothing written beside."""
+    pad = 9
+    book = books.generate(n + pad, seed=9)
+    arrays = [np.ascontiguousarray(a) for a in book.arrays()]
+    with Context(0, n + pad) as ctx:
+        for mode, lo in (("fast", 0), ("libm_ref", 3), ("fast", 1)):
+            dev = [torch.from_numpy(a[lo:lo + n].copy()).cuda() for a in arrays]
+            out = torch.zeros(n, device="cuda:0")
+            torch.cuda.synchronize()
+            ctx.price_soa(*dev, out, n=n, mode=mode, device=True)
+            whole = np.full(n + pad, -1, np.float32)
+            ctx.price_soa(*[a[lo:lo + n] for a in arrays], whole[lo:lo + n], mode=mode)
+            assert np.array_equal(whole[lo:lo + n].view(np.uint32), out.cpu().numpy().view(np.uint32)), mode
+            assert (whole[:lo] == -1).all() and (whole[lo + n:] == -1).all()
