@@ -123,7 +123,9 @@ int bsg_BlkSchlsEqEuroNoDiv(float* OptionPrice, int numOptions, float* sptprice,
 
 /* FP64 product mode: double storage in and out, the types of the
  * reference's SIMD variant built with NCO = 2 (blackscholes.simd.c:68-81,
- * 221-298), num_runs passes.  Bound by the GPU's FP64 rate.  Host or device
+ * 221-298), num_runs passes.  Elementary functions in 64-bit fixed point, N
+ * rounded to 2^-53 as in doubles (errors below the double evaluation's; a price
+ * that is only that rounding may differ from it by a unit).  Host or device
  * pointers as bsg_price_soa (host calls stage through temporary device
  * memory). */
 int bsg_price_soa_f64(bsg_ctx* ctx, const double* sptprice, const double* strike,
