@@ -231,15 +231,20 @@ __global__ void __launch_bounds__(M == MODE_LIBM_REF ? 256 : 512,
 // (about 500 clocks each) overlap.
 // What bounds a short book is that chain and the interval between dependent
 // launches, not its bytes (65,536 options: 1.8 MB).  The whole call, 65,536
-// options x 100 passes: 41 us, 58 with one pass in flight, 91 as a graph of
-// programmatic launches, 212 as a graph of plain ones; 100 options: 31, 47,
-// 78, 155.  Of a host book of 65,536 pinned options x 100 passes a launch that
-// first gathered it (14 us), this kernel (29) and a copy of the prices took 65;
-// with HOST, the kernel that does all three, 54; x 2, 40 and 30.
+// options x 100 passes: 41 us (two options a thread and four passes in flight
+// 45, one pass 58), 91 as a graph of programmatic launches, 212 as a graph of
+// plain ones; 100 options: 27 (31, 47), 78, 155.  Of a host book of 65,536 pinned
+// options x 100 passes a launch that first gathered it (14 us), the passes (29)
+// and a copy of the prices took 65; with HOST, the kernel that does all three,
+// 49; x 2, 40 and 30.
 template <int W, bool OWN>  // OWN: written by this thread before
 __device__ __forceinline__ Raw<W> ld_again(const void* p) {
     Raw<W> r;
-    if constexpr (W == 2 && OWN)
+    if constexpr (W == 1 && OWN)
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(r.v[0]) : "l"(p) : "memory");
+    else if constexpr (W == 1)
+        asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(r.v[0]) : "l"(p));
+    else if constexpr (W == 2 && OWN)
         asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(r.v[0]), "=r"(r.v[1]) : "l"(p) : "memory");
     else if constexpr (W == 2)
         asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.v[0]), "=r"(r.v[1]) : "l"(p));
@@ -261,7 +266,7 @@ __device__ __forceinline__ float2 price2(float2 s, float2 k, float2 r, float2 v,
 // W words from host memory (s + o) to device memory (d + o).
 template <int W>
 __device__ __forceinline__ void take_words(const void* s, const void* d, int64_t o) {
-    using V = typename std::conditional<W == 2, uint2, uint4>::type;
+    using V = typename std::conditional<W == 1, uint32_t, typename std::conditional<W == 2, uint2, uint4>::type>::type;
     const uint32_t* from = static_cast<const uint32_t*>(s) + o;
     uint32_t* to = const_cast<uint32_t*>(static_cast<const uint32_t*>(d)) + o;
     if ((reinterpret_cast<uintptr_t>(s) & (4 * W - 1)) == 0) {
@@ -278,7 +283,8 @@ __device__ __forceinline__ void take_words(const void* s, const void* d, int64_t
 template <int W>
 __device__ __forceinline__ void give_words(float* to, const float* p) {
     if ((reinterpret_cast<uintptr_t>(to) & (4 * W - 1)) == 0) {
-        if constexpr (W == 2) *reinterpret_cast<float2*>(to) = make_float2(p[0], p[1]);
+        if constexpr (W == 1) *to = p[0];
+        else if constexpr (W == 2) *reinterpret_cast<float2*>(to) = make_float2(p[0], p[1]);
         else *reinterpret_cast<float4*>(to) = make_float4(p[0], p[1], p[2], p[3]);
     } else {
 #pragma unroll
@@ -315,25 +321,28 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
                     O[u] = ld_again<W, HOST>(a.ot + o);
                 }
             float p[U][W];
+            // two evaluations at a time: neighbouring options, or (W = 1) an
+            // option's neighbouring passes
+            constexpr int kPassStep = W == 1 ? 2 : 1;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
+            for (int u = 0; u < U; u += kPassStep) {
 #pragma unroll
                 for (int e = 0; e < W; e += 2) {
-                    const float2 q = price2<M>(
-                        make_float2(__uint_as_float(S[u].v[e]), __uint_as_float(S[u].v[e + 1])),
-                        make_float2(__uint_as_float(K[u].v[e]), __uint_as_float(K[u].v[e + 1])),
-                        make_float2(__uint_as_float(R[u].v[e]), __uint_as_float(R[u].v[e + 1])),
-                        make_float2(__uint_as_float(V[u].v[e]), __uint_as_float(V[u].v[e + 1])),
-                        make_float2(__uint_as_float(T[u].v[e]), __uint_as_float(T[u].v[e + 1])),
-                        (int)O[u].v[e], (int)O[u].v[e + 1]);
+                    const int u2 = W == 1 ? u + 1 : u, e2 = W == 1 ? e : e + 1;
+                    auto two = [&](const Raw<W>* x) {
+                        return make_float2(__uint_as_float(x[u].v[e]), __uint_as_float(x[u2].v[e2]));
+                    };
+                    const float2 q = price2<M>(two(S), two(K), two(R), two(V), two(T), (int)O[u].v[e], (int)O[u2].v[e2]);
                     p[u][e] = q.x;
-                    p[u][e + 1] = q.y;
+                    p[u2][e2] = q.y;
                 }
             }
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (j + u < runs) {
-                    if constexpr (W == 2)
+                    if constexpr (W == 1)
+                        asm volatile("st.global.f32 [%0], %1;" :: "l"(a.out + o), "f"(p[u][0]) : "memory");
+                    else if constexpr (W == 2)
                         asm volatile("st.global.v2.f32 [%0], {%1,%2};"
                                      :: "l"(a.out + o), "f"(p[u][0]), "f"(p[u][1]) : "memory");
                     else
@@ -864,22 +873,25 @@ cudaError_t launch_map(const SoA& a, int64_t n, int mode, const MapCfg& cfg,
 
 template <int M>
 static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cudaStream_t st, const HostBook* host) {
-    const int head = peel(&a, &n, 16);
+    // one, then two options per thread while that needs no more than 512 threads
+    // an SM: 40,000 options x 100 36 us with one, 44 with two (half the warps);
+    // 155,000 57 with two.  One option's passes are evaluated in pairs, four in
+    // flight (two 40, eight 39).
+    const int w = n <= (int64_t)sm_count * 512 ? 1 : n <= (int64_t)sm_count * 1024 ? 2 : 4;
+    const int head = w == 1 ? 0 : peel(&a, &n, 16);
     if (head < 0 || (host && head)) return cudaErrorInvalidValue;
-    // two options per thread while that needs no more than 512 threads an SM
-    // (155,000 options x 100: 57 us; four a thread would leave half the warps)
-    const bool pairs = n <= (int64_t)sm_count * 1024;
-    const int64_t ngroups = n / (pairs ? 2 : 4);
+    const int64_t ngroups = n / w;
     int64_t block = (((ngroups + sm_count - 1) / sm_count) + 31) / 32 * 32;
     block = block < 64 ? 64 : block > 512 ? 512 : block;
     // (a block of its own for the options before and after the vectors, so that
     // their passes run beside the others': 20,001 options x 100 on the device 49 us without)
-    const bool odd = head || n % (pairs ? 2 : 4);
+    const bool odd = head || n % w;
     int64_t grid = (ngroups + block - 1) / block + odd;
     if (grid < 1) grid = 1;
     const HostBook h = host ? *host : HostBook{};
-    auto* kernel = pairs ? (host ? map_runs_kernel<M, 2, 4, true> : map_runs_kernel<M, 2, 4, false>)
-                         : (host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>);
+    auto* kernel = w == 1   ? (host ? map_runs_kernel<M, 1, 4, true> : map_runs_kernel<M, 1, 4, false>)
+                   : w == 2 ? (host ? map_runs_kernel<M, 2, 4, true> : map_runs_kernel<M, 2, 4, false>)
+                            : (host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>);
     kernel<<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs, h);
     return cudaGetLastError();
 }

@@ -53,3 +53,22 @@ def test_pageable_book_in_two_launches(n):
             ctx.price_soa(*[a[lo:lo + n] for a in arrays], whole[lo:lo + n], mode=mode)
             assert np.array_equal(whole[lo:lo + n].view(np.uint32), out.cpu().numpy().view(np.uint32)), mode
             assert (whole[:lo] == -1).all() and (whole[lo + n:] == -1).all()
+
+
+@pytest.mark.parametrize("n", [1, 63, 77_824, 77_825])
+def test_passes_of_one_option_in_pairs(n):
+    """Up to 512 options an SM (152) a thread owns one option and evaluates its
+    passes two at a time: whatever their number, from any alignment, the bits of
+    one pass."""
+    book = books.generate(n + 3, seed=10)
+    with Context(0, 1) as ctx:
+        for mode, lo in (("fast", 0), ("sfu_ref", 3), ("fast", 1)):
+            dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda()[lo:lo + n] for a in book.arrays()]
+            want, got = (torch.full((n + 3,), -1.0, device="cuda:0") for _ in range(2))
+            torch.cuda.synchronize()
+            ctx.price_soa(*dev, want[lo:lo + n], n=n, mode=mode, device=True)
+            for runs in (2, 3, 4, 5, 9):
+                got.fill_(-1)
+                torch.cuda.synchronize()
+                ctx.price_soa(*dev, got[lo:lo + n], n=n, num_runs=runs, mode=mode, device=True)
+                assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (mode, lo, runs)
