@@ -260,6 +260,7 @@ __device__ __forceinline__ Raw<W> ld_again(const void* p) {
 template <int M>
 __device__ __forceinline__ float2 price2(float2 s, float2 k, float2 r, float2 v, float2 t, int o0, int o1) {
     if constexpr (M == MODE_FAST) return price_fast2(s, k, r, v, t, o0, o1);
+    else if constexpr (M == MODE_LIBM_REF) return price_libm_ref2(s, k, r, v, t, o0, o1);
     else return make_float2(price<M>(s.x, k.x, r.x, v.x, t.x, o0), price<M>(s.y, k.y, r.y, v.y, t.y, o1));
 }
 
@@ -889,9 +890,12 @@ static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cu
     int64_t grid = (ngroups + block - 1) / block + odd;
     if (grid < 1) grid = 1;
     const HostBook h = host ? *host : HostBook{};
-    auto* kernel = w == 1   ? (host ? map_runs_kernel<M, 1, 4, true> : map_runs_kernel<M, 1, 4, false>)
-                   : w == 2 ? (host ? map_runs_kernel<M, 2, 4, true> : map_runs_kernel<M, 2, 4, false>)
-                            : (host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>);
+    void (*kernel)(SoA, int64_t, int, int, HostBook) = nullptr;
+    constexpr int kPairs = M == MODE_LIBM_REF ? 2 : 4;  // passes of two options in flight
+    if (w == 1) kernel = host ? map_runs_kernel<M, 1, 4, true> : map_runs_kernel<M, 1, 4, false>;
+    else if (w == 2) kernel = host ? map_runs_kernel<M, 2, kPairs, true> : map_runs_kernel<M, 2, kPairs, false>;
+    else if constexpr (M != MODE_LIBM_REF) kernel = host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>;
+    if (!kernel) return cudaErrorInvalidValue;
     kernel<<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs, h);
     return cudaGetLastError();
 }
@@ -909,12 +913,13 @@ static bool in_place(const SoA& a, int64_t n) {
 
 // Up to 2048 options an SM (4 options a thread, 512 threads): 311,000 options x
 // 100 passes take 100 us, 117 as programmatic launches; at 622,592 both took
-// 222.  The reference-order libm mode stays with those: its evaluation fills
-// the SMs (65,536 x 100: 97 us against 140).
+// 222.  The reference-order libm mode up to 1024 (2 a thread): 155,648 options
+// 128 us against 141, 65,536 75 against 96, 1,000 42 against 70; at 200,000, four
+// a thread, 184 against 170.
 bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count) {
     SoA b = a;
     int64_t m = n;
-    return runs > 1 && mode != MODE_LIBM_REF && n <= (int64_t)sm_count * 2048 && !in_place(a, n) &&
+    return runs > 1 && n <= (int64_t)sm_count * (mode == MODE_LIBM_REF ? 1024 : 2048) && !in_place(a, n) &&
            peel(&b, &m, 16) >= 0;
 }
 
@@ -924,6 +929,7 @@ cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_
     switch (mode) {
         case MODE_FAST: return launch_runs_mode<MODE_FAST>(a, n, runs, sm_count, st, host);
         case MODE_SFU_REF: return launch_runs_mode<MODE_SFU_REF>(a, n, runs, sm_count, st, host);
+        case MODE_LIBM_REF: return launch_runs_mode<MODE_LIBM_REF>(a, n, runs, sm_count, st, host);
         default: return cudaErrorInvalidValue;
     }
 }

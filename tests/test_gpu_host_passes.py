@@ -17,7 +17,7 @@ def test_host_passes(n, pinned):
     pad = 9
     book = books.generate(n + pad, seed=8)
     with Context(0, n + pad) as ctx:
-        for mode, lo in (("fast", 0), ("sfu_ref", 1), ("fast", 2)):
+        for mode, lo in (("fast", 0), ("sfu_ref", 1), ("libm_ref", 2)):
             dev = [torch.from_numpy(a[lo:lo + n].copy()).cuda() for a in book.arrays()]
             out = torch.zeros(n, device="cuda:0")
             torch.cuda.synchronize()
@@ -55,14 +55,14 @@ def test_pageable_book_in_two_launches(n):
             assert (whole[:lo] == -1).all() and (whole[lo + n:] == -1).all()
 
 
-@pytest.mark.parametrize("n", [1, 63, 77_824, 77_825])
+@pytest.mark.parametrize("n", [1, 63, 77_824, 77_825, 155_648, 155_649])
 def test_passes_of_one_option_in_pairs(n):
     """Up to 512 options an SM (152) a thread owns one option and evaluates its
     passes two at a time: whatever their number, from any alignment, the bits of
     one pass."""
     book = books.generate(n + 3, seed=10)
     with Context(0, 1) as ctx:
-        for mode, lo in (("fast", 0), ("sfu_ref", 3), ("fast", 1)):
+        for mode, lo in (("fast", 0), ("sfu_ref", 3), ("libm_ref", 1)):
             dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda()[lo:lo + n] for a in book.arrays()]
             want, got = (torch.full((n + 3,), -1.0, device="cuda:0") for _ in range(2))
             torch.cuda.synchronize()
