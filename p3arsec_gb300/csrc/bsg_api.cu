@@ -119,8 +119,8 @@ struct bsg_ctx {
     std::string err;
     uint64_t launches = 0;
     std::vector<GraphEntry> graphs;
-    // batch scratch: per-tile [begin, end) of the batch (2 entries per tile),
-    // device and pinned staging
+    // batch scratch: a zero (a single pass's work counter) and a pad, then
+    // [begin, end) of each tile; device and pinned staging
     uint64_t* d_tb = nullptr;
     uint64_t* h_tb = nullptr;
     size_t tb_cap = 0;  // tiles
@@ -690,8 +690,9 @@ int grow_tile_scratch(bsg_ctx* c, size_t ntiles) {
     c->d_tb = nullptr;
     c->h_tb = nullptr;
     c->tb_cap = 0;
-    BSG_CK(c, cudaMalloc(&c->d_tb, 2 * cap * sizeof(uint64_t)));
-    BSG_CK(c, cudaMallocHost(&c->h_tb, 2 * cap * sizeof(uint64_t)));
+    BSG_CK(c, cudaMalloc(&c->d_tb, (2 + 2 * cap) * sizeof(uint64_t)));
+    BSG_CK(c, cudaMallocHost(&c->h_tb, (2 + 2 * cap) * sizeof(uint64_t)));
+    c->h_tb[0] = c->h_tb[1] = 0;
     c->tb_cap = cap;
     return BSG_OK;
 }
@@ -735,7 +736,7 @@ int build_segments(bsg_ctx* c, const bsg_segment* segs, size_t nseg, size_t pool
         for (const Span& x : v) total += (x.second - x.first + tile - 1) / tile;
     }
     if (int st = grow_tile_scratch(c, total)) return st;
-    uint64_t* tb = c->h_tb;
+    uint64_t* tb = c->h_tb + 2;
     for (const Span& x : v)
         for (uint64_t b = x.first; b < x.second; b += tile, tb += 2) {
             tb[0] = b;
@@ -1121,8 +1122,21 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
         uint64_t ntiles = 0;
         if ((st = build_segments(c, segs, nseg, pool_len, topt, &ntiles))) return st;
         if (ntiles == 0) return finish(c, flags);
-        BSG_CK(c, cudaMemcpyAsync(c->d_tb, c->h_tb, ntiles * 16, cudaMemcpyHostToDevice, c->stream));
-        BSG_CK(c, cudaEventRecord(c->seg_ev, c->stream));
+        BSG_CK(c, cudaMemcpyAsync(c->d_tb, c->h_tb, (1 + ntiles) * 16, cudaMemcpyHostToDevice, c->stream));
+        // (a synchronous call is through with the staging when it returns)
+        if (flags & BSG_ASYNC) BSG_CK(c, cudaEventRecord(c->seg_ev, c->stream));
+        if (num_runs == 1) {
+            // one pass: its work counter is the zero in front of the table (64
+            // books of up to 4,096 options 26 us; with a memset of a counter 29)
+            cudaError_t e = bsg::launch_batch(a, c->d_tb + 2, ntiles, reinterpret_cast<unsigned long long*>(c->d_tb),
+                                              mode, grid, 0, c->stream);
+            if (e != cudaSuccess) {
+                cudaStreamSynchronize(c->stream);  // the staging is free again
+                return cuda_fail(c, e, "launch_batch");
+            }
+            c->launches++;
+            return finish(c, flags);
+        }
         // one work counter per pass, zeroed together, so that pass j + 1 can
         // start (PDL) while pass j drains
         if ((size_t)num_runs > c->cursor_cap) {
@@ -1139,11 +1153,11 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
         auto all_runs = [&]() -> cudaError_t {
             cudaError_t e = cudaMemsetAsync(c->d_cursor, 0, (size_t)num_runs * 8, c->stream);
             for (int j = 0; j < num_runs && e == cudaSuccess; ++j)
-                e = bsg::launch_batch(a, c->d_tb, ntiles, c->d_cursor + j,
+                e = bsg::launch_batch(a, c->d_tb + 2, ntiles, c->d_cursor + j,
                                       mode, grid, j > 0 ? 1 : 0, c->stream);
             return e;
         };
-        if (num_runs == 1 || (flags & BSG_NO_GRAPH)) {
+        if (flags & BSG_NO_GRAPH) {
             cudaError_t e = all_runs();
             if (e != cudaSuccess) return cuda_fail(c, e, "launch_batch");
             c->launches += (uint64_t)num_runs;
