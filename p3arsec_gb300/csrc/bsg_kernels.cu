@@ -915,11 +915,11 @@ static bool in_place(const SoA& a, int64_t n) {
 // 100 passes take 100 us, 117 as programmatic launches; at 622,592 both took
 // 222.  The reference-order libm mode up to 1024 (2 a thread): 155,648 options
 // 128 us against 141, 65,536 75 against 96, 1,000 42 against 70; at 200,000, four
-// a thread, 184 against 170.
+// a thread, 184 against 170.  (The kernel's pass counter runs a step past `runs`.)
 bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count) {
     SoA b = a;
     int64_t m = n;
-    return runs > 1 && n <= (int64_t)sm_count * (mode == MODE_LIBM_REF ? 1024 : 2048) && !in_place(a, n) &&
+    return runs > 1 && runs <= 1 << 30 && n <= (int64_t)sm_count * (mode == MODE_LIBM_REF ? 1024 : 2048) && !in_place(a, n) &&
            peel(&b, &m, 16) >= 0;
 }
 
