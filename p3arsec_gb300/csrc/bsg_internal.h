@@ -83,18 +83,19 @@ inline MapCfg pass_cfg(MapCfg c, int j, int runs) {
 MapCfg map_default_cfg(const SoA& a, int64_t n, int runs);
 // Whether launch_map_runs takes `runs` passes of this book (in one launch).
 bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count);
-// A host book's arrays, as the device sees them, and how to tell the host that
-// the prices are there (signal_host).
-struct HostBook {
-    SoA at;
+// How a kernel tells the host that it is done (signal_host): a device counter,
+// zero, left zero, and a word in pinned memory that gets seq.  flag NULL: not.
+struct Signal {
     unsigned* count;
     unsigned* flag;
     unsigned seq;
 };
-// All passes in one launch; with `host` over its book, by way of the device
-// arrays a (16-byte aligned), where the kernel stores seq to *flag at its end.
+// All passes in one launch; with `host` (the device's addresses of a host book)
+// over that book, by way of the device arrays a (16-byte aligned).
 cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st,
-                            const HostBook* host = nullptr);
+                            const Signal& sig = Signal{}, const SoA* host = nullptr);
+// Whether the n prices share memory with an input array.
+bool in_place(const SoA& a, int64_t n);
 #if defined(__CUDACC__)
 // One thread of each of `parts` parts of a kernel, once the part's stores are
 // made (and seen by this thread): the last one zeroes the count and stores seq
@@ -111,11 +112,9 @@ __device__ __forceinline__ void signal_host(unsigned* count, unsigned parts, uns
 }
 #endif
 
-// One pass over n options of pinned, 16-byte aligned host arrays (device
-// addresses) that stores seq to *flag (pinned) at its end; count: a device
-// counter, zero, left zero.
-cudaError_t launch_map_stage(const SoA& a, int n, int mode, unsigned* count, unsigned* flag, unsigned seq,
-                             cudaStream_t st);
+// One pass over n options of 16-byte aligned arrays, in device memory or pinned
+// host memory (its device addresses).
+cudaError_t launch_map_stage(const SoA& a, int n, int mode, const Signal& sig, cudaStream_t st);
 // Copies n options' six input arrays from src (pinned host memory, its device
 // addresses) into dst's, by one kernel.
 cudaError_t launch_gather(const SoA& src, const SoA& dst, int64_t n, int sm_count, cudaStream_t st);
@@ -130,10 +129,10 @@ cudaError_t launch_bulk_wait_selftest(const SoA& a, int64_t n, int sm_count, uin
 // True when launch_map would take the vector path for these pointers.
 bool map_vectorizable(const SoA& a, const MapCfg& cfg);
 
-cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count,
-                        cudaStream_t st);
+cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count, cudaStream_t st,
+                        const Signal& sig = Signal{});
 // One pass of the FP64 product mode over n options.
-cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st);
+cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st, const Signal& sig = Signal{});
 
 // Persistent batched pricing over a device table of ntiles tiles, each its
 // [begin, end) in the pool.  cursor is a device counter that must be 0 at

@@ -297,17 +297,17 @@ __device__ __forceinline__ void give_words(float* to, const float* p) {
 // (device arrays, aligned), and the last pass's prices go to the host too.
 template <int M, int W, int U, bool HOST>
 __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int head, int runs,
-                                                                        HostBook host) {
+                                                                        SoA host, Signal sig) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t o = g * W;
     if (o + W <= n) {
         if constexpr (HOST) {
-            take_words<W>(host.at.s, a.s, o);
-            take_words<W>(host.at.k, a.k, o);
-            take_words<W>(host.at.r, a.r, o);
-            take_words<W>(host.at.v, a.v, o);
-            take_words<W>(host.at.t, a.t, o);
-            take_words<W>(host.at.ot, a.ot, o);
+            take_words<W>(host.s, a.s, o);
+            take_words<W>(host.k, a.k, o);
+            take_words<W>(host.r, a.r, o);
+            take_words<W>(host.v, a.v, o);
+            take_words<W>(host.t, a.t, o);
+            take_words<W>(host.ot, a.ot, o);
         }
         for (int j = 0; j < runs; j += U) {
             Raw<W> S[U], K[U], R[U], V[U], T[U], O[U];
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
                         asm volatile("st.global.v4.f32 [%0], {%1,%2,%3,%4};"
                                      :: "l"(a.out + o), "f"(p[u][0]), "f"(p[u][1]), "f"(p[u][2]), "f"(p[u][3])
                                      : "memory");
-                    if (HOST && j + u == runs - 1) give_words<W>(host.at.out + o, p[u]);
+                    if (HOST && j + u == runs - 1) give_words<W>(host.out + o, p[u]);
                 }
         }
     }
@@ -360,12 +360,12 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
         const int64_t i = threadIdx.x < 32 ? n / W * W + threadIdx.x : (int64_t)threadIdx.x - 32 - head;
         if (threadIdx.x < 32 ? i < n : i < 0) {
             if constexpr (HOST) {
-                const_cast<float*>(a.s)[i] = host.at.s[i];
-                const_cast<float*>(a.k)[i] = host.at.k[i];
-                const_cast<float*>(a.r)[i] = host.at.r[i];
-                const_cast<float*>(a.v)[i] = host.at.v[i];
-                const_cast<float*>(a.t)[i] = host.at.t[i];
-                const_cast<int32_t*>(a.ot)[i] = host.at.ot[i];
+                const_cast<float*>(a.s)[i] = host.s[i];
+                const_cast<float*>(a.k)[i] = host.k[i];
+                const_cast<float*>(a.r)[i] = host.r[i];
+                const_cast<float*>(a.v)[i] = host.v[i];
+                const_cast<float*>(a.t)[i] = host.t[i];
+                const_cast<int32_t*>(a.ot)[i] = host.ot[i];
             }
             auto f = [&](const float* x) { return *const_cast<const volatile float*>(x + i); };
             constexpr int kTail = 4;  // passes in flight
@@ -389,25 +389,24 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
                 for (int u = 0; u < kTail; ++u)
                     if (j + u < runs) *const_cast<volatile float*>(a.out + i) = p = q[u];
             }
-            if constexpr (HOST) host.at.out[i] = p;
+            if constexpr (HOST) host.out[i] = p;
         }
     }
-    if constexpr (HOST) {
+    if (sig.flag) {
         __syncthreads();
-        if (threadIdx.x == 0) signal_host(host.count, gridDim.x, host.flag, host.seq);
+        if (threadIdx.x == 0) signal_host(sig.count, gridDim.x, sig.flag, sig.seq);
     }
 }
 
-// One pass over a short host book in the context's staging (16-byte aligned
-// pinned arrays), which tells the host itself that it is done: the block that
-// finishes last stores `seq` to *flag, in pinned memory, after every price is
-// there.  The host polls that word: a call of 16 options takes 11.7 us, 13.7 with
-// a stream synchronisation.
+// One pass over a short book, in device memory or staged by the host (16-byte
+// aligned arrays), which tells the host itself that it is done: the block that
+// finishes last stores the call's number to a word in pinned memory, after every
+// price is there.  The host polls that word: a call of 16 options takes 11.7 us,
+// 13.7 with a stream synchronisation.
 constexpr int kStageThreads = 128;
 
 template <int M>
-__global__ void __launch_bounds__(kStageThreads) map_stage_kernel(SoA a, int n, unsigned* count, unsigned* flag,
-                                                                  unsigned seq) {
+__global__ void __launch_bounds__(kStageThreads) map_stage_kernel(SoA a, int n, Signal sig) {
     const int g = blockIdx.x * kStageThreads + threadIdx.x;
     if (4 * g + 4 <= n) {
         const float4 q = price4<M>(__ldg(reinterpret_cast<const float4*>(a.s) + g),
@@ -421,17 +420,16 @@ __global__ void __launch_bounds__(kStageThreads) map_stage_kernel(SoA a, int n, 
         for (int i = 4 * g; i < n; ++i) price_scalar<M>(a, i);
     }
     __syncthreads();
-    if (threadIdx.x == 0) signal_host(count, gridDim.x, flag, seq);
+    if (threadIdx.x == 0) signal_host(sig.count, gridDim.x, sig.flag, sig.seq);
 }
 
-cudaError_t launch_map_stage(const SoA& a, int n, int mode, unsigned* count, unsigned* flag, unsigned seq,
-                             cudaStream_t st) {
-    if (n <= 0) return cudaErrorInvalidValue;
+cudaError_t launch_map_stage(const SoA& a, int n, int mode, const Signal& sig, cudaStream_t st) {
+    if (n <= 0 || !sig.flag) return cudaErrorInvalidValue;
     const unsigned grid = (unsigned)((n + 4 * kStageThreads - 1) / (4 * kStageThreads));
     switch (mode) {
-        case MODE_FAST: map_stage_kernel<MODE_FAST><<<grid, kStageThreads, 0, st>>>(a, n, count, flag, seq); break;
-        case MODE_SFU_REF: map_stage_kernel<MODE_SFU_REF><<<grid, kStageThreads, 0, st>>>(a, n, count, flag, seq); break;
-        case MODE_LIBM_REF: map_stage_kernel<MODE_LIBM_REF><<<grid, kStageThreads, 0, st>>>(a, n, count, flag, seq); break;
+        case MODE_FAST: map_stage_kernel<MODE_FAST><<<grid, kStageThreads, 0, st>>>(a, n, sig); break;
+        case MODE_SFU_REF: map_stage_kernel<MODE_SFU_REF><<<grid, kStageThreads, 0, st>>>(a, n, sig); break;
+        case MODE_LIBM_REF: map_stage_kernel<MODE_LIBM_REF><<<grid, kStageThreads, 0, st>>>(a, n, sig); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -873,7 +871,8 @@ cudaError_t launch_map(const SoA& a, int64_t n, int mode, const MapCfg& cfg,
 }
 
 template <int M>
-static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cudaStream_t st, const HostBook* host) {
+static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cudaStream_t st, const Signal& sig,
+                                    const SoA* host) {
     // one, then two options per thread while that needs no more than 512 threads
     // an SM: 40,000 options x 100 36 us with one, 44 with two (half the warps);
     // 155,000 57 with two.  One option's passes are evaluated in pairs, four in
@@ -889,19 +888,19 @@ static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cu
     const bool odd = head || n % w;
     int64_t grid = (ngroups + block - 1) / block + odd;
     if (grid < 1) grid = 1;
-    const HostBook h = host ? *host : HostBook{};
-    void (*kernel)(SoA, int64_t, int, int, HostBook) = nullptr;
+    const SoA h = host ? *host : SoA{};
+    void (*kernel)(SoA, int64_t, int, int, SoA, Signal) = nullptr;
     constexpr int kPairs = M == MODE_LIBM_REF ? 2 : 4;  // passes of two options in flight
     if (w == 1) kernel = host ? map_runs_kernel<M, 1, 4, true> : map_runs_kernel<M, 1, 4, false>;
     else if (w == 2) kernel = host ? map_runs_kernel<M, 2, kPairs, true> : map_runs_kernel<M, 2, kPairs, false>;
     else if constexpr (M != MODE_LIBM_REF) kernel = host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>;
     if (!kernel) return cudaErrorInvalidValue;
-    kernel<<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs, h);
+    kernel<<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs, h, sig);
     return cudaGetLastError();
 }
 
 // Whether the n prices share memory with an input array.
-static bool in_place(const SoA& a, int64_t n) {
+bool in_place(const SoA& a, int64_t n) {
     const uintptr_t o = reinterpret_cast<uintptr_t>(a.out), b = (uintptr_t)n * 4;
     const void* p[6] = {a.s, a.k, a.r, a.v, a.t, a.ot};
     for (const void* q : p) {
@@ -924,12 +923,12 @@ bool map_runs_fit(const SoA& a, int64_t n, int mode, int runs, int sm_count) {
 }
 
 cudaError_t launch_map_runs(const SoA& a, int64_t n, int mode, int runs, int sm_count, cudaStream_t st,
-                            const HostBook* host) {
-    if (n <= 0 || runs <= 0) return host ? cudaErrorInvalidValue : cudaSuccess;
+                            const Signal& sig, const SoA* host) {
+    if (n <= 0 || runs <= 0) return host || sig.flag ? cudaErrorInvalidValue : cudaSuccess;
     switch (mode) {
-        case MODE_FAST: return launch_runs_mode<MODE_FAST>(a, n, runs, sm_count, st, host);
-        case MODE_SFU_REF: return launch_runs_mode<MODE_SFU_REF>(a, n, runs, sm_count, st, host);
-        case MODE_LIBM_REF: return launch_runs_mode<MODE_LIBM_REF>(a, n, runs, sm_count, st, host);
+        case MODE_FAST: return launch_runs_mode<MODE_FAST>(a, n, runs, sm_count, st, sig, host);
+        case MODE_SFU_REF: return launch_runs_mode<MODE_SFU_REF>(a, n, runs, sm_count, st, sig, host);
+        case MODE_LIBM_REF: return launch_runs_mode<MODE_LIBM_REF>(a, n, runs, sm_count, st, sig, host);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1038,7 +1037,7 @@ __device__ __forceinline__ void copy_async(T* dst, const T* src) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kF64Threads, 1) map_f64_kernel(F64View<T> a, int64_t n) {
+__global__ void __launch_bounds__(kF64Threads, 1) map_f64_kernel(F64View<T> a, int64_t n, Signal sig) {
     extern __shared__ __align__(16) char f64_smem[];
     F64Shared<T>& sh = *reinterpret_cast<F64Shared<T>*>(f64_smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1114,25 +1113,28 @@ __global__ void __launch_bounds__(kF64Threads, 1) map_f64_kernel(F64View<T> a, i
     __syncthreads();
     for (int q = threadIdx.x; q < kF64Queue; q += kF64Threads)
         if (sh.queue[q] != kEmpty) price_left(sh.queue[q]);
+    if (sig.flag) {
+        __syncthreads();
+        if (threadIdx.x == 0) signal_host(sig.count, gridDim.x, sig.flag, sig.seq);
+    }
 }
 
 template <typename T>
-static cudaError_t launch_f64_view(const F64View<T>& a, int64_t n, int sm_count, cudaStream_t st) {
+static cudaError_t launch_f64_view(const F64View<T>& a, int64_t n, int sm_count, cudaStream_t st, const Signal& sig) {
     if (n <= 0) return cudaSuccess;
     cudaError_t e = opt_in_smem<map_f64_kernel<T>>(sizeof(F64Shared<T>));
     if (e != cudaSuccess) return e;
     const int64_t grid = std::min<int64_t>((n + 31) / 32, sm_count);
-    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, sizeof(F64Shared<T>), st>>>(a, n);
+    map_f64_kernel<T><<<(unsigned)grid, kF64Threads, sizeof(F64Shared<T>), st>>>(a, n, sig);
     return cudaGetLastError();
 }
 
-cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st) {
-    return launch_f64_view(F64View<double>{a.s, a.k, a.r, a.v, a.t, a.ot, a.out}, n, sm_count, st);
+cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t st, const Signal& sig) {
+    return launch_f64_view(F64View<double>{a.s, a.k, a.r, a.v, a.t, a.ot, a.out}, n, sm_count, st, sig);
 }
 
-cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count,
-                        cudaStream_t st) {
-    return launch_f64_view(F64View<float>{a.s, a.k, a.r, a.v, a.t, a.ot, out}, n, sm_count, st);
+cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count, cudaStream_t st, const Signal& sig) {
+    return launch_f64_view(F64View<float>{a.s, a.k, a.r, a.v, a.t, a.ot, out}, n, sm_count, st, sig);
 }
 
 // ------------------------------------------------------------ batched books

@@ -1,0 +1,36 @@
+"""Short synchronous device calls wait for a word that their kernel stores; the
+asynchronous call of the same book goes the other way.  Same bits, nothing
+written beside, and a synchronous call leaves nothing of an asynchronous one
+before it unfinished."""
+import numpy as np
+import pytest
+
+from p3arsec_gb300 import Context, books
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+N_MAX = 1 << 18  # kFlagOptions
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 511, 513, N_MAX, N_MAX + 1])
+def test_short_device_calls(n):
+    book = books.generate(n + 4, seed=14)
+    cols = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in book.arrays()]
+    wide = [c.double() for c in cols[:5]] + [cols[5]]
+    with Context(0, 1) as ctx:
+        for mode in ("fast", "sfu_ref", "libm_ref"):
+            one, two = (torch.full((n + 4,), -1.0, device="cuda:0") for _ in range(2))
+            torch.cuda.synchronize()
+            ctx.price_soa(*cols, one, n=n, mode=mode, device=True, asynchronous=True)
+            ctx.price_soa(*cols, two, n=n, mode=mode, device=True)
+            assert torch.equal(one.view(torch.int32), two.view(torch.int32)), mode
+            assert (two[n:] == -1).all()
+        one, two, three = (torch.full((n + 4,), -1.0, device="cuda:0", dtype=torch.float64) for _ in range(3))
+        torch.cuda.synchronize()
+        ctx.price_soa_f64(*wide, one, n=n, device=True, asynchronous=True)
+        ctx.price_soa_f64(*wide, two, n=n, num_runs=2, device=True)
+        ctx.price_fp64(*cols, three, n=n, device=True)
+        assert torch.equal(one.view(torch.int64), two.view(torch.int64))
+        assert torch.equal(one.view(torch.int64), three.view(torch.int64))
+        assert (two[n:] == -1).all()
