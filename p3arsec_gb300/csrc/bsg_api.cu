@@ -85,7 +85,9 @@ constexpr size_t kOverlapOptions = (size_t)1 << 17;
 // Synchronous device calls of one pass up to this many options wait for a word
 // that the kernel stores to pinned memory, not for the stream: 1,000 options 11.9
 // us against 13.7, 65,536 12.2 against 13.6, 262,144 13.8 against 14.7 (each block
-// of 512 options counts itself; beyond, map_vec_kernel's shapes are ahead).
+// of 512 options counts itself; beyond, map_vec_kernel's shapes are ahead), from
+// option 3 of a book 12.0 against 13.7.  The libm mode up to half of it (131,072
+// from option 3 15.5 against 15.9, 262,144 16.7 against 16.2).
 constexpr size_t kFlagOptions = (size_t)1 << 18;
 constexpr size_t kStageBytes = 7 * kStageOptions * sizeof(float);
 // Host arrays in pinned memory, or in pageable memory whose page tables the
@@ -525,13 +527,6 @@ int ensure_pipeline(bsg_ctx* c) {
 // The next call's number, and where its kernel stores it.
 bsg::Signal next_signal(bsg_ctx* c) { return bsg::Signal{c->d_parts, c->h_flag, ++c->call}; }
 
-bool aligned16(const bsg::SoA& a) {
-    const void* p[7] = {a.s, a.k, a.r, a.v, a.t, a.ot, a.out};
-    uintptr_t x = 0;
-    for (const void* q : p) x |= reinterpret_cast<uintptr_t>(q);
-    return (x & 15) == 0;
-}
-
 // Waits for the kernel of this call (number c->call) to store that number to
 // *h_flag: by polling the word, which sees it 2 us before the driver's stream
 // synchronisation would return, and after 2 ms by that (which also returns
@@ -930,12 +925,12 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
         if (flags & BSG_DEVICE_PTRS) {
             if ((st = check_soa_dev(c, a, n, 4))) return st;
             if (!(flags & BSG_ASYNC) && !c->tuned && !c->debug) {
-                cudaError_t e = cudaErrorNotReady;
-                if (num_runs == 1 && n <= kFlagOptions && aligned16(a) && !bsg::in_place(a, (int64_t)n))
-                    e = bsg::launch_map_stage(a, (int)n, mode, next_signal(c), c->stream);
+                cudaError_t e = cudaErrorNotSupported;
+                if (num_runs == 1 && n <= kFlagOptions >> (mode == bsg::MODE_LIBM_REF) && !bsg::in_place(a, (int64_t)n))
+                    e = bsg::launch_map_stage(a, (int64_t)n, mode, next_signal(c), c->stream);
                 else if (!(flags & BSG_NO_GRAPH) && bsg::map_runs_fit(a, (int64_t)n, mode, num_runs, c->sm_count))
                     e = bsg::launch_map_runs(a, (int64_t)n, mode, num_runs, c->sm_count, c->stream, next_signal(c));
-                if (e != cudaErrorNotReady) {
+                if (e != cudaErrorNotSupported) {
                     if (e != cudaSuccess) return cuda_fail(c, e, "launch_map");
                     c->launches++;
                     BSG_CK(c, wait_flag(c));
@@ -958,7 +953,7 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
             const bsg::SoA h{f, f + al, f + 2 * al, f + 3 * al, f + 4 * al,
                              reinterpret_cast<const int32_t*>(f + 5 * al), f + 6 * al};
             if (num_runs == 1) {
-                cudaError_t e = bsg::launch_map_stage(h, (int)n, mode, next_signal(c), c->stream);
+                cudaError_t e = bsg::launch_map_stage(h, (int64_t)n, mode, next_signal(c), c->stream);
                 if (e != cudaSuccess) return cuda_fail(c, e, "launch_map_stage");
                 c->launches++;
                 BSG_CK(c, wait_flag(c));

@@ -112,9 +112,10 @@ __device__ __forceinline__ void signal_host(unsigned* count, unsigned parts, uns
 }
 #endif
 
-// One pass over n options of 16-byte aligned arrays, in device memory or pinned
-// host memory (its device addresses).
-cudaError_t launch_map_stage(const SoA& a, int n, int mode, const Signal& sig, cudaStream_t st);
+// One pass over n options of arrays equally far from a 16-byte boundary (else
+// cudaErrorNotSupported), in device memory or pinned host memory (its device
+// addresses).
+cudaError_t launch_map_stage(SoA a, int64_t n, int mode, const Signal& sig, cudaStream_t st);
 // Copies n options' six input arrays from src (pinned host memory, its device
 // addresses) into dst's, by one kernel.
 cudaError_t launch_gather(const SoA& src, const SoA& dst, int64_t n, int sm_count, cudaStream_t st);

@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(512, 1) map_runs_kernel(SoA a, int64_t n, int 
 // 13.7 with a stream synchronisation.
 constexpr int kStageThreads = 128;
 
-template <int M>
-__global__ void __launch_bounds__(kStageThreads) map_stage_kernel(SoA a, int n, Signal sig) {
+template <int M, bool HEAD>  // (HEAD's code alone costs a call without one 0.4 us)
+__global__ void __launch_bounds__(kStageThreads) map_stage_kernel(SoA a, int n, int head, Signal sig) {
     const int g = blockIdx.x * kStageThreads + threadIdx.x;
     if (4 * g + 4 <= n) {
         const float4 q = price4<M>(__ldg(reinterpret_cast<const float4*>(a.s) + g),
@@ -419,20 +419,10 @@ __global__ void __launch_bounds__(kStageThreads) map_stage_kernel(SoA a, int n, 
     } else {
         for (int i = 4 * g; i < n; ++i) price_scalar<M>(a, i);
     }
+    // the options before the vectors: a block of their own, the last
+    if (HEAD && blockIdx.x == gridDim.x - 1 && (int)threadIdx.x < head) price_scalar<M>(a, (int)threadIdx.x - head);
     __syncthreads();
     if (threadIdx.x == 0) signal_host(sig.count, gridDim.x, sig.flag, sig.seq);
-}
-
-cudaError_t launch_map_stage(const SoA& a, int n, int mode, const Signal& sig, cudaStream_t st) {
-    if (n <= 0 || !sig.flag) return cudaErrorInvalidValue;
-    const unsigned grid = (unsigned)((n + 4 * kStageThreads - 1) / (4 * kStageThreads));
-    switch (mode) {
-        case MODE_FAST: map_stage_kernel<MODE_FAST><<<grid, kStageThreads, 0, st>>>(a, n, sig); break;
-        case MODE_SFU_REF: map_stage_kernel<MODE_SFU_REF><<<grid, kStageThreads, 0, st>>>(a, n, sig); break;
-        case MODE_LIBM_REF: map_stage_kernel<MODE_LIBM_REF><<<grid, kStageThreads, 0, st>>>(a, n, sig); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
 }
 
 // Host arrays into device arrays: blockIdx.y picks the array, so that the link
@@ -896,6 +886,22 @@ static cudaError_t launch_runs_mode(SoA a, int64_t n, int runs, int sm_count, cu
     else if constexpr (M != MODE_LIBM_REF) kernel = host ? map_runs_kernel<M, 4, 2, true> : map_runs_kernel<M, 4, 2, false>;
     if (!kernel) return cudaErrorInvalidValue;
     kernel<<<(unsigned)grid, (unsigned)block, 0, st>>>(a, n, head, runs, h, sig);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_map_stage(SoA a, int64_t n, int mode, const Signal& sig, cudaStream_t st) {
+    if (n <= 0 || n > 1 << 30 || !sig.flag) return cudaErrorInvalidValue;
+    const int head = peel(&a, &n, 16);
+    if (head < 0) return cudaErrorNotSupported;
+    const unsigned grid = (unsigned)((n + 4 * kStageThreads - 1) / (4 * kStageThreads)) + (head > 0);
+    void (*kernel)(SoA, int, int, Signal) = nullptr;
+    switch (mode) {
+        case MODE_FAST: kernel = head ? map_stage_kernel<MODE_FAST, true> : map_stage_kernel<MODE_FAST, false>; break;
+        case MODE_SFU_REF: kernel = head ? map_stage_kernel<MODE_SFU_REF, true> : map_stage_kernel<MODE_SFU_REF, false>; break;
+        case MODE_LIBM_REF: kernel = head ? map_stage_kernel<MODE_LIBM_REF, true> : map_stage_kernel<MODE_LIBM_REF, false>; break;
+        default: return cudaErrorInvalidValue;
+    }
+    kernel<<<grid, kStageThreads, 0, st>>>(a, (int)n, head, sig);
     return cudaGetLastError();
 }
 

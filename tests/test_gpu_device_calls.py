@@ -13,7 +13,7 @@ torch = pytest.importorskip("torch")
 N_MAX = 1 << 18  # kFlagOptions
 
 
-@pytest.mark.parametrize("n", [1, 3, 4, 511, 513, N_MAX, N_MAX + 1])
+@pytest.mark.parametrize("n", [1, 3, 4, 511, 513, N_MAX // 2, N_MAX // 2 + 1, N_MAX, N_MAX + 1])
 def test_short_device_calls(n):
     book = books.generate(n + 4, seed=14)
     cols = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in book.arrays()]
@@ -26,6 +26,15 @@ def test_short_device_calls(n):
             ctx.price_soa(*cols, two, n=n, mode=mode, device=True)
             assert torch.equal(one.view(torch.int32), two.view(torch.int32)), mode
             assert (two[n:] == -1).all()
+            for lo in (1, 3):  # a slice: up to three options in front of the vectors
+                two.fill_(-1)
+                torch.cuda.synchronize()
+                ctx.price_soa(*[c[lo:lo + n] for c in cols], two[lo:lo + n], n=n, mode=mode, device=True)
+                ctx.price_soa(*[c[lo:lo + n] for c in cols], one[lo:lo + n], n=n, mode=mode, device=True,
+                              asynchronous=True)
+                ctx.synchronize()
+                assert torch.equal(one[lo:lo + n].view(torch.int32), two[lo:lo + n].view(torch.int32)), (mode, lo)
+                assert (two[:lo] == -1).all() and (two[lo + n:] == -1).all()
         one, two, three = (torch.full((n + 4,), -1.0, device="cuda:0", dtype=torch.float64) for _ in range(3))
         torch.cuda.synchronize()
         ctx.price_soa_f64(*wide, one, n=n, device=True, asynchronous=True)
