@@ -140,7 +140,8 @@ cudaError_t launch_map_f64(const SoA64& a, int64_t n, int sm_count, cudaStream_t
 // launch.  pdl: launch with programmatic stream serialization (the next pass
 // may start while this one drains; it must use its own cursor).
 cudaError_t launch_batch(const SoA& pool, const uint64_t* tiles, uint64_t ntiles,
-                         unsigned long long* cursor, int mode, int grid, int pdl, cudaStream_t st);
+                         unsigned long long* cursor, int mode, int grid, int pdl, cudaStream_t st,
+                         const Signal& sig = Signal{});
 // The same over device arrays of nseg segments (tile_prefix: nseg + 1 entries,
 // exclusive prefix of tiles of tile_opts options per segment).
 cudaError_t launch_batch_segments(const SoA& pool, const uint64_t* seg_off, const uint64_t* seg_len,

@@ -1176,7 +1176,7 @@ __device__ __forceinline__ void price_range(const SoA& pool, uint64_t b, uint64_
 // exp/log get up to 128.)
 template <int M, int W>
 __global__ void __launch_bounds__(kBatchBlock, M == MODE_LIBM_REF ? 2 : 4) batch_kernel(
-    SoA pool, const uint64_t* __restrict__ tiles, uint64_t ntiles, unsigned long long* cursor) {
+    SoA pool, const uint64_t* __restrict__ tiles, uint64_t ntiles, unsigned long long* cursor, Signal sig) {
     __shared__ uint64_t sh_b, sh_e;
     __shared__ int sh_done;
     pdl_trigger();
@@ -1199,6 +1199,8 @@ __global__ void __launch_bounds__(kBatchBlock, M == MODE_LIBM_REF ? 2 : 4) batch
         if (done) break;
         price_range<M, W>(pool, b, e, threadIdx.x, kBatchBlock);
     }
+    // (the barriers above are behind every price of the block)
+    if (sig.flag && threadIdx.x == 0) signal_host(sig.count, gridDim.x, sig.flag, sig.seq);
     pdl_wait();
 }
 
@@ -1256,8 +1258,9 @@ static bool batch_w8(const SoA& pool, int mode) {
 }
 
 cudaError_t launch_batch(const SoA& pool, const uint64_t* tiles, uint64_t ntiles,
-                         unsigned long long* cursor, int mode, int grid, int pdl, cudaStream_t st) {
-    if (ntiles == 0) return cudaSuccess;
+                         unsigned long long* cursor, int mode, int grid, int pdl, cudaStream_t st,
+                         const Signal& sig) {
+    if (ntiles == 0) return sig.flag ? cudaErrorInvalidValue : cudaSuccess;
     if ((uint64_t)grid > ntiles) grid = (int)ntiles;  // no block without a tile
     if (grid < 1) grid = 1;
     cudaLaunchConfig_t lc = {};
@@ -1271,8 +1274,8 @@ cudaError_t launch_batch(const SoA& pool, const uint64_t* tiles, uint64_t ntiles
     lc.numAttrs = pdl ? 1 : 0;
     const bool w8 = batch_w8(pool, mode);
 #define BSG_BATCH(M_) \
-    (w8 ? cudaLaunchKernelEx(&lc, batch_kernel<M_, 8>, pool, tiles, ntiles, cursor) \
-        : cudaLaunchKernelEx(&lc, batch_kernel<M_, 4>, pool, tiles, ntiles, cursor))
+    (w8 ? cudaLaunchKernelEx(&lc, batch_kernel<M_, 8>, pool, tiles, ntiles, cursor, sig) \
+        : cudaLaunchKernelEx(&lc, batch_kernel<M_, 4>, pool, tiles, ntiles, cursor, sig))
     switch (mode) {
         case MODE_FAST: return BSG_BATCH(MODE_FAST);
         case MODE_SFU_REF: return BSG_BATCH(MODE_SFU_REF);

@@ -43,3 +43,26 @@ def test_short_device_calls(n):
         assert torch.equal(one.view(torch.int64), two.view(torch.int64))
         assert torch.equal(one.view(torch.int64), three.view(torch.int64))
         assert (two[n:] == -1).all()
+
+
+@pytest.mark.parametrize("count", [1, 3, 3000])
+def test_batch_of_one_pass_waits_for_its_kernel(count):
+    """The last block of a synchronous batch stores the word; calls in a row take
+    their work counter from the table each uploads."""
+    rng = np.random.default_rng(count)
+    lens = rng.integers(0, 5000, count)
+    lens[0] = 7
+    gaps = rng.integers(0, 9, count)
+    at = np.concatenate([[0], np.cumsum(lens + gaps)[:-1]])
+    segs = [(int(o), int(l)) for o, l in zip(at, lens)]
+    n = int(at[-1] + lens[-1]) + 1
+    cols = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in books.generate(n, seed=15).arrays()]
+    one, two = (torch.full((n,), -1.0, device="cuda:0") for _ in range(2))
+    with Context(0, 1) as ctx:
+        torch.cuda.synchronize()
+        ctx.price_batch(cols, one, n, segs, num_runs=2)
+        for _ in range(3):
+            two.fill_(-1)
+            torch.cuda.synchronize()
+            ctx.price_batch(cols, two, n, segs)
+            assert torch.equal(one.view(torch.int32), two.view(torch.int32))
