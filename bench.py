@@ -891,7 +891,8 @@ def fp64_record(args, local, n=None, runs=None, steps=None, warmup=None):
         # leave (of either sign): there any relative figure is noise against noise
         spot = np.maximum(book.sptprice, book.strike).astype(np.float64)
         of_spot = float(np.max(np.abs(got - want) / spot))
-        held = float(np.max((np.abs(got - want) / np.abs(want))[np.abs(want) > 1e-6 * spot]))
+        big = np.abs(want) > 1e-6 * spot
+        held = float(np.max(np.abs(got - want)[big] / np.abs(want)[big]))
         cpu = {"value": n / cpu_s, "unit": UNIT, "cores": 1, "kind": "port",
                "sample": f"{n} options, one pass of the FP64 oracle (the same formula in double)"}
     value = n * runs * steps / secs
