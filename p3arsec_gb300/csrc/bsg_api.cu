@@ -1329,14 +1329,16 @@ int bsg_price_books_plain(bsg_ctx* c, const float* s, const float* k, const floa
         if (o > pool_len || l > pool_len - o)
             return fail(c, BSG_ERR_INVALID_ARG, "segment " + std::to_string(i) + " lies outside the pool");
     }
+    bool first = true;  // of the call: it alone waits for what the stream holds
     for (int j = 0; j < num_runs; ++j) {
         for (size_t i = 0; i < nseg; ++i) {
             if (!segs[i].len) continue;
             const uint64_t o = segs[i].offset;
             bsg::SoA b{s + o, k + o, r + o, v + o, t + o, otype + o, prices + o};
-            cudaError_t e = bsg::launch_map(b, (int64_t)segs[i].len, mode,
-                                            bsg::pass_cfg(c->tune, j, num_runs), c->sm_count,
-                                            c->stream);
+            bsg::MapCfg cfg = bsg::pass_cfg(c->tune, j, num_runs);
+            if (!first) cfg.pdl = c->tune.pdl;
+            first = false;
+            cudaError_t e = bsg::launch_map(b, (int64_t)segs[i].len, mode, cfg, c->sm_count, c->stream);
             if (e != cudaSuccess) return cuda_fail(c, e, "launch_map (per book)");
             c->launches++;
         }
@@ -1845,7 +1847,9 @@ extern "C" int bsg_autotune(bsg_ctx* c, size_t n, bsg_tune* out) {
     // warm-up pass; a negative result: the launch failed or a bounded wait of
     // the staged kernel expired (never pick such a shape).
     auto time_cfg = [&](const bsg::MapCfg& cfg, int reps) -> float {
-        e = bsg::launch_map(a, (int64_t)n, bsg::MODE_FAST, cfg, c->sm_count, c->stream);
+        bsg::MapCfg warm = cfg;
+        warm.pdl = 0;  // behind the fill
+        e = bsg::launch_map(a, (int64_t)n, bsg::MODE_FAST, warm, c->sm_count, c->stream);
         if (e != cudaSuccess) return -1.0f;
         cudaEventRecord(e0, c->stream);
         for (int i = 0; i < reps && e == cudaSuccess; ++i)

@@ -73,7 +73,14 @@ cudaError_t launch_map(const SoA& a, int64_t n, int mode, const MapCfg& cfg,
 // The alternating load path (8) walks odd passes from the book's last tile
 // to its first, so each pass starts on the lines the previous pass touched
 // last, which the L2 still holds.
+// Pass 0 is never a programmatic launch: a kernel with that attribute loads its
+// inputs, and stores prices, while the kernel before it on the stream may still
+// be writing (map_vec_kernel and batch_kernel let their dependents start at
+// once).  Passes of one book may overlap; the first waits for whatever the
+// stream holds: a call that wrote its inputs or writes the same prices, a
+// gather, the caller's own kernels.
 inline MapCfg pass_cfg(MapCfg c, int j, int runs) {
+    if (j == 0) c.pdl = 0;
     if (c.load_path == 7 && j == runs - 1) c.load_path = 6;
     c.rev = (c.load_path == 8) ? (j & 1) : 0;
     return c;
