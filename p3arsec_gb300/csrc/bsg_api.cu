@@ -403,7 +403,8 @@ int enqueue_map_runs(bsg_ctx* c, const bsg::SoA& a, int64_t n, int runs, int mod
         c->launches++;
         return BSG_OK;
     }
-    const bsg::MapCfg cfg = c->tuned ? c->tune : bsg::map_default_cfg(a, n, runs);
+    bsg::MapCfg cfg = c->tuned ? c->tune : bsg::map_default_cfg(a, n, runs);
+    if (bsg::in_place(a, n)) cfg.pdl = 0;  // a pass reads what the one before it wrote
     if (runs == 1 || (flags & BSG_NO_GRAPH)) {
         for (int j = 0; j < runs; ++j) {
             cudaError_t e = bsg::launch_map(a, n, mode, bsg::pass_cfg(cfg, j, runs), c->sm_count,
@@ -1177,7 +1178,8 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
             return finish(c, flags);
         }
         // one work counter per pass, zeroed together, so that pass j + 1 can
-        // start (PDL) while pass j drains
+        // start (PDL) while pass j drains, unless it reads what pass j writes
+        const bool overlap = !bsg::in_place(a, (int64_t)pool_len);
         if ((size_t)num_runs > c->cursor_cap) {
             BSG_CK(c, cudaStreamSynchronize(c->stream));
             graph_drop_all(c);
@@ -1193,7 +1195,7 @@ int price_batch_impl(bsg_ctx* c, const float* s, const float* k, const float* r,
             cudaError_t e = cudaMemsetAsync(c->d_cursor, 0, (size_t)num_runs * 8, c->stream);
             for (int j = 0; j < num_runs && e == cudaSuccess; ++j)
                 e = bsg::launch_batch(a, c->d_tb + 2, ntiles, c->d_cursor + j,
-                                      mode, grid, j > 0 ? 1 : 0, c->stream);
+                                      mode, grid, j > 0 && overlap, c->stream);
             return e;
         };
         if (flags & BSG_NO_GRAPH) {
@@ -1329,14 +1331,17 @@ int bsg_price_books_plain(bsg_ctx* c, const float* s, const float* k, const floa
         if (o > pool_len || l > pool_len - o)
             return fail(c, BSG_ERR_INVALID_ARG, "segment " + std::to_string(i) + " lies outside the pool");
     }
-    bool first = true;  // of the call: it alone waits for what the stream holds
+    // the call's first launch waits for what the stream holds; prices over an
+    // input make every pass an input of the next
+    const int pdl = c->tune.pdl && !bsg::in_place(a, (int64_t)pool_len);
+    bool first = true;
     for (int j = 0; j < num_runs; ++j) {
         for (size_t i = 0; i < nseg; ++i) {
             if (!segs[i].len) continue;
             const uint64_t o = segs[i].offset;
             bsg::SoA b{s + o, k + o, r + o, v + o, t + o, otype + o, prices + o};
             bsg::MapCfg cfg = bsg::pass_cfg(c->tune, j, num_runs);
-            if (!first) cfg.pdl = c->tune.pdl;
+            cfg.pdl = pdl && !first;
             first = false;
             cudaError_t e = bsg::launch_map(b, (int64_t)segs[i].len, mode, cfg, c->sm_count, c->stream);
             if (e != cudaSuccess) return cuda_fail(c, e, "launch_map (per book)");

@@ -130,3 +130,26 @@ def test_plain_books_after_a_call_that_writes_the_pool():
         outs.append((x, y))
     for one, two in zip(*outs):
         assert torch.equal(one.view(torch.int32), two.view(torch.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+@pytest.mark.parametrize("call", ["graph", "direct", "batch", "batch direct", "plain books"])
+def test_prices_over_an_input(shape, call):
+    """Each pass takes the prices of the one before it as its spot prices."""
+    torch = pytest.importorskip("torch")
+    s, k, r, v, t, o = _book(torch, N, 42)
+    segs = [(i, min(1_000_000, N - i)) for i in range(0, N, 1_000_000)]
+    one, two = s.clone(), s.clone()
+    torch.cuda.synchronize()
+    with Context(0, 1) as ctx:
+        for _ in range(3):
+            ctx.price_soa(one, k, r, v, t, o, one, n=N, device=True)
+        if shape:
+            ctx.set_tune(*shape)
+        if call in ("graph", "direct"):
+            ctx.price_soa(two, k, r, v, t, o, two, n=N, num_runs=3, device=True, graph=call == "graph")
+        else:
+            ctx.price_batch([two, k, r, v, t, o], two, N, segs, num_runs=3, plain=call == "plain books",
+                            graph=call != "batch direct")
+    assert torch.equal(one.view(torch.int32), two.view(torch.int32))
