@@ -577,6 +577,29 @@ bool pinned_view(const bsg::SoA& h, size_t n, bsg::SoA* d) {
     return true;
 }
 
+// Whether the host may read and write all seven arrays itself.  Not where one is
+// device memory: a call without BSG_DEVICE_PTRS that is given such a pointer is
+// served by the driver's copies, which go by the address.  An array that begins
+// on the page where another one does is not looked up again (0.11 us each: a
+// call of 16 options 11.6 us, 12.0 with all seven looked up, 11.4 with none).
+bool host_book(const bsg::SoA& h) {
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const void* p[7] = {h.s, h.k, h.r, h.v, h.t, h.ot, h.out};
+    for (int i = 0; i < 7; ++i) {
+        bool seen = false;
+        for (int j = 0; j < i; ++j)
+            seen = seen || (reinterpret_cast<uintptr_t>(p[i]) ^ reinterpret_cast<uintptr_t>(p[j])) < page;
+        if (seen) continue;
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p[i]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type == cudaMemoryTypeDevice) return false;
+    }
+    return true;
+}
+
 // Whether the GPU may read a pageable host book's inputs, and write its prices
 // when `write`, in place: it walks the process's own page tables
 // (bsg_ctx::host_tables), and the kernel has just made every page of the
@@ -946,7 +969,7 @@ int bsg_price_soa(bsg_ctx* c, const float* s, const float* k, const float* r,
         if (flags & BSG_ASYNC) return enqueue_host_pipelined(c, a, n, num_runs, mode, flags);
         if ((st = drain_pipeline(c))) return st;
         const size_t b = n * 4;
-        if (!c->debug && n <= kStageOptions) {
+        if (!c->debug && n <= kStageOptions && host_book(a)) {
             float* f = reinterpret_cast<float*>(c->h_stage);
             const size_t al = round_up(n, 64);
             const void* in[6] = {s, k, r, v, t, otype};

@@ -111,3 +111,26 @@ def test_host_and_asynchronous_calls_in_turn(ctx, book):
     ctx.synchronize()
     for p in piped + [dout.cpu().numpy()]:
         assert np.array_equal(p.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [1, 16, STAGE, STAGE + 1, 200_000])
+def test_device_memory_without_the_device_flag(ctx, book, n):
+    """A C caller that leaves BSG_DEVICE_PTRS out has its arrays copied by the
+    driver, wherever they are: every array in device memory, and each one alone."""
+    arrays = [np.ascontiguousarray(a[:n]) for a in book.arrays()] + [np.zeros(n, np.float32)]
+    want = _want(ctx, book, 0, n, "fast")
+    dev = [torch.from_numpy(a).cuda() for a in arrays]
+    torch.cuda.synchronize()
+    for which in [set(range(7))] + [{i} for i in range(7)]:
+        ptrs = [dev[i].data_ptr() if i in which else arrays[i].ctypes.data for i in range(7)]
+        for runs in (1, 3):
+            arrays[6][:] = -1
+            dev[6].fill_(-1)
+            torch.cuda.synchronize()
+            assert ctx.lib.bsg_price_soa(ctx.h, *ptrs, n, runs, 0) == 0
+            got = dev[6].cpu().numpy() if 6 in which else arrays[6]
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (which, runs)
+    dev[6].fill_(-1)
+    torch.cuda.synchronize()
+    assert ctx.lib.bsg_BlkSchlsEqEuroNoDiv(dev[6].data_ptr(), n, *[d.data_ptr() for d in dev[:6]], 0.0) == 0
+    assert np.array_equal(dev[6].cpu().numpy().view(np.uint32), want.view(np.uint32))
