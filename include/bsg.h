@@ -47,7 +47,7 @@ typedef enum bsg_status {
     BSG_ERR_CUDA = -3,          /* a CUDA runtime call failed */
     BSG_ERR_OUT_OF_MEMORY = -4, /* device or pinned host allocation failed */
     BSG_ERR_CAPACITY = -5,      /* n exceeds the context's max_options */
-    BSG_ERR_MISALIGNED = -6,    /* device pointer not 4-byte aligned */
+    BSG_ERR_MISALIGNED = -6,    /* device pointer not aligned to its element (4 or 8 bytes) */
     BSG_ERR_TIMEOUT = -7,       /* a bounded wait expired */
     BSG_ERR_BUDGET = -8,        /* request larger than the admission budget */
     BSG_ERR_CANCELLED = -9,     /* request cancelled while queued */

@@ -308,11 +308,12 @@ namespace {
 // range (bsg::device_extent).  seen: the allocation that the previous array of
 // the same call was found in, which the next often shares (a look-up in the
 // driver takes 0.3 us).
-int check_dev_range(bsg_ctx* c, const void* p, size_t bytes, const char* name,
+// elem: the array's element size, to a multiple of which it must be aligned.
+int check_dev_range(bsg_ctx* c, const void* p, size_t bytes, size_t elem, const char* name,
                     bsg::Range* seen = nullptr) {
     if (!p) return fail(c, BSG_ERR_INVALID_ARG, std::string(name) + " is NULL");
-    if ((reinterpret_cast<uintptr_t>(p) & 3) != 0)
-        return fail(c, BSG_ERR_MISALIGNED, std::string(name) + " is not 4-byte aligned");
+    if ((reinterpret_cast<uintptr_t>(p) & (elem - 1)) != 0)
+        return fail(c, BSG_ERR_MISALIGNED, std::string(name) + " is not " + std::to_string(elem) + "-byte aligned");
     const uintptr_t x = reinterpret_cast<uintptr_t>(p);
     if (seen && x >= seen->b && x < seen->e && bytes <= seen->e - x) return BSG_OK;
     switch (bsg::device_extent(p, bytes, c->device, seen)) {
@@ -334,13 +335,13 @@ int check_soa_dev(bsg_ctx* c, const bsg::SoA& a, size_t n, size_t out_elem) {
     const size_t b = n * 4;
     int st;
     bsg::Range seen;
-    if ((st = check_dev_range(c, a.s, b, "sptprice", &seen))) return st;
-    if ((st = check_dev_range(c, a.k, b, "strike", &seen))) return st;
-    if ((st = check_dev_range(c, a.r, b, "rate", &seen))) return st;
-    if ((st = check_dev_range(c, a.v, b, "volatility", &seen))) return st;
-    if ((st = check_dev_range(c, a.t, b, "otime", &seen))) return st;
-    if ((st = check_dev_range(c, a.ot, b, "otype", &seen))) return st;
-    if (out_elem && (st = check_dev_range(c, a.out, n * out_elem, "prices", &seen))) return st;
+    if ((st = check_dev_range(c, a.s, b, 4, "sptprice", &seen))) return st;
+    if ((st = check_dev_range(c, a.k, b, 4, "strike", &seen))) return st;
+    if ((st = check_dev_range(c, a.r, b, 4, "rate", &seen))) return st;
+    if ((st = check_dev_range(c, a.v, b, 4, "volatility", &seen))) return st;
+    if ((st = check_dev_range(c, a.t, b, 4, "otime", &seen))) return st;
+    if ((st = check_dev_range(c, a.ot, b, 4, "otype", &seen))) return st;
+    if (out_elem && (st = check_dev_range(c, a.out, n * out_elem, out_elem, "prices", &seen))) return st;
     return BSG_OK;
 }
 
@@ -1056,7 +1057,7 @@ int bsg_price_fp64(bsg_ctx* c, const float* s, const float* k, const float* r,
     int st;
     if (flags & BSG_DEVICE_PTRS) {
         if ((st = check_soa_dev(c, a, n, 0))) return st;
-        if ((st = check_dev_range(c, out, n * 8, "out"))) return st;
+        if ((st = check_dev_range(c, out, n * 8, 8, "out"))) return st;
         const bool wait = !(flags & BSG_ASYNC) && !c->debug;
         cudaError_t e = bsg::launch_fp64(a, out, (int64_t)n, c->sm_count, c->stream,
                                          wait ? next_signal(c) : bsg::Signal{});
@@ -1104,10 +1105,10 @@ int bsg_price_soa_f64(bsg_ctx* c, const double* s, const double* k, const double
     if (flags & BSG_DEVICE_PTRS) {
         const size_t b = n * 8;
         bsg::Range seen;
-        if ((st = check_dev_range(c, s, b, "sptprice", &seen)) || (st = check_dev_range(c, k, b, "strike", &seen)) ||
-            (st = check_dev_range(c, r, b, "rate", &seen)) || (st = check_dev_range(c, v, b, "volatility", &seen)) ||
-            (st = check_dev_range(c, t, b, "otime", &seen)) || (st = check_dev_range(c, otype, n * 4, "otype", &seen)) ||
-            (st = check_dev_range(c, prices, b, "prices", &seen)))
+        if ((st = check_dev_range(c, s, b, 8, "sptprice", &seen)) || (st = check_dev_range(c, k, b, 8, "strike", &seen)) ||
+            (st = check_dev_range(c, r, b, 8, "rate", &seen)) || (st = check_dev_range(c, v, b, 8, "volatility", &seen)) ||
+            (st = check_dev_range(c, t, b, 8, "otime", &seen)) || (st = check_dev_range(c, otype, n * 4, 4, "otype", &seen)) ||
+            (st = check_dev_range(c, prices, b, 8, "prices", &seen)))
             return st;
         const bsg::SoA64 a{s, k, r, v, t, otype, prices};
         const bool wait = !(flags & BSG_ASYNC) && !c->debug;  // for the last pass's kernel itself
@@ -1389,7 +1390,7 @@ int bsg_error_report(bsg_ctx* c, const float* s, const float* k, const float* r,
     int st;
     if (n) {
         if ((st = check_soa_dev(c, a, n, 0))) return st;
-        if ((st = check_dev_range(c, prices, n * 4, "prices"))) return st;
+        if ((st = check_dev_range(c, prices, n * 4, 4, "prices"))) return st;
     }
     BSG_CK(c, cudaMemsetAsync(c->d_acc, 0, sizeof(bsg::ErrAcc) * nbuckets, c->stream));
     BSG_CK(c, cudaMemcpyAsync(c->d_edges, edges, sizeof(double) * (nbuckets + 1), cudaMemcpyHostToDevice, c->stream));

@@ -1,0 +1,39 @@
+"""Arrays that are not aligned to their elements are a status, before anything is
+launched."""
+import numpy as np
+import pytest
+
+from p3arsec_gb300 import BsgError, Context, books
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+MISALIGNED = -6
+
+
+def test_doubles_off_their_alignment_are_refused():
+    """An array of doubles four bytes off is a status before anything is launched
+    (the kernel copies and stores eight bytes at a time); four bytes are enough
+    for the types."""
+    n = 100
+    book = books.generate(n + 2, seed=16)
+    cols = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in book.arrays()]
+    wide = [c.double() for c in cols[:5]] + [cols[5]]
+    out = torch.full((n + 2,), -1.0, device="cuda:0", dtype=torch.float64)
+    torch.cuda.synchronize()
+    with Context(0, 1) as ctx:
+        at = [x.data_ptr() for x in wide + [out]]
+        for i in (0, 1, 2, 3, 4, 6):
+            ptrs = list(at)
+            ptrs[i] += 4
+            for asynchronous in (False, True):
+                with pytest.raises(BsgError) as e:
+                    ctx.price_soa_f64(*ptrs, n=n, device=True, asynchronous=asynchronous)
+                assert e.value.status == MISALIGNED
+        with pytest.raises(BsgError) as e:
+            ctx.price_fp64(*[x.data_ptr() for x in cols], out.data_ptr() + 4, n=n, device=True)
+        assert e.value.status == MISALIGNED
+        assert ctx.launches == 0
+        ctx.price_soa_f64(*at[:5], at[5] + 4, at[6], n=n, device=True)
+        ctx.price_soa_f64(*[p + 8 for p in at[:5]], at[5] + 4, at[6] + 8, n=n, device=True)
+        assert ctx.launches == 2
