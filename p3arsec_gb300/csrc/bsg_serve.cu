@@ -1194,7 +1194,11 @@ int submit_impl(bsg_server* s, const bsg_request* r, uint64_t* id, bool auto_rel
                 return BSG_ERR_INVALID_ARG;  // not inside registered host memory
             }
             const uintptr_t dev = reinterpret_cast<uintptr_t>(arrs[j]) + h->delta;
-            const uint64_t v = (dev & 3) ? 0 : 1 + ((16 - (dev & 15)) & 15) / 4;
+            if (dev & 3) {
+                delete q;
+                return BSG_ERR_MISALIGNED;  // the kernels read and write whole options
+            }
+            const uint64_t v = 1 + ((16 - (dev & 15)) & 15) / 4;
             vec = (j == 0 || vec == v) ? v : 0;
             if (j < 5) q->desc.src[j] = reinterpret_cast<const float*>(dev);
             else if (j == 5) q->desc.ot = reinterpret_cast<const int32_t*>(dev);

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from p3arsec_gb300 import BsgError, Context, books
+from p3arsec_gb300.abi import Server
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -37,3 +38,31 @@ def test_doubles_off_their_alignment_are_refused():
         ctx.price_soa_f64(*at[:5], at[5] + 4, at[6], n=n, device=True)
         ctx.price_soa_f64(*[p + 8 for p in at[:5]], at[5] + 4, at[6] + 8, n=n, device=True)
         assert ctx.launches == 2
+
+
+@pytest.mark.parametrize("kind", [dict(fused=False), dict(fused=True), dict(persistent=True)], ids=str)
+def test_requests_off_their_alignment_are_refused(kind):
+    """The serving kernels read the caller's arrays in place; the plain loop copies
+    them, from wherever they begin."""
+    n = 100
+    book = books.generate(n, seed=17)
+    keep = [torch.zeros(n + 1).pin_memory() for _ in range(7)]
+    bytes_of = [k.numpy().view(np.uint8) for k in keep]
+    at = [k.data_ptr() for k in keep]
+    for b, a in zip(bytes_of, book.arrays()):
+        b[:4 * n] = a.view(np.uint8)
+    with Server(budget_bytes=1 << 24, **kind) as srv:
+        for k in keep:
+            srv.register(k.numpy())
+        for i in range(7):
+            with pytest.raises(BsgError) as e:
+                srv.submit(*[p + 2 * (j == i) for j, p in enumerate(at)], n=n)
+            assert e.value.status == MISALIGNED
+        assert srv.wait(srv.submit(*at, n=n), timeout_s=60.0)[0] == 0
+        want = keep[6].numpy()[:n].copy()
+        assert srv.stats()["completed"] == 1
+    for b in bytes_of[:6]:
+        b[2:4 * n + 2] = b[:4 * n].copy()
+    with Server(budget_bytes=1 << 24, plain=True) as srv:
+        assert srv.wait(srv.submit(*[p + 2 for p in at], n=n), timeout_s=60.0)[0] == 0
+    assert np.array_equal(bytes_of[6][2:4 * n + 2].view(np.uint32), want.view(np.uint32))
