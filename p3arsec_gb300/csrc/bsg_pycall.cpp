@@ -95,20 +95,23 @@ bool host_array(PyObject* x, char fmt, size_t n, Py_buffer* b) {
     return false;
 }
 
-bool whole(PyObject* x, uint64_t* out) {  // int(x), modulo 2^64 as ctypes stores it
+// A whole number modulo 2^64, as ctypes takes one: an int or what has
+// __index__ (numpy's integers); no float and no text.
+bool whole(PyObject* x, uint64_t* out) {
     if (PyLong_CheckExact(x) && PyUnstable_Long_IsCompact((PyLongObject*)x)) {
         *out = (uint64_t)PyUnstable_Long_CompactValue((PyLongObject*)x);
         return true;
     }
-    if (PyLong_Check(x)) {
-        *out = PyLong_AsUnsignedLongLongMask(x);
-        return !PyErr_Occurred();
-    }
-    PyObject* i = PyNumber_Long(x);
-    if (!i) return false;
-    *out = PyLong_AsUnsignedLongLongMask(i);
-    Py_DECREF(i);
+    *out = PyLong_AsUnsignedLongLongMask(x);  // through __index__
     return !PyErr_Occurred();
+}
+
+bool as_int(PyObject* x, uint64_t* out) {  // int(x), for a segment's two entries
+    if (PyLong_Check(x)) return whole(x, out);
+    PyObject* i = PyNumber_Long(x);
+    const bool ok = i && whole(i, out);
+    Py_XDECREF(i);
+    return ok;
 }
 
 bool six_and_one(PyObject* const* a, uintptr_t* p) {  // six inputs and the prices
@@ -149,10 +152,8 @@ PyObject* py_ptr(PyObject*, PyObject* x) {
 PyObject* price_soa(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (!arg_count(na, 12)) return nullptr;
     uintptr_t ctx, p[7];
-    uint64_t n, flags;
-    const long runs = PyLong_AsLong(a[9]);
-    if ((runs == -1 && PyErr_Occurred()) || !address(a[0], &ctx) || !whole(a[8], &n) || !whole(a[10], &flags))
-        return nullptr;
+    uint64_t n, runs, flags;
+    if (!address(a[0], &ctx) || !whole(a[8], &n) || !whole(a[9], &runs) || !whole(a[10], &flags)) return nullptr;
     const bool f64 = a[11] == Py_True;
     Py_buffer held[7];
     int m = 0;
@@ -192,15 +193,15 @@ bool read_segments(PyObject* list, std::vector<bsg_segment>* out) {
         PyObject* item = PySequence_Fast_GET_ITEM(seq, i);
         uint64_t o = 0, l = 0;
         if (PyTuple_CheckExact(item) && PyTuple_GET_SIZE(item) == 2) {
-            ok = whole(PyTuple_GET_ITEM(item, 0), &o) && whole(PyTuple_GET_ITEM(item, 1), &l);
+            ok = as_int(PyTuple_GET_ITEM(item, 0), &o) && as_int(PyTuple_GET_ITEM(item, 1), &l);
         } else {
             PyObject* pair = PySequence_Fast(item, "a segment is an (offset, length) pair");
             if (pair && PySequence_Fast_GET_SIZE(pair) != 2) {
                 PyErr_SetString(PyExc_ValueError, "a segment is an (offset, length) pair");
                 ok = false;
             } else {
-                ok = pair && whole(PySequence_Fast_GET_ITEM(pair, 0), &o) &&
-                     whole(PySequence_Fast_GET_ITEM(pair, 1), &l);
+                ok = pair && as_int(PySequence_Fast_GET_ITEM(pair, 0), &o) &&
+                     as_int(PySequence_Fast_GET_ITEM(pair, 1), &l);
             }
             Py_XDECREF(pair);
         }
@@ -214,10 +215,8 @@ bool read_segments(PyObject* list, std::vector<bsg_segment>* out) {
 PyObject* price_batch(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (!arg_count(na, 8)) return nullptr;
     uintptr_t ctx, p[7];
-    uint64_t pool_len, flags;
-    const long runs = PyLong_AsLong(a[5]);
-    if ((runs == -1 && PyErr_Occurred()) || !address(a[0], &ctx) || !whole(a[3], &pool_len) ||
-        !whole(a[6], &flags))
+    uint64_t pool_len, runs, flags;
+    if (!address(a[0], &ctx) || !whole(a[3], &pool_len) || !whole(a[5], &runs) || !whole(a[6], &flags))
         return nullptr;
     PyObject* pool = PySequence_Fast(a[1], "the pool is six arrays");
     if (!pool) return nullptr;
@@ -307,8 +306,8 @@ PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
                 *d[j] = PyFloat_AsDouble(v);
                 ok = !PyErr_Occurred();
             } else if (j < 8) {
-                const long x = PyLong_AsLong(v);
-                ok = !PyErr_Occurred();
+                uint64_t x = 0;
+                ok = whole(v, &x);
                 (j == 6 ? s->n_steps : s->n_factors) = (int)x;
             } else if (j < 10) {
                 PyObject* y = doubles(v, j == 8 ? &s->yield : &s->factors);

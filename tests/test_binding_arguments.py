@@ -1,0 +1,69 @@
+"""What the binding's native half takes as an argument, without a GPU: the calls
+go to no context (status -1), so an argument that is refused raises before."""
+import ctypes
+import dataclasses
+
+import numpy as np
+import pytest
+
+from p3arsec_gb300 import abi, build
+from p3arsec_gb300 import swaptions as S
+
+INVALID = -1
+
+
+@pytest.fixture(scope="module")
+def call():
+    build.build()
+    abi.load()
+    return abi._call
+
+
+def _host(n):
+    return [np.ones(n, np.float32) for _ in range(5)] + [np.zeros(n, np.int32), np.zeros(n, np.float32)]
+
+
+COUNTS = {"float": 100.0, "fraction": 2.5, "text": "100", "bytes": b"100", "numpy float": np.float64(2)}
+TAKEN = {"int": 3, "bool": True, "numpy int": np.int64(3), "numpy unsigned": np.uint8(3)}
+
+
+def _calls(call):
+    """Every count of every call, as a function of its value."""
+    host, sw = _host(100), S.generate(1, 1)
+    one = np.zeros(1)
+    price = lambda n=1, runs=1, flags=0: call.price_soa(0, *host, n, runs, flags, False)  # noqa: E731
+    batch = lambda n=1, runs=1, flags=1: call.price_batch(0, (0,) * 6, 0, n, [(0, 1)], runs, flags, False)  # noqa: E731
+    return {
+        "n": lambda x: price(n=x), "num_runs": lambda x: price(runs=x), "flags": lambda x: price(flags=x),
+        "pool_len": lambda x: batch(n=x), "batch num_runs": lambda x: batch(runs=x),
+        "batch flags": lambda x: batch(flags=x),
+        "request n": lambda x: call.server_submit(0, *[a.ctypes.data for a in host], x)[0],
+        "request id": lambda x: call.server_wait(0, x, 0.0)[0],
+        "trials": lambda x: call.price_swaptions(0, sw, x, one, one),
+        "seed": lambda x: call.price_swaptions(0, [dataclasses.replace(sw[0], seed=x)], 2, one, one),
+    }
+
+
+@pytest.mark.parametrize("value", list(COUNTS.values()), ids=list(COUNTS))
+def test_counts_that_are_not_whole_are_refused(call, value):
+    with pytest.raises(TypeError):
+        ctypes.c_size_t(value)  # as ctypes refuses them
+    for name, f in _calls(call).items():
+        with pytest.raises(TypeError):
+            print(name, f(value))
+
+
+@pytest.mark.parametrize("value", list(TAKEN.values()), ids=list(TAKEN))
+def test_whole_counts_are_taken(call, value):
+    for name, f in _calls(call).items():
+        assert f(value) == INVALID, name
+
+
+def test_segments_take_what_int_takes(call):
+    batch = lambda segs: call.price_batch(0, (0,) * 6, 0, 100, segs, 1, 1, False)  # noqa: E731
+    for segs in ([(0, 5)], [(0.0, 5.5)], [("0", "5")], [[0, 5]], np.array([[0, 5], [7, 2]]), (), [(np.int32(0), 2)]):
+        assert batch(segs) == INVALID
+    for segs, e in (([(0,)], ValueError), ([(0, 1, 2)], ValueError), ([(0, "x")], ValueError), ([(0, None)], TypeError),
+                    ([5], TypeError), (5, TypeError)):
+        with pytest.raises(e):
+            batch(segs)
