@@ -84,8 +84,10 @@ bool host_array(PyObject* x, char fmt, size_t n, Py_buffer* b) {
     const int arr = PyObject_IsInstance(x, g_ndarray);
     if (arr < 0) return false;
     if (arr && PyObject_GetBuffer(x, b, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) == 0) {
-        if (b->format && b->format[0] == fmt && b->format[1] == 0 && b->itemsize == 4 && b->ndim >= 1 &&
-            b->shape[0] >= 0 && (size_t)b->shape[0] >= n)
+        const char* f = b->format;
+        if (f && f[0] == '=') ++f;  // so where the array is not aligned; the calls copy it
+        if (f && f[0] == fmt && f[1] == 0 && b->itemsize == 4 && b->ndim >= 1 && b->shape[0] >= 0 &&
+            (size_t)b->shape[0] >= n)
             return true;
         PyBuffer_Release(b);
     }

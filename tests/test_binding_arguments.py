@@ -67,3 +67,17 @@ def test_segments_take_what_int_takes(call):
                     ([5], TypeError), (5, TypeError)):
         with pytest.raises(e):
             batch(segs)
+
+
+def test_host_arrays_at_any_address(call):
+    """Arrays of the right type that begin at an odd address (a field of a packed
+    record, a view of a file's bytes) are taken; the other byte order is not."""
+    for off in (1, 2, 3):
+        odd = [np.zeros(44, np.uint8)[off:off + 40].view(a.dtype) for a in _host(10)]
+        assert not odd[0].flags.aligned
+        assert call.price_soa(0, *odd, 10, 1, 0, False) == INVALID
+        for i in range(7):
+            swapped = list(odd)
+            swapped[i] = odd[i].view(odd[i].dtype.newbyteorder())
+            with pytest.raises(TypeError):
+                call.price_soa(0, *swapped, 10, 1, 0, False)
