@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import atexit
 import ctypes
+import importlib.util
 import os
 import sys
 import weakref
@@ -206,6 +207,19 @@ _lib = None
 _call = None  # p3arsec_gb300._pycall, bound to _lib
 
 
+def _load_pycall():
+    """The binding's native half, from the file that this interpreter's build()
+    writes (an import would also take a module of the name without an ABI tag)."""
+    from . import build  # (not at import: python -m p3arsec_gb300.build runs it as a script)
+    if not os.path.exists(build.PYCALL):
+        raise RuntimeError(f"{build.PYCALL} is missing: build it with this Python first "
+                           "(python -m p3arsec_gb300.build)")
+    spec = importlib.util.spec_from_file_location(__package__ + "._pycall", build.PYCALL)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
 def load(path: str = LIB_PATH) -> ctypes.CDLL:
     """Load libbsgpu.so (once).  Raises if it has not been built."""
     global _lib, _call
@@ -220,7 +234,7 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
-    from . import _pycall
+    _pycall = _load_pycall()
     _pycall.bind(*[ctypes.cast(getattr(lib, name), _P).value for name in _PYCALL])
     _call = _pycall
     _lib = lib

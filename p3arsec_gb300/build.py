@@ -21,7 +21,9 @@ HOST = os.path.join(PKG, "host")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libbsgpu.so")
 CLI = os.path.join(PKG, "bin", "blackscholes_gpu")
-PYCALL = os.path.join(PKG, "_pycall.so")  # the Python binding's native half
+# The Python binding's native half, named for the interpreter that it is built
+# for: another one's is neither fresh to build() nor found by abi.load().
+PYCALL = os.path.join(PKG, "_pycall" + sysconfig.get_config_var("EXT_SUFFIX"))
 SWAPTIONS_CLI = os.path.join(PKG, "bin", "swaptions_gpu")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

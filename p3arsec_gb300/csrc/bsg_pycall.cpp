@@ -100,10 +100,12 @@ bool host_array(PyObject* x, char fmt, size_t n, Py_buffer* b) {
 // A whole number modulo 2^64, as ctypes takes one: an int or what has
 // __index__ (numpy's integers); no float and no text.
 bool whole(PyObject* x, uint64_t* out) {
+#if PY_VERSION_HEX >= 0x030C0000
     if (PyLong_CheckExact(x) && PyUnstable_Long_IsCompact((PyLongObject*)x)) {
         *out = (uint64_t)PyUnstable_Long_CompactValue((PyLongObject*)x);
         return true;
     }
+#endif
     *out = PyLong_AsUnsignedLongLongMask(x);  // through __index__
     return !PyErr_Occurred();
 }
