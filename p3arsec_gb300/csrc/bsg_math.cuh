@@ -495,11 +495,12 @@ __device__ __forceinline__ float2 dmul_finite2(float2 x, FF c) {
 // comes near those.  The corrections are P. W. Markstein's ("Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34(1), 1990): a residual that one fma gives exactly, times the
-// approximate reciprocal.  1/b: every float in [2^-60, 2^110], and sqrt(t):
-// every float in [2^-40, 2^40], compared with the functions above.  a/b: from
-// a correctly rounded 1/b and a quotient within an ulp (which the first
-// correction makes of q) the second correction is his theorem; 2^36 random
-// and near-power-of-two pairs compared.
+// approximate reciprocal.  a/b: from a correctly rounded 1/b and a quotient
+// within an ulp (which the first correction makes of q) the second correction
+// is his theorem.  tests/test_rounding.py compares them with the functions
+// above: 1/b for every float in [2^-60, 2^110), sqrt(t) for every one in
+// [2^-40, 2^40), a/b for 2^36 pairs, random, next to powers of two and with
+// quotients next to the middle of two floats.
 __device__ __forceinline__ float2 rcp2_rn(float2 b) {
     const float2 y = make_float2(rcp_approx(b.x), rcp_approx(b.y));
     return fma2(fma2(neg2(b), y, f2(1.0f)), y, y);
