@@ -23,6 +23,9 @@
  *    (e.g. torch.cuda.ExternalStream(bsg_stream(ctx))).  A synchronous
  *    call's results are complete when it returns; a BSG_ASYNC call's after
  *    bsg_synchronize() or in work ordered after bsg_stream().
+ *  - A waiting call spins, for up to 2 ms itself and then as the driver does,
+ *    unless the device's schedule flags (cudaSetDeviceFlags) asked to yield or
+ *    to block when the context was created.
  *  - No call ever falls back to a CPU computation: without a usable GPU,
  *    bsg_create fails with BSG_ERR_NO_DEVICE.
  */

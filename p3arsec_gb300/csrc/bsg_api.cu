@@ -156,6 +156,7 @@ struct bsg_ctx {
     unsigned* h_flag = nullptr;
     unsigned* d_parts = nullptr;
     unsigned call = 0;
+    bool poll = true;  // unless the device's schedule flags ask to yield or block while waiting
     // debug guards (BSG_DEBUG set at bsg_create): every resident array is
     // followed by at least kGuardWords words of kGuardByte, checked after
     // each synchronous call; d_guard holds the check's {count, first index}
@@ -532,8 +533,11 @@ bsg::Signal next_signal(bsg_ctx* c) { return bsg::Signal{c->d_parts, c->h_flag, 
 // Waits for the kernel of this call (number c->call) to store that number to
 // *h_flag: by polling the word, which sees it 2 us before the driver's stream
 // synchronisation would return, and after 2 ms by that (which also returns
-// the error of a kernel that failed).
+// the error of a kernel that failed).  The driver's own wait spins too unless
+// the program has set cudaDeviceScheduleYield or BlockingSync, which then hold
+// here as well.
 cudaError_t wait_flag(bsg_ctx* c) {
+    if (!c->poll) return cudaStreamSynchronize(c->stream);
     const auto t0 = std::chrono::steady_clock::now();
     for (unsigned i = 1;; ++i) {
         if (__atomic_load_n(c->h_flag, __ATOMIC_ACQUIRE) == c->call) return cudaSuccess;
@@ -842,6 +846,9 @@ int bsg_create(bsg_ctx** out, int device, size_t max_options) {
         int ats = 0;
         c->host_tables = cudaDeviceGetAttribute(&ats, cudaDevAttrPageableMemoryAccessUsesHostPageTables,
                                                 device) == cudaSuccess && ats != 0;
+        unsigned df = 0;
+        if (cudaGetDeviceFlags(&df) == cudaSuccess)
+            c->poll = (df & (cudaDeviceScheduleYield | cudaDeviceScheduleBlockingSync)) == 0;
         c->cap = max_options;
         c->debug = debug_env();
         // 256-byte aligned arrays, each followed by guard words in debug mode
