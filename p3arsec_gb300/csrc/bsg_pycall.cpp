@@ -13,6 +13,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "bsg.h"
@@ -187,12 +188,22 @@ PyObject* price_soa(PyObject*, PyObject* const* a, Py_ssize_t na) {
     return PyLong_FromLong(st);
 }
 
+template <typename T>
+bool resized(std::vector<T>* v, Py_ssize_t n) {
+    try {
+        v->resize((size_t)n);
+        return true;
+    } catch (const std::bad_alloc&) {
+        PyErr_NoMemory();
+        return false;
+    }
+}
+
 bool read_segments(PyObject* list, std::vector<bsg_segment>* out) {
     PyObject* seq = PySequence_Fast(list, "segments must be a sequence of (offset, length) pairs");
     if (!seq) return false;
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
-    out->resize((size_t)n);
-    bool ok = true;
+    bool ok = resized(out, n);
     for (Py_ssize_t i = 0; i < n && ok; ++i) {
         PyObject* item = PySequence_Fast_GET_ITEM(seq, i);
         uint64_t o = 0, l = 0;
@@ -295,9 +306,9 @@ PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
     PyObject* seq = PySequence_Fast(a[1], "swaptions must be a sequence");
     if (!seq) return nullptr;
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
-    std::vector<bsg_swaption> sw((size_t)(n > 0 ? n : 1));
-    std::vector<PyObject*> keep;
-    bool ok = true;
+    std::vector<bsg_swaption> sw;
+    std::vector<PyObject*> keep;  // two arrays a swaption, NULL where not there yet
+    bool ok = resized(&sw, n > 0 ? n : 1) && resized(&keep, 2 * n);
     for (Py_ssize_t i = 0; i < n && ok; ++i) {
         PyObject* w = PySequence_Fast_GET_ITEM(seq, i);
         bsg_swaption* s = &sw[(size_t)i];
@@ -314,9 +325,8 @@ PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
                 ok = whole(v, &x);
                 (j == 6 ? s->n_steps : s->n_factors) = (int)x;
             } else if (j < 10) {
-                PyObject* y = doubles(v, j == 8 ? &s->yield : &s->factors);
-                ok = y != nullptr;
-                if (ok) keep.push_back(y);
+                keep[(size_t)(2 * i + j - 8)] = doubles(v, j == 8 ? &s->yield : &s->factors);
+                ok = keep[(size_t)(2 * i + j - 8)] != nullptr;
             } else {
                 ok = whole(v, &s->seed);
             }
@@ -330,7 +340,7 @@ PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
         st = f_swaptions((bsg_ctx*)ctx, sw.data(), (size_t)n, trials, (double*)price, (double*)err);
         Py_END_ALLOW_THREADS
     }
-    for (PyObject* y : keep) Py_DECREF(y);
+    for (PyObject* y : keep) Py_XDECREF(y);
     return ok ? PyLong_FromLong(st) : nullptr;
 }
 

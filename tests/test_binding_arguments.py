@@ -2,10 +2,14 @@
 go to no context (status -1), so an argument that is refused raises before."""
 import ctypes
 import dataclasses
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 
+from conftest import ROOT
 from p3arsec_gb300 import abi, build
 from p3arsec_gb300 import swaptions as S
 
@@ -81,3 +85,31 @@ def test_host_arrays_at_any_address(call):
             swapped[i] = odd[i].view(odd[i].dtype.newbyteorder())
             with pytest.raises(TypeError):
                 call.price_soa(0, *swapped, 10, 1, 0, False)
+
+
+MEMORY = r"""
+import resource, sys
+from p3arsec_gb300 import abi, swaptions
+abi.load()
+kind = sys.argv[1]
+if kind == "segments":
+    items = [(0, 1)] * (1 << 24)   # 128 MB here, 256 MB as segments
+    call = lambda: abi._call.price_batch(0, (0,) * 6, 0, 100, items, 1, 1, False)
+else:
+    items = swaptions.generate(1, 1) * (1 << 22)  # 32 MB here, 400 MB as structs
+    call = lambda: abi._call.price_swaptions(0, items, 2, 0, 0)
+used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (used + (128 << 20),) * 2)
+try:
+    call()
+except MemoryError:
+    print("refused")
+"""
+
+
+@pytest.mark.parametrize("kind", ["segments", "swaptions"])
+def test_no_memory_is_an_exception(call, kind):
+    """In a process with too little address space for the call's own table."""
+    r = subprocess.run([sys.executable, "-c", MEMORY, kind], cwd=ROOT, env=dict(os.environ, PYTHONPATH=ROOT),
+                       stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "refused", (r.returncode, r.stderr[-500:])
