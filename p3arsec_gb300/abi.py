@@ -443,6 +443,7 @@ class Context:
     def price_swaptions(self, swaptions, trials: int):
         """bsg_price_swaptions over p3arsec_gb300.swaptions.Swaption objects;
         returns (prices, standard errors) as float64 arrays."""
+        swaptions = tuple(swaptions)  # the caller's list may change while its items are read
         n = len(swaptions)
         price = np.empty(n)
         err = np.empty(n)

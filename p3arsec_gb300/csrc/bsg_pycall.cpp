@@ -207,22 +207,27 @@ bool read_segments(PyObject* list, std::vector<bsg_segment>* out) {
     for (Py_ssize_t i = 0; i < n && ok; ++i) {
         PyObject* item = PySequence_Fast_GET_ITEM(seq, i);
         uint64_t o = 0, l = 0;
-        if (PyTuple_CheckExact(item) && PyTuple_GET_SIZE(item) == 2) {
-            ok = as_int(PyTuple_GET_ITEM(item, 0), &o) && as_int(PyTuple_GET_ITEM(item, 1), &l);
+        if (PyTuple_CheckExact(item) && PyTuple_GET_SIZE(item) == 2 && PyLong_CheckExact(PyTuple_GET_ITEM(item, 0)) &&
+            PyLong_CheckExact(PyTuple_GET_ITEM(item, 1))) {
+            ok = whole(PyTuple_GET_ITEM(item, 0), &o) && whole(PyTuple_GET_ITEM(item, 1), &l);
         } else {
-            PyObject* pair = PySequence_Fast(item, "a segment is an (offset, length) pair");
-            if (pair && PySequence_Fast_GET_SIZE(pair) != 2) {
+            // reading this one may run Python code, which may change the caller's
+            // list or the pair: go on with tuples of what is in them now
+            PyObject* now = PySequence_Tuple(seq);
+            Py_DECREF(seq);
+            seq = now;
+            PyObject* pair = seq ? PySequence_Tuple(PyTuple_GET_ITEM(seq, i)) : nullptr;
+            if (pair && PyTuple_GET_SIZE(pair) != 2) {
                 PyErr_SetString(PyExc_ValueError, "a segment is an (offset, length) pair");
                 ok = false;
             } else {
-                ok = pair && as_int(PySequence_Fast_GET_ITEM(pair, 0), &o) &&
-                     as_int(PySequence_Fast_GET_ITEM(pair, 1), &l);
+                ok = pair && as_int(PyTuple_GET_ITEM(pair, 0), &o) && as_int(PyTuple_GET_ITEM(pair, 1), &l);
             }
             Py_XDECREF(pair);
         }
         (*out)[(size_t)i] = bsg_segment{o, l};
     }
-    Py_DECREF(seq);
+    Py_XDECREF(seq);
     return ok;
 }
 
@@ -233,11 +238,11 @@ PyObject* price_batch(PyObject*, PyObject* const* a, Py_ssize_t na) {
     uint64_t pool_len, runs, flags;
     if (!address(a[0], &ctx) || !whole(a[3], &pool_len) || !whole(a[5], &runs) || !whole(a[6], &flags))
         return nullptr;
-    PyObject* pool = PySequence_Fast(a[1], "the pool is six arrays");
+    PyObject* pool = PySequence_Tuple(a[1]);
     if (!pool) return nullptr;
-    bool ok = PySequence_Fast_GET_SIZE(pool) == 6;
+    bool ok = PyTuple_GET_SIZE(pool) == 6;
     if (!ok) PyErr_SetString(PyExc_TypeError, "the pool is six arrays");
-    for (int i = 0; i < 6 && ok; ++i) ok = address(PySequence_Fast_GET_ITEM(pool, i), &p[i]);
+    for (int i = 0; i < 6 && ok; ++i) ok = address(PyTuple_GET_ITEM(pool, i), &p[i]);
     Py_DECREF(pool);
     std::vector<bsg_segment> segs;
     if (!ok || !address(a[2], &p[6]) || !read_segments(a[4], &segs)) return nullptr;
@@ -296,21 +301,25 @@ PyObject* doubles(PyObject* x, const double** data) {
     return y;
 }
 
-// price_swaptions(ctx, swaptions, trials, prices, errors)
+// price_swaptions(ctx, swaptions, trials, prices, errors): a tuple of swaptions,
+// prices and errors of its length
 PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (!arg_count(na, 5)) return nullptr;
     uintptr_t ctx, price, err;
     uint64_t trials;
     if (!address(a[0], &ctx) || !whole(a[2], &trials) || !address(a[3], &price) || !address(a[4], &err))
         return nullptr;
-    PyObject* seq = PySequence_Fast(a[1], "swaptions must be a sequence");
-    if (!seq) return nullptr;
-    const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
+    PyObject* const seq = a[1];
+    if (!PyTuple_Check(seq)) {
+        PyErr_SetString(PyExc_TypeError, "swaptions must be a tuple");
+        return nullptr;
+    }
+    const Py_ssize_t n = PyTuple_GET_SIZE(seq);
     std::vector<bsg_swaption> sw;
     std::vector<PyObject*> keep;  // two arrays a swaption, NULL where not there yet
     bool ok = resized(&sw, n > 0 ? n : 1) && resized(&keep, 2 * n);
     for (Py_ssize_t i = 0; i < n && ok; ++i) {
-        PyObject* w = PySequence_Fast_GET_ITEM(seq, i);
+        PyObject* w = PyTuple_GET_ITEM(seq, i);
         bsg_swaption* s = &sw[(size_t)i];
         double* const d[6] = {&s->strike, &s->compounding, &s->maturity, &s->tenor, &s->payment_interval, &s->years};
         for (int j = 0; j < 11 && ok; ++j) {
@@ -333,7 +342,6 @@ PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
             Py_XDECREF(v);
         }
     }
-    Py_DECREF(seq);
     int st = 0;
     if (ok) {
         Py_BEGIN_ALLOW_THREADS

@@ -43,8 +43,8 @@ def _calls(call):
         "batch flags": lambda x: batch(flags=x),
         "request n": lambda x: call.server_submit(0, *[a.ctypes.data for a in host], x)[0],
         "request id": lambda x: call.server_wait(0, x, 0.0)[0],
-        "trials": lambda x: call.price_swaptions(0, sw, x, one, one),
-        "seed": lambda x: call.price_swaptions(0, [dataclasses.replace(sw[0], seed=x)], 2, one, one),
+        "trials": lambda x: call.price_swaptions(0, tuple(sw), x, one, one),
+        "seed": lambda x: call.price_swaptions(0, (dataclasses.replace(sw[0], seed=x),), 2, one, one),
     }
 
 
@@ -96,7 +96,7 @@ if kind == "segments":
     items = [(0, 1)] * (1 << 24)   # 128 MB here, 256 MB as segments
     call = lambda: abi._call.price_batch(0, (0,) * 6, 0, 100, items, 1, 1, False)
 else:
-    items = swaptions.generate(1, 1) * (1 << 22)  # 32 MB here, 400 MB as structs
+    items = tuple(swaptions.generate(1, 1)) * (1 << 22)  # 32 MB here, 400 MB as structs
     call = lambda: abi._call.price_swaptions(0, items, 2, 0, 0)
 used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
 resource.setrlimit(resource.RLIMIT_AS, (used + (128 << 20),) * 2)
@@ -113,3 +113,39 @@ def test_no_memory_is_an_exception(call, kind):
     r = subprocess.run([sys.executable, "-c", MEMORY, kind], cwd=ROOT, env=dict(os.environ, PYTHONPATH=ROOT),
                        stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "refused", (r.returncode, r.stderr[-500:])
+
+
+def test_items_that_change_the_callers_list(call):
+    """Reading a segment or a swaption may run Python code; what the call reads is
+    what the list held when it was given."""
+    segs = []
+
+    class Clears:
+        def __init__(self, x):
+            self.x = x
+
+        def __int__(self):
+            segs.clear()
+            return self.x
+
+    for pair in (lambda o: (Clears(o), 1), lambda o: [Clears(o), 1]):
+        segs[:] = [(0, 1)] * 100 + [pair(500 + i) for i in range(1000)]
+        assert call.price_batch(0, (0,) * 6, 0, 2000, segs, 1, 1, False) == INVALID
+        assert segs == []
+    mine = []
+
+    @dataclasses.dataclass
+    class Shrinks(S.Swaption):
+        @property
+        def n_steps(self):
+            mine.clear()
+            return 11
+
+    class NoGpu(abi.Context):
+        def __init__(self):
+            self.lib, self.h, self._addr = abi.load(), None, None
+
+    mine[:] = [Shrinks(strike=0.1, years=5.5, seed=i) for i in range(500)]
+    with pytest.raises(abi.BsgError):
+        NoGpu().price_swaptions(mine, 2)
+    assert mine == []
