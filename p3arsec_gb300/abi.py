@@ -551,19 +551,6 @@ def serve_trace(host_pool, prices, rate_per_s, duration_s, min_n=16, max_n=1 << 
     return res.as_dict()
 
 
-def swaption_structs(swaptions):
-    """bsg_swaption array for p3arsec_gb300.swaptions.Swaption objects, and the
-    numpy arrays it points into (keep them alive while the array is used)."""
-    keep, arr = [], (SwaptionC * max(len(swaptions), 1))()
-    for i, w in enumerate(swaptions):
-        y = np.ascontiguousarray(w.yield_curve, dtype=np.float64)
-        f = np.ascontiguousarray(w.factors, dtype=np.float64)
-        keep += [y, f]
-        arr[i] = SwaptionC(w.strike, w.compounding, w.maturity, w.tenor, w.payment_interval,
-                           w.years, w.n_steps, w.n_factors, y.ctypes.data, f.ctypes.data, w.seed)
-    return arr, keep
-
-
 def HJM_Swaption_Blocking(w, trials: int):
     """The reference's per-swaption call shape (bsg_HJM_Swaption_Blocking):
     returns (status, price, standard error); status 1 = success."""

@@ -154,8 +154,6 @@ cudaError_t launch_batch(const SoA& pool, const uint64_t* tiles, uint64_t ntiles
 cudaError_t launch_batch_segments(const SoA& pool, const uint64_t* seg_off, const uint64_t* seg_len,
                                   const uint64_t* tile_prefix, int nseg, uint64_t ntiles, uint64_t tile_opts,
                                   unsigned long long* cursor, int mode, int grid, cudaStream_t st);
-// Default options per batch tile.
-uint64_t batch_tile_options();
 // Resident blocks per SM of the batch kernel (its persistent grid = this x SMs).
 int batch_blocks_per_sm();
 
@@ -213,10 +211,6 @@ struct SwHead {
     int disc_varies;          // 0, 1
     int wide;                 // 0, 1
 };
-// s steps to maturity and p payments share a grid of at most 32 points:
-// n_exp (2 + n_normals) <= 32 (2 + 8 s) and (p + 1) 8 s <= 8 s (32 - s)
-constexpr int kSwMaxWords = 2 * kSwMaxExp + 8 * 256;
-
 // A table small enough to travel with the launch (a copy before the kernel
 // costs 3 us of a 20 us call).
 constexpr int kSwInlineWords = 480;

@@ -1147,9 +1147,6 @@ cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count, cuda
 // A tile is 8192 options; a block covers it in passes of kBatchBlock
 // threads x kBatchVpt v4 groups.
 constexpr int kBatchVpt = 1;
-constexpr uint64_t kBatchTileOptions = 8192;
-
-uint64_t batch_tile_options() { return kBatchTileOptions; }
 
 // Prices options [b, e) of the pool as thread `tid` of `nt` that share them: an
 // unaligned head and tail one option per thread, the aligned body in groups of

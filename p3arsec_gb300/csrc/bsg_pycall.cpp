@@ -148,11 +148,6 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Py_RETURN_NONE;
 }
 
-PyObject* py_ptr(PyObject*, PyObject* x) {
-    uintptr_t p;
-    return address(x, &p) ? PyLong_FromUnsignedLongLong(p) : nullptr;
-}
-
 // price_soa(ctx, s, k, r, v, t, otype, prices, n, num_runs, flags, f64)
 PyObject* price_soa(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (!arg_count(na, 12)) return nullptr;
@@ -355,7 +350,7 @@ PyObject* price_swaptions(PyObject*, PyObject* const* a, Py_ssize_t na) {
 #define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST(bind), FAST(price_soa), FAST(price_batch), FAST(server_submit),
                          FAST(server_wait), FAST(price_swaptions),
-                         {"ptr", py_ptr, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
+                         {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pycall", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
