@@ -26,8 +26,10 @@ records measured in the same run:
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--config map|batch|precision|serve|serve-blocks|io|fp64|prefix-sweep|swaptions]
+                    [--records FILE]
 
-One JSON line on stdout (rank 0).  Under torchrun each rank prices its own
+One JSON line on stdout (rank 0), with the figures of each nested record;
+--records FILE keeps the records whole.  Under torchrun each rank prices its own
 book on its own GPU (weak scaling, no collective on the data path); the
 nested records are measured at one GPU only.
 """
@@ -405,9 +407,70 @@ def run_ours(args, rank, world, local):
     if rank == 0 and world == 1 and not args.no_cpu:
         line["cpu_baseline"] = cpu_baseline(book)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        if args.records:
+            with open(args.records, "w") as f:
+                json.dump(line, f, indent=1)
+        print(printed_line(line), flush=True)
     if dist is not None:
         dist.destroy_process_group()
+
+
+LINE_LIMIT = 2800  # characters: a reader that keeps a log's last 3,000 gets all of the line
+
+
+def _short(record, *keys):
+    """A nested record's figures under these keys ("a.b": of its part a), or its error."""
+    out = {}
+    for key in ("error",) + keys:
+        x = record
+        for part in key.split("."):
+            x = x.get(part) if isinstance(x, dict) else None
+        if x is not None:
+            out[key.replace("modes.", "").replace(".", "_")] = x
+    return out
+
+
+def _rounded(x):
+    if isinstance(x, float):
+        return float(f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: _rounded(v) for k, v in x.items()}
+    return [_rounded(v) for v in x] if isinstance(x, list) else x
+
+
+def printed_line(line, limit=LINE_LIMIT):
+    """The map's JSON line as it is printed: the headline whole but for its prose,
+    of each nested record the figures it is read for (--records FILE keeps
+    everything).  Nested records, the last first, give way to the limit."""
+    line = dict(line)
+    for key, what in (("roofline", ("traffic_note", "note")), ("cpu_baseline", ("note",)), ("repeats", ("values", "note"))):
+        if line.get(key):
+            line[key] = {k: v for k, v in line[key].items() if k not in what}
+    pick = {
+        "roofline_2p28": ("value", "frac", "max_abs_vs_fp64", "gpu_launches"),
+        "batch": ("value", "roofline.frac", "speedup_vs_plain", "bit_identical", "gpu_launches"),
+        "serve": ("trace.batched.p99_ms", "trace.batched.options_per_s", "trace.plain.options_per_s"),
+        "swaptions": ("value", "ms_per_step", "vs_oracle.max_rel_price_diff", "cpu_baseline.value", "gpu_launches"),
+        "precision": ("modes.fast.max_abs", "modes.fast.rms_abs", "modes.fast.options_per_s",
+                      "modes.libm_ref.max_abs", "modes.libm_ref.options_per_s"),
+        "fp64": ("value", "max_diff_over_max_s_k", "max_rel_above_1e-6_of_max_s_k", "max_rel_vs_cpu_fp64"),
+        "io": ("parse.speedup", "write.speedup", "parse.bit_identical", "write.byte_identical"),
+    }
+    nested = [k for k in pick if k in line]
+    for key in nested:
+        full = line[key]
+        line[key] = _short(full, *pick[key])
+        if key == "serve" and "throughput_at_equal_p99" in full:
+            line[key]["equal_p99"] = [[e["p99_bound_ms"], e["batched_options_per_s"], e["plain_options_per_s"],
+                                       e["ratio"]] for e in full["throughput_at_equal_p99"]]
+    keep = {k: line[k] for k in ("value", "ms_per_step")}
+    dump = lambda: json.dumps({**_rounded(line), **keep}, separators=(",", ":"))  # noqa: E731
+    text = dump()
+    while len(text) > limit and nested:
+        line[nested[-1]] = "in --records"
+        nested.pop()
+        text = dump()
+    return text
 
 
 def _nested(fn, *a, **kw):
@@ -1228,6 +1291,8 @@ def main(argv=None):
                     help="map: extra timed windows of the same steps (their spread is reported)")
     ap.add_argument("--no-nested", action="store_true",
                     help="map: skip the nested 2^28, batch and serve records")
+    ap.add_argument("--records", default=None, metavar="FILE",
+                    help="map: write the line with every nested record in full to FILE")
     ap.add_argument("--tune", default=None,
                     help="vec_per_thread,block,blocks_per_sm,load_path[,pdl[,resident_32nds]] "
                          "instead of autotuning")
