@@ -68,7 +68,7 @@ typedef enum bsg_status {
 #define BSG_MODE_LIBM_REF 0x020u /* reference operation order, correctly rounded exp/log,
                                     IEEE division and square root: the reference's own
                                     FP32 prices wherever glibc's expf/logf round correctly
-                                    (99.7 % of options); compute-bound, ~3x slower */
+                                    (99.7 % of options); compute-bound, 2x slower */
 #define BSG_MODE_MASK     0x0F0u
 #define BSG_NO_GRAPH      0x100u /* launch NUM_RUNS kernels directly, no graph */
 
@@ -89,7 +89,8 @@ int bsg_create(bsg_ctx** out, int device, size_t max_options);
 void bsg_destroy(bsg_ctx* ctx);
 const char* bsg_strerror(int status);
 const char* bsg_last_error(const bsg_ctx* ctx);
-/* The context's cudaStream_t (as void*): work of every call is ordered on it. */
+/* The context's cudaStream_t (as void*): work of every call is ordered on it,
+ * behind everything that the stream holds. */
 void* bsg_stream(bsg_ctx* ctx);
 /* Waits for every call enqueued on the context (pipelined host calls too). */
 int bsg_synchronize(bsg_ctx* ctx);
@@ -107,7 +108,8 @@ void bsg_host_free(void* p);
  * reference's NUM_RUNS loop, blackscholes.c:315-348 / 607-658).
  * Replaces bs_thread (blackscholes.c:607) and the FastFlow map's svc
  * (blackscholes.c:316-346).  n == 0 or num_runs == 0 is a no-op.
- * BSG_ASYNC with device pointers: returns once enqueued on bsg_stream().
+ * Prices may overlap an input: each pass then reads what the one before it
+ * wrote.  BSG_ASYNC with device pointers: returns once enqueued on bsg_stream().
  * BSG_ASYNC with host pointers (pipelined): returns once enqueued; successive
  * calls alternate between two resident buffer sets and overlap one call's
  * host<->device copies with another's passes.  The caller keeps the host
@@ -408,7 +410,10 @@ int bsg_price_swaptions(bsg_ctx* ctx, const bsg_swaption* swaptions, size_t n,
  * words[4 i .. 4 i + 3] (host array) -> z[2 i], z[2 i + 1] (host array), by
  * the device's Box-Muller transform (u1 from words 0-1, u2 from words 2-3,
  * u = (2k + 1) 2^-53 with k = the top 20 bits of the first word and all of
- * the second).  For checking the transform against a host evaluation. */
+ * the second).  For checking the transform against a host evaluation: each is
+ * within 1.5e-16 of max(1, |z|), the kernel's fixed point having 58 fraction
+ * bits; a variate next to zero is that close to the exact one, but is not
+ * accurate relative to itself (one of 1e-5 to 41 bits). */
 int bsg_swaption_normals(bsg_ctx* ctx, const uint32_t* words, size_t n_pairs, double* z);
 
 /* The reference's per-swaption signature (HJM_Swaption_Blocking.cpp:19-41;
@@ -458,7 +463,10 @@ int bsg_read_soa(const char* path, bsg_book* out);
 /* ---- tuning ------------------------------------------------------------
  * A context that was never tuned picks a shape by the size of the book and the
  * number of passes (all passes of a short book in one launch); a chosen or
- * autotuned shape is used as it is, one launch per pass.
+ * autotuned shape is used as it is, one launch per pass.  The tuner compares
+ * shapes of one launch per pass only: for several passes over a short book (up
+ * to 2048 options per SM) no shape is as fast as not tuning (65,536 options x
+ * 100: 62-71 us against 41).
  * The plain map is a family of kernels: vector width per thread, block size,
  * grid size, load path and, for the resident-prefix load path, the prefix
  * size.  bsg_autotune times the candidates on the context's device for n

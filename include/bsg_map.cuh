@@ -28,7 +28,8 @@ namespace bsg {
 struct MapShape {
     int block = 256;         // threads per block
     int blocks_per_sm = 4;   // persistent grid = blocks_per_sm x SMs
-    bool pdl = false;        // programmatic dependent launch
+    bool pdl = false;        // programmatic dependent launch: only where no work before it
+                             // on the stream writes its inputs, or its output otherwise
 };
 
 namespace map_detail {

@@ -59,9 +59,10 @@ struct ErrAcc {
 constexpr int kMaxErrBuckets = 32;
 constexpr int kBatchBlock = 256;
 
-// Launches one pass of the plain map over n options.  Picks the vector
-// kernel when every pointer is aligned for the configured width, else the
-// scalar kernel.  Returns the launch error.
+// Launches one pass of the plain map over n options.  Picks the vector kernel
+// when all pointers are equally far from a boundary of the configured width
+// (the options before it are priced one by one), or else of 16 bytes, and
+// otherwise the scalar kernel.  Returns the launch error.
 cudaError_t launch_map(const SoA& a, int64_t n, int mode, const MapCfg& cfg,
                        int sm_count, cudaStream_t st);
 // The shape of pass j of `runs` consecutive passes over the same book.  The
@@ -134,7 +135,8 @@ unsigned bulk_error_take();
 // the bounded waits; the copies themselves complete normally).
 cudaError_t launch_bulk_wait_selftest(const SoA& a, int64_t n, int sm_count, uint64_t wait_ns,
                                       cudaStream_t st);
-// True when launch_map would take the vector path for these pointers.
+// True when every pointer is aligned for cfg's load path (the batch kernel's
+// choice of 256-bit loads).
 bool map_vectorizable(const SoA& a, const MapCfg& cfg);
 
 cudaError_t launch_fp64(const SoA& a, double* out, int64_t n, int sm_count, cudaStream_t st,

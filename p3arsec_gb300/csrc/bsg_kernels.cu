@@ -186,8 +186,9 @@ __device__ __forceinline__ void price_groups(const SoA& a, int64_t g0, int64_t g
 // instructions are no-ops for a launch without the PDL attribute.
 // Registers: one-group shapes (VPT = 1) are held to 64 per thread (1024
 // threads per SM, no spills); more groups per thread need up to 128.  The
-// reference-order libm mode (compute-bound, float-float exp/log) always runs
-// 256-thread blocks, four per SM (59 registers, no spills).
+// reference-order libm mode (compute-bound, float-float exp/log) runs blocks of
+// up to 256 threads (untuned contexts: 128), 1024 threads per SM (59
+// registers, no spills).
 __device__ __forceinline__ void pdl_trigger() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -736,9 +737,9 @@ static cudaError_t launch_map_mode(const SoA& a_in, int64_t n, const MapCfg& cfg
     MapCfg cfg = cfg_in;
     SoA a = a_in;
     if constexpr (M == MODE_LIBM_REF) {
-        // compute-bound (float-float exp/log): 128-bit loads and one
-        // 256-thread block per tile (four resident per SM), whatever shape
-        // the memory-bound tuning chose
+        // compute-bound (float-float exp/log): 128-bit loads and one block of
+        // up to 256 threads per tile (1024 threads resident per SM), whatever
+        // shape the memory-bound tuning chose
         cfg.load_path = 0;
         cfg.vpt = 1;
         cfg.blocks_per_sm = 0;

@@ -4,9 +4,9 @@
 // HJM_Swaption_Blocking (parsec-ff/pkgs/apps/swaptions/src/
 // HJM_Swaption_Blocking.cpp:19-223), one swaption per FastFlow worker
 // iteration (HJM_Securities.cpp:312-323), trials in blocks on one core.  Here
-// one launch prices every swaption: a grid of (trial chunk, swaption) blocks,
-// one path per thread at a time, in double precision as the reference's
-// FTYPE.
+// one launch prices every swaption: persistent blocks whose warps take the next
+// paths of the next swaption from a queue, one path a lane at a time, in 64-bit
+// fixed point and doubles, to the double precision of the reference's FTYPE.
 //
 // Per path (the driver's arithmetic, HJM_Swaption_Blocking.cpp:160-204, on
 // a discrete HJM model in the time-to-maturity parameterisation):

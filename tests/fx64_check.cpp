@@ -1,6 +1,5 @@
 // CPU check of the fixed-point double price (p3arsec_gb300/csrc/bsg_fx64.h,
-// the same code the GPU runs but for its reciprocal seed's last bits)
-// against the formula in long double and in double.
+// the same code the GPU runs) against the formula in long double and in double.
 //
 //   fx64_check <n> <seed> <dist>     dist: 0 plain, 1 tails, 2 wide
 // prints "priced <a> left <b> fixed <max> <rms> double <max> <rms> test <d>":
