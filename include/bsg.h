@@ -108,8 +108,10 @@ void bsg_host_free(void* p);
  * reference's NUM_RUNS loop, blackscholes.c:315-348 / 607-658).
  * Replaces bs_thread (blackscholes.c:607) and the FastFlow map's svc
  * (blackscholes.c:316-346).  n == 0 or num_runs == 0 is a no-op.
- * Prices may overlap an input: each pass then reads what the one before it
- * wrote.  BSG_ASYNC with device pointers: returns once enqueued on bsg_stream().
+ * With device pointers the prices may be one of the input arrays: each pass
+ * then reads what the one before it wrote.  (A host call reads its inputs
+ * before it writes a price.)
+ * BSG_ASYNC with device pointers: returns once enqueued on bsg_stream().
  * BSG_ASYNC with host pointers (pipelined): returns once enqueued; successive
  * calls alternate between two resident buffer sets and overlap one call's
  * host<->device copies with another's passes.  The caller keeps the host
